@@ -1,30 +1,32 @@
-// Packed causal attention forward on the sm_100a tensor path: S = Q K^T and O = P V are
-// tcgen05.mma instructions with FP32 accumulators in tensor memory, operands arrive by TMA.
+// Packed causal attention forward on the sm_100a tensor path: S = Q K^T and O += P V are tcgen05.mma instructions with FP32
+// accumulators in tensor memory; Q, K and V arrive by TMA, P never leaves tensor memory (it is the A operand of the second
+// product), O stays there for the whole item.
 //
-// Fast path of gd_backend_sdpa_varlen for 16-bit storage, head_dim 64, causal (+ optional sliding
-// window), no prefix. A work item is 128 consecutive rows of the PACKED token stream for one head;
-// the mask is evaluated in packed coordinates exactly as in the mma.sync kernels (attention_flash.cu):
+// Fast path of gd_backend_sdpa_varlen for 16-bit storage, head_dim 64 or 128, causal (+ optional sliding window), no prefix. A
+// work item is 128 consecutive rows of the PACKED token stream for one head; the mask is evaluated in packed coordinates:
 //   allowed(i, j)  <=>  seg_start(i) <= j <= i  and  (window == 0 or i - j < window)
 // (src/ops/sdpa_varlen/metal_sdpa_varlen.metal:30-55, prefix 0), so a tile may span sequences.
 //
-// The kernel is persistent: two CTAs per SM stay resident and draw items from a launch-wide ticket counter
-// (an item costs 1-5 key tiles, so a fixed deal leaves CTAs up to 1.6x out of balance), so tensor-memory
-// allocation, barrier set-up and the cu_seqlens copy are paid once per CTA, and the TMA producer and
-// the MMA issuer run ahead into the next item while the softmax warps finish the current one (at the
-// model's sequence lengths an item has only 1-5 key tiles).
+// The kernel is persistent: two CTAs per SM stay resident and draw items from a launch-wide ticket counter (an item costs 1-5
+// key tiles at the model's sequence lengths, so a fixed deal leaves CTAs up to 1.6x out of balance). Tensor-memory allocation,
+// barrier set-up and the cu_seqlens copy are paid once per CTA, and producer and issuer run ahead into the next item.
 //
-// Roles (320 threads): warp 0 = TMA producer (Q per item, K double-buffered, V single-buffered);
-// warp 1 = MMA issuer; warps 2-9 = softmax. A query row is shared by TWO threads of the same
-// tensor-memory lane quadrant (warps w and w + 4): each owns 64 of the 128 key columns of S and 32 of
-// the 64 output columns, reads them with tcgen05.ld 32x32b (no shuffles) and the two exchange only
-// the row maximum through shared memory. Per key tile:
-//   pass 1: row max of S over the allowed columns (+ exchange)
-//   (deferred) o += alpha * O_part of the previous tile, read back from tensor memory
-//   pass 2: p = exp2(s * scale * log2e - m), written as 16-bit into the 128-byte-swizzled K-major
-//           shared tile that the P V MMA reads as its A operand; running partial sum l
-// Tensor memory: 2 buffers of 128 columns; S[g] lives in buffer g & 1 and, once consumed, the same
-// buffer receives O_part[g] (64 columns), so 256 columns suffice for a CTA. The MMA issuer keeps one
-// S tile ahead: S[g+1] is issued while the softmax warps work on S[g].
+// What bounds it: the special-function unit (one exp2 per score at 16 per cycle and SM: 512 cycles of a 128 x 64 step), as long
+// as the chain S -> softmax -> P V does not. The softmax of a 64-key step takes a warp 741 cycles by itself and 581 when two
+// warps share a scheduler (measured with the loop alone), a hand-over between roles 300-500, so the chain is taken apart:
+//   * S has two buffers: S of the next step (also of the next item) is formed while the softmax warps work on this one, and
+//     P V runs behind them; a softmax warp never waits for a product of its own step;
+//   * one thread per query row (192 threads: warp 0 = TMA producer, warp 1 = MMA issuer, warps 2-5 = softmax) holds the row's
+//     64 scores in registers: no exchange between threads, S is read from tensor memory once;
+//   * P (16-bit) is written over the S columns it came from with tcgen05.st: no shared-memory tile, no proxy fence. A later S
+//     may overwrite it because one thread issues all products and they execute in order;
+//   * O is rescaled in tensor memory only when a row's maximum has grown by more than 2^8 since the last rescale (the sum is
+//     kept relative to the same stale maximum, so the result is the same); after the first tile that is rare;
+//   * the code of all roles stays near the 32 KB of the first-level instruction cache (waits and searches are not unrolled, a
+//     step has one masked and one unmasked way to the same exponentials): at 57 KB the kernel ran at a third of this speed.
+// 32768 tokens in sequences of 16-512, 8 heads of 64: 72 us (one step at a time, P through shared memory: 124 us); 8191 tokens
+// in sequences of 256-2048, 16 heads of 128, window 1024: 78 us (mma.sync kernel: 286 us).
+// Tensor memory per CTA (256 columns): S / P 2 x 64, O head_dim.
 //
 // Statistics written for the backward pass: (row max in natural-log units, sum of exp, 0).
 // Every mbarrier wait is bounded and reports through gd_backend::err_flag.
@@ -36,22 +38,26 @@ using namespace gdb_t5;
 
 constexpr float LOG2E_F = 1.4426950408889634f;
 constexpr float LN2_F = 0.6931471805599453f;
-constexpr int A_BQ = 128, A_DH = 64, A_BKV = 128;
+constexpr int A_BQ = 128, A_BKV = 64;   // query rows of an item, keys of a step
 constexpr int A_MAX_CU = 1024;
-constexpr int A_THREADS = 320;
+constexpr int A_THREADS = 192;
+constexpr float A_RESCALE = 8.0f;   // log2 of the growth of a row maximum that triggers a rescale of O
 
 struct attn5_params {
     int n_tokens, batch, hq, hkv, window, n_items;
     float scale;
 };
 
+template <int DH>
 struct attn5_plan {
-    static constexpr int Q_BYTES = A_BQ * 128;          // 128 rows x 64 x 2 B
-    static constexpr int KV_BYTES = A_BKV * 128;
-    static constexpr int P_BYTES = A_BQ * A_BKV * 2;    // two blocks (64 keys each) of [128 rows x 128 B]
-    static constexpr int OFF_K = Q_BYTES, OFF_V = OFF_K + 2 * KV_BYTES, OFF_P = OFF_V + KV_BYTES, OFF_BAR = OFF_P + P_BYTES;
-    static constexpr int TOTAL = OFF_BAR + 256 + 1024;
-    static constexpr int TMEM_COLS = 2 * A_BKV;
+    static constexpr int STAGES = DH == 64 ? 4 : 2;               // K and V stages
+    static constexpr int QSTAGES = DH == 64 ? 2 : 1;              // (two CTAs share 227 KB)
+    static constexpr int QBLOCK = A_BQ * 128, BLOCK = A_BKV * 128;  // 64 x 2 B per row: one 128-byte-swizzled block
+    static constexpr int QTILE = QBLOCK * (DH / 64), TILE = BLOCK * (DH / 64);
+    static constexpr int OFF_K = QSTAGES * QTILE, OFF_V = OFF_K + STAGES * TILE, OFF_BAR = OFF_V + STAGES * TILE;
+    static constexpr int TOTAL = OFF_BAR + 512 + 1024;
+    static constexpr int TMEM_COLS = 256;
+    static constexpr uint32_t COL_S = 0, COL_O = 2 * A_BKV;       // S / P: two buffers of A_BKV columns
 };
 
 __device__ __forceinline__ float ex2_approx(float x)
@@ -64,6 +70,7 @@ __device__ __forceinline__ float ex2_approx(float x)
 __device__ __forceinline__ int seg_start_of(const int *cu_s, int batch, int row)
 {
     int lo = 0, hi = batch;
+#pragma unroll 1
     while (lo + 1 < hi) {
         const int mid = (lo + hi) >> 1;
         if (cu_s[mid] <= row) lo = mid; else hi = mid;
@@ -71,7 +78,7 @@ __device__ __forceinline__ int seg_start_of(const int *cu_s, int batch, int row)
     return cu_s[lo];
 }
 
-// Key range of a work item: first key and number of 128-key tiles (0 when the rows lie behind the last sequence).
+// Key range of a work item: first key and number of key tiles (0 when the rows lie behind the last sequence).
 __device__ __forceinline__ void item_range(const int *cu_s, const attn5_params &p, int n_valid, int q0, int *kv_begin, int *n_tiles)
 {
     *kv_begin = 0;
@@ -85,28 +92,49 @@ __device__ __forceinline__ void item_range(const int *cu_s, const attn5_params &
     }
 }
 
+// pairs of FP32 values in one register pair
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 f2_make(float lo, float hi)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void f2_split(f32x2 p, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p)); }
+__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
 __device__ __forceinline__ void mbar_arrive_local(uint32_t bar)
 {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-template <typename T>
+template <typename T, int DH>
 __global__ void __launch_bounds__(A_THREADS, 2)
 attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
                  const __grid_constant__ CUtensorMap tma_v, T *__restrict__ out,
                  const int *__restrict__ cu, float *__restrict__ stats, attn5_params p, int *err_flag, unsigned *work_counter,
                  unsigned *done_counter)
 {
-    using plan = attn5_plan;
+    using plan = attn5_plan<DH>;
+    constexpr uint32_t ST = plan::STAGES, QST = plan::QSTAGES;
     extern __shared__ unsigned char smem_raw[];
     __shared__ int cu_s[A_MAX_CU + 1];
-    __shared__ float xch[2][2][A_BQ];   // [tile parity][column half][row]: row maxima of the two column halves
-    __shared__ float xsum[2][2][A_BQ];  // [item parity][column half][row]: partial sums of exp, exchanged once per item
     __shared__ int sched_item[4];       // work items handed out by the producer thread (-1: no more work)
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023U) & ~(uintptr_t)1023U);
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + plan::OFF_BAR);
-    enum { Q_FULL = 0, Q_EMPTY = 1, K_FULL = 2, K_EMPTY = 4, V_FULL = 6, V_EMPTY = 7, S_FULL = 8, P_FULL = 10, P_EMPTY = 11, O_FULL = 12, BUF_FREE = 14,
-           SCHED_FULL = 16, SCHED_EMPTY = 20, PAIR = 24, N_BARS = 28 };
+    enum { Q_FULL = 0, Q_EMPTY = 2, K_FULL = 4, K_EMPTY = 8, V_FULL = 12, V_EMPTY = 16, S_FULL = 20, P_FULL = 22, PV_DONE = 24, O_FREE = 26,
+           SCHED_FULL = 27, SCHED_EMPTY = 31, N_BARS = 35 };
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + N_BARS);
     const uint32_t bar0 = smem_u32(bars);
     auto bar = [&](int i) { return bar0 + 8U * (uint32_t)i; };
@@ -115,10 +143,10 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
     const int group = p.hq / p.hkv;
 
     if (threadIdx.x == 0) {
+#pragma unroll 1
         for (int i = 0; i < N_BARS; ++i) {
-            const bool eight = i == P_FULL || i == BUF_FREE || i == BUF_FREE + 1;
-            // schedule slots are released by the MMA thread and the 8 softmax warps; pair barriers by 2 warps
-            const uint32_t count = eight ? 8U : (i >= SCHED_EMPTY && i < SCHED_EMPTY + 4 ? 9U : (i >= PAIR ? 2U : 1U));
+            // schedule slots are released by the MMA thread and the four softmax warps
+            const uint32_t count = (i == P_FULL || i == P_FULL + 1 || i == O_FREE) ? 4U : (i >= SCHED_EMPTY ? 5U : 1U);
             mbar_init(bar(i), count);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -133,6 +161,7 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
     const uint32_t tmem_base = *tmem_slot;
     // barrier set-up and tensor-memory allocation may overlap the preceding kernel; global memory is read from here on
     gdb_pdl_sync();
+#pragma unroll 1
     for (int i = threadIdx.x; i <= p.batch; i += blockDim.x) cu_s[i] = cu[i];
     __syncthreads();
     const int n_valid = min(cu_s[p.batch], p.n_tokens);
@@ -160,7 +189,7 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                 return it;
             };
             // The schedule runs one item ahead of the loads: the MMA thread looks up the next item right after the
-            // last S of the current one, while this thread may still wait for a V slot that only a later P V frees.
+            // last P V of the current one, while this thread may still wait for a stage that only a later product frees.
             int item = draw(), next = -1;
             for (; ok && item >= 0; item = next) {
                 next = draw();
@@ -168,29 +197,39 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                 int kv_begin, n_tiles;
                 item_range(cu_s, p, n_valid, q0, &kv_begin, &n_tiles);
                 if (n_tiles == 0) continue;
-                if (!mbar_wait(bar(Q_EMPTY), (iq & 1U) ^ 1U)) {
+                const uint32_t qs = iq % QST;
+                if (!mbar_wait(bar(Q_EMPTY + qs), ((iq / QST) & 1U) ^ 1U)) {
                     atomicExch(err_flag, 300);
                     break;
                 }
-                mbar_expect_tx(bar(Q_FULL), plan::Q_BYTES);
-                tma_load_2d(smem_u32(smem), &tma_q, h * A_DH, q0, bar(Q_FULL));
+                mbar_expect_tx(bar(Q_FULL + qs), plan::QTILE);
+#pragma unroll
+                for (int b = 0; b < DH / 64; ++b) tma_load_2d(smem_u32(smem + qs * plan::QTILE + b * plan::QBLOCK), &tma_q, h * DH + b * 64, q0, bar(Q_FULL + qs));
                 ++iq;
+#pragma unroll 1
                 for (int t = 0; t < n_tiles; ++t, ++g) {
-                    const int key0 = kv_begin + t * A_BKV, ks = g & 1U;
-                    if (!mbar_wait(bar(K_EMPTY + ks), ((g >> 1) & 1U) ^ 1U)) {
+                    const int key0 = kv_begin + t * A_BKV;
+                    const uint32_t s = g % ST, ph = ((g / ST) & 1U) ^ 1U;
+                    if (!mbar_wait(bar(K_EMPTY + s), ph)) {
                         atomicExch(err_flag, 301);
                         ok = false;
                         break;
                     }
-                    mbar_expect_tx(bar(K_FULL + ks), plan::KV_BYTES);
-                    tma_load_2d(smem_u32(smem + plan::OFF_K + ks * plan::KV_BYTES), &tma_k, hk * A_DH, key0, bar(K_FULL + ks));
-                    if (!mbar_wait(bar(V_EMPTY), (g & 1U) ^ 1U)) {
+                    mbar_expect_tx(bar(K_FULL + s), plan::TILE);
+#pragma unroll
+                    for (int b = 0; b < DH / 64; ++b) {
+                        tma_load_2d(smem_u32(smem + plan::OFF_K + s * plan::TILE + b * plan::BLOCK), &tma_k, hk * DH + b * 64, key0, bar(K_FULL + s));
+                    }
+                    if (!mbar_wait(bar(V_EMPTY + s), ph)) {
                         atomicExch(err_flag, 302);
                         ok = false;
                         break;
                     }
-                    mbar_expect_tx(bar(V_FULL), plan::KV_BYTES);
-                    tma_load_2d(smem_u32(smem + plan::OFF_V), &tma_v, hk * A_DH, key0, bar(V_FULL));
+                    mbar_expect_tx(bar(V_FULL + s), plan::TILE);
+#pragma unroll
+                    for (int b = 0; b < DH / 64; ++b) {
+                        tma_load_2d(smem_u32(smem + plan::OFF_V + s * plan::TILE + b * plan::BLOCK), &tma_v, hk * DH + b * 64, key0, bar(V_FULL + s));
+                    }
                 }
             }
         }
@@ -198,123 +237,116 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
         // ---------------- MMA issuer ----------------
         if (lane == 0) {
             constexpr uint32_t FMT = std::is_same<T, __nv_bfloat16>::value ? 1U : 0U;
-            constexpr uint32_t IDESC_S = (1U << 4) | (FMT << 7) | (FMT << 10) | ((uint32_t)(A_BKV >> 3) << 17) | ((uint32_t)(A_BQ >> 4) << 24);
-            constexpr uint32_t IDESC_PV = (1U << 4) | (FMT << 7) | (FMT << 10) | (1U << 16) | ((uint32_t)(A_DH >> 3) << 17) | ((uint32_t)(A_BQ >> 4) << 24);
-            const uint32_t q_base = smem_u32(smem), p_base = smem_u32(smem + plan::OFF_P), v_base = smem_u32(smem + plan::OFF_V);
-            // Walks the same (item, tile) sequence twice: `s_*` is the cursor of the S issue (one tile ahead),
-            // `pv_g` the cursor of the P V issue.
-            int s_item = -1, s_t = 0, s_tiles = 0;
-            uint32_t s_g = 0, s_iq = 0, s_si = 0;
+            constexpr uint32_t ID_BASE = (1U << 4) | (FMT << 7) | (FMT << 10) | ((uint32_t)(A_BQ >> 4) << 24);
+            constexpr uint32_t IDESC_S = ID_BASE | ((uint32_t)(A_BKV >> 3) << 17);             // A, B K-major
+            constexpr uint32_t IDESC_PV = ID_BASE | (1U << 16) | ((uint32_t)(DH >> 3) << 17);     // A in tensor memory, B MN-major
+            const uint64_t q_d = make_smem_desc(smem_u32(smem), 16, 1024), k_d = make_smem_desc(smem_u32(smem + plan::OFF_K), 16, 1024);
+            // V stored [key][dh] in blocks of 64 dh: 16 keys = 2048 B per MMA
+            const uint64_t v_d = make_smem_desc(smem_u32(smem + plan::OFF_V), plan::BLOCK, 1024);
+            constexpr uint64_t QBLOCK16 = plan::QBLOCK >> 4, BLOCK16 = plan::BLOCK >> 4, TILE16 = plan::TILE >> 4, QTILE16 = plan::QTILE >> 4;
+            // Two cursors over the same sequence of steps: `s_*` issues S one step ahead (across items), `g` issues P V.
+            uint32_t s_g = 0, s_item = 0, s_si = 0, s_tile = 0;
+            int s_tiles = 0;
             bool ok = true;
-            auto s_seek = [&]() {   // position the S cursor on the next scheduled item that has tiles
+            auto fail = [&](int code) {
+                atomicExch(err_flag, code);
+                ok = false;
+            };
+            auto seek = [&]() {   // number of key tiles of the next scheduled item that has any; 0: no more work
+                s_tile = 0;
+#pragma unroll 1
                 for (;;) {
                     const uint32_t slot = s_si & 3U;
-                    if (!mbar_wait(bar(SCHED_FULL + slot), (s_si >> 2) & 1U)) {
-                        atomicExch(err_flag, 311);
-                        s_item = -1;
-                    } else {
-                        s_item = *reinterpret_cast<volatile int *>(&sched_item[slot]);
-                        mbar_arrive_local(bar(SCHED_EMPTY + slot));
-                        ++s_si;
-                    }
                     s_tiles = 0;
-                    if (s_item < 0) return;
+                    if (!mbar_wait(bar(SCHED_FULL + slot), (s_si >> 2) & 1U)) {
+                        fail(311);
+                        return;
+                    }
+                    const int item = *reinterpret_cast<volatile int *>(&sched_item[slot]);
+                    mbar_arrive_local(bar(SCHED_EMPTY + slot));
+                    ++s_si;
+                    if (item < 0) return;
                     int kb;
-                    item_range(cu_s, p, n_valid, (s_item / p.hq) * A_BQ, &kb, &s_tiles);
+                    item_range(cu_s, p, n_valid, (item / p.hq) * A_BQ, &kb, &s_tiles);
                     if (s_tiles > 0) return;
                 }
             };
-            auto issue_s = [&]() -> bool {   // S[s_g] = Q K^T for tile s_t of item s_item
-                const uint32_t ks = s_g & 1U, b = s_g & 1U;
-                if (s_t == 0 && !mbar_wait(bar(Q_FULL), s_iq & 1U)) {
-                    atomicExch(err_flag, 305);
-                    return false;
-                }
-                if (!mbar_wait(bar(K_FULL + ks), (s_g >> 1) & 1U)) {
-                    atomicExch(err_flag, 303);
-                    return false;
-                }
-                if (s_g >= 2U && !mbar_wait(bar(BUF_FREE + b), ((s_g - 2U) >> 1) & 1U)) {   // O_part[s_g - 2] has been read back
-                    atomicExch(err_flag, 304);
-                    return false;
-                }
+            auto issue_s = [&]() {
+                // S[s_g] goes into buffer s_g & 1, over P of two steps before: P V of that step was issued by this thread
+                // already and executes first
+                const uint32_t s = s_g % ST, qs = s_item % QST;
+                if (s_tile == 0 && !mbar_wait(bar(Q_FULL + qs), (s_item / QST) & 1U)) return fail(305);
+                if (!mbar_wait(bar(K_FULL + s), (s_g / ST) & 1U)) return fail(303);
                 tcgen05_fence_after();
-                const uint32_t k_base = smem_u32(smem + plan::OFF_K + ks * plan::KV_BYTES);
 #pragma unroll
-                for (int kk = 0; kk < A_DH / UMMA_K; ++kk) {
-                    tcgen05_mma_f16(tmem_base + b * A_BKV, make_smem_desc(q_base + kk * 32, 16, 1024), make_smem_desc(k_base + kk * 32, 16, 1024),
-                                    IDESC_S, kk != 0 ? 1U : 0U);
+                for (int kk = 0; kk < DH / UMMA_K; ++kk) {
+                    const uint64_t step = (uint64_t)((kk & 3) * 2);
+                    tcgen05_mma_f16(tmem_base + plan::COL_S + (s_g & 1U) * A_BKV, q_d + qs * QTILE16 + (kk >> 2) * QBLOCK16 + step,
+                                    k_d + s * TILE16 + (kk >> 2) * BLOCK16 + step, IDESC_S, kk != 0 ? 1U : 0U);
                 }
-                tcgen05_commit(bar(S_FULL + b));
-                tcgen05_commit(bar(K_EMPTY + ks));
+                tcgen05_commit(bar(S_FULL + (s_g & 1U)));
+                tcgen05_commit(bar(K_EMPTY + s));
                 ++s_g;
-                if (++s_t == s_tiles) {   // last S of the item: the Q tile may be replaced
-                    tcgen05_commit(bar(Q_EMPTY));
-                    ++s_iq;
-                    s_t = 0;
-                    s_seek();
+                if (++s_tile == (uint32_t)s_tiles) {
+                    tcgen05_commit(bar(Q_EMPTY + qs));
+                    ++s_item;
+                    seek();
                 }
-                return true;
             };
-            s_seek();
-            uint32_t pv_g = 0;
-            if (s_tiles > 0) ok = issue_s();
-            while (ok && pv_g < s_g) {
-                // The next S is issued ahead of the pending P V only inside an item. The first S of the NEXT
-                // item waits for that item's Q tile, and must not hold back the last P V of this one.
-                const bool s_first = s_tiles > 0 && s_t != 0;
-                if (s_first) {
-                    ok = issue_s();
-                    if (!ok) break;
+            // P V walks behind S: the tiles of the item it is in, and of the one S has moved on to
+            uint32_t n_item = 0;
+            int tiles = 0, t = 0;
+            seek();
+            tiles = s_tiles;
+            if (ok && s_tiles > 0) issue_s();
+#pragma unroll 1
+            for (uint32_t g = 0; ok && g < s_g; ++g) {
+                const int ahead = s_tiles;
+                if (s_tiles > 0) issue_s();
+                if (!ok) break;
+                const uint32_t s = g % ST;
+                if (t == 0 && !mbar_wait(bar(O_FREE), (n_item & 1U) ^ 1U)) {   // O of the previous item has been read back
+                    fail(304);
+                    break;
                 }
-                const uint32_t b = pv_g & 1U;
-                if (!mbar_wait(bar(P_FULL), pv_g & 1U) || !mbar_wait(bar(V_FULL), pv_g & 1U)) {
-                    atomicExch(err_flag, 306);
+                if (!mbar_wait(bar(V_FULL + s), (g / ST) & 1U) || !mbar_wait(bar(P_FULL + (g & 1U)), (g >> 1) & 1U)) {
+                    fail(306);
                     break;
                 }
                 tcgen05_fence_after();
 #pragma unroll
                 for (int kk = 0; kk < A_BKV / UMMA_K; ++kk) {
-                    // A = P, K-major, blocks of 64 keys 16 KB apart; B = V stored [key][dh]: MN-major, 16 keys = 2048 B
-                    tcgen05_mma_f16(tmem_base + b * A_BKV, make_smem_desc(p_base + (kk >> 2) * (A_BQ * 128) + (kk & 3) * 32, 16, 1024),
-                                    make_smem_desc(v_base + kk * 2048, A_BKV * 128, 1024), IDESC_PV, kk != 0 ? 1U : 0U);
+                    tcgen05_mma_f16_ts(tmem_base + plan::COL_O, tmem_base + plan::COL_S + (g & 1U) * A_BKV + kk * 8, v_d + s * TILE16 + (uint64_t)(kk * 128),
+                                       IDESC_PV, (t != 0 || kk != 0) ? 1U : 0U);
                 }
-                tcgen05_commit(bar(O_FULL + b));
-                tcgen05_commit(bar(V_EMPTY));
-                tcgen05_commit(bar(P_EMPTY));
-                ++pv_g;
-                if (!s_first && s_tiles > 0) {
-                    ok = issue_s();
+                tcgen05_commit(bar(V_EMPTY + s));
+                tcgen05_commit(bar(PV_DONE + (g & 1U)));
+                if (++t == tiles) {
+                    // the S cursor is one step ahead, so it already stands in the next item
+                    t = 0;
+                    ++n_item;
+                    tiles = ahead;
                 }
             }
         }
     } else {
-        // ---------------- softmax: two threads per query row ----------------
-        const int quad = warp & 3, half = (warp - 2) >> 2;          // half 0: key columns 0..63, output columns 0..31
+        // ---------------- softmax: one thread per query row ----------------
+        const int quad = warp & 3;
         const int r = quad * 32 + lane;
         const float sl2 = p.scale * LOG2E_F;
         const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
-        unsigned char *p_row = smem + plan::OFF_P + half * (A_BQ * 128) + r * 128;   // this thread's 64 keys = one 128-byte row of block `half`
-        uint32_t g = 0, n_item = 0;
-        // A wait that gives up makes the warp "dead": it records the error, stops waiting and reading
-        // tensor memory, but keeps walking the loops so that its partner warp never blocks on a named barrier.
+        uint32_t g = 0;
+        // A wait that gives up ends the warp's work (error recorded); the other roles then run into their own limits.
         bool dead = false;
         auto wait_or_die = [&](int which, uint32_t parity, int code) {
-            if (!dead && !mbar_wait(bar(which), parity)) {
+            int ok = 1;
+            if (lane == 0) ok = mbar_wait(bar(which), parity) ? 1 : 0;
+            if (!__shfl_sync(0xffffffffU, ok, 0)) {
                 dead = true;
                 if (lane == 0) atomicExch(err_flag, code);
             }
         };
-        // bounded rendezvous of the two warps of a lane quadrant (mbarrier with two arrivals per phase)
-        uint32_t pair_phase = 0;
-        auto pair_sync = [&]() {
-            __syncwarp();
-            if (lane == 0) mbar_arrive_local(bar(PAIR + quad));
-            wait_or_die(PAIR + quad, pair_phase & 1U, 312);
-            ++pair_phase;
-        };
-        for (uint32_t si = 0;; ++si) {
-            // next scheduled item; a dead warp stops consuming (its partner then gives up at the next rendezvous)
+        for (uint32_t si = 0; !dead; ++si) {
             const uint32_t slot = si & 3U;
             wait_or_die(SCHED_FULL + slot, (si >> 2) & 1U, 313);
             if (dead) break;
@@ -331,123 +363,127 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                 lo_key = seg_start_of(cu_s, p.batch, qi);
                 if (p.window > 0) lo_key = max(lo_key, qi - p.window + 1);
             }
-            float m = -INFINITY, l = 0.0f, alpha_pending = 1.0f;
-            float o[32];
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = 0.0f;
-            auto accumulate_o = [&](uint32_t g_prev) {
-                const uint32_t b = g_prev & 1U;
-                wait_or_die(O_FULL + b, (g_prev >> 1) & 1U, 307);
-                if (dead) return;
-                tcgen05_fence_after();
-                uint32_t v[32];
-                tmem_ld_32x32b_x32(lane_base + b * A_BKV + half * 32, v);
-                tcgen05_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_local(bar(BUF_FREE + b));
-#pragma unroll
-                for (int i = 0; i < 32; ++i) o[i] = o[i] * alpha_pending + __uint_as_float(v[i]);
-            };
+            // m: the maximum O and l are relative to (log2 units, may lag the true maximum by up to A_RESCALE); m_true: the maximum
+            float m = -INFINITY, m_true = -INFINITY, l = 0.0f;
+#pragma unroll 1
             for (int t = 0; t < n_tiles; ++t, ++g) {
-                const uint32_t b = g & 1U;
-                const int key0 = kv_begin + t * A_BKV + half * 64;   // first key of this thread's 64 columns
-                wait_or_die(S_FULL + b, (g >> 1) & 1U, 308);
+                const int key0 = kv_begin + t * A_BKV;
+                const uint32_t s_col = lane_base + plan::COL_S + (g & 1U) * A_BKV;
+                // allowed local columns [c_lo, c_hi] of this row
+                const int c_lo = valid ? max(0, lo_key - key0) : A_BKV, c_hi = valid ? min(A_BKV - 1, qi - key0) : -1;
+                const bool live = __any_sync(0xffffffffU, c_lo <= c_hi), full = __all_sync(0xffffffffU, c_lo == 0 && c_hi == A_BKV - 1);
+                wait_or_die(S_FULL + (g & 1U), (g >> 1) & 1U, 308);
+                if (dead) break;
                 tcgen05_fence_after();
-                // allowed local columns [c_lo, c_hi] of this thread's half
-                const int c_lo = valid ? max(0, lo_key - key0) : 64, c_hi = valid ? min(63, qi - key0) : -1;
-                const uint32_t s_addr = lane_base + b * A_BKV + half * 64;
-                const bool any0 = !dead && __any_sync(0xffffffffU, c_lo <= 31 && c_hi >= 0), any1 = !dead && __any_sync(0xffffffffU, c_lo <= 63 && c_hi >= 32);
-                const bool all0 = __all_sync(0xffffffffU, c_lo <= 0 && c_hi >= 31), all1 = __all_sync(0xffffffffU, c_lo <= 32 && c_hi >= 63);
-                float tmax = -INFINITY;
+                if (live) {
+                    uint32_t v[2][32];
+                    tmem_ld_32x32b_x32_nowait(s_col, v[0]);
+                    tmem_ld_32x32b_x32_nowait(s_col + 32, v[1]);
+                    tmem_ld_wait();
+                    if (!full) {
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    if (!(c == 0 ? any0 : any1)) continue;
-                    uint32_t v[32];
-                    tmem_ld_32x32b_x32(s_addr + c * 32, v);
-                    if (c == 0 ? all0 : all1) {
+                        for (int c = 0; c < 2; ++c) {
+                            const int lo = max(c_lo - c * 32, 0), hi = min(c_hi - c * 32, 31);
+                            const uint32_t allowed = lo <= hi ? (0xffffffffU << lo) & (0xffffffffU >> (31 - hi)) : 0U;
 #pragma unroll
-                        for (int i = 0; i < 32; i += 2) tmax = fmaxf(tmax, fmaxf(__uint_as_float(v[i]), __uint_as_float(v[i + 1])));
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) tmax = (c * 32 + i >= c_lo && c * 32 + i <= c_hi) ? fmaxf(tmax, __uint_as_float(v[i])) : tmax;
+                            for (int i = 0; i < 32; ++i) v[c][i] = (allowed & (1U << i)) ? v[c][i] : 0xff800000U;
+                        }
                     }
-                }
-                // exchange the row maximum with the thread that owns the other 64 columns
-                xch[g & 1U][half][r] = tmax;
-                pair_sync();
-                tmax = fmaxf(tmax, xch[g & 1U][half ^ 1][r]);
-                if (t >= 1) accumulate_o(g - 1U);
-                const float m_new = fmaxf(m, tmax * sl2);
-                const float alpha = m == -INFINITY ? (m_new == -INFINITY ? 1.0f : 0.0f) : ex2_approx(m - m_new);
-                const float m_use = m_new == -INFINITY ? 0.0f : m_new;
-                wait_or_die(P_EMPTY, (g & 1U) ^ 1U, 309);       // P V of the previous tile has read the P tile
-                float rsum = 0.0f;
+                    float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    const bool anyc = c == 0 ? any0 : any1, allc = c == 0 ? all0 : all1;
-                    uint32_t packed[16];
-                    if (anyc) {
-                        uint32_t v[32];
-                        tmem_ld_32x32b_x32(s_addr + c * 32, v);
-                        if (allc) {
+                    for (int i = 0; i < 64; i += 8) {
 #pragma unroll
-                            for (int i = 0; i < 32; i += 2) {
-                                const float p0 = ex2_approx(fmaf(__uint_as_float(v[i]), sl2, -m_use));
-                                const float p1 = ex2_approx(fmaf(__uint_as_float(v[i + 1]), sl2, -m_use));
-                                rsum += p0 + p1;
-                                packed[i >> 1] = half_pack<T>::pack(p0, p1);
-                            }
-                        } else {
+                        for (int e = 0; e < 4; ++e) mx[e] = fmaxf(mx[e], fmaxf(__uint_as_float(v[i >> 5][(i & 31) + 2 * e]), __uint_as_float(v[i >> 5][(i & 31) + 2 * e + 1])));
+                    }
+                    const float m_cand = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl2;
+                    m_true = fmaxf(m_true, m_cand);
+                    const bool bump = m_cand > m + A_RESCALE || (m == -INFINITY && m_cand != -INFINITY);
+                    if (__any_sync(0xffffffffU, bump)) {
+                        const float alpha = bump ? ex2_approx(m - m_cand) : 1.0f;   // m = -inf: 0
+                        if (__any_sync(0xffffffffU, bump && m != -INFINITY)) {
+                            wait_or_die(PV_DONE + ((g - 1U) & 1U), ((g - 1U) >> 1) & 1U, 309);   // O holds every step before this one
+                            if (dead) break;
+                            tcgen05_fence_after();
+#pragma unroll 1
+                            for (int c = 0; c < DH / 8; ++c) {
+                                uint32_t o[8];
+                                tmem_ld_32x32b_x8(lane_base + plan::COL_O + c * 8, o);
 #pragma unroll
-                            for (int i = 0; i < 32; i += 2) {
-                                const int col = c * 32 + i;
-                                const float p0 = (col >= c_lo && col <= c_hi) ? ex2_approx(fmaf(__uint_as_float(v[i]), sl2, -m_use)) : 0.0f;
-                                const float p1 = (col + 1 >= c_lo && col + 1 <= c_hi) ? ex2_approx(fmaf(__uint_as_float(v[i + 1]), sl2, -m_use)) : 0.0f;
-                                rsum += p0 + p1;
-                                packed[i >> 1] = half_pack<T>::pack(p0, p1);
+                                for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                                tmem_st_32x32b_x8(lane_base + plan::COL_O + c * 8, o);
                             }
                         }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) packed[i] = 0U;
+                        l *= alpha;
+                        if (bump) m = m_cand;
                     }
+                    const f32x2 scale2 = f2_make(sl2, sl2), shift2 = m == -INFINITY ? f2_make(0.0f, 0.0f) : f2_make(-m, -m);
+                    f32x2 sum0 = f2_make(0.0f, 0.0f), sum1 = sum0;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int chunk = c * 4 + j;
-                        *reinterpret_cast<uint4 *>(p_row + ((chunk ^ (r & 7)) << 4)) = make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
+                    for (int c = 0; c < 2; ++c) {
+                        uint32_t packed[16];
+#pragma unroll
+                        for (int i = 0; i < 32; i += 2) {
+                            float p0, p1;
+                            f2_split(f2_fma(f2_make(__uint_as_float(v[c][i]), __uint_as_float(v[c][i + 1])), scale2, shift2), p0, p1);
+                            p0 = ex2_approx(p0);
+                            p1 = ex2_approx(p1);
+                            f32x2 &sum = (i & 2) ? sum1 : sum0;
+                            sum = f2_add(sum, f2_make(p0, p1));
+                            packed[i >> 1] = half_pack<T>::pack(p0, p1);
+                        }
+                        tmem_st_32x32b_x16(s_col + c * 16, packed);
                     }
+                    float a0, a1;
+                    f2_split(f2_add(sum0, sum1), a0, a1);
+                    l += a0 + a1;
+                } else {
+                    const uint32_t zero[16] = {0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U};
+                    tmem_st_32x32b_x16(s_col, zero);
+                    tmem_st_32x32b_x16(s_col + 16, zero);
                 }
-                l = l * alpha + rsum;
-                m = m_new;
-                alpha_pending = alpha;
+                tmem_st_wait();
                 tcgen05_fence_before();
-                fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_local(bar(P_FULL));
+                if (lane == 0) mbar_arrive_local(bar(P_FULL + (g & 1U)));
             }
-            if (n_tiles > 0) accumulate_o(g - 1U);   // also implies that every MMA of this item has completed
-            // ---- total row sum, normalise, store this thread's 32 output columns (two full 32-byte sectors) ----
-            xsum[n_item & 1U][half][r] = l;
-            pair_sync();
-            const float l_tot = l + xsum[n_item & 1U][half ^ 1][r];
-            ++n_item;
-            const float inv = (!dead && l_tot > 0.0f) ? 1.0f / l_tot : 0.0f;
-            if (qi < p.n_tokens) {
-                T *dst = out + ((size_t)qi * p.hq + h) * A_DH + half * 32;
+            if (dead) break;
+            // ---- normalise and store this row ----
+            const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+            T *dst = out + ((size_t)qi * p.hq + h) * DH;
+            if (n_tiles > 0) {
+                wait_or_die(PV_DONE + ((g - 1U) & 1U), ((g - 1U) >> 1) & 1U, 307);
+                if (dead) break;
+                tcgen05_fence_after();
+#pragma unroll 1
+                for (int c = 0; c < DH / 32; ++c) {
+                    uint32_t o[32];
+                    tmem_ld_32x32b_x32(lane_base + plan::COL_O + c * 32, o);
+                    if (c == DH / 32 - 1) {
+                        tcgen05_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive_local(bar(O_FREE));
+                    }
+                    if (qi < p.n_tokens) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    uint4 w;
-                    w.x = half_pack<T>::pack(o[8 * j] * inv, o[8 * j + 1] * inv);
-                    w.y = half_pack<T>::pack(o[8 * j + 2] * inv, o[8 * j + 3] * inv);
-                    w.z = half_pack<T>::pack(o[8 * j + 4] * inv, o[8 * j + 5] * inv);
-                    w.w = half_pack<T>::pack(o[8 * j + 6] * inv, o[8 * j + 7] * inv);
-                    *reinterpret_cast<uint4 *>(dst + 8 * j) = w;
+                        for (int j = 0; j < 4; ++j) {
+                            // (a row without allowed keys has only zero probabilities; its inverse is zero)
+                            uint4 w;
+                            w.x = half_pack<T>::pack(__uint_as_float(o[8 * j]) * inv, __uint_as_float(o[8 * j + 1]) * inv);
+                            w.y = half_pack<T>::pack(__uint_as_float(o[8 * j + 2]) * inv, __uint_as_float(o[8 * j + 3]) * inv);
+                            w.z = half_pack<T>::pack(__uint_as_float(o[8 * j + 4]) * inv, __uint_as_float(o[8 * j + 5]) * inv);
+                            w.w = half_pack<T>::pack(__uint_as_float(o[8 * j + 6]) * inv, __uint_as_float(o[8 * j + 7]) * inv);
+                            *reinterpret_cast<uint4 *>(dst + c * 32 + 8 * j) = w;
+                        }
+                    }
                 }
+            } else if (qi < p.n_tokens) {
+#pragma unroll
+                for (int j = 0; j < DH / 8; ++j) *reinterpret_cast<uint4 *>(dst + 8 * j) = make_uint4(0U, 0U, 0U, 0U);
             }
-            if (stats != nullptr && valid && half == 0) {
+            if (stats != nullptr && valid) {
                 float *s = stats + ((size_t)qi * p.hq + h) * 3;
-                s[0] = m == -INFINITY ? m : m * LN2_F;
-                s[1] = l_tot;
+                s[0] = m_true == -INFINITY ? m_true : m_true * LN2_F;
+                s[1] = m_true == -INFINITY ? l : l * ex2_approx(m - m_true);
                 s[2] = 0.0f;
             }
         }
@@ -468,25 +504,25 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
     }
 }
 
-template <typename T>
+template <typename T, int DH>
 gd_status launch_fwd(gd_backend *be, const gdb_flash_args *a)
 {
-    using plan = attn5_plan;
-    auto kern = attn5_fwd_kernel<T>;
+    using plan = attn5_plan<DH>;
+    auto kern = attn5_fwd_kernel<T, DH>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, plan::TOTAL);
         if (e != cudaSuccess) return gdb_fail(be, e, "tcgen05 attention smem attribute");
         configured = true;
     }
-    // Two CTAs fit an SM by construction (2 x 256 tensor-memory columns, 2 x 106 KB shared memory, 2 x 30720
+    // Two CTAs fit an SM by construction (2 x 256 tensor-memory columns, 2 x at most 104 KB shared memory, 2 x 32256
     // registers). Nothing waits across CTAs, so if fewer were co-resident the rest would simply run later.
     const int resident = 2 * (be->sm_count - be->sm_reserve);
     CUtensorMap mq, mk, mv;
     const uint64_t n = (uint64_t)a->n_tokens;
-    const bool ok = make_tmap(&mq, a->dtype, a->q, n, (uint64_t)a->hq * A_DH, (uint64_t)a->hq * A_DH * 2U, 64, A_BQ) &&
-                    make_tmap(&mk, a->dtype, a->k, n, (uint64_t)a->hkv * A_DH, (uint64_t)a->hkv * A_DH * 2U, 64, A_BKV) &&
-                    make_tmap(&mv, a->dtype, a->v, n, (uint64_t)a->hkv * A_DH, (uint64_t)a->hkv * A_DH * 2U, 64, A_BKV);
+    const bool ok = make_tmap(&mq, a->dtype, a->q, n, (uint64_t)a->hq * DH, (uint64_t)a->hq * DH * 2U, 64, A_BQ) &&
+                    make_tmap(&mk, a->dtype, a->k, n, (uint64_t)a->hkv * DH, (uint64_t)a->hkv * DH * 2U, 64, A_BKV) &&
+                    make_tmap(&mv, a->dtype, a->v, n, (uint64_t)a->hkv * DH, (uint64_t)a->hkv * DH * 2U, 64, A_BKV);
     if (!ok) {
         return GD_ERR_UNSUPPORTED;
     }
@@ -503,9 +539,10 @@ gd_status launch_fwd(gd_backend *be, const gdb_flash_args *a)
 gd_status gdb_attn5_forward(gd_backend *be, const gdb_flash_args *a)
 {
     const uintptr_t al = (uintptr_t)a->q | (uintptr_t)a->k | (uintptr_t)a->v | (uintptr_t)a->out_or_dq;
-    if ((a->dtype != GDB_DTYPE_F16 && a->dtype != GDB_DTYPE_BF16) || a->dh != A_DH || a->causal == 0 || a->prefix != 0 || a->window < 0 ||
-        (al % 16U) != 0U || a->hkv <= 0 || (a->hq % a->hkv) != 0 || a->hq > 65535 || a->batch > A_MAX_CU || a->n_tokens < A_BQ) {
+    if ((a->dtype != GDB_DTYPE_F16 && a->dtype != GDB_DTYPE_BF16) || (a->dh != 64 && a->dh != 128) || a->causal == 0 || a->prefix != 0 ||
+        a->window < 0 || (al % 16U) != 0U || a->hkv <= 0 || (a->hq % a->hkv) != 0 || a->hq > 65535 || a->batch > A_MAX_CU || a->n_tokens < A_BQ) {
         return GD_ERR_UNSUPPORTED;
     }
-    return a->dtype == GDB_DTYPE_F16 ? launch_fwd<__half>(be, a) : launch_fwd<__nv_bfloat16>(be, a);
+    if (a->dh == 64) return a->dtype == GDB_DTYPE_F16 ? launch_fwd<__half, 64>(be, a) : launch_fwd<__nv_bfloat16, 64>(be, a);
+    return a->dtype == GDB_DTYPE_F16 ? launch_fwd<__half, 128>(be, a) : launch_fwd<__nv_bfloat16, 128>(be, a);
 }
