@@ -669,7 +669,7 @@ gd_status gd_backend_sdpa_varlen(gd_backend *be, const gd_backend_tensor_view *q
 }
 
 // `out` (the forward output) and `dq_accum` (FP32 scratch of q's element count) are optional: with both, forward
-// statistics and head_dim 64 the backward runs as one attention pass.
+// statistics and head_dim 64 or 128 the backward runs as one attention pass.
 static gd_status sdpa_varlen_backward_impl(gd_backend *be, const gd_backend_tensor_view *grad_out, const gd_backend_tensor_view *q, const gd_backend_tensor_view *k, const gd_backend_tensor_view *v, const gd_backend_tensor_view *cu_seqlens, const gd_backend_tensor_view *grad_q, const gd_backend_tensor_view *grad_k, const gd_backend_tensor_view *grad_v, const gd_backend_tensor_view *stats, const gd_backend_sdpa_varlen_args *args, const gd_backend_tensor_view *out, const gd_backend_tensor_view *dq_accum,
                                            int32_t *query_grad_in_accum = NULL)
 {
@@ -721,10 +721,11 @@ static gd_status sdpa_varlen_backward_impl(gd_backend *be, const gd_backend_tens
         if (op == NULL || acc == NULL) {
             return GD_ERR_INVALID_ARGUMENT;
         }
-        fa.keep_dq32 = query_grad_in_accum != NULL ? 1 : 0;
+        // (head_dim 128: the query gradient is rounded here, the entry's contract leaves it in the accumulator at 64 only)
+        fa.keep_dq32 = query_grad_in_accum != NULL && p.dh == 64 ? 1 : 0;
         st = gdb_flash_varlen_backward_with_out(be, &fa, op, acc);
         if (st != GD_ERR_UNSUPPORTED) {
-            if (st == GD_OK && query_grad_in_accum != NULL) {
+            if (st == GD_OK && fa.keep_dq32 != 0) {
                 *query_grad_in_accum = 1;
             }
             return st;

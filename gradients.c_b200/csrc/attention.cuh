@@ -20,12 +20,18 @@ struct gdb_flash_args {
 // then runs the general kernels.
 gd_status gdb_flash_varlen_forward(gd_backend *be, const gdb_flash_args *a);
 gd_status gdb_flash_varlen_backward(gd_backend *be, const gdb_flash_args *a, bool have_forward_stats);
-// Single-pass backward when the forward output is available (attention_flash.cu); dq32: FP32 scratch [N, Hq, 64].
+// Single-pass backward when the forward output is available (attention_flash.cu); dq32: FP32 scratch [N, Hq, Dh].
 gd_status gdb_flash_varlen_backward_with_out(gd_backend *be, const gdb_flash_args *a, const void *out, float *dq32);
 // tcgen05 / tensor-memory forward (attention_tcgen05.cu); GD_ERR_UNSUPPORTED outside its fast path.
 gd_status gdb_attn5_forward(gd_backend *be, const gdb_flash_args *a);
+// What the preparation kernel (attention_flash.cu) leaves for the tensor-memory backward, all in device memory:
+struct gdb_attn_bwd_meta {
+    int n_pad;         // tokens rounded up to the query tile of 64: row pitch of the two arrays of statistics
+    float *neg_m2;     // [Hq, n_pad]  -(m log2e + log2 l)
+    float *neg_d;      // [Hq, n_pad]  -D scale
+    int *row_hi;       // [N]  last query that may see this key (-1: none)
+    int *tile_nqt;     // [ceil(N / 128)]  64-row query tiles, from the key tile's own first row on, that may see one of its keys
+};
 // tcgen05 / tensor-memory key-stationary backward (attention_tcgen05_bwd.cu): dK, dV and the FP32 dQ accumulator dq32
-// [N, Hq, 64] (zero on entry) from complete statistics (max, sum, D) and the mask bounds `meta` (int [N + ceil(N / 128)]:
-// first allowed key per query row, query tiles per key tile; written by the preparation kernel in attention_flash.cu).
-// GD_ERR_UNSUPPORTED outside its fast path.
-gd_status gdb_attn5_backward(gd_backend *be, const gdb_flash_args *a, float *dq32, const int *meta);
+// [N, Hq, Dh] (zero on entry). GD_ERR_UNSUPPORTED outside its fast path.
+gd_status gdb_attn5_backward(gd_backend *be, const gdb_flash_args *a, float *dq32, const gdb_attn_bwd_meta *m);

@@ -688,69 +688,106 @@ __global__ void dq_convert_kernel(const float4 *__restrict__ src, uint4 *__restr
     }
 }
 
-// Preparation of the single-pass backward: D[row, head] = sum_c dO * O (stats[.., 2]) and dq32 = 0.
-// Eight threads per (row, head) of 64 elements, 16 bytes of dO and of O each. With `meta` != NULL it also leaves the mask
-// bounds the tensor-memory kernel reads instead of searching cu_seqlens per step: meta[row] = first key row `row` may
-// attend to (start of its sequence, moved up by the window; INT_MAX behind the last sequence), and, for every tile of 128
-// keys, meta[n_tokens + tile] = number of 128-row query tiles, starting with the tile's own, that hold a query allowed to
-// see one of its keys (0 behind the last sequence).
-template <typename T>
+// Preparation of the single-pass backward, 16 rows per block: D[row, head] = sum_c dO * O (stats[.., 2]) and dq32 = 0. With
+// m.row_hi != NULL it also leaves what the tensor-memory kernel reads per step instead of forming it from cu_seqlens and the
+// statistics (see gdb_attn_bwd_meta): the statistics per head with consecutive rows, so that a step's 64 rows are one
+// copy, last allowed query per key, and the number of query tiles per key tile. dO, O and the statistics are read in
+// memory order; D crosses shared memory to be written by head.
+constexpr int PREP_ROWS = 16;
+template <typename T, int DH>
 __global__ void bwd_prep_kernel(const uint4 *__restrict__ go, const uint4 *__restrict__ out, float *__restrict__ stats, float4 *__restrict__ dq32,
-                                size_t n_vec, const int *__restrict__ cu, int batch, int n_tokens, int hq, int window, int *__restrict__ meta)
+                                const int *__restrict__ cu, int batch, int n_tokens, int hq, int window, float scale, gdb_attn_bwd_meta m)
 {
     gdb_pdl_sync();
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;   // one 8-element piece; n_vec is a multiple of 8
-    float s = 0.0f;
-    if (i < n_vec) {
-        gdb_vec8<T> a, b;
-        a.raw = go[i];
-        b.raw = out[i];
+    constexpr int PIECES = DH / 8;                      // 16-byte pieces of a (row, head)
+    extern __shared__ float d_s[];                      // [PREP_ROWS][hq]
+    const int row0 = (int)blockIdx.x * PREP_ROWS, rows = min(PREP_ROWS, n_tokens - row0);
+    const int n_vec = max(rows, 0) * hq * PIECES;
+    const size_t base = (size_t)row0 * hq * PIECES;
+    for (int i = threadIdx.x; i < ((n_vec + 31) & ~31); i += blockDim.x) {
+        float s = 0.0f;
+        if (i < n_vec) {
+            gdb_vec8<T> a, b;
+            a.raw = go[base + i];
+            b.raw = out[base + i];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) s += a.get(e) * b.get(e);
-        dq32[2 * i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        dq32[2 * i + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) s += __shfl_xor_sync(0xffffffffU, s, o);
-    if (i < n_vec && (threadIdx.x & 7) == 0) stats[(i >> 3) * 3U + 2U] = s;
-    if (meta != nullptr && i < n_vec && (i % ((size_t)hq * 8U)) == 0U) {
-        const int row = (int)(i / ((size_t)hq * 8U));
-        const int n_valid = min(cu[batch], n_tokens);
-        int lo = 0x7fffffff;
-        if (row < n_valid) {
-            lo = cu[seg_of(cu, batch, row)];
-            if (window > 0) lo = max(lo, row - window + 1);
+            for (int e = 0; e < 8; ++e) s += a.get(e) * b.get(e);
+            dq32[2 * (base + i)] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            dq32[2 * (base + i) + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
-        meta[row] = lo;
+#pragma unroll
+        for (int o = 1; o < PIECES; o <<= 1) s += __shfl_xor_sync(0xffffffffU, s, o);
+        if (i < n_vec && (i % PIECES) == 0) d_s[i / PIECES] = s;
+    }
+    __syncthreads();
+    const int n_valid = min(cu[batch], n_tokens);
+    for (int i = threadIdx.x; i < PREP_ROWS * hq; i += blockDim.x) {
+        const int r = i / hq, row = row0 + r;
+        float m2 = 0.0f, d = 0.0f;
+        if (row < n_tokens) {
+            float *st = stats + ((size_t)row0 * hq + i) * 3U;
+            const float mx = st[0], l = st[1];
+            st[2] = d_s[i];
+            if (row < n_valid) {
+                // P = exp(s scale - max) / sum = exp2(s scale log2e - m2); a row without keys has no products either
+                m2 = l > 0.0f && mx != -INFINITY ? -fmaf(mx, 1.4426950408889634f, __log2f(l)) : -INFINITY;
+                d = -d_s[i] * scale;
+            }
+        }
+        if (m.neg_m2 != nullptr && row < m.n_pad) {
+            const size_t at = (size_t)(i - r * hq) * m.n_pad + row;
+            m.neg_m2[at] = m2;
+            m.neg_d[at] = d;
+        }
+    }
+    if (m.row_hi != nullptr && threadIdx.x < PREP_ROWS && row0 + (int)threadIdx.x < n_tokens) {
+        const int row = row0 + (int)threadIdx.x;
+        int hi = -1;
+        if (row < n_valid) {
+            hi = min(cu[seg_of(cu, batch, row) + 1], n_valid) - 1;
+            if (window > 0) hi = min(hi, row + window - 1);
+        }
+        m.row_hi[row] = hi;
         if ((row & 127) == 0) {
             int n_qt = 0;
             if (row < n_valid) {
                 const int last_key = min(row + 128, n_valid) - 1;
-                int q_hi = cu[seg_of(cu, batch, last_key) + 1];       // exclusive
+                int q_hi = min(cu[seg_of(cu, batch, last_key) + 1], n_valid);   // exclusive
                 if (window > 0) q_hi = min(q_hi, last_key + window);
-                q_hi = min(q_hi, n_valid);
-                n_qt = (q_hi - 1) / 128 - row / 128 + 1;
+                n_qt = (q_hi - 1 - row) / 64 + 1;
             }
-            meta[n_tokens + (row >> 7)] = n_qt;
+            m.tile_nqt[row >> 7] = n_qt;
         }
     }
 }
 
-// Backward in one attention pass (head_dim 64, statistics (max, sum) saved by the forward): D from dO and the forward
-// output, then the key-stationary kernel forms dK, dV and accumulates dQ in FP32, then dQ is rounded.
-template <typename T>
+// Backward in one attention pass (statistics (max, sum) saved by the forward): D from dO and the forward output, then the
+// key-stationary kernel forms dK, dV and accumulates dQ in FP32, then dQ is rounded. head_dim 128 has the tensor-memory kernel only.
+template <typename T, int DH>
 gd_status backward_single_pass(gd_backend *be, const gdb_flash_args *a, const flash_params &p, const void *out, float *dq32)
 {
-    const size_t n = (size_t)a->n_tokens * a->hq * 64U, n_vec = n / 8U;
-    // mask bounds for the tensor-memory kernel live at the start of the backend workspace between the two launches
-    const size_t meta_bytes = ((size_t)a->n_tokens + (size_t)(a->n_tokens + 127) / 128U) * sizeof(int);
-    int *meta = (be->attn_mode == 0 && meta_bytes <= be->ws_bytes) ? (int *)be->ws : nullptr;
-    gdb_launch(bwd_prep_kernel<T>, (unsigned)((n_vec + 255U) / 256U), 256, 0, be->stream, (const uint4 *)a->grad_out, (const uint4 *)out, a->stats,
-               (float4 *)dq32, n_vec, a->cu, a->batch, a->n_tokens, a->hq, a->window, meta);
+    const size_t n = (size_t)a->n_tokens * a->hq * DH, n_vec = n / 8U;
+    // statistics by head and mask bounds live at the start of the backend workspace between the two launches
+    gdb_attn_bwd_meta m;
+    memset(&m, 0, sizeof(m));
+    m.n_pad = (a->n_tokens + 63) & ~63;
+    const size_t per_head = (size_t)m.n_pad * a->hq, tiles = (size_t)(a->n_tokens + 127) / 128U;
+    const bool tensor = be->attn_mode == 0 && a->n_tokens >= 128 && (2U * per_head + (size_t)m.n_pad + tiles) * sizeof(float) <= be->ws_bytes;
+    if (!tensor && DH != 64) {
+        return GD_ERR_UNSUPPORTED;
+    }
+    if (tensor) {
+        m.neg_m2 = (float *)be->ws;
+        m.neg_d = m.neg_m2 + per_head;
+        m.row_hi = (int *)(m.neg_d + per_head);
+        m.tile_nqt = m.row_hi + m.n_pad;
+    }
+    gdb_launch(bwd_prep_kernel<T, DH>, (unsigned)((m.n_pad + PREP_ROWS - 1) / PREP_ROWS), 256, (size_t)PREP_ROWS * a->hq * sizeof(float), be->stream,
+               (const uint4 *)a->grad_out, (const uint4 *)out, a->stats, (float4 *)dq32, a->cu, a->batch, a->n_tokens, a->hq, a->window, a->scale, m);
     gd_status st = gdb_launched(be, "flash_backward_prep");
     if (st != GD_OK) return st;
-    st = meta != nullptr ? gdb_attn5_backward(be, a, dq32, meta) : GD_ERR_UNSUPPORTED;   // tensor-memory kernel where the shape allows
-    if (st == GD_ERR_UNSUPPORTED) st = launch_kv<T, 64, 64, true>(be, a, p, dq32);
+    st = tensor ? gdb_attn5_backward(be, a, dq32, &m) : GD_ERR_UNSUPPORTED;   // tensor-memory kernel where the shape allows
+    if (st == GD_ERR_UNSUPPORTED && DH == 64) st = launch_kv<T, 64, 64, true>(be, a, p, dq32);
     if (st != GD_OK) return st;
     if (a->keep_dq32 != 0) {
         return GD_OK;   // the caller's next kernel reads the accumulator and rounds on load
@@ -801,13 +838,17 @@ gd_status gdb_flash_varlen_backward(gd_backend *be, const gdb_flash_args *a, boo
 }
 
 // Backward with the forward output at hand (not part of the reference's entry, src/core/backend.h:699-709): D = rowsum(dO o O)
-// replaces the query-stationary pass. `dq32`: FP32 scratch [N, Hq, 64]. GD_ERR_UNSUPPORTED outside head_dim 64 / the fast path.
+// replaces the query-stationary pass. `dq32`: FP32 scratch [N, Hq, Dh]. GD_ERR_UNSUPPORTED outside the fast path.
 gd_status gdb_flash_varlen_backward_with_out(gd_backend *be, const gdb_flash_args *a, const void *out, float *dq32)
 {
     const uintptr_t al = (uintptr_t)a->grad_out | (uintptr_t)a->out_or_dq | (uintptr_t)a->dk | (uintptr_t)a->dv | (uintptr_t)out | (uintptr_t)dq32;
-    if (!fast_path(a) || a->dh != 64 || (al % 16U) != 0U || a->stats == NULL || out == NULL || dq32 == NULL) {
+    // (16 rows of D per block in shared memory: up to 48 KB)
+    if (!fast_path(a) || (al % 16U) != 0U || a->stats == NULL || out == NULL || dq32 == NULL || a->hq > 768) {
         return GD_ERR_UNSUPPORTED;
     }
     const flash_params p = make_params(a);
-    return a->dtype == GDB_DTYPE_F16 ? backward_single_pass<__half>(be, a, p, out, dq32) : backward_single_pass<__nv_bfloat16>(be, a, p, out, dq32);
+    if (a->dh == 64) {
+        return a->dtype == GDB_DTYPE_F16 ? backward_single_pass<__half, 64>(be, a, p, out, dq32) : backward_single_pass<__nv_bfloat16, 64>(be, a, p, out, dq32);
+    }
+    return a->dtype == GDB_DTYPE_F16 ? backward_single_pass<__half, 128>(be, a, p, out, dq32) : backward_single_pass<__nv_bfloat16, 128>(be, a, p, out, dq32);
 }

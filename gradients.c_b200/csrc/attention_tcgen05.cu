@@ -22,8 +22,8 @@
 //     may overwrite it because one thread issues all products and they execute in order;
 //   * O is rescaled in tensor memory only when a row's maximum has grown by more than 2^8 since the last rescale (the sum is
 //     kept relative to the same stale maximum, so the result is the same); after the first tile that is rare;
-//   * the code of all roles stays near the 32 KB of the first-level instruction cache (waits and searches are not unrolled, a
-//     step has one masked and one unmasked way to the same exponentials): at 57 KB the kernel ran at a third of this speed.
+//   * the code of all roles stays near the 32 KB of the first-level instruction cache: waits and searches are not unrolled (57 KB
+//     before), a step has one masked and one unmasked way to the same exponentials.
 // 32768 tokens in sequences of 16-512, 8 heads of 64: 72 us (one step at a time, P through shared memory: 124 us); 8191 tokens
 // in sequences of 256-2048, 16 heads of 128, window 1024: 78 us (mma.sync kernel: 286 us).
 // Tensor memory per CTA (256 columns): S / P 2 x 64, O head_dim.
@@ -90,28 +90,6 @@ __device__ __forceinline__ void item_range(const int *cu_s, const attn5_params &
         *kv_begin = kb;
         *n_tiles = (kv_end - kb + A_BKV - 1) / A_BKV;
     }
-}
-
-// pairs of FP32 values in one register pair
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 f2_make(float lo, float hi)
-{
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void f2_split(f32x2 p, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p)); }
-__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b)
-{
-    f32x2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c)
-{
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
 }
 
 __device__ __forceinline__ void mbar_arrive_local(uint32_t bar)
