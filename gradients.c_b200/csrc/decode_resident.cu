@@ -1,0 +1,590 @@
+// The greedy KV-cache decode of decode_mega.cu for at most 16 sequences and a model that fits the shared memory of the GPU:
+// ONE cooperative launch whose CTAs keep their share of all weights in shared memory for the whole run.
+//
+// What bounds a step of few sequences is the chain of its 5 L + 1 dependent phases, each an exchange of activations through L2.
+// The benchmark model's weights are 22 MB = 149 KB per SM, so every unit of 16 output columns of every projection is given to one
+// CTA, loaded once per launch, and a phase is: wait for the previous phase, read the activation rows (B KB), [RMSNorm,] multiply
+// from shared memory, add the eight k ranges, epilogue, publish. Against decode_mega.cu, which serves up to 64 sequences and
+// models of any size from L2, that removes 16-48 KB of weight copies and the 64-row tile from every phase; further:
+//   * a phase waits only for the CTAs that had work in the phase before it, and CTAs without work in a phase neither wait
+//     nor arrive (one counter per phase, monotone over the steps);
+//   * the logits are not written: a unit's epilogue takes the maximum of its 16 columns per row (soft cap included) and merges
+//     it with a 64-bit atomic maximum whose low half orders equal values by first index, so sampling is no phase of its own;
+//   * norm weights, biases, residuals and cos / sin values are read ahead of the wait.
+// Every sum is formed as in decode_parts.cuh (eight k ranges, k16 products in order, ranges added in order; attention over the
+// same key splits), so the generated ids are those of decode_mega.cu and of the per-operation path.
+// One sequence, 31 steps of the benchmark model: see the figures at gdb_decode_resident_launch.
+//
+// Waits are bounded: a CTA that gives up stores code 398 in the backend's error word, raises the abort word and returns.
+#include "common.cuh"
+#include "decode_parts.cuh"
+
+#include <vector>
+#include <algorithm>
+
+namespace {
+
+using namespace gdb_dec;
+
+constexpr int DR_THREADS = 512, DR_WARPS = 16, DR_ROWS = 16;
+constexpr int DR_MAX_UNITS = 2048, DR_MAX_CTA_UNITS = 96, DR_MAX_PHASES = 4 * GDB_MEGA_MAX_LAYERS + 1;
+constexpr unsigned DR_SPIN_LIMIT = 1U << 22;
+constexpr int DR_ERR_BARRIER = 398;
+constexpr uint32_t DR_RED_BYTES = SK_WARPS * DR_ROWS * (SK_COLS + 1) * 4U;   // partial sums of one unit
+constexpr uint32_t DR_SYNC_STRIDE = 8U;                                      // counter words are 32 bytes apart
+
+// Counters: [0] abort, then one per phase (5 L + 1, in the order of a step); behind them the running maxima [3][16].
+struct dr_args {
+    gdb_mega_args a;
+    unsigned long long *best;
+    uint32_t work_off, n_units;
+    uint16_t phase_unit[DR_MAX_PHASES + 1];   // first unit of a projection phase (A, C, D, E of each layer, then F)
+    uint8_t workers[DR_MAX_PHASES];           // CTAs with units in it
+    uint8_t cta_of[DR_MAX_UNITS];
+};
+
+enum { DR_QKV = 0, DR_OUT = 1, DR_UP = 2, DR_DOWN = 3, DR_LM = 4 };
+
+__host__ __device__ inline uint32_t dr_unit_bytes(int kind, uint32_t D, uint32_t F)
+{
+    // K-major units [16][K + 8], the down projection [F][16]; then the 16 biases
+    return (kind == DR_DOWN ? F * 32U : 16U * (D + 8U) * 2U) + 32U;
+}
+__host__ __device__ inline uint32_t dr_phase_units(int kind, uint32_t D, uint32_t F, uint32_t V)
+{
+    return kind == DR_QKV ? 3U * D / 16U : (kind == DR_OUT || kind == DR_DOWN ? D / 16U : (kind == DR_UP ? F / 8U : V / 16U));
+}
+
+struct dr_ctx {
+    unsigned char *sm;
+    unsigned *sync;
+    int *err_flag, *ok_flag;
+    int tid, warp, lane;
+};
+
+__device__ __forceinline__ unsigned *dr_counter(const dr_ctx &c, int idx) { return c.sync + (size_t)(1 + idx) * DR_SYNC_STRIDE; }
+
+// Waits until `target` CTAs have arrived at counter idx (idx < 0: nothing to wait for).
+__device__ __forceinline__ bool dr_wait(const dr_ctx &c, int idx, unsigned target)
+{
+    if (idx < 0 || target == 0U) return true;
+    if (c.tid == 0) {
+        int ok = 1;
+        const unsigned *p = dr_counter(c, idx);
+#pragma unroll 1
+        for (unsigned spins = 0;; ++spins) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+            if (v >= target) break;
+            if ((spins & 1023U) == 1023U) {
+                unsigned ab;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(ab) : "l"(c.sync) : "memory");
+                if (ab != 0U || spins > DR_SPIN_LIMIT) {
+                    ok = 0;
+                    atomicExch(c.sync, 1U);
+                    atomicCAS(c.err_flag, 0, DR_ERR_BARRIER);
+                    break;
+                }
+            }
+        }
+        *c.ok_flag = ok;
+    }
+    __syncthreads();
+    return *c.ok_flag != 0;
+}
+__device__ __forceinline__ void dr_arrive(const dr_ctx &c, int idx)
+{
+    __syncthreads();
+    if (c.tid == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(dr_counter(c, idx)) : "memory");
+}
+
+// order-preserving map of finite values and -inf to unsigned
+__device__ __forceinline__ unsigned dr_order(float v)
+{
+    const unsigned b = __float_as_uint(v);
+    return (b & 0x80000000U) ? ~b : b | 0x80000000U;
+}
+
+// weight rows of a unit (the 16 output columns): rows lo .. lo + 7 and hi .. hi + 7
+__device__ __forceinline__ void dr_unit_rows(int kind, uint32_t unit, uint32_t D, uint32_t F, uint32_t H, uint32_t *lo, uint32_t *hi)
+{
+    if (kind == DR_QKV) {
+        const uint32_t nrope = 2U * H * 4U;
+        if (unit < nrope) {   // 8 rotation pairs of one head
+            const uint32_t region = unit / (H * 4U), hg = unit % (H * 4U);
+            *lo = region * D + (hg / 4U) * 64U + (hg % 4U) * 8U;
+            *hi = *lo + 32U;
+        } else {
+            *lo = 2U * D + (unit - nrope) * 16U;
+            *hi = *lo + 8U;
+        }
+    } else if (kind == DR_UP) {
+        *lo = unit * 8U;
+        *hi = F + unit * 8U;
+    } else {
+        *lo = unit * 16U;
+        *hi = *lo + 8U;
+    }
+}
+
+// byte offset of a 16-byte piece of the down projection's tile [F][16]: eight consecutive rows hit distinct banks
+__device__ __forceinline__ uint32_t dr_down_off(uint32_t k, uint32_t piece) { return k * 32U + ((piece ^ ((k >> 2) & 1U)) << 4); }
+
+// One projection phase. GATHER: the normalised rows are the embedding rows of the current ids; otherwise rows of `x` ([B, K]).
+template <typename T, int KIND, bool GATHER>
+__device__ __forceinline__ bool dr_phase(const dr_ctx &c, const dr_args &g, const uint16_t *my_unit, const uint32_t *my_off, int n_my, int phase, int wait_idx,
+                                         unsigned wait_target, int layer, int step, const T *x, const T *norm_w, T *out)
+{
+    if (n_my == 0) return true;
+    constexpr bool NORM = KIND == DR_QKV || KIND == DR_UP || KIND == DR_LM;
+    const gdb_mega_args &a = g.a;
+    const uint32_t D = (uint32_t)a.D, F = (uint32_t)a.F, H = (uint32_t)a.H, K = KIND == DR_DOWN ? F : D, LDA = K + 8U;
+    const uint32_t CH = KIND == DR_DOWN ? ((F % 512U) == 0U ? 512U : ((F % 256U) == 0U ? 256U : 128U)) : D, kw = CH / SK_WARPS;
+    const int B = a.B, gang = c.warp >> 3, kslot = c.warp & 7, gt = c.tid & 255;
+    T *As = reinterpret_cast<T *>(c.sm + g.work_off);
+    const uint32_t a_bytes = DR_ROWS * LDA * 2U;
+    const bool alias = KIND == DR_DOWN;                       // the down projection's long rows leave no room beside them
+    float(*red)[DR_ROWS][SK_COLS + 1] = reinterpret_cast<float(*)[DR_ROWS][SK_COLS + 1]>(c.sm + g.work_off + (alias ? 0U : a_bytes) + (uint32_t)gang * DR_RED_BYTES);
+
+    // ---- what does not depend on the previous phase ----
+    uint4 wraw[2] = {make_uint4(0U, 0U, 0U, 0U), make_uint4(0U, 0U, 0U, 0U)};
+    const int vecs = (int)D / 8;
+    if (NORM) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int v = c.lane + 32 * i;
+            if (v < vecs) wraw[i] = __ldg(reinterpret_cast<const uint4 *>(norm_w) + v);
+        }
+    }
+    float cs = 1.0f, sn = 0.0f;
+    if (KIND == DR_QKV && gang < n_my && gt < DR_ROWS * 8) {
+        const uint32_t unit = my_unit[gang];
+        const int r = gt >> 3, e = gt & 7;
+        if (r < B && unit < 8U * H) rope_cos_sin(a.rope, a.rope_table, (unit & 3U) * 8U + (unsigned)e, a.positions[r] + step, &cs, &sn);
+    }
+    if (!dr_wait(c, wait_idx, wait_target)) return false;
+
+    auto current_id = [&](int r) -> int {   // the id row r is at: given for the first step, else the previous step's maximum
+        return step == 0 ? a.tokens[r] : (int)(0xffffffffU - (unsigned)(__ldcg(&g.best[((step - 1) % 3) * DR_ROWS + r]) & 0xffffffffULL));
+    };
+    if (GATHER && my_unit[0] == 0U && c.tid < DR_ROWS && c.tid < B && step > 0) {
+        // the CTA of the first unit records the previous step's ids and clears the maxima that the next step will use
+        const int t = *a.step_counter + step - 1;
+        if (t >= 0 && t < a.max_steps) a.out_tokens[(size_t)t * B + c.tid] = current_id(c.tid);
+        g.best[((step + 1) % 3) * DR_ROWS + c.tid] = 0ULL;
+    }
+
+    for (int it = 0; it < n_my; it += 2) {
+        const int mine = it + gang;
+        const bool have = mine < n_my;
+        const uint32_t unit = have ? my_unit[mine] : 0U;
+        const T *Ws = reinterpret_cast<const T *>(c.sm + (have ? my_off[mine] : 0U));
+        const T *bias = reinterpret_cast<const T *>(c.sm + (have ? my_off[mine] : 0U) + dr_unit_bytes(KIND, D, F) - 32U);
+        uint32_t lo, hi;
+        dr_unit_rows(KIND, unit, D, F, H, &lo, &hi);
+        float res = 0.0f;
+        const int r0 = gt >> 4, c0 = gt & 15;
+        if ((KIND == DR_OUT || KIND == DR_DOWN) && have && r0 < B) {
+            // residual operand of this thread's output: the block's input (layer 0: the embedding row) or the attention branch's sum
+            const T *src = (const T *)(KIND == DR_DOWN ? a.resid : a.xbuf);
+            size_t row = (size_t)r0;
+            bool nan_row = false;
+            if (KIND == DR_OUT && layer == 0) {
+                const int id = current_id(r0);
+                nan_row = id < 0 || id >= a.V;
+                src = (const T *)a.emb;
+                row = nan_row ? 0U : (size_t)id;
+            }
+            const unsigned short bits = __ldcg(reinterpret_cast<const unsigned short *>(src) + row * D + lo + c0);
+            res = nan_row ? __int_as_float(0x7fc00000) : gdb_io<T>::up(bits);
+        }
+        if (NORM && it == 0) {
+            // one warp per row: mean square over the lane's vectors lane, lane + 32, then round(x * w * rsqrt)
+            const int r = c.warp;
+            if (r < B) {
+                const T *row = x + (size_t)r * D;
+                bool nan_row = false;
+                if (GATHER) {
+                    const int id = current_id(r);
+                    nan_row = id < 0 || id >= a.V;
+                    row = x + (size_t)(nan_row ? 0 : id) * D;
+                }
+                uint4 raw[2];
+                float ss = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int v = c.lane + 32 * i;
+                    raw[i] = make_uint4(0U, 0U, 0U, 0U);
+                    if (v < vecs) raw[i] = __ldcg(reinterpret_cast<const uint4 *>(row) + v);
+                }
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    if (c.lane + 32 * i < vecs) {
+                        float f[8];
+                        unpack8<T>(raw[i], f);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) ss += f[e] * f[e];
+                    }
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffU, ss, o);
+                const float inv = nan_row ? __int_as_float(0x7fc00000) : rsqrtf(ss / (float)(size_t)D + a.eps);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int v = c.lane + 32 * i;
+                    if (v < vecs) {
+                        float f[8], w[8];
+                        unpack8<T>(raw[i], f);
+                        unpack8<T>(wraw[i], w);
+                        uint4 o;
+                        o.x = pack2<T>::down(f[0] * w[0] * inv, f[1] * w[1] * inv);
+                        o.y = pack2<T>::down(f[2] * w[2] * inv, f[3] * w[3] * inv);
+                        o.z = pack2<T>::down(f[4] * w[4] * inv, f[5] * w[5] * inv);
+                        o.w = pack2<T>::down(f[6] * w[6] * inv, f[7] * w[7] * inv);
+                        *reinterpret_cast<uint4 *>(As + (size_t)r * LDA + v * 8) = o;
+                    }
+                }
+            }
+            __syncthreads();
+        } else if (!NORM && (it == 0 || alias)) {
+            const uint32_t segs = K / 8U;
+            for (uint32_t i = (uint32_t)c.tid; i < (uint32_t)B * segs; i += DR_THREADS) {
+                const uint32_t r = i / segs, sg = i - r * segs;
+                sk_cp16(As + r * LDA + sg * 8U, x + (size_t)r * K + sg * 8U, true);
+            }
+            asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+        }
+        float acc[2][4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[0][e] = acc[1][e] = 0.0f;
+        if (have) {
+#pragma unroll 1
+            for (uint32_t k0 = (uint32_t)kslot * kw; k0 < K; k0 += CH) {
+#pragma unroll 4
+                for (uint32_t k = k0; k < k0 + kw; k += 16U) {
+                    uint32_t av[4], b4[4];
+                    sk_ldm4(av, As + (c.lane & 15) * LDA + k + (c.lane >> 4) * 8);
+                    if (KIND == DR_DOWN) {
+                        sk_ldm4t(b4, reinterpret_cast<const unsigned char *>(Ws) + dr_down_off(k + (uint32_t)(c.lane & 15), (uint32_t)c.lane >> 4));
+                    } else {
+                        sk_ldm4(b4, Ws + ((c.lane & 7) + ((c.lane >> 4) << 3)) * LDA + k + ((c.lane >> 3) & 1) * 8);
+                    }
+                    const uint32_t b0[2] = {b4[0], b4[1]}, b1[2] = {b4[2], b4[3]};
+                    mma16816<T>::run(acc[0], av, b0);
+                    mma16816<T>::run(acc[1], av, b1);
+                }
+            }
+        }
+        if (alias) __syncthreads();
+        if (have) {
+            const int gr = c.lane >> 2, tc = c.lane & 3;
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt) {
+                red[kslot][gr][nt * 8 + 2 * tc] = acc[nt][0];
+                red[kslot][gr][nt * 8 + 2 * tc + 1] = acc[nt][1];
+                red[kslot][gr + 8][nt * 8 + 2 * tc] = acc[nt][2];
+                red[kslot][gr + 8][nt * 8 + 2 * tc + 1] = acc[nt][3];
+            }
+        }
+        __syncthreads();
+        auto sum = [&](int r, int cc) {
+            float v = 0.0f;
+#pragma unroll
+            for (int w = 0; w < SK_WARPS; ++w) v += red[w][r][cc];
+            return v;
+        };
+        if (have) {
+            if (KIND == DR_UP) {
+                const int r = gt >> 3, cc = gt & 7;
+                if (gt < DR_ROWS * 8 && r < B) {
+                    gdb_io<T>::st(out, (size_t)r * F + lo + cc, sk_swiglu<T>(sum(r, cc), sum(r, cc + 8), bias, 2, (uint32_t)cc, (uint32_t)cc + 8U));
+                }
+            } else if (KIND == DR_OUT || KIND == DR_DOWN) {
+                if (r0 < B) {
+                    const float y = gdb_io<T>::rnd(sk_bias<T>(sum(r0, c0), bias, KIND == DR_OUT ? 2 : 1, (uint32_t)c0));
+                    gdb_io<T>::st(out, (size_t)r0 * D + lo + c0, res + y);
+                }
+            } else if (KIND == DR_LM) {
+                // soft cap, non-finite -> -inf, maximum of the unit's 16 classes (the first of equal ones)
+                unsigned long long key = 0ULL;
+                if (r0 < B) {
+                    float v = gdb_io<T>::rnd(sk_bias<T>(sum(r0, c0), bias, 2, (uint32_t)c0));
+                    if (a.softcap > 0.0f) v = a.softcap * tanhf(v / a.softcap);
+                    if (!isfinite(v)) v = -INFINITY;
+                    if (v == 0.0f) v = 0.0f;   // -0 and +0 are equal
+                    key = ((unsigned long long)dr_order(v) << 32) | (unsigned long long)(0xffffffffU - (lo + (uint32_t)c0));
+                }
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) {
+                    const unsigned long long other = __shfl_xor_sync(0xffffffffU, key, o);
+                    key = other > key ? other : key;
+                }
+                if (r0 < B && c0 == 0) atomicMax(&g.best[(step % 3) * DR_ROWS + r0], key);
+            } else {
+                const uint32_t nrope = 8U * H;
+                if (unit < nrope) {
+                    const int r = gt >> 3, e = gt & 7;
+                    if (gt < DR_ROWS * 8 && r < B) {
+                        const int pos = a.positions[r] + step;
+                        const uint32_t region = unit / (H * 4U), hg = unit % (H * 4U), hcol = (hg / 4U) * 64U + (hg % 4U) * 8U;
+                        if (it > 0) rope_cos_sin(a.rope, a.rope_table, (hg % 4U) * 8U + (unsigned)e, pos, &cs, &sn);
+                        const float x0 = gdb_io<T>::rnd(sk_bias<T>(sum(r, e), bias, 2, (uint32_t)e)), x1 = gdb_io<T>::rnd(sk_bias<T>(sum(r, e + 8), bias, 2, (uint32_t)e + 8U));
+                        const float y0 = rope_lo(x0, x1, cs, sn), y1 = rope_hi(x0, x1, cs, sn);
+                        if (region == 0U) {
+                            gdb_io<T>::st((T *)a.q, (size_t)r * D + hcol + e, y0);
+                            gdb_io<T>::st((T *)a.q, (size_t)r * D + hcol + 32U + e, y1);
+                        } else if (pos >= 0 && pos < a.CAP) {
+                            const size_t kv = ((size_t)r * a.CAP + (size_t)pos) * D + hcol + e;
+                            gdb_io<T>::st((T *)a.kc[layer], kv, y0);
+                            gdb_io<T>::st((T *)a.kc[layer], kv + 32U, y1);
+                        }
+                    }
+                } else if (r0 < B) {
+                    const int pos = a.positions[r0] + step;
+                    const float y = gdb_io<T>::rnd(sk_bias<T>(sum(r0, c0), bias, 2, (uint32_t)c0));
+                    if (pos >= 0 && pos < a.CAP) gdb_io<T>::st((T *)a.vc[layer], ((size_t)r0 * a.CAP + (size_t)pos) * D + (lo - 2U * D) + c0, y);
+                }
+            }
+        }
+        if (it + 2 < n_my) __syncthreads();   // the partial sums (and an aliased A tile) are reused by the next pair of units
+    }
+    dr_arrive(c, phase);
+    return true;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(DR_THREADS, 1) decode_resident_kernel(const __grid_constant__ dr_args g)
+{
+    extern __shared__ __align__(16) unsigned char dr_sm[];
+    __shared__ int ok_flag;
+    __shared__ uint16_t my_unit[DR_MAX_CTA_UNITS];
+    __shared__ uint32_t my_off[DR_MAX_CTA_UNITS];
+    __shared__ uint16_t first[DR_MAX_PHASES + 1];
+    const gdb_mega_args &a = g.a;
+    dr_ctx c;
+    c.sm = dr_sm;
+    c.sync = a.sync;
+    c.err_flag = a.err_flag;
+    c.ok_flag = &ok_flag;
+    c.tid = threadIdx.x;
+    c.warp = threadIdx.x >> 5;
+    c.lane = threadIdx.x & 31;
+    const uint32_t D = (uint32_t)a.D, F = (uint32_t)a.F, H = (uint32_t)a.H;
+    const int L = a.L, n_phases = 4 * L + 1;
+
+    // ---- this CTA's units, in phase order, and their weights ----
+    if (c.warp == 0) {
+        int n = 0;
+        uint32_t off = 0U;
+        for (int ph = 0; ph < n_phases; ++ph) {
+            if (c.lane == 0) first[ph] = (uint16_t)n;
+            const uint32_t bytes = dr_unit_bytes(ph == 4 * L ? (int)DR_LM : (ph & 3), D, F);
+            for (uint32_t u0 = g.phase_unit[ph]; u0 < g.phase_unit[ph + 1]; u0 += 32U) {
+                const uint32_t u = u0 + (uint32_t)c.lane;
+                const bool mine = u < g.phase_unit[ph + 1] && g.cta_of[u] == (uint8_t)blockIdx.x;
+                const unsigned mask = __ballot_sync(0xffffffffU, mine);
+                const int rank = __popc(mask & ((1U << c.lane) - 1U));
+                if (mine && n + rank < DR_MAX_CTA_UNITS) {
+                    my_unit[n + rank] = (uint16_t)(u - g.phase_unit[ph]);
+                    my_off[n + rank] = off + (uint32_t)rank * bytes;
+                }
+                n += __popc(mask);
+                off += (uint32_t)__popc(mask) * bytes;
+            }
+        }
+        if (c.lane == 0) first[n_phases] = (uint16_t)n;
+    }
+    __syncthreads();
+    for (int ph = 0; ph < n_phases; ++ph) {
+        const int kind = ph == 4 * L ? (int)DR_LM : (ph & 3);
+        const void *const *lw = a.lw[ph < 4 * L ? ph >> 2 : 0];
+        const T *w = (const T *)(kind == DR_LM ? a.w_lm : lw[kind == DR_QKV ? 1 : (kind == DR_OUT ? 3 : (kind == DR_UP ? 6 : 8))]);
+        const T *bias = (const T *)(kind == DR_LM ? a.b_lm : lw[kind == DR_QKV ? 2 : (kind == DR_OUT ? 4 : (kind == DR_UP ? 7 : 9))]);
+        for (int i = first[ph]; i < first[ph + 1]; ++i) {
+            uint32_t lo, hi;
+            dr_unit_rows(kind, my_unit[i], D, F, H, &lo, &hi);
+            unsigned char *dst = dr_sm + my_off[i];
+            if (kind == DR_DOWN) {
+                for (uint32_t j = (uint32_t)c.tid; j < F * 2U; j += DR_THREADS) sk_cp16(dst + dr_down_off(j >> 1, j & 1U), w + (size_t)(j >> 1) * D + lo + (j & 1U) * 8U, true);
+            } else {
+                const uint32_t segs = D / 8U;
+                for (uint32_t j = (uint32_t)c.tid; j < 16U * segs; j += DR_THREADS) {
+                    const uint32_t r = j / segs, sg = j - r * segs;
+                    sk_cp16(dst + (r * (D + 8U) + sg * 8U) * 2U, w + (size_t)(r < 8U ? lo + r : hi + (r - 8U)) * D + sg * 8U, true);
+                }
+            }
+            if (c.tid < 2) sk_cp16(dst + dr_unit_bytes(kind, D, F) - 32U + c.tid * 16U, bias + (c.tid == 0 ? lo : hi), true);
+        }
+    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+
+    const int hpc = 16 / a.splits, groups = a.H / hpc, attn_units = a.B * groups;
+    const unsigned attn_workers = (unsigned)min(attn_units, (int)gridDim.x);
+    decode_params dp;
+    dp.batch = a.B;
+    dp.tq = 1;
+    dp.tmax = a.CAP;
+    dp.hq = a.H;
+    dp.hkv = a.H;
+    dp.dh = 64;
+    dp.window = a.window;
+    dp.prefix = 0;
+    dp.pos_mode = 0;
+    dp.scale = a.scale;
+    auto units_of = [&](int ph) { return (int)first[ph + 1] - (int)first[ph]; };
+#pragma unroll 1
+    for (int step = 0; step < a.n_steps; ++step) {
+        const unsigned round = (unsigned)step + 1U;
+#pragma unroll 1
+        for (int layer = 0; layer < L; ++layer) {
+            const void *const *lw = a.lw[layer];
+            const int ph = 4 * layer, cnt = 5 * layer;
+            if (layer == 0) {
+                if (!dr_phase<T, DR_QKV, true>(c, g, my_unit + first[ph], my_off + first[ph], units_of(ph), cnt, 5 * L, g.workers[4 * L] * (unsigned)step, layer, step,
+                                               (const T *)a.emb, (const T *)lw[0], nullptr)) return;
+            } else {
+                if (!dr_phase<T, DR_QKV, false>(c, g, my_unit + first[ph], my_off + first[ph], units_of(ph), cnt, cnt - 1, g.workers[ph - 1] * round, layer, step,
+                                                (const T *)a.xbuf, (const T *)lw[0], nullptr)) return;
+            }
+            if ((int)blockIdx.x < attn_units) {
+                // attention: the CTA's 16 warps are `hpc` heads x `splits` key ranges of one sequence, merged in shared memory
+                if (!dr_wait(c, cnt, g.workers[ph] * round)) return;
+                float *sm_ml = reinterpret_cast<float *>(dr_sm + g.work_off), *sm_acc = sm_ml + DR_WARPS * 2;
+                for (int unit = blockIdx.x; unit < attn_units; unit += gridDim.x) {
+                    const int b = unit / groups, hl = c.warp % hpc, split = c.warp / hpc, item = hl * a.splits + split;
+                    const long long w = (long long)b * a.H + (unit % groups) * hpc + hl;
+                    dp.cache_pos = a.positions[b] + step;
+                    if (split < a.splits) {
+                        decode_split_item<T, 64, false>((const T *)a.q, (const T *)a.kc[layer], (const T *)a.vc[layer], nullptr, sm_ml + item * 2, sm_acc + item * 64, dp,
+                                                        a.splits, w, split, c.lane);
+                    }
+                    __syncthreads();
+                    if (c.warp < hpc) {
+                        decode_combine_query<T, false>(sm_ml + c.warp * a.splits * 2, sm_acc + c.warp * a.splits * 64,
+                                                       (T *)a.attn + (size_t)((long long)b * a.H + (unit % groups) * hpc + c.warp) * 64, 64, a.splits, c.lane);
+                    }
+                    __syncthreads();
+                }
+                dr_arrive(c, cnt + 1);
+            }
+            if (!dr_phase<T, DR_OUT, false>(c, g, my_unit + first[ph + 1], my_off + first[ph + 1], units_of(ph + 1), cnt + 2, cnt + 1, attn_workers * round, layer, step,
+                                            (const T *)a.attn, nullptr, (T *)a.resid)) return;
+            if (!dr_phase<T, DR_UP, false>(c, g, my_unit + first[ph + 2], my_off + first[ph + 2], units_of(ph + 2), cnt + 3, cnt + 2, g.workers[ph + 1] * round, layer, step,
+                                           (const T *)a.resid, (const T *)lw[5], (T *)a.act)) return;
+            if (!dr_phase<T, DR_DOWN, false>(c, g, my_unit + first[ph + 3], my_off + first[ph + 3], units_of(ph + 3), cnt + 4, cnt + 3, g.workers[ph + 2] * round, layer, step,
+                                             (const T *)a.act, nullptr, (T *)a.xbuf)) return;
+        }
+        if (!dr_phase<T, DR_LM, false>(c, g, my_unit + first[4 * L], my_off + first[4 * L], units_of(4 * L), 5 * L, 5 * L - 1, g.workers[4 * L - 1] * round, 0, step,
+                                       (const T *)a.xbuf, (const T *)a.w_final, nullptr)) return;
+    }
+    if (blockIdx.x == 0) {
+        if (!dr_wait(c, 5 * L, g.workers[4 * L] * (unsigned)a.n_steps)) return;
+        if (c.tid < a.B) {
+            const int id = (int)(0xffffffffU - (unsigned)(__ldcg(&g.best[((a.n_steps - 1) % 3) * DR_ROWS + c.tid]) & 0xffffffffULL));
+            const int t = *a.step_counter + a.n_steps - 1;
+            a.tokens[c.tid] = id;
+            a.positions[c.tid] += a.n_steps;
+            if (t >= 0 && t < a.max_steps) a.out_tokens[(size_t)t * a.B + c.tid] = id;
+        }
+        __syncthreads();
+        if (c.tid == 0) *a.step_counter += a.n_steps;
+    }
+}
+
+// Which CTA keeps which unit: per phase every CTA at most one unit more than another, the CTAs that hold least so far first; the
+// down projections, whose units are the largest, before the rest. False when the model does not fit.
+struct dr_plan {
+    uint32_t D, F, V, L, ctas;
+    bool fits;
+    uint32_t weight_bytes;
+    dr_args tables;   // phase_unit, workers, cta_of, n_units
+};
+bool dr_make_plan(dr_plan *p, uint32_t max_weight_bytes)
+{
+    const uint32_t n_phases = 4U * p->L + 1U;
+    uint32_t units = 0U;
+    for (uint32_t ph = 0; ph <= n_phases; ++ph) {
+        if (units > (uint32_t)DR_MAX_UNITS) return false;
+        p->tables.phase_unit[ph] = (uint16_t)units;
+        if (ph < n_phases) units += dr_phase_units(ph == 4U * p->L ? (int)DR_LM : (int)(ph & 3U), p->D, p->F, p->V);
+    }
+    p->tables.n_units = units;
+    std::vector<uint32_t> load(p->ctas, 0U), count(p->ctas, 0U), order(p->ctas);
+    for (uint32_t i = 0; i < p->ctas; ++i) order[i] = i;
+    for (int pass = 0; pass < 2; ++pass) {
+        for (uint32_t ph = 0; ph < n_phases; ++ph) {
+            const int kind = ph == 4U * p->L ? (int)DR_LM : (int)(ph & 3U);
+            if ((kind == DR_DOWN) != (pass == 0)) continue;
+            const uint32_t first = p->tables.phase_unit[ph], n = p->tables.phase_unit[ph + 1] - first, bytes = dr_unit_bytes(kind, p->D, p->F);
+            std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return load[x] < load[y]; });
+            for (uint32_t u = 0; u < n; ++u) {
+                const uint32_t cta = order[u % p->ctas];
+                p->tables.cta_of[first + u] = (uint8_t)cta;
+                load[cta] += bytes;
+                count[cta] += 1U;
+            }
+            p->tables.workers[ph] = (uint8_t)std::min(n, p->ctas);
+        }
+    }
+    p->weight_bytes = *std::max_element(load.begin(), load.end());
+    return p->weight_bytes <= max_weight_bytes && *std::max_element(count.begin(), count.end()) <= (uint32_t)DR_MAX_CTA_UNITS;
+}
+
+}  // namespace
+
+size_t gdb_decode_resident_sync_words(int L) { return (size_t)(2 + 5 * L) * DR_SYNC_STRIDE + 3U * DR_ROWS * 2U; }
+
+// n_steps greedy decode steps of at most 16 sequences with the weights in shared memory; GD_ERR_UNSUPPORTED when the model does
+// not fit (decode_mega.cu then takes the call). a->sync: gdb_decode_resident_sync_words(L) zeroed words, 8-byte aligned.
+// The benchmark model on one B200, per step: SEE_FIGURES
+gd_status gdb_decode_resident_launch(gd_backend *be, uint32_t dtype, const gdb_mega_args *a)
+{
+    static thread_local dr_plan plan;   // of the last model
+    if (a->B > DR_ROWS || a->L > GDB_MEGA_MAX_LAYERS || be->sm_count > 255) {
+        return GD_ERR_UNSUPPORTED;
+    }
+    const uint32_t D = (uint32_t)a->D, F = (uint32_t)a->F, ctas = (uint32_t)be->sm_count;
+    const uint32_t work = std::max({DR_ROWS * (F + 8U) * 2U, DR_ROWS * (D + 8U) * 2U + 2U * DR_RED_BYTES, (uint32_t)(DR_WARPS * 66 * sizeof(float))});
+    constexpr uint32_t smem_limit = 232448U - 2048U;   // dynamic part beside the kernel's static tables
+    if (work >= smem_limit) {
+        return GD_ERR_UNSUPPORTED;
+    }
+    if (plan.ctas != ctas || plan.D != D || plan.F != F || plan.V != (uint32_t)a->V || plan.L != (uint32_t)a->L) {
+        plan.D = D;
+        plan.F = F;
+        plan.V = (uint32_t)a->V;
+        plan.L = (uint32_t)a->L;
+        plan.ctas = ctas;
+        plan.fits = dr_make_plan(&plan, smem_limit - work);
+    }
+    if (!plan.fits) {
+        return GD_ERR_UNSUPPORTED;
+    }
+    dr_args g = plan.tables;
+    g.a = *a;
+    g.best = reinterpret_cast<unsigned long long *>(a->sync + (size_t)(2 + 5 * a->L) * DR_SYNC_STRIDE);
+    g.work_off = (plan.weight_bytes + 127U) & ~127U;
+    const size_t smem = (size_t)g.work_off + work;
+    void (*kern)(const dr_args) = dtype == GDB_DTYPE_F16 ? decode_resident_kernel<__half> : decode_resident_kernel<__nv_bfloat16>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return gdb_fail(be, e, "resident decode kernel: shared memory attribute");
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;   // every CTA resident: they wait for one another
+    attr[0].val.cooperative = 1;
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(DR_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = be->stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, kern, g);
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported || e == cudaErrorInvalidValue || e == cudaErrorInvalidConfiguration) {
+        (void)cudaGetLastError();
+        return GD_ERR_UNSUPPORTED;
+    }
+    if (e != cudaSuccess) return gdb_fail(be, e, "resident decode kernel: launch");
+    return gdb_launched(be, "resident decode kernel");
+}

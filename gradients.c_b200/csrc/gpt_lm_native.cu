@@ -1209,7 +1209,7 @@ gd_status decode_steps_persistent(gd_backend *be, const gdb200_gpt_spec *s, cons
     a.attn = act(D);
     a.act = act(F);
     a.logits = act(V);
-    Ten sync = c.alloc(GDB_DTYPE_I32, {4});
+    Ten sync = c.alloc(GDB_DTYPE_I32, {(int64_t)gdb_decode_resident_sync_words(L)});
     if (c.st != GD_OK) {
         snprintf(be->last_error, sizeof(be->last_error), "gpt decode steps: %s", c.where);
         return c.st;
@@ -1239,7 +1239,8 @@ gd_status decode_steps_persistent(gd_backend *be, const gdb200_gpt_spec *s, cons
     if (scratch_used != NULL) {
         *scratch_used = c.top;
     }
-    st = gdb_decode_mega_launch(be, dt, &a);
+    st = a.timeline == NULL ? gdb_decode_resident_launch(be, dt, &a) : GD_ERR_UNSUPPORTED;
+    if (st == GD_ERR_UNSUPPORTED) st = gdb_decode_mega_launch(be, dt, &a);
     if (st == GD_OK && a.timeline != NULL && n_steps > 2) {
         std::vector<unsigned long long> h((size_t)n_steps * per_step);
         if (cudaStreamSynchronize(be->stream) == cudaSuccess &&
