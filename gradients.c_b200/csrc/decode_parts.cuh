@@ -455,6 +455,7 @@ __device__ __forceinline__ void decode_split_item(const T *q, const T *kc, const
             auto key_base = [&](int j) { return (((size_t)b * p.tmax + (size_t)j) * p.hkv + hk) * DH + sub * 16; };
 #pragma unroll
             for (int c = 0; c < 16; ++c) qr[c] = gdb_io<T>::ld(q, qb + c) * p.scale;
+#pragma unroll 1
             for (int jb = s_lo; jb < s_hi; jb += TILE) {
                 uint4 k0[2], k1[2], v0[2], v1[2];
                 bool valid[2];

@@ -130,13 +130,13 @@ __device__ __forceinline__ void dr_unit_rows(int kind, uint32_t unit, uint32_t D
 // byte offset of a 16-byte piece of the down projection's tile [F][16]: eight consecutive rows hit distinct banks
 __device__ __forceinline__ uint32_t dr_down_off(uint32_t k, uint32_t piece) { return k * 32U + ((piece ^ ((k >> 2) & 1U)) << 4); }
 
-// One projection phase. GATHER: the normalised rows are the embedding rows of the current ids; otherwise rows of `x` ([B, K]).
-template <typename T, int KIND, bool GATHER>
-__device__ __forceinline__ bool dr_phase(const dr_ctx &c, const dr_args &g, const uint16_t *my_unit, const uint32_t *my_off, int n_my, int phase, int wait_idx,
+// One projection phase (one body of code for all kinds: a step must not run through much more than the 32 KB instruction cache). GATHER: the normalised rows are the embedding rows of the current ids; otherwise rows of `x` ([B, K]).
+template <typename T>
+__device__ __forceinline__ bool dr_phase(const dr_ctx &c, const dr_args &g, const int KIND, const bool GATHER, const uint16_t *my_unit, const uint32_t *my_off, int n_my, int phase, int wait_idx,
                                          unsigned wait_target, int layer, int step, const T *x, const T *norm_w, T *out)
 {
     if (n_my == 0) return true;
-    constexpr bool NORM = KIND == DR_QKV || KIND == DR_UP || KIND == DR_LM;
+    const bool NORM = KIND == DR_QKV || KIND == DR_UP || KIND == DR_LM;
     const gdb_mega_args &a = g.a;
     const uint32_t D = (uint32_t)a.D, F = (uint32_t)a.F, H = (uint32_t)a.H, K = KIND == DR_DOWN ? F : D, LDA = K + 8U;
     const uint32_t CH = KIND == DR_DOWN ? ((F % 512U) == 0U ? 512U : ((F % 256U) == 0U ? 256U : 128U)) : D, kw = CH / SK_WARPS;
@@ -174,6 +174,7 @@ __device__ __forceinline__ bool dr_phase(const dr_ctx &c, const dr_args &g, cons
         g.best[((step + 1) % 3) * DR_ROWS + c.tid] = 0ULL;
     }
 
+#pragma unroll 1
     for (int it = 0; it < n_my; it += 2) {
         const int mine = it + gang;
         const bool have = mine < n_my;
@@ -248,9 +249,14 @@ __device__ __forceinline__ bool dr_phase(const dr_ctx &c, const dr_args &g, cons
             __syncthreads();
         } else if (!NORM && (it == 0 || alias)) {
             const uint32_t segs = K / 8U;
-            for (uint32_t i = (uint32_t)c.tid; i < (uint32_t)B * segs; i += DR_THREADS) {
-                const uint32_t r = i / segs, sg = i - r * segs;
+            uint32_t r = 0U, sg = (uint32_t)c.tid;
+#pragma unroll 1
+            for (;;) {
+#pragma unroll 1
+                for (; sg >= segs; sg -= segs) ++r;
+                if (r >= (uint32_t)B) break;
                 sk_cp16(As + r * LDA + sg * 8U, x + (size_t)r * K + sg * 8U, true);
+                sg += DR_THREADS;
             }
             asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
             __syncthreads();
@@ -377,9 +383,11 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decode_resident_kernel(const __
     if (c.warp == 0) {
         int n = 0;
         uint32_t off = 0U;
+#pragma unroll 1
         for (int ph = 0; ph < n_phases; ++ph) {
             if (c.lane == 0) first[ph] = (uint16_t)n;
             const uint32_t bytes = dr_unit_bytes(ph == 4 * L ? (int)DR_LM : (ph & 3), D, F);
+#pragma unroll 1
             for (uint32_t u0 = g.phase_unit[ph]; u0 < g.phase_unit[ph + 1]; u0 += 32U) {
                 const uint32_t u = u0 + (uint32_t)c.lane;
                 const bool mine = u < g.phase_unit[ph + 1] && g.cta_of[u] == (uint8_t)blockIdx.x;
@@ -396,19 +404,23 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decode_resident_kernel(const __
         if (c.lane == 0) first[n_phases] = (uint16_t)n;
     }
     __syncthreads();
+#pragma unroll 1
     for (int ph = 0; ph < n_phases; ++ph) {
         const int kind = ph == 4 * L ? (int)DR_LM : (ph & 3);
         const void *const *lw = a.lw[ph < 4 * L ? ph >> 2 : 0];
         const T *w = (const T *)(kind == DR_LM ? a.w_lm : lw[kind == DR_QKV ? 1 : (kind == DR_OUT ? 3 : (kind == DR_UP ? 6 : 8))]);
         const T *bias = (const T *)(kind == DR_LM ? a.b_lm : lw[kind == DR_QKV ? 2 : (kind == DR_OUT ? 4 : (kind == DR_UP ? 7 : 9))]);
+#pragma unroll 1
         for (int i = first[ph]; i < first[ph + 1]; ++i) {
             uint32_t lo, hi;
             dr_unit_rows(kind, my_unit[i], D, F, H, &lo, &hi);
             unsigned char *dst = dr_sm + my_off[i];
             if (kind == DR_DOWN) {
+#pragma unroll 1
                 for (uint32_t j = (uint32_t)c.tid; j < F * 2U; j += DR_THREADS) sk_cp16(dst + dr_down_off(j >> 1, j & 1U), w + (size_t)(j >> 1) * D + lo + (j & 1U) * 8U, true);
             } else {
                 const uint32_t segs = D / 8U;
+#pragma unroll 1
                 for (uint32_t j = (uint32_t)c.tid; j < 16U * segs; j += DR_THREADS) {
                     const uint32_t r = j / segs, sg = j - r * segs;
                     sk_cp16(dst + (r * (D + 8U) + sg * 8U) * 2U, w + (size_t)(r < 8U ? lo + r : hi + (r - 8U)) * D + sg * 8U, true);
@@ -437,47 +449,56 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decode_resident_kernel(const __
 #pragma unroll 1
     for (int step = 0; step < a.n_steps; ++step) {
         const unsigned round = (unsigned)step + 1U;
+        // counters in the order of a step: QKV, attention, OUT, UP, DOWN of every layer, then LM
 #pragma unroll 1
-        for (int layer = 0; layer < L; ++layer) {
-            const void *const *lw = a.lw[layer];
-            const int ph = 4 * layer, cnt = 5 * layer;
-            if (layer == 0) {
-                if (!dr_phase<T, DR_QKV, true>(c, g, my_unit + first[ph], my_off + first[ph], units_of(ph), cnt, 5 * L, g.workers[4 * L] * (unsigned)step, layer, step,
-                                               (const T *)a.emb, (const T *)lw[0], nullptr)) return;
-            } else {
-                if (!dr_phase<T, DR_QKV, false>(c, g, my_unit + first[ph], my_off + first[ph], units_of(ph), cnt, cnt - 1, g.workers[ph - 1] * round, layer, step,
-                                                (const T *)a.xbuf, (const T *)lw[0], nullptr)) return;
-            }
-            if ((int)blockIdx.x < attn_units) {
+        for (int i = 0; i <= 5 * L; ++i) {
+            const int layer = i / 5, sub = i - 5 * layer;
+            if (sub == 1 && i < 5 * L) {
                 // attention: the CTA's 16 warps are `hpc` heads x `splits` key ranges of one sequence, merged in shared memory
-                if (!dr_wait(c, cnt, g.workers[ph] * round)) return;
+                if ((int)blockIdx.x >= attn_units) continue;
+                if (!dr_wait(c, i - 1, g.workers[4 * layer] * round)) return;
                 float *sm_ml = reinterpret_cast<float *>(dr_sm + g.work_off), *sm_acc = sm_ml + DR_WARPS * 2;
+#pragma unroll 1
                 for (int unit = blockIdx.x; unit < attn_units; unit += gridDim.x) {
-                    const int b = unit / groups, hl = c.warp % hpc, split = c.warp / hpc, item = hl * a.splits + split;
-                    const long long w = (long long)b * a.H + (unit % groups) * hpc + hl;
+                    const int b = unit / groups, h0 = (unit - b * groups) * hpc, hl = c.warp % hpc, split = c.warp / hpc, item = hl * a.splits + split;
                     dp.cache_pos = a.positions[b] + step;
                     if (split < a.splits) {
                         decode_split_item<T, 64, false>((const T *)a.q, (const T *)a.kc[layer], (const T *)a.vc[layer], nullptr, sm_ml + item * 2, sm_acc + item * 64, dp,
-                                                        a.splits, w, split, c.lane);
+                                                        a.splits, (long long)b * a.H + h0 + hl, split, c.lane);
                     }
                     __syncthreads();
-                    if (c.warp < hpc) {
-                        decode_combine_query<T, false>(sm_ml + c.warp * a.splits * 2, sm_acc + c.warp * a.splits * 64,
-                                                       (T *)a.attn + (size_t)((long long)b * a.H + (unit % groups) * hpc + c.warp) * 64, 64, a.splits, c.lane);
+                    // merge of the splits (decode_combine_query), one thread per output: weights, sum and output over the splits in order
+                    if (c.tid < hpc * 64) {
+                        const int hh = c.tid >> 6, col = c.tid & 63;
+                        const float2 *ml = reinterpret_cast<const float2 *>(sm_ml) + hh * a.splits;
+                        const float *acc = sm_acc + hh * a.splits * 64 + col;
+                        float m = -INFINITY, l = 0.0f, o = 0.0f;
+#pragma unroll 4
+                        for (int s = 0; s < a.splits; ++s) m = fmaxf(m, ml[s].x);
+#pragma unroll 4
+                        for (int s = 0; s < a.splits; ++s) {
+                            const float2 p = ml[s];
+                            const float w = p.x == -INFINITY ? 0.0f : __expf(p.x - m);
+                            l = fmaf(p.y, w, l);
+                            if (p.x != -INFINITY) o = fmaf(acc[s * 64], w, o);
+                        }
+                        gdb_io<T>::st((T *)a.attn, ((size_t)b * a.H + h0 + hh) * 64 + col, o * (l > 0.0f ? 1.0f / l : 0.0f));
                     }
                     __syncthreads();
                 }
-                dr_arrive(c, cnt + 1);
+                dr_arrive(c, i);
+                continue;
             }
-            if (!dr_phase<T, DR_OUT, false>(c, g, my_unit + first[ph + 1], my_off + first[ph + 1], units_of(ph + 1), cnt + 2, cnt + 1, attn_workers * round, layer, step,
-                                            (const T *)a.attn, nullptr, (T *)a.resid)) return;
-            if (!dr_phase<T, DR_UP, false>(c, g, my_unit + first[ph + 2], my_off + first[ph + 2], units_of(ph + 2), cnt + 3, cnt + 2, g.workers[ph + 1] * round, layer, step,
-                                           (const T *)a.resid, (const T *)lw[5], (T *)a.act)) return;
-            if (!dr_phase<T, DR_DOWN, false>(c, g, my_unit + first[ph + 3], my_off + first[ph + 3], units_of(ph + 3), cnt + 4, cnt + 3, g.workers[ph + 2] * round, layer, step,
-                                             (const T *)a.act, nullptr, (T *)a.xbuf)) return;
+            const int kind = i == 5 * L ? (int)DR_LM : (sub == 0 ? (int)DR_QKV : sub - 1), ph = i == 5 * L ? 4 * L : 4 * layer + kind;
+            // the counter of the phase in front: the attention for OUT, the previous step's last phase for the first
+            const int wait_idx = i == 0 ? 5 * L : i - 1;
+            const unsigned wait_n = kind == DR_OUT ? attn_workers : (unsigned)g.workers[i == 0 ? 4 * L : ph - 1], wait_rounds = i == 0 ? (unsigned)step : round;
+            const void *src = kind == DR_OUT ? a.attn : (kind == DR_UP ? a.resid : (kind == DR_DOWN ? a.act : (i == 0 ? a.emb : a.xbuf)));
+            void *dst = kind == DR_OUT ? a.resid : (kind == DR_UP ? a.act : a.xbuf);
+            const void *nw = kind == DR_LM ? a.w_final : a.lw[layer < L ? layer : 0][kind == DR_UP ? 5 : 0];
+            if (!dr_phase<T>(c, g, kind, i == 0, my_unit + first[ph], my_off + first[ph], units_of(ph), i, wait_idx, wait_n * wait_rounds, layer, step, (const T *)src,
+                             (const T *)nw, (T *)dst)) return;
         }
-        if (!dr_phase<T, DR_LM, false>(c, g, my_unit + first[4 * L], my_off + first[4 * L], units_of(4 * L), 5 * L, 5 * L - 1, g.workers[4 * L - 1] * round, 0, step,
-                                       (const T *)a.xbuf, (const T *)a.w_final, nullptr)) return;
     }
     if (blockIdx.x == 0) {
         if (!dr_wait(c, 5 * L, g.workers[4 * L] * (unsigned)a.n_steps)) return;
