@@ -1267,6 +1267,135 @@ gd_status decode_steps_persistent(gd_backend *be, const gdb200_gpt_spec *s, cons
 
 }  // namespace
 
+// Packed prefill of a batch of prompts (gpt_lm_prefill_last_logits, examples/gpt_lm/gpt_lm_shared.c:1117-1202) with the caches filled
+// and the first sampled id of every prompt fed back: one native call instead of some sixty op capsules, whose host time exceeded
+// the device's for short prompts. Same entries and rounding points as GptLm.prefill_last_logits; residual adds and the norms behind
+// them are one launch, the gate is formed in the up / gate contraction, the last rows are gathered by one embedding gather.
+extern "C" gd_status gdb200_gpt_prefill(gd_backend *be, const gdb200_gpt_spec *s, const gdb200_gpt_batch *batch, size_t cache_pos_offset,
+                                        size_t last_rows_offset, const gdb200_gpt_decode_state *d, size_t *scratch_used)
+{
+    if (be == NULL || s == NULL || batch == NULL || d == NULL || batch->n_tokens <= 0 || d->batch <= 0 || batch->n_cu != d->batch + 1 || s->n_layers <= 0 ||
+        s->n_layers > GDB200_GPT_MAX_LAYERS || s->n_heads * s->head_dim != s->d_model || d->cache_buffer == NULL || d->io_buffer == NULL) {
+        return GD_ERR_INVALID_ARGUMENT;
+    }
+    const size_t io_bytes = gd_backend_buffer_nbytes(d->io_buffer);
+    if (((d->tokens_offset | d->positions_offset | d->out_tokens_offset | d->step_counter_offset) % 4U) != 0U ||
+        d->tokens_offset + (size_t)d->batch * 4U > io_bytes || d->positions_offset + (size_t)d->batch * 4U > io_bytes ||
+        d->step_counter_offset + 4U > io_bytes || d->out_tokens_offset + (size_t)d->max_steps * (size_t)d->batch * 4U > io_bytes) {
+        return GD_ERR_INVALID_ARGUMENT;
+    }
+    Step c;
+    c.be = be;
+    c.s = s;
+    c.top = 0;
+    c.st = GD_OK;
+    c.where = "";
+    const int64_t T = batch->n_tokens, B = d->batch, D = s->d_model, F = s->mlp_hidden, V = s->vocab_size, H = s->n_heads, Dh = s->head_dim, CAP = d->capacity;
+    const int L = s->n_layers;
+    const uint32_t dt = s->dtype;
+    const int P_FINAL = 1 + 10 * L, P_LMW = s->tied_lm_head ? 0 : P_FINAL + 1, P_LMB = P_FINAL + (s->tied_lm_head ? 1 : 2);
+    const Ten ids = i32_tensor(batch->buffer, batch->input_ids_offset, T), pos = i32_tensor(batch->buffer, batch->positions_offset, T);
+    const Ten cu = i32_tensor(batch->buffer, batch->cu_seqlens_offset, B + 1), cpos = i32_tensor(batch->buffer, cache_pos_offset, B);
+    const Ten last = i32_tensor(batch->buffer, last_rows_offset, B);
+    auto gather = [&](const Ten &table, int64_t rows, const Ten &index, int64_t n) {
+        Ten out = c.alloc(dt, {n, D});
+        gd_backend_embedding_args ea = {(uint64_t)n, (uint64_t)rows, (uint64_t)D};
+        gd_backend_tensor_view a = tv(table), b = tv(index), o = tv(out);
+        c.ok(gd_backend_embedding_forward(be, &a, &b, &o, &ea), "embedding_forward");
+        return out;
+    };
+    auto rms = [&](const Ten &x, const Ten &w, int64_t rows) {
+        Ten out = c.alloc(dt, {rows, D});
+        gd_backend_rms_norm_args a = rms_args(rows, D, s->rms_eps);
+        gd_backend_tensor_view xv = tv(x), wv = tv(w), ov = tv(out);
+        c.ok(gd_backend_rms_norm_forward(be, &xv, &wv, &ov, &a), "rms_norm_forward");
+        return out;
+    };
+    auto add_then_rms = [&](const Ten &xa, const Ten &ya, const Ten &w, Ten *sum, Ten *normed) {
+        *sum = c.alloc(dt, {T, D});
+        *normed = c.alloc(dt, {T, D});
+        gd_backend_tensor_view xv = tv(xa), yv = tv(ya), wv = tv(w), sv = tv(*sum), nv = tv(*normed);
+        gd_status r = gdb_add_rms_norm(be, &xv, &yv, &wv, &sv, &nv, (size_t)T, (size_t)D, s->rms_eps);
+        if (r == GD_ERR_UNSUPPORTED) {
+            c.ok(gd_backend_add(be, &xv, &yv, &sv), "add");
+            gd_backend_rms_norm_args a = rms_args(T, D, s->rms_eps);
+            r = gd_backend_rms_norm_forward(be, &sv, &wv, &nv, &a);
+        }
+        c.ok(r, "add + rms_norm");
+    };
+    gd_backend_rope_args rope = {s->rope_theta, (uint32_t)Dh, 0U};
+    gd_backend_sdpa_varlen_args sa;
+    memset(&sa, 0, sizeof(sa));
+    sa.scale = (float)(1.0 / sqrt((double)Dh));
+    sa.causal = 1;
+    sa.sliding_window = (uint32_t)s->sdpa_window;
+    sa.max_seqlen = (uint32_t)s->context_length;
+    gd_backend_kv_cache_append_args ka = {0};
+    Ten x = gather(c.param(0, {V, D}), V, ids, T), normed = rms(x, c.param(1, {D}), T);
+    for (int i = 0; i < L && c.st == GD_OK; ++i) {
+        const int pb = 1 + 10 * i;
+        Ten qkv = linear_t(c, normed, c.param(pb + 1, {3 * D, D}), c.param(pb + 2, {3 * D}), T, D, 3 * D);
+        Ten q = c.alloc(dt, {T, H, Dh}), k = c.alloc(dt, {T, H, Dh}), v = c.alloc(dt, {T, H, Dh}), attn = c.alloc(dt, {T, H, Dh}), kc;
+        memset(&kc, 0, sizeof(kc));
+        kc.buf = d->cache_buffer;
+        kc.dt = dt;
+        kc.rank = 4;
+        kc.shape[0] = B;
+        kc.shape[1] = CAP;
+        kc.shape[2] = H;
+        kc.shape[3] = Dh;
+        Ten vc = kc;
+        kc.off = d->k_cache_offset[i];
+        vc.off = d->v_cache_offset[i];
+        {
+            gd_backend_tensor_view a = tv(qkv), p = tv(pos), qv = tv(q), kv = tv(k), vv_ = tv(v), kcv = tv(kc), vcv = tv(vc), cp = tv(cpos), cuv = tv(cu), ov = tv(attn);
+            c.ok(gd_backend_qkv_split_rope_forward(be, &a, &p, &qv, &kv, &vv_, (uint32_t)H, (uint32_t)Dh, &rope), "qkv_split_rope_forward");
+            c.ok(gd_backend_kv_cache_append_packed(be, &kcv, &vcv, &cp, &cuv, &kv, &vv_, &ka), "kv_cache_append_packed");
+            c.ok(gd_backend_sdpa_varlen(be, &qv, &kv, &vv_, &cuv, &ov, NULL, &sa), "sdpa_varlen");
+        }
+        Ten proj = linear_t(c, attn, c.param(pb + 3, {D, D}), c.param(pb + 4, {D}), T, D, D), resid, normed2;
+        add_then_rms(x, proj, c.param(pb + 5, {D}), &resid, &normed2);
+        Ten up_gate = c.alloc(dt, {T, 2 * F}), act = c.alloc(dt, {T, F}), mlp = c.alloc(dt, {T, D});
+        {
+            const Ten w = c.param(pb + 6, {2 * F, D}), b = c.param(pb + 7, {2 * F}), wd = c.param(pb + 8, {F, D}), bd = c.param(pb + 9, {D});
+            gd_backend_matrix_view xm = mv(normed2, (uint32_t)T, (uint32_t)D), wm = mv(w, (uint32_t)(2 * F), (uint32_t)D), um = mv(up_gate, (uint32_t)T, (uint32_t)(2 * F));
+            gd_backend_matrix_view am = mv(act, (uint32_t)T, (uint32_t)F), dm = mv(wd, (uint32_t)F, (uint32_t)D), ym = mv(mlp, (uint32_t)T, (uint32_t)D);
+            gd_backend_vector_view bv = vv(b, 0, (uint32_t)(2 * F)), bdv = vv(bd, 0, (uint32_t)D);
+            gd_status r = T <= 64 ? gdb200_matmul_nt_bias_swiglu(be, &xm, &wm, &bv, &am) : GD_ERR_UNSUPPORTED;
+            if (r == GD_ERR_UNSUPPORTED) r = gdb200_matmul_nt_bias_swiglu_both(be, &xm, &wm, &bv, &um, &am);
+            c.ok(r, "matmul_nt_bias + swiglu_split");
+            c.ok(gd_backend_linear(be, &am, &dm, &bdv, &ym), "linear(down_proj)");
+        }
+        if (i + 1 < L) {
+            Ten out;
+            add_then_rms(resid, mlp, c.param(1 + 10 * (i + 1), {D}), &out, &normed);
+            x = out;
+        } else {
+            x = c.alloc(dt, {T, D});
+            gd_backend_tensor_view rv = tv(resid), yv = tv(mlp), ov = tv(x);
+            c.ok(gd_backend_add(be, &rv, &yv, &ov), "add");
+        }
+    }
+    Ten final_norm = rms(gather(x, T, last, B), c.param(P_FINAL, {D}), B);
+    Ten logits = linear_t(c, final_norm, c.param(P_LMW, {V, D}), c.param(P_LMB, {V}), B, D, V);
+    if (c.st == GD_OK) {
+        gd_backend_tensor_view lv = tv(logits);
+        int32_t *io = (int32_t *)gdb_raw_ptr(d->io_buffer, 0, io_bytes);
+        if (io == NULL) {
+            return GD_ERR_INVALID_ARGUMENT;
+        }
+        c.ok(argmax_launch(be, &lv, s->logits_softcap, io + d->tokens_offset / 4U, io + d->out_tokens_offset / 4U, io + d->step_counter_offset / 4U, d->max_steps,
+                           io + d->positions_offset / 4U), "argmax_rows");
+    }
+    if (scratch_used != NULL) {
+        *scratch_used = c.top;
+    }
+    if (c.st != GD_OK) {
+        snprintf(be->last_error, sizeof(be->last_error), "gpt prefill: %s", c.where);
+    }
+    return c.st;
+}
+
 extern "C" gd_status gdb200_argmax_rows(gd_backend *be, const gd_backend_tensor_view *logits, float softcap, const gd_backend_tensor_view *out_ids)
 {
     if (be == NULL || logits == NULL || out_ids == NULL || logits->rank != 2 || out_ids->count != (size_t)logits->shape[0]) {

@@ -311,6 +311,7 @@ PROTOTYPES = {
     "gdb200_lm_cross_entropy_fused_rows": (_ST, [P, TV, TV, TV, TV, TV, TV, F, F, I32_T]),
     "gdb200_matmul_tn_colsum": (_ST, [P, MV, MV, MV, VV]),
     "gdb200_argmax_rows": (_ST, [P, TV, F, TV]),
+    "gdb200_gpt_prefill": (_ST, [P, C.POINTER(GptSpec), C.POINTER(GptBatch), SZ, SZ, C.POINTER(GptDecodeState), C.POINTER(SZ)]),
     "gdb200_gpt_decode_steps": (_ST, [P, C.POINTER(GptSpec), C.POINTER(GptDecodeState), I32_T, I32_T, C.POINTER(SZ)]),
     "gdb200_inject_device_error": (_ST, [P, I32_T]),
     "gdb200_selftest_bounded_wait": (_ST, [P, U32]),

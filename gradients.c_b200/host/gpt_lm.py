@@ -341,9 +341,13 @@ class GptLm:
 
     # ---- KV-cache generation ----
     def alloc_kv_cache(self, batch: int, capacity: int) -> None:
+        """Zeroed K and V caches of every layer, next to each other (one clear)."""
         cfg, ctx = self.cfg, self.ctx
-        self.k_cache = [ctx.zeros(ctx.state, cfg.dtype, (batch, capacity, cfg.n_heads, cfg.head_dim), f"k_cache.{i}") for i in range(cfg.n_layers)]
-        self.v_cache = [ctx.zeros(ctx.state, cfg.dtype, (batch, capacity, cfg.n_heads, cfg.head_dim), f"v_cache.{i}") for i in range(cfg.n_layers)]
+        shape = (batch, capacity, cfg.n_heads, cfg.head_dim)
+        caches = [ctx.empty(ctx.state, cfg.dtype, shape, f"{kv}_cache.{i}") for kv in "kv" for i in range(cfg.n_layers)]
+        first, last = caches[0], caches[-1]
+        ctx.check(ctx.lib.gd_backend_fill(ctx.backend, first.buffer, first.offset, (last.offset + last.nbytes - first.offset) // 2, 2, 0), "fill")
+        self.k_cache, self.v_cache = caches[:cfg.n_layers], caches[cfg.n_layers:]
 
     def _mlp_infer(self, pre: str, resid: Tensor) -> Tensor:
         ctx, cfg, p = self.ctx, self.cfg, self.params
@@ -565,7 +569,12 @@ def greedy_generate(model: GptLm, prompts: np.ndarray, new_tokens: int, capacity
 def model_spec(model: GptLm) -> "abi.GptSpec":
     """gdb200_gpt_spec with the model fields and parameter locations only (what the decode driver reads)."""
     mc, ctx = model.cfg, model.ctx
+    # a model's parameters do not move: the description is kept until the arenas or the configuration change
+    key = (ctx.params, ctx.state, ctx.scratch, tuple(vars(mc).values()))
+    if getattr(model, "_spec_key", None) == key:
+        return model._spec
     s = abi.GptSpec()
+    model._spec_key, model._spec = key, s
     s.params_buffer, s.state_buffer, s.scratch_buffer = ctx.params.buffer, ctx.state.buffer, ctx.scratch.buffer
     s.scratch_bytes = ctx.scratch.capacity
     s.vocab_size, s.context_length, s.d_model, s.n_layers = mc.vocab_size, mc.context_length, mc.d_model, mc.n_layers
@@ -599,32 +608,31 @@ def greedy_generate_native(model: GptLm, prompts: np.ndarray, new_tokens: int, c
     b, plen = prompts.shape
     model.alloc_kv_cache(b, capacity)
     lib, be = ctx.lib, ctx.backend
+    # one upload: prompt ids, positions [b * plen], cu_seqlens [b + 1], first cache slots, packed rows of the last prompt tokens [b], then
+    # the words the device works on: tokens, positions (of the last prompt token) [b], out_tokens [new_tokens, b], step counter
+    n = b * plen
+    at = np.cumsum([0, n, n, b + 1, b, b, b, b, new_tokens * b, 1])
+    words = np.zeros(int(at[-1]), dtype=np.int32)
+    words[:n] = prompts.reshape(-1)
+    words[n:2 * n].reshape(b, plen)[:] = np.arange(plen, dtype=np.int32)
+    words[at[2]:at[3]] = np.arange(b + 1, dtype=np.int32) * plen
+    words[at[4]:at[5]] = np.arange(1, b + 1, dtype=np.int32) * plen - 1
+    words[at[6]:at[7]] = plen - 1
     ctx.begin_step()
-    ids = ctx.from_numpy(ctx.data, I32, prompts.reshape(-1).astype(np.int32))
-    pos = ctx.from_numpy(ctx.data, I32, np.tile(np.arange(plen, dtype=np.int32), b))
-    cu = ctx.from_numpy(ctx.data, I32, (np.arange(b + 1, dtype=np.int32) * plen))
-    cpos = ctx.from_numpy(ctx.data, I32, np.zeros(b, dtype=np.int32))
-    ev = [lib.gdb200_event_record(be)] if timing is not None else None
-    logits = model.prefill_last_logits(ids, pos, cu, cpos, np.arange(b) * plen + plen - 1)
-    first = device_argmax(ctx, logits, cfg.logits_softcap)
-    if ev is not None:
-        ev.append(lib.gdb200_event_record(be))
-    ctx.end_step()
-    # io words: tokens [b] = argmax of the prefill logits, positions [b] = prompt length,
-    # out_tokens [new_tokens, b] with row 0 filled, step counter = 1 (one read-back per generation)
-    first_ids = first.read().astype(np.int32)
-    words = np.zeros(2 * b + new_tokens * b + 1, dtype=np.int32)
-    words[:b], words[b:2 * b], words[2 * b:3 * b], words[-1] = first_ids, plen, first_ids, 1
-    io = ctx.from_numpy(ctx.state, I32, words)
+    io = ctx.from_numpy(ctx.data, I32, words)
+    off = [io.offset + 4 * int(i) for i in at]
+    batch = abi.GptBatch(io.buffer, off[0], 0, off[1], off[2], n, b + 1)
     d = abi.GptDecodeState()
-    d.cache_buffer, d.io_buffer = ctx.state.buffer, ctx.state.buffer
+    d.cache_buffer, d.io_buffer = ctx.state.buffer, io.buffer
     for i in range(cfg.n_layers):
         d.k_cache_offset[i], d.v_cache_offset[i] = model.k_cache[i].offset, model.v_cache[i].offset
-    d.tokens_offset, d.positions_offset = io.offset, io.offset + 4 * b
-    d.out_tokens_offset, d.step_counter_offset = io.offset + 8 * b, io.offset + 8 * b + 4 * new_tokens * b
+    d.tokens_offset, d.positions_offset, d.out_tokens_offset, d.step_counter_offset = off[5], off[6], off[7], off[8]
     d.batch, d.capacity, d.max_steps = b, capacity, new_tokens
-    ctx.begin_step()
     spec = model_spec(model)
+    ev = [lib.gdb200_event_record(be)] if timing is not None else None
+    ctx.check(lib.gdb200_gpt_prefill(be, C.byref(spec), C.byref(batch), off[3], off[4], C.byref(d), None), "gpt_prefill")
+    if ev is not None:
+        ev.append(lib.gdb200_event_record(be))
     launches0 = ctx.launch_count()
     if ev is not None:
         ev.append(lib.gdb200_event_record(be))
@@ -632,15 +640,15 @@ def greedy_generate_native(model: GptLm, prompts: np.ndarray, new_tokens: int, c
     if ev is not None:
         ev.append(lib.gdb200_event_record(be))
     ctx.end_step()
-    ctx.flush()
     if ev is not None:
+        ctx.flush()
         timing["prefill_ms"] = float(lib.gdb200_event_elapsed_ms(ev[0], ev[1]))
         timing["decode_ms"] = float(lib.gdb200_event_elapsed_ms(ev[2], ev[3]))
         timing["decode_launches"] = int(ctx.launch_count() - launches0)
         for e in ev:
             lib.gdb200_event_destroy(e)
-    flat = io.read()
-    return flat[2 * b:2 * b + new_tokens * b].reshape(new_tokens, b).T.copy()
+    ctx.flush()   # the ids are complete; reports a bounded wait that ran out
+    return Tensor(ctx, io.arena, off[7], I32, (new_tokens, b)).read().T.copy()
 
 
 def host_argmax(logits: np.ndarray, softcap: float) -> np.ndarray:

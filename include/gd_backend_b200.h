@@ -628,6 +628,13 @@ typedef struct gdb200_gpt_decode_state {
     size_t tokens_offset, positions_offset, out_tokens_offset, step_counter_offset;
     int32_t batch, capacity, max_steps;
 } gdb200_gpt_decode_state;
+/* Packed prefill in one call (gpt_lm_prefill_last_logits, examples/gpt_lm/gpt_lm_shared.c:1117-1202): `batch` holds the packed
+ * prompts (input ids, positions, cu_seqlens [batch + 1]; no targets), cache_pos_offset / last_rows_offset I32 [batch] words of its
+ * buffer (first cache slot per prompt, packed row of its last token). Fills the caches; per prompt the argmax of its last row's logits
+ * goes to tokens and to row *step_counter of out_tokens, positions and the step counter advance by one (the caller sets positions
+ * to the last prompt position and the counter to zero). Nothing is waited for. */
+gd_status gdb200_gpt_prefill(gd_backend *backend, const gdb200_gpt_spec *spec, const gdb200_gpt_batch *batch, size_t cache_pos_offset,
+                             size_t last_rows_offset, const gdb200_gpt_decode_state *state, size_t *scratch_used);
 /* Enqueues n_steps decode steps without any host synchronisation. use_graph == 0: one launch per operation, step after
  * step. use_graph != 0: where the shapes allow (16-bit storage, at most 64 sequences, head_dim 64, d_model 128 / 256 / 512,
  * mlp_hidden a multiple of 128, the cos / sin table of the rotation in use) ALL steps run in one persistent cooperative
