@@ -1,6 +1,6 @@
 // Packed causal attention forward on the sm_100a tensor path: S = Q K^T and O += P V are tcgen05.mma instructions with FP32
 // accumulators in tensor memory; Q, K and V arrive by TMA, P never leaves tensor memory (it is the A operand of the second
-// product), O stays there for the whole item.
+// product).
 //
 // Fast path of gd_backend_sdpa_varlen for 16-bit storage, head_dim 64 or 128, causal (+ optional sliding window), no prefix. A
 // work item is 128 consecutive rows of the PACKED token stream for one head; the mask is evaluated in packed coordinates:
@@ -14,19 +14,22 @@
 // What bounds it: the special-function unit (one exp2 per score at 16 per cycle and SM: 512 cycles of a 128 x 64 step), as long
 // as the chain S -> softmax -> P V does not. The softmax of a 64-key step takes a warp 741 cycles by itself and 581 when two
 // warps share a scheduler (measured with the loop alone), a hand-over between roles 300-500, so the chain is taken apart:
-//   * S has two buffers: S of the next step (also of the next item) is formed while the softmax warps work on this one, and
-//     P V runs behind them; a softmax warp never waits for a product of its own step;
+//   * S has two or three buffers: S of the next steps (also of the next item) is formed while the softmax warps work on this one,
+//     and P V runs behind them; a softmax warp never waits for a product of its own step;
 //   * one thread per query row (192 threads: warp 0 = TMA producer, warp 1 = MMA issuer, warps 2-5 = softmax) holds the row's
-//     64 scores in registers: no exchange between threads, S is read from tensor memory once;
+//     64 scores in registers: no exchange between threads;
 //   * P (16-bit) is written over the S columns it came from with tcgen05.st: no shared-memory tile, no proxy fence. A later S
 //     may overwrite it because one thread issues all products and they execute in order;
-//   * O is rescaled in tensor memory only when a row's maximum has grown by more than 2^8 since the last rescale (the sum is
-//     kept relative to the same stale maximum, so the result is the same); after the first tile that is rare;
-//   * the code of all roles stays near the 32 KB of the first-level instruction cache: waits and searches are not unrolled (57 KB
-//     before), a step has one masked and one unmasked way to the same exponentials.
-// 32768 tokens in sequences of 16-512, 8 heads of 64: 72 us (one step at a time, P through shared memory: 124 us); 8191 tokens
-// in sequences of 256-2048, 16 heads of 128, window 1024: 78 us (mma.sync kernel: 286 us).
-// Tensor memory per CTA (256 columns): S / P 2 x 64, O head_dim.
+//   * the code of all roles stays near the 32 KB of the first-level instruction cache: waits and searches are not unrolled.
+// head_dim 64: P is relative to the exact running maximum of every 128 keys of the item, and O is a fused multiply-add of the
+// finished product of those 128 keys in registers. That fixes every rounding (the output does not depend on how the work is split),
+// at the price of a second read of S: 83 us for 32768 tokens in sequences of 16-512, 8 heads, against 72 with O in tensor memory and
+// a maximum that may lag (124 with 128-key tiles one at a time, P through shared memory). Also measured: the product added before
+// the next exponentials instead of after them 89 us, two warps per row 95 us, skipping masked halves of a step by a branch 88 us.
+// head_dim 128: O (128 columns) does not fit the registers. It stays in tensor memory for the whole item and is rescaled there only
+// when a row's maximum has grown by more than 2^8 since the last rescale (the sum is kept relative to the same stale maximum);
+// after the first tile that is rare. 8191 tokens in sequences of 256-2048, 16 heads, window 1024: 78 us (mma.sync kernel: 286 us).
+// Tensor memory per CTA (256 columns): S / P 3 x 64 or 2 x 64, O head_dim.
 //
 // Statistics written for the backward pass: (row max in natural-log units, sum of exp, 0).
 // Every mbarrier wait is bounded and reports through gd_backend::err_flag.
@@ -41,7 +44,6 @@ constexpr float LN2_F = 0.6931471805599453f;
 constexpr int A_BQ = 128, A_BKV = 64;   // query rows of an item, keys of a step
 constexpr int A_MAX_CU = 1024;
 constexpr int A_THREADS = 192;
-constexpr float A_RESCALE = 8.0f;   // log2 of the growth of a row maximum that triggers a rescale of O
 
 struct attn5_params {
     int n_tokens, batch, hq, hkv, window, n_items;
@@ -57,7 +59,10 @@ struct attn5_plan {
     static constexpr int OFF_K = QSTAGES * QTILE, OFF_V = OFF_K + STAGES * TILE, OFF_BAR = OFF_V + STAGES * TILE;
     static constexpr int TOTAL = OFF_BAR + 512 + 1024;
     static constexpr int TMEM_COLS = 256;
-    static constexpr uint32_t COL_S = 0, COL_O = 2 * A_BKV;       // S / P: two buffers of A_BKV columns
+    static constexpr uint32_t SBUF = DH == 64 ? 3 : 2;            // S / P buffers of A_BKV columns
+    static constexpr uint32_t COL_S = 0, COL_O = SBUF * A_BKV;
+    static constexpr bool PAIRED = DH == 64;                      // O in registers, one maximum per 128 keys
+    static constexpr float RESCALE = 8.0f;                        // (otherwise) log2 of the growth of a row maximum that triggers a rescale of O
 };
 
 __device__ __forceinline__ float ex2_approx(float x)
@@ -92,6 +97,25 @@ __device__ __forceinline__ void item_range(const int *cu_s, const attn5_params &
     }
 }
 
+// Scores of 32 keys: those outside [lo, hi] become -inf.
+__device__ __forceinline__ void mask_keys(uint32_t (&v)[32], int lo, int hi)
+{
+    lo = max(lo, 0);
+    hi = min(hi, 31);
+    const uint32_t allowed = lo <= hi ? (0xffffffffU << lo) & (0xffffffffU >> (31 - hi)) : 0U;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = (allowed & (1U << i)) ? v[i] : 0xff800000U;
+}
+
+__device__ __forceinline__ void max_keys(const uint32_t (&v)[32], float (&mx)[4])
+{
+#pragma unroll
+    for (int i = 0; i < 32; i += 8) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) mx[e] = fmaxf(mx[e], fmaxf(__uint_as_float(v[i + 2 * e]), __uint_as_float(v[i + 2 * e + 1])));
+    }
+}
+
 __device__ __forceinline__ void mbar_arrive_local(uint32_t bar)
 {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
@@ -105,14 +129,14 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                  unsigned *done_counter)
 {
     using plan = attn5_plan<DH>;
-    constexpr uint32_t ST = plan::STAGES, QST = plan::QSTAGES;
+    constexpr uint32_t ST = plan::STAGES, QST = plan::QSTAGES, NS = plan::SBUF;
     extern __shared__ unsigned char smem_raw[];
     __shared__ int cu_s[A_MAX_CU + 1];
     __shared__ int sched_item[4];       // work items handed out by the producer thread (-1: no more work)
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023U) & ~(uintptr_t)1023U);
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + plan::OFF_BAR);
-    enum { Q_FULL = 0, Q_EMPTY = 2, K_FULL = 4, K_EMPTY = 8, V_FULL = 12, V_EMPTY = 16, S_FULL = 20, P_FULL = 22, PV_DONE = 24, O_FREE = 26,
-           SCHED_FULL = 27, SCHED_EMPTY = 31, N_BARS = 35 };
+    enum { Q_FULL = 0, Q_EMPTY = 2, K_FULL = 4, K_EMPTY = 8, V_FULL = 12, V_EMPTY = 16, S_FULL = 20, P_FULL = 23, PV_DONE = 26, O_FREE = 29,
+           SCHED_FULL = 30, SCHED_EMPTY = 34, N_BARS = 38 };
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + N_BARS);
     const uint32_t bar0 = smem_u32(bars);
     auto bar = [&](int i) { return bar0 + 8U * (uint32_t)i; };
@@ -124,7 +148,7 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
 #pragma unroll 1
         for (int i = 0; i < N_BARS; ++i) {
             // schedule slots are released by the MMA thread and the four softmax warps
-            const uint32_t count = (i == P_FULL || i == P_FULL + 1 || i == O_FREE) ? 4U : (i >= SCHED_EMPTY ? 5U : 1U);
+            const uint32_t count = ((i >= P_FULL && i < P_FULL + 3) || i == O_FREE) ? 4U : (i >= SCHED_EMPTY ? 5U : 1U);
             mbar_init(bar(i), count);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -222,9 +246,10 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
             // V stored [key][dh] in blocks of 64 dh: 16 keys = 2048 B per MMA
             const uint64_t v_d = make_smem_desc(smem_u32(smem + plan::OFF_V), plan::BLOCK, 1024);
             constexpr uint64_t QBLOCK16 = plan::QBLOCK >> 4, BLOCK16 = plan::BLOCK >> 4, TILE16 = plan::TILE >> 4, QTILE16 = plan::QTILE >> 4;
-            // Two cursors over the same sequence of steps: `s_*` issues S one step ahead (across items), `g` issues P V.
+            // Two cursors over the same sequence of steps: `s_*` issues S, NS - 1 steps ahead (across items), `g` issues P V.
             uint32_t s_g = 0, s_item = 0, s_si = 0, s_tile = 0;
             int s_tiles = 0;
+            int ahead[3] = {0, 0, 0}, n_ahead = 0;   // key tiles of the items S has moved on to, which P V has not reached
             bool ok = true;
             auto fail = [&](int code) {
                 atomicExch(err_flag, code);
@@ -250,8 +275,7 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                 }
             };
             auto issue_s = [&]() {
-                // S[s_g] goes into buffer s_g & 1, over P of two steps before: P V of that step was issued by this thread
-                // already and executes first
+                // S[s_g] goes over P of NS steps before: P V of that step was issued by this thread already and executes first
                 const uint32_t s = s_g % ST, qs = s_item % QST;
                 if (s_tile == 0 && !mbar_wait(bar(Q_FULL + qs), (s_item / QST) & 1U)) return fail(305);
                 if (!mbar_wait(bar(K_FULL + s), (s_g / ST) & 1U)) return fail(303);
@@ -259,27 +283,30 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
 #pragma unroll
                 for (int kk = 0; kk < DH / UMMA_K; ++kk) {
                     const uint64_t step = (uint64_t)((kk & 3) * 2);
-                    tcgen05_mma_f16(tmem_base + plan::COL_S + (s_g & 1U) * A_BKV, q_d + qs * QTILE16 + (kk >> 2) * QBLOCK16 + step,
+                    tcgen05_mma_f16(tmem_base + plan::COL_S + (s_g % NS) * A_BKV, q_d + qs * QTILE16 + (kk >> 2) * QBLOCK16 + step,
                                     k_d + s * TILE16 + (kk >> 2) * BLOCK16 + step, IDESC_S, kk != 0 ? 1U : 0U);
                 }
-                tcgen05_commit(bar(S_FULL + (s_g & 1U)));
+                tcgen05_commit(bar(S_FULL + s_g % NS));
                 tcgen05_commit(bar(K_EMPTY + s));
                 ++s_g;
                 if (++s_tile == (uint32_t)s_tiles) {
                     tcgen05_commit(bar(Q_EMPTY + qs));
                     ++s_item;
                     seek();
+                    ahead[0] = n_ahead == 0 ? s_tiles : ahead[0];
+                    ahead[1] = n_ahead == 1 ? s_tiles : ahead[1];
+                    ahead[2] = n_ahead == 2 ? s_tiles : ahead[2];
+                    ++n_ahead;
                 }
             };
-            // P V walks behind S: the tiles of the item it is in, and of the one S has moved on to
             uint32_t n_item = 0;
             int tiles = 0, t = 0;
             seek();
             tiles = s_tiles;
-            if (ok && s_tiles > 0) issue_s();
+#pragma unroll 1
+            for (uint32_t i = 1; i < NS && ok && s_tiles > 0; ++i) issue_s();
 #pragma unroll 1
             for (uint32_t g = 0; ok && g < s_g; ++g) {
-                const int ahead = s_tiles;
                 if (s_tiles > 0) issue_s();
                 if (!ok) break;
                 const uint32_t s = g % ST;
@@ -287,23 +314,26 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                     fail(304);
                     break;
                 }
-                if (!mbar_wait(bar(V_FULL + s), (g / ST) & 1U) || !mbar_wait(bar(P_FULL + (g & 1U)), (g >> 1) & 1U)) {
+                if (!mbar_wait(bar(V_FULL + s), (g / ST) & 1U) || !mbar_wait(bar(P_FULL + g % NS), (g / NS) & 1U)) {
                     fail(306);
                     break;
                 }
                 tcgen05_fence_after();
 #pragma unroll
                 for (int kk = 0; kk < A_BKV / UMMA_K; ++kk) {
-                    tcgen05_mma_f16_ts(tmem_base + plan::COL_O, tmem_base + plan::COL_S + (g & 1U) * A_BKV + kk * 8, v_d + s * TILE16 + (uint64_t)(kk * 128),
-                                       IDESC_PV, (t != 0 || kk != 0) ? 1U : 0U);
+                    tcgen05_mma_f16_ts(tmem_base + plan::COL_O, tmem_base + plan::COL_S + (g % NS) * A_BKV + kk * 8, v_d + s * TILE16 + (uint64_t)(kk * 128),
+                                       IDESC_PV, ((plan::PAIRED ? (t & 1) : t) != 0 || kk != 0) ? 1U : 0U);
                 }
                 tcgen05_commit(bar(V_EMPTY + s));
-                tcgen05_commit(bar(PV_DONE + (g & 1U)));
+                tcgen05_commit(bar(PV_DONE + g % NS));   // (of NS steps before: complete once S of this step was seen, so a parity is never mistaken)
                 if (++t == tiles) {
-                    // the S cursor is one step ahead, so it already stands in the next item
+                    // the S cursor is ahead, so it already stands in the next item
                     t = 0;
                     ++n_item;
-                    tiles = ahead;
+                    tiles = ahead[0];
+                    ahead[0] = ahead[1];
+                    ahead[1] = ahead[2];
+                    --n_ahead;
                 }
             }
         }
@@ -341,127 +371,252 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                 lo_key = seg_start_of(cu_s, p.batch, qi);
                 if (p.window > 0) lo_key = max(lo_key, qi - p.window + 1);
             }
-            // m: the maximum O and l are relative to (log2 units, may lag the true maximum by up to A_RESCALE); m_true: the maximum
-            float m = -INFINITY, m_true = -INFINITY, l = 0.0f;
+            float m = -INFINITY, l;
+            T *dst = out + ((size_t)qi * p.hq + h) * DH;
+            // eight finished values of a row
+            auto store8 = [&](int col, float a0, float a1, float a2, float a3, float a4, float a5, float a6, float a7) {
+                uint4 w;
+                w.x = half_pack<T>::pack(a0, a1);
+                w.y = half_pack<T>::pack(a2, a3);
+                w.z = half_pack<T>::pack(a4, a5);
+                w.w = half_pack<T>::pack(a6, a7);
+                *reinterpret_cast<uint4 *>(dst + col) = w;
+            };
+            if constexpr (plan::PAIRED) {
+                // Two steps, 128 keys, share a maximum, the exact running one. Their product P V is formed from zero and added to the row's
+                // O, which is held in registers (O * alpha of the pair the product belongs to), during the next pair: after its first P
+                // is written and before that step's product may start, so the wait for the product is never on the chain.
+                f32x2 o[DH / 2];
+#pragma unroll
+                for (int i = 0; i < DH / 2; ++i) o[i] = f2_make(0.0f, 0.0f);
+                float part[2] = {0.0f, 0.0f}, alpha = 1.0f;   // sums over the even and over the odd steps' keys
+                auto take_o = [&](uint32_t last, float scale) {
+                    wait_or_die(PV_DONE + last % NS, (last / NS) & 1U, 309);
+                    if (dead) return;
+                    tcgen05_fence_after();
+                    const f32x2 scale2 = f2_make(scale, scale);
+#pragma unroll
+                    for (int c = 0; c < DH / 32; ++c) {
+                        uint32_t w[32];
+                        tmem_ld_32x32b_x32(lane_base + plan::COL_O + c * 32, w);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) o[c * 16 + i] = f2_fma(o[c * 16 + i], scale2, f2_make(__uint_as_float(w[2 * i]), __uint_as_float(w[2 * i + 1])));
+                    }
+                };
 #pragma unroll 1
-            for (int t = 0; t < n_tiles; ++t, ++g) {
-                const int key0 = kv_begin + t * A_BKV;
-                const uint32_t s_col = lane_base + plan::COL_S + (g & 1U) * A_BKV;
-                // allowed local columns [c_lo, c_hi] of this row
-                const int c_lo = valid ? max(0, lo_key - key0) : A_BKV, c_hi = valid ? min(A_BKV - 1, qi - key0) : -1;
-                const bool live = __any_sync(0xffffffffU, c_lo <= c_hi), full = __all_sync(0xffffffffU, c_lo == 0 && c_hi == A_BKV - 1);
-                wait_or_die(S_FULL + (g & 1U), (g >> 1) & 1U, 308);
-                if (dead) break;
-                tcgen05_fence_after();
-                if (live) {
-                    uint32_t v[2][32];
-                    tmem_ld_32x32b_x32_nowait(s_col, v[0]);
-                    tmem_ld_32x32b_x32_nowait(s_col + 32, v[1]);
-                    tmem_ld_wait();
-                    if (!full) {
-#pragma unroll
-                        for (int c = 0; c < 2; ++c) {
-                            const int lo = max(c_lo - c * 32, 0), hi = min(c_hi - c * 32, 31);
-                            const uint32_t allowed = lo <= hi ? (0xffffffffU << lo) & (0xffffffffU >> (31 - hi)) : 0U;
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) v[c][i] = (allowed & (1U << i)) ? v[c][i] : 0xff800000U;
-                        }
-                    }
-                    float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-                    for (int i = 0; i < 64; i += 8) {
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) mx[e] = fmaxf(mx[e], fmaxf(__uint_as_float(v[i >> 5][(i & 31) + 2 * e]), __uint_as_float(v[i >> 5][(i & 31) + 2 * e + 1])));
-                    }
-                    const float m_cand = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl2;
-                    m_true = fmaxf(m_true, m_cand);
-                    const bool bump = m_cand > m + A_RESCALE || (m == -INFINITY && m_cand != -INFINITY);
-                    if (__any_sync(0xffffffffU, bump)) {
-                        const float alpha = bump ? ex2_approx(m - m_cand) : 1.0f;   // m = -inf: 0
-                        if (__any_sync(0xffffffffU, bump && m != -INFINITY)) {
-                            wait_or_die(PV_DONE + ((g - 1U) & 1U), ((g - 1U) >> 1) & 1U, 309);   // O holds every step before this one
+                for (int t = 0; t < n_tiles; ++t, ++g) {
+                    float taken = alpha;   // what the product of the pair before is combined with
+                    if ((t & 1) == 0) {
+                        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll 1
+                        for (int u = 0; u < 2 && t + u < n_tiles; ++u) {
+                            const uint32_t gu = g + (uint32_t)u;
+                            const int key0 = kv_begin + (t + u) * A_BKV;
+                            // allowed local columns [c_lo, c_hi] of this row
+                            const int c_lo = valid ? max(0, lo_key - key0) : A_BKV, c_hi = valid ? min(A_BKV - 1, qi - key0) : -1;
+                            wait_or_die(S_FULL + gu % NS, (gu / NS) & 1U, 308);
                             if (dead) break;
                             tcgen05_fence_after();
-#pragma unroll 1
-                            for (int c = 0; c < DH / 8; ++c) {
-                                uint32_t o[8];
-                                tmem_ld_32x32b_x8(lane_base + plan::COL_O + c * 8, o);
-#pragma unroll
-                                for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                                tmem_st_32x32b_x8(lane_base + plan::COL_O + c * 8, o);
+                            if (__any_sync(0xffffffffU, c_lo <= c_hi)) {
+                                uint32_t v[2][32];
+                                tmem_ld_32x32b_x32_nowait(lane_base + plan::COL_S + (gu % NS) * A_BKV, v[0]);
+                                tmem_ld_32x32b_x32_nowait(lane_base + plan::COL_S + (gu % NS) * A_BKV + 32, v[1]);
+                                tmem_ld_wait();
+                                if (!__all_sync(0xffffffffU, c_lo == 0 && c_hi == A_BKV - 1)) {
+                                    mask_keys(v[0], c_lo, c_hi);
+                                    mask_keys(v[1], c_lo - 32, c_hi - 32);
+                                }
+                                max_keys(v[0], mx);
+                                max_keys(v[1], mx);
                             }
                         }
-                        l *= alpha;
-                        if (bump) m = m_cand;
+                        if (dead) break;
+                        const float m_new = fmaxf(m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl2);
+                        alpha = m == m_new ? 1.0f : ex2_approx(m - m_new);   // (m = -inf: 0)
+                        m = m_new;
                     }
-                    const f32x2 scale2 = f2_make(sl2, sl2), shift2 = m == -INFINITY ? f2_make(0.0f, 0.0f) : f2_make(-m, -m);
-                    f32x2 sum0 = f2_make(0.0f, 0.0f), sum1 = sum0;
-#pragma unroll
-                    for (int c = 0; c < 2; ++c) {
-                        uint32_t packed[16];
-#pragma unroll
-                        for (int i = 0; i < 32; i += 2) {
-                            float p0, p1;
-                            f2_split(f2_fma(f2_make(__uint_as_float(v[c][i]), __uint_as_float(v[c][i + 1])), scale2, shift2), p0, p1);
-                            p0 = ex2_approx(p0);
-                            p1 = ex2_approx(p1);
-                            f32x2 &sum = (i & 2) ? sum1 : sum0;
-                            sum = f2_add(sum, f2_make(p0, p1));
-                            packed[i >> 1] = half_pack<T>::pack(p0, p1);
+                    const int key0 = kv_begin + t * A_BKV;
+                    const int c_lo = valid ? max(0, lo_key - key0) : A_BKV, c_hi = valid ? min(A_BKV - 1, qi - key0) : -1;
+                    const uint32_t s_col = lane_base + plan::COL_S + (g % NS) * A_BKV;
+                    float rsum = 0.0f;
+                    if (__any_sync(0xffffffffU, c_lo <= c_hi)) {
+                        uint32_t v[2][32];
+                        tmem_ld_32x32b_x32_nowait(s_col, v[0]);
+                        tmem_ld_32x32b_x32_nowait(s_col + 32, v[1]);
+                        tmem_ld_wait();
+                        if (!__all_sync(0xffffffffU, c_lo == 0 && c_hi == A_BKV - 1)) {
+                            mask_keys(v[0], c_lo, c_hi);
+                            mask_keys(v[1], c_lo - 32, c_hi - 32);
                         }
-                        tmem_st_32x32b_x16(s_col + c * 16, packed);
+                        const f32x2 scale2 = f2_make(sl2, sl2), shift2 = m == -INFINITY ? f2_make(0.0f, 0.0f) : f2_make(-m, -m);
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) {
+                            uint32_t packed[16];
+#pragma unroll
+                            for (int i = 0; i < 32; i += 4) {
+                                float q0, q1, q2, q3;
+                                f2_split(f2_fma(f2_make(__uint_as_float(v[c][i]), __uint_as_float(v[c][i + 1])), scale2, shift2), q0, q1);
+                                f2_split(f2_fma(f2_make(__uint_as_float(v[c][i + 2]), __uint_as_float(v[c][i + 3])), scale2, shift2), q2, q3);
+                                q0 = ex2_approx(q0);
+                                q1 = ex2_approx(q1);
+                                q2 = ex2_approx(q2);
+                                q3 = ex2_approx(q3);
+                                packed[i >> 1] = half_pack<T>::pack(q0, q1);
+                                packed[(i >> 1) + 1] = half_pack<T>::pack(q2, q3);
+                                float s01, s23;
+                                f2_split(f2_add(f2_make(q0, q2), f2_make(q1, q3)), s01, s23);
+                                rsum += s01;
+                                rsum += s23;
+                            }
+                            tmem_st_32x32b_x16(s_col + c * 16, packed);
+                        }
+                    } else {
+                        const uint32_t zero[16] = {0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U};
+                        tmem_st_32x32b_x16(s_col, zero);
+                        tmem_st_32x32b_x16(s_col + 16, zero);
                     }
-                    float a0, a1;
-                    f2_split(f2_add(sum0, sum1), a0, a1);
-                    l += a0 + a1;
-                } else {
-                    const uint32_t zero[16] = {0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U};
-                    tmem_st_32x32b_x16(s_col, zero);
-                    tmem_st_32x32b_x16(s_col + 16, zero);
+                    if ((t & 1) == 0) {
+                        part[0] = fmaf(part[0], alpha, rsum);
+                        part[1] *= t + 1 < n_tiles ? 1.0f : alpha;   // (no odd step follows)
+                        if (t > 0) take_o(g - 1U, taken);
+                        if (dead) break;
+                    } else {
+                        part[1] = fmaf(part[1], alpha, rsum);
+                    }
+                    tmem_st_wait();
+                    tcgen05_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_local(bar(P_FULL + g % NS));
                 }
-                tmem_st_wait();
-                tcgen05_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_local(bar(P_FULL + (g & 1U)));
-            }
-            if (dead) break;
-            // ---- normalise and store this row ----
-            const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-            T *dst = out + ((size_t)qi * p.hq + h) * DH;
-            if (n_tiles > 0) {
-                wait_or_die(PV_DONE + ((g - 1U) & 1U), ((g - 1U) >> 1) & 1U, 307);
                 if (dead) break;
-                tcgen05_fence_after();
-#pragma unroll 1
-                for (int c = 0; c < DH / 32; ++c) {
-                    uint32_t o[32];
-                    tmem_ld_32x32b_x32(lane_base + plan::COL_O + c * 32, o);
-                    if (c == DH / 32 - 1) {
-                        tcgen05_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive_local(bar(O_FREE));
-                    }
-                    if (qi < p.n_tokens) {
+                if (n_tiles > 0) {
+                    take_o(g - 1U, alpha);
+                    if (dead) break;
+                    tcgen05_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_local(bar(O_FREE));
+                }
+                l = part[0] + part[1];
+                const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+                if (qi < p.n_tokens) {
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            // (a row without allowed keys has only zero probabilities; its inverse is zero)
-                            uint4 w;
-                            w.x = half_pack<T>::pack(__uint_as_float(o[8 * j]) * inv, __uint_as_float(o[8 * j + 1]) * inv);
-                            w.y = half_pack<T>::pack(__uint_as_float(o[8 * j + 2]) * inv, __uint_as_float(o[8 * j + 3]) * inv);
-                            w.z = half_pack<T>::pack(__uint_as_float(o[8 * j + 4]) * inv, __uint_as_float(o[8 * j + 5]) * inv);
-                            w.w = half_pack<T>::pack(__uint_as_float(o[8 * j + 6]) * inv, __uint_as_float(o[8 * j + 7]) * inv);
-                            *reinterpret_cast<uint4 *>(dst + c * 32 + 8 * j) = w;
-                        }
+                    for (int j = 0; j < DH / 8; ++j) {
+                        float a[8];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) f2_split(o[4 * j + e], a[2 * e], a[2 * e + 1]);
+                        store8(8 * j, a[0] * inv, a[1] * inv, a[2] * inv, a[3] * inv, a[4] * inv, a[5] * inv, a[6] * inv, a[7] * inv);
                     }
                 }
-            } else if (qi < p.n_tokens) {
+            } else {
+                // m: the maximum O and l are relative to (log2 units, may lag the true maximum by up to RESCALE); m_true: the maximum
+                float m_true = -INFINITY;
+                l = 0.0f;
+#pragma unroll 1
+                for (int t = 0; t < n_tiles; ++t, ++g) {
+                    const int key0 = kv_begin + t * A_BKV;
+                    const uint32_t s_col = lane_base + plan::COL_S + (g % NS) * A_BKV;
+                    const int c_lo = valid ? max(0, lo_key - key0) : A_BKV, c_hi = valid ? min(A_BKV - 1, qi - key0) : -1;
+                    const bool live = __any_sync(0xffffffffU, c_lo <= c_hi), full = __all_sync(0xffffffffU, c_lo == 0 && c_hi == A_BKV - 1);
+                    wait_or_die(S_FULL + g % NS, (g / NS) & 1U, 308);
+                    if (dead) break;
+                    tcgen05_fence_after();
+                    if (live) {
+                        uint32_t v[2][32];
+                        tmem_ld_32x32b_x32_nowait(s_col, v[0]);
+                        tmem_ld_32x32b_x32_nowait(s_col + 32, v[1]);
+                        tmem_ld_wait();
+                        if (!full) {
+                            mask_keys(v[0], c_lo, c_hi);
+                            mask_keys(v[1], c_lo - 32, c_hi - 32);
+                        }
+                        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+                        max_keys(v[0], mx);
+                        max_keys(v[1], mx);
+                        const float m_cand = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl2;
+                        m_true = fmaxf(m_true, m_cand);
+                        const bool bump = m_cand > m + plan::RESCALE || (m == -INFINITY && m_cand != -INFINITY);
+                        if (__any_sync(0xffffffffU, bump)) {
+                            const float alpha = bump ? ex2_approx(m - m_cand) : 1.0f;   // m = -inf: 0
+                            if (__any_sync(0xffffffffU, bump && m != -INFINITY)) {
+                                wait_or_die(PV_DONE + (g - 1U) % NS, ((g - 1U) / NS) & 1U, 309);   // O holds every step before this one
+                                if (dead) break;
+                                tcgen05_fence_after();
+#pragma unroll 1
+                                for (int c = 0; c < DH / 16; ++c) {
+                                    uint32_t o[16];
+                                    tmem_ld_32x32b_x16_nowait(lane_base + plan::COL_O + c * 16, o);
+                                    tmem_ld_wait();
 #pragma unroll
-                for (int j = 0; j < DH / 8; ++j) *reinterpret_cast<uint4 *>(dst + 8 * j) = make_uint4(0U, 0U, 0U, 0U);
+                                    for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                                    tmem_st_32x32b_x16(lane_base + plan::COL_O + c * 16, o);
+                                }
+                            }
+                            l *= alpha;
+                            if (bump) m = m_cand;
+                        }
+                        const f32x2 scale2 = f2_make(sl2, sl2), shift2 = m == -INFINITY ? f2_make(0.0f, 0.0f) : f2_make(-m, -m);
+                        f32x2 sum0 = f2_make(0.0f, 0.0f), sum1 = sum0;
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) {
+                            uint32_t packed[16];
+#pragma unroll
+                            for (int i = 0; i < 32; i += 2) {
+                                float p0, p1;
+                                f2_split(f2_fma(f2_make(__uint_as_float(v[c][i]), __uint_as_float(v[c][i + 1])), scale2, shift2), p0, p1);
+                                p0 = ex2_approx(p0);
+                                p1 = ex2_approx(p1);
+                                f32x2 &sum = (i & 2) ? sum1 : sum0;
+                                sum = f2_add(sum, f2_make(p0, p1));
+                                packed[i >> 1] = half_pack<T>::pack(p0, p1);
+                            }
+                            tmem_st_32x32b_x16(s_col + c * 16, packed);
+                        }
+                        float a0, a1;
+                        f2_split(f2_add(sum0, sum1), a0, a1);
+                        l += a0 + a1;
+                    } else {
+                        const uint32_t zero[16] = {0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U};
+                        tmem_st_32x32b_x16(s_col, zero);
+                        tmem_st_32x32b_x16(s_col + 16, zero);
+                    }
+                    tmem_st_wait();
+                    tcgen05_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_local(bar(P_FULL + g % NS));
+                }
+                if (dead) break;
+                // ---- normalise and store this row ----
+                const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+                if (n_tiles > 0) {
+                    wait_or_die(PV_DONE + (g - 1U) % NS, ((g - 1U) / NS) & 1U, 307);
+                    if (dead) break;
+                    tcgen05_fence_after();
+#pragma unroll 1
+                    for (int c = 0; c < DH / 32; ++c) {
+                        uint32_t o[32];
+                        tmem_ld_32x32b_x32(lane_base + plan::COL_O + c * 32, o);
+                        if (c == DH / 32 - 1) {
+                            tcgen05_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive_local(bar(O_FREE));
+                        }
+                        if (qi < p.n_tokens) {
+                            auto f = [&](int i) { return __uint_as_float(o[i]) * inv; };   // (a row without allowed keys: zeros, its inverse is zero)
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) store8(c * 32 + 8 * j, f(8 * j), f(8 * j + 1), f(8 * j + 2), f(8 * j + 3), f(8 * j + 4), f(8 * j + 5), f(8 * j + 6), f(8 * j + 7));
+                        }
+                    }
+                } else if (qi < p.n_tokens) {
+#pragma unroll
+                    for (int j = 0; j < DH / 8; ++j) *reinterpret_cast<uint4 *>(dst + 8 * j) = make_uint4(0U, 0U, 0U, 0U);
+                }
+                l = m_true == -INFINITY ? l : l * ex2_approx(m - m_true);
+                m = m_true;
             }
             if (stats != nullptr && valid) {
                 float *s = stats + ((size_t)qi * p.hq + h) * 3;
-                s[0] = m_true == -INFINITY ? m_true : m_true * LN2_F;
-                s[1] = m_true == -INFINITY ? l : l * ex2_approx(m - m_true);
+                s[0] = m == -INFINITY ? m : m * LN2_F;
+                s[1] = l;
                 s[2] = 0.0f;
             }
         }
