@@ -72,6 +72,83 @@ __global__ void cast_from_f32_kernel(const float *src, T *dst, size_t n)
         gdb_io<T>::st(dst, i, src[i]);
     }
 }
+// Vector forms for rows of a multiple of eight 16-bit elements on 16-byte boundaries: one 16-byte load of the gradient and two
+// four-element reductions per thread instead of eight loads, divisions and atomics (18.4 k rows of 512: 26 us before).
+template <typename T>
+__global__ void embedding_scatter_vec8_kernel(const uint4 *__restrict__ grad, const int *__restrict__ ids, float *acc, unsigned n_vec, unsigned vpr, unsigned vocab)
+{
+    gdb_pdl_sync();
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n_vec; i += gridDim.x * blockDim.x) {
+        const unsigned row = i / vpr, v = i - row * vpr;
+        const int id = __ldg(&ids[row]);
+        if (id < 0 || (unsigned)id >= vocab) continue;
+        gdb_vec8<T> g;
+        g.raw = grad[i];
+        float *p = acc + ((size_t)id * vpr + v) * 8U;
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(g.get(0)), "f"(g.get(1)), "f"(g.get(2)), "f"(g.get(3)) : "memory");
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p + 4), "f"(g.get(4)), "f"(g.get(5)), "f"(g.get(6)), "f"(g.get(7)) : "memory");
+    }
+}
+// dst = round(src) eight elements at a time; with `ids`, only the rows named by them (a row named twice is written twice, alike).
+template <typename T>
+__global__ void cast_from_f32_vec8_kernel(const float4 *__restrict__ src, uint4 *__restrict__ dst, size_t n_vec, const int *__restrict__ ids, unsigned vpr, unsigned vocab)
+{
+    gdb_pdl_sync();
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_vec; i += stride) {
+        size_t at = i;
+        if (ids != nullptr) {
+            const unsigned row = (unsigned)i / vpr;
+            const int id = __ldg(&ids[row]);
+            if (id < 0 || (unsigned)id >= vocab) continue;
+            at = (size_t)id * vpr + ((unsigned)i - row * vpr);
+        }
+        const float4 a = src[2 * at], b = src[2 * at + 1];
+        gdb_vec8<T> o;
+        o.set(0, a.x);
+        o.set(1, a.y);
+        o.set(2, a.z);
+        o.set(3, a.w);
+        o.set(4, b.x);
+        o.set(5, b.y);
+        o.set(6, b.z);
+        o.set(7, b.w);
+        dst[at] = o.raw;
+    }
+}
+__global__ void clear_rows_kernel(float4 *acc, const int *__restrict__ ids, unsigned n, unsigned quads, unsigned vocab)
+{
+    gdb_pdl_sync();
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const unsigned row = i / quads;
+        const int id = __ldg(&ids[row]);
+        if (id >= 0 && (unsigned)id < vocab) acc[(size_t)id * quads + (i - row * quads)] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+}
+// Gradient of a 16-bit table, vector path. With fewer tokens than table rows the FP32 accumulator is cleared and rounded only in the
+// rows the tokens name and the rest of the gradient is one clear; else the accumulator is cleared and rounded as a whole.
+template <typename T>
+gd_status embedding_backward_vec8(gd_backend *be, const void *grad, const int *ids, float *acc, void *table, const gd_backend_embedding_args *a)
+{
+    const unsigned vpr = (unsigned)(a->dim / 8U), n_vec = (unsigned)(a->ids_count * vpr), vocab = (unsigned)a->vocab;
+    const size_t total = a->vocab * a->dim;
+    const bool by_row = a->ids_count < a->vocab;
+    cudaError_t e = by_row ? cudaMemsetAsync(table, 0, total * sizeof(T), be->stream) : cudaMemsetAsync(acc, 0, total * sizeof(float), be->stream);
+    be->launches += 1U;
+    if (e != cudaSuccess) return gdb_fail(be, e, "embedding_backward zero");
+    if (by_row) {
+        gdb_launch(clear_rows_kernel, gdb_grid_for(n_vec * 2U, 256, be, 8), 256, 0, be->stream, (float4 *)acc, ids, n_vec * 2U, vpr * 2U, vocab);
+        gd_status st = gdb_launched(be, "embedding_backward clear");
+        if (st != GD_OK) return st;
+    }
+    gdb_launch(embedding_scatter_vec8_kernel<T>, gdb_grid_for(n_vec, 256, be, 8), 256, 0, be->stream, (const uint4 *)grad, ids, acc, n_vec, vpr, vocab);
+    gd_status st = gdb_launched(be, "embedding_backward scatter");
+    if (st != GD_OK) return st;
+    const size_t n_cast = by_row ? (size_t)n_vec : total / 8U;
+    gdb_launch(cast_from_f32_vec8_kernel<T>, gdb_grid_for(n_cast, 256, be, 8), 256, 0, be->stream, (const float4 *)acc, (uint4 *)table, n_cast, by_row ? ids : (const int *)nullptr,
+               vpr, vocab);
+    return gdb_launched(be, "embedding_backward cast");
+}
 
 // ------------------------------------------------------------------ rope
 // One thread per (token, head, pair). FWD: src = qkv [N, 3*H*Dh] -> q,k,v [N,H,Dh].
@@ -529,6 +606,10 @@ gd_status gd_backend_embedding_backward(gd_backend *be, const gd_backend_tensor_
         }
     }
     const size_t total = a->vocab * a->dim;
+    if (dt != GDB_DTYPE_F32 && a->ids_count != 0U && (a->dim % 8U) == 0U && (((uintptr_t)gp | (uintptr_t)acc | (uintptr_t)tp) % 16U) == 0U &&
+        a->ids_count * a->dim < ((uint64_t)1 << 31) && total < ((uint64_t)1 << 34) && a->vocab < ((uint64_t)1 << 31)) {
+        return dt == GDB_DTYPE_F16 ? embedding_backward_vec8<__half>(be, gp, ip, acc, tp, a) : embedding_backward_vec8<__nv_bfloat16>(be, gp, ip, acc, tp, a);
+    }
     cudaError_t e = cudaMemsetAsync(acc, 0, total * sizeof(float), be->stream);
     be->launches += 1U;
     if (e != cudaSuccess) {
