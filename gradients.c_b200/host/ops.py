@@ -30,7 +30,7 @@ SDPA_BACKWARD_WITH_OUTPUT = True
 
 
 def _tvp(t: Optional[Tensor]):
-    return byref(t.tv()) if t is not None else None
+    return t.ref() if t is not None else None
 
 
 def _flat2(t: Tensor) -> tuple[int, int]:

@@ -149,6 +149,7 @@ class AdamW:
         self.n = n
         self._norm_descs = (abi.GradNormDesc * n)()
         self._adamw_descs = (abi.AdamwDesc * n)()
+        self._laid_out: list = [None] * n   # per descriptor: what its step-independent fields were written for
 
     def _f32_off(self, field: int, index: int) -> int:
         return self.state_f32.offset + (field * self.n + index) * 4
@@ -171,15 +172,17 @@ class AdamW:
         found_buf, found_off = scaler.flag_state.buffer, scaler.flag_state.offset + 4
         count = 0
         partial_index = 0
+        partial_buffer, partial_offset = self.partials.buffer, self.partials.offset
         active = []
         for i, s in enumerate(self.slots):
             g = s.param.grad
             if g is None:
                 continue
-            groups = (s.param.count + NORM_BLOCK - 1) // NORM_BLOCK
+            p = s.param
+            groups = (p.count + NORM_BLOCK - 1) // NORM_BLOCK
             d = self._norm_descs[count]
-            d.grad_buffer, d.grad_offset, d.count, d.grad_dtype = g.buffer, g.offset, g.count, g.dtype
-            d.partial_buffer, d.partial_offset, d.partial_count = self.partials.buffer, self.partials.offset + partial_index * 4, groups
+            d.grad_buffer, d.grad_offset, d.count, d.grad_dtype = g.arena.buffer, g.offset, g.count, g.dtype
+            d.partial_buffer, d.partial_offset, d.partial_count = partial_buffer, partial_offset + partial_index * 4, groups
             d.grad_scale_buffer, d.grad_scale_offset = inv_buf, inv_off
             d.found_inf_buffer, d.found_inf_offset, d.has_found_inf = found_buf, found_off, 1
             partial_index += groups
@@ -191,32 +194,41 @@ class AdamW:
         ctx.check(lib.gd_backend_grad_clip_scale(ctx.backend, self._norm_descs, count, self.grad_clip_scale.buffer,
                                                  self.grad_clip_scale.offset, max_grad_norm, GRAD_CLIP_SCALE_EPS), "grad_clip_scale")
         cfg = self.config
+        bias_correction = 1 if cfg.bias_correction else 0
         for j, i in enumerate(active):
             s = self.slots[i]
             g = s.param.grad
             d = self._adamw_descs[j]
-            C.memset(byref(d), 0, C.sizeof(d))
-            d.param_buffer, d.param_offset = s.param.buffer, s.param.offset
-            if s.master is not None:
-                d.master_buffer, d.master_offset, d.has_master = s.master.buffer, s.master.offset, 1
-            d.grad_buffer, d.grad_offset = g.buffer, g.offset
-            d.grad_scale_buffer, d.grad_scale_offset, d.has_grad_scale = self.grad_clip_scale.buffer, self.grad_clip_scale.offset, 1
-            d.found_inf_buffer, d.found_inf_offset, d.has_found_inf = found_buf, found_off, 1
-            d.m_buffer, d.m_offset, d.v_buffer, d.v_offset = s.m.buffer, s.m.offset, s.v.buffer, s.v.offset
-            d.state_f32_buffer = self.state_f32.buffer
-            d.beta1_power_offset, d.beta2_power_offset = self._f32_off(self.F_BETA1, i), self._f32_off(self.F_BETA2, i)
-            d.step_scale_offset, d.decay_scale_offset = self._f32_off(self.F_STEP, i), self._f32_off(self.F_DECAY, i)
-            d.eps_scaled_offset = self._f32_off(self.F_EPS, i)
-            d.state_i32_buffer = self.state_i32.buffer
-            d.param_step_offset = self.state_i32.offset + i * 4
-            d.optimizer_step_offset = self.state_i32.offset + self.n * 4
-            d.count, d.param_dtype, d.grad_dtype = s.param.count, s.param.dtype, g.dtype
-            d.has_device_state, d.bias_correction = 1, 1 if cfg.bias_correction else 0
-            d.update_optimizer_step = 1 if j == 0 else 0
+            if self._laid_out[j] != (i, s.param, s.master, s.m, s.v):
+                self._lay_out(d, i, s, first=j == 0)
+                self._laid_out[j] = (i, s.param, s.master, s.m, s.v)
+            d.grad_buffer, d.grad_offset, d.grad_dtype = g.arena.buffer, g.offset, g.dtype
+            d.found_inf_buffer, d.found_inf_offset = found_buf, found_off
+            d.bias_correction = bias_correction
             d.lr, d.beta1, d.beta2, d.eps, d.weight_decay = lr * s.lr_mult, cfg.beta1, cfg.beta2, cfg.eps, s.weight_decay
-            d.bias_correction1 = d.bias_correction2 = 1.0
         ctx.check(lib.gd_backend_adamw_batch(ctx.backend, self._adamw_descs, count), "adamw_batch")
         scaler.finish_step()
+
+    def _lay_out(self, d: abi.AdamwDesc, i: int, s: ParamSlot, first: bool) -> None:
+        """The fields of slot i's descriptor that stay as they are from step to step."""
+        C.memset(byref(d), 0, C.sizeof(d))
+        d.param_buffer, d.param_offset = s.param.buffer, s.param.offset
+        if s.master is not None:
+            d.master_buffer, d.master_offset, d.has_master = s.master.buffer, s.master.offset, 1
+        d.grad_scale_buffer, d.grad_scale_offset, d.has_grad_scale = self.grad_clip_scale.buffer, self.grad_clip_scale.offset, 1
+        d.has_found_inf = 1
+        d.m_buffer, d.m_offset, d.v_buffer, d.v_offset = s.m.buffer, s.m.offset, s.v.buffer, s.v.offset
+        d.state_f32_buffer = self.state_f32.buffer
+        d.beta1_power_offset, d.beta2_power_offset = self._f32_off(self.F_BETA1, i), self._f32_off(self.F_BETA2, i)
+        d.step_scale_offset, d.decay_scale_offset = self._f32_off(self.F_STEP, i), self._f32_off(self.F_DECAY, i)
+        d.eps_scaled_offset = self._f32_off(self.F_EPS, i)
+        d.state_i32_buffer = self.state_i32.buffer
+        d.param_step_offset = self.state_i32.offset + i * 4
+        d.optimizer_step_offset = self.state_i32.offset + self.n * 4
+        d.count, d.param_dtype = s.param.count, s.param.dtype
+        d.has_device_state = 1
+        d.update_optimizer_step = 1 if first else 0
+        d.bias_correction1 = d.bias_correction2 = 1.0
 
     def zero_grad(self) -> None:
         for s in self.slots:

@@ -10,6 +10,7 @@ produced by a gd_backend_* call.
 from __future__ import annotations
 
 import ctypes as C
+import math
 from typing import Callable, Optional, Sequence
 
 import numpy as np
@@ -45,44 +46,60 @@ class Arena:
         self.buffer = out
         self.top = 0
         self.high_water = 0
+        self._views: dict = {}   # (dtype, shape) -> image of a tensor view without its offset
 
     def alloc(self, nbytes: int, align: int = ALIGN) -> int:
         off = (self.top + align - 1) & ~(align - 1)
         if off + nbytes > self.capacity:
             raise MemoryError(f"arena {self.name}: need {off + nbytes} bytes, capacity {self.capacity}")
-        self.top = off + int(nbytes)
-        self.high_water = max(self.high_water, self.top)
+        self.top = top = off + int(nbytes)
+        if top > self.high_water:
+            self.high_water = top
         return off
 
     def reset(self) -> None:
         self.top = 0
 
+    def view(self, offset: int, dtype: int, shape: tuple, count: int) -> abi.TensorView:
+        """gd_backend_tensor_view of contiguous bytes of this arena. The image of a (dtype, shape) is kept and copied: filling the
+        sixteen array fields of a new structure was a quarter of the host time of a small attention call."""
+        image = self._views.get((dtype, shape))
+        if image is None:
+            v = abi.TensorView()
+            v.buffer, v.count, v.dtype, v.rank = self.buffer, count, dtype, len(shape)
+            stride = 1
+            for d in range(len(shape) - 1, -1, -1):
+                v.shape[d] = shape[d]
+                v.strides[d] = stride
+                stride *= shape[d]
+            if len(self._views) >= 1024:   # shapes follow the batch: bounded
+                self._views.clear()
+            image = self._views[(dtype, shape)] = bytes(v)
+        v = abi.TensorView.from_buffer_copy(image)
+        v.offset = offset
+        return v
+
     def destroy(self) -> None:
         if self.buffer:
             self.ctx.lib.gd_backend_buffer_destroy(self.buffer)
             self.buffer = None
+            self._views.clear()
 
 
 class Tensor:
     """Descriptor of contiguous tensor bytes inside an arena (reference gd_tensor)."""
 
-    __slots__ = ("ctx", "arena", "offset", "dtype", "shape", "requires_grad", "grad", "is_leaf", "name", "_tv")
+    __slots__ = ("ctx", "arena", "offset", "dtype", "shape", "count", "requires_grad", "grad", "is_leaf", "name", "_tv", "_ref")
 
     def __init__(self, ctx: "Context", arena: Arena, offset: int, dtype: int, shape: Sequence[int], name: str = ""):
         self.ctx, self.arena, self.offset, self.dtype = ctx, arena, int(offset), dtype
-        self.shape = tuple(int(s) for s in shape)
+        self.shape = shape = tuple(map(int, shape))
+        self.count = math.prod(shape)
         self.requires_grad = False
         self.grad: Optional[Tensor] = None
         self.is_leaf = False
         self.name = name
-        self._tv = None
-
-    @property
-    def count(self) -> int:
-        n = 1
-        for s in self.shape:
-            n *= s
-        return n
+        self._tv = self._ref = None
 
     @property
     def nbytes(self) -> int:
@@ -95,28 +112,22 @@ class Tensor:
     def tv(self) -> abi.TensorView:
         """gd_backend_tensor_view of the whole tensor (cached; descriptors are immutable)."""
         if self._tv is None:
-            v = abi.TensorView()
-            v.buffer, v.offset, v.count, v.dtype, v.rank = self.arena.buffer, self.offset, self.count, self.dtype, len(self.shape)
-            stride = 1
-            for d in range(len(self.shape) - 1, -1, -1):
-                v.shape[d] = self.shape[d]
-                v.strides[d] = stride
-                stride *= self.shape[d]
-            self._tv = v
+            self._tv = self.arena.view(self.offset, self.dtype, self.shape, self.count)
         return self._tv
+
+    def ref(self):
+        """Pointer argument to tv() (cached with it)."""
+        if self._ref is None:
+            self._ref = C.byref(self.tv())
+        return self._ref
 
     def mv(self, rows: int, cols: int, row_offset: int = 0, row_bytes: Optional[int] = None) -> abi.MatrixView:
         es = DTYPE_SIZE[self.dtype]
         rb = cols * es if row_bytes is None else row_bytes
-        v = abi.MatrixView()
-        v.buffer, v.offset, v.rows, v.cols, v.row_bytes, v.dtype = self.arena.buffer, self.offset + row_offset * rb, rows, cols, rb, self.dtype
-        return v
+        return abi.MatrixView(self.arena.buffer, self.offset + row_offset * rb, rows, cols, rb, self.dtype)
 
     def vv(self, start: int = 0, length: Optional[int] = None) -> abi.VectorView:
-        v = abi.VectorView()
-        v.buffer, v.offset = self.arena.buffer, self.offset + start * DTYPE_SIZE[self.dtype]
-        v.length, v.dtype = (self.count - start) if length is None else length, self.dtype
-        return v
+        return abi.VectorView(self.arena.buffer, self.offset + start * DTYPE_SIZE[self.dtype], self.count - start if length is None else length, self.dtype)
 
     def reshape(self, shape: Sequence[int]) -> "Tensor":
         t = Tensor(self.ctx, self.arena, self.offset, self.dtype, shape, self.name)
@@ -143,13 +154,13 @@ class Tensor:
         keep its contents until a fence recorded after this call has completed."""
         assert pinned.dtype == NP_DTYPES[self.dtype] and pinned.size == self.count and pinned.flags.c_contiguous
         self.ctx.check(self.ctx.lib.gdb200_upload_async(self.ctx.backend, self.buffer, self.offset,
-                                                        pinned.ctypes.data_as(C.c_void_p), pinned.nbytes), "upload_async")
+                                                        pinned.ctypes.data, pinned.nbytes), "upload_async")
 
     def read_async(self, pinned_out: np.ndarray) -> None:
         """Stream-ordered download into page-locked memory; valid once a later fence has completed."""
         assert pinned_out.dtype == NP_DTYPES[self.dtype] and pinned_out.size == self.count and pinned_out.flags.c_contiguous
         self.ctx.check(self.ctx.lib.gdb200_download_async(self.ctx.backend, self.buffer, self.offset,
-                                                          pinned_out.ctypes.data_as(C.c_void_p), pinned_out.nbytes), "download_async")
+                                                          pinned_out.ctypes.data, pinned_out.nbytes), "download_async")
 
     def read(self) -> np.ndarray:
         out = np.empty(self.shape, dtype=NP_DTYPES[self.dtype])
@@ -266,11 +277,9 @@ class Context:
 
     # ---- tensors ----
     def empty(self, arena: Arena, dtype: int, shape: Sequence[int], name: str = "") -> Tensor:
-        n = 1
-        for s in shape:
-            n *= int(s)
-        off = arena.alloc(max(n, 1) * DTYPE_SIZE[dtype])
-        return Tensor(self, arena, off, dtype, shape, name)
+        t = Tensor(self, arena, 0, dtype, shape, name)
+        t.offset = arena.alloc((t.count or 1) * DTYPE_SIZE[dtype])
+        return t
 
     def scratch_empty(self, dtype: int, shape: Sequence[int], name: str = "") -> Tensor:
         return self.empty(self.scratch, dtype, shape, name)
