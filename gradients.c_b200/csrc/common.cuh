@@ -332,6 +332,11 @@ gd_status gdb_embedding_dropout_rms_norm(gd_backend *be, const gd_backend_tensor
 gd_status gdb_lm_ce_count_valid(gd_backend *be, const gd_backend_tensor_view *targets, int32_t ignore_index, const gd_backend_tensor_view *counts);
 gd_status gdb_lm_ce_reduce_normalize_global(gd_backend *be, const gd_backend_tensor_view *row_loss, const gd_backend_tensor_view *counts,
                                             const gd_backend_tensor_view *loss, const gd_backend_tensor_view *inv_valid_count);
+// gdb200_lm_cross_entropy_fused_rows for up to 32768 classes.
+gd_status gdb_lm_ce_fused_rows(gd_backend *be, const gd_backend_tensor_view *logits, const gd_backend_tensor_view *bias,
+                               const gd_backend_tensor_view *targets, const gd_backend_tensor_view *grad_loss,
+                               const gd_backend_tensor_view *counts, const gd_backend_tensor_view *row_loss, float scale,
+                               float logits_softcap, int32_t ignore_index);
 gd_status gdb_rms_norm_backward_with_weight(gd_backend *be, const gd_backend_tensor_view *x, const gd_backend_tensor_view *weight,
                                             const gd_backend_tensor_view *inv_rms, const gd_backend_tensor_view *grad_out,
                                             const gd_backend_tensor_view *grad_x, bool add_to_dx, const gd_backend_tensor_view *grad_weight,

@@ -313,7 +313,6 @@ __global__ void lmce_backward_chunk_kernel(const T *logits, const T *bias, const
 // target only has its gradient cleared. A block walks over the rows with the grid's stride; the vectors of its next
 // row are already in flight while the current one is worked on, so the loads never wait for the arithmetic.
 constexpr int LMF_BLOCK = 256;
-constexpr int LMF_MAX_WPR = LMF_BLOCK / 32;
 // Vectors per thread. Measured on 18432 rows of 2048 classes: 4 (126 registers, 16 warps per SM) 60 us inside the train step,
 // 2 (80 registers, 24 warps) 63 us, 8 (one warp per row, 8 warps per SM) 28 us more than 4.
 constexpr int LMF_VECTORS = 4;
@@ -403,19 +402,26 @@ __device__ __forceinline__ void row_barrier(int id, int threads)
 }
 
 constexpr int LMF_NO_ROW = INT_MIN;   // target value standing for "no such row" in the row loop
+// Rows of more than LMF_BLOCK * LMF_VECTORS vectors (8192 classes) take blocks of LMF_BIG_BLOCK threads, up to 32768 classes. One such
+// block fills an SM's registers, so the next row waits in shared memory (cp.async, every thread reads back only what it copied)
+// instead of in registers. 9.7 k rows of 32768 classes: 3 special-function calls per class are 3.2 us of a row's time on an SM.
+constexpr int LMF_BIG_BLOCK = 1024;
 
-template <typename T, int NV, bool CAP>
-__global__ void __launch_bounds__(LMF_BLOCK, 2) lmce_fused_rows_kernel(T *logits, const T *bias, const int *targets,
+template <typename T, int NV, bool CAP, int BLOCK>
+__global__ void __launch_bounds__(BLOCK, BLOCK == LMF_BLOCK ? 2 : 1) lmce_fused_rows_kernel(T *logits, const T *bias, const int *targets,
                                                                                      const float *grad_loss, const float *counts, float *row_loss,
                                                                                      size_t rows, int nvec, int wpr, float scale, float cap,
                                                                                      float inv_cap, int ignore_index)
 {
     gdb_pdl_sync();
-    __shared__ float red[2][LMF_MAX_WPR][LMF_MAX_WPR];
-    __shared__ float target_soft[LMF_MAX_WPR];
+    constexpr bool STAGED = BLOCK != LMF_BLOCK;
+    constexpr int MAX_WPR = BLOCK / 32;
+    extern __shared__ uint4 staged[];                      // STAGED: two row sets of BLOCK * NV vectors
+    __shared__ float red[2][MAX_WPR][MAX_WPR];
+    __shared__ float target_soft[MAX_WPR];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rib = warp / wpr, wr = warp - rib * wpr;     // row within the block, warp within the row
-    const int rpb = (LMF_BLOCK / 32) / wpr;                // rows a block works on at a time
+    const int rpb = MAX_WPR / wpr;                         // rows a block works on at a time
     const int tpr = wpr * 32, tr = wr * 32 + lane;
     const size_t groups = (rows + (size_t)rpb - 1U) / (size_t)rpb;
     const uint4 *bv = reinterpret_cast<const uint4 *>(bias);
@@ -423,7 +429,7 @@ __global__ void __launch_bounds__(LMF_BLOCK, 2) lmce_fused_rows_kernel(T *logits
     const float seed = grad_loss[0] * scale * (valid > 0.0f ? 1.0f / valid : 0.0f);
 
     // the row's vectors of this thread and its target; a row without a usable target is not read
-    auto fetch = [&](size_t group, uint4 (&dst)[NV], int &t) {
+    auto fetch = [&](size_t group, uint4 (&dst)[NV], int &t, int set) {
         const size_t row = group * (size_t)rpb + (size_t)rib;
         t = (group < groups && row < rows) ? targets[row] : LMF_NO_ROW;
         const bool usable = t >= 0 && t != ignore_index && t < nvec * 8;
@@ -431,15 +437,24 @@ __global__ void __launch_bounds__(LMF_BLOCK, 2) lmce_fused_rows_kernel(T *logits
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int v = tr + i * tpr;
-            dst[i] = (usable && v < nvec) ? rv[v] : make_uint4(0U, 0U, 0U, 0U);
+            if (STAGED) {
+                if (usable && v < nvec) {
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(staged + (set * NV + i) * BLOCK + threadIdx.x)),
+                                 "l"(rv + v) : "memory");
+                }
+            } else {
+                dst[i] = (usable && v < nvec) ? rv[v] : make_uint4(0U, 0U, 0U, 0U);
+            }
         }
+        if (STAGED) asm volatile("cp.async.commit_group;" ::: "memory");
     };
 
     uint4 cur[NV], nxt[NV];
-    int t, t_next;
-    fetch(blockIdx.x, cur, t);
+    int t, t_next, set = 0;
+    fetch(blockIdx.x, cur, t, 0);
     for (size_t group = blockIdx.x; group < groups; group += gridDim.x) {
-        fetch(group + gridDim.x, nxt, t_next);             // in flight while this row is worked on
+        fetch(group + gridDim.x, nxt, t_next, set ^ 1);    // in flight while this row is worked on
+        if (STAGED) asm volatile("cp.async.wait_group 1;" ::: "memory");
         const size_t row = group * (size_t)rpb + (size_t)rib;
         uint4 *rv = reinterpret_cast<uint4 *>(logits) + row * (size_t)nvec;
         if (t == LMF_NO_ROW) {
@@ -466,7 +481,7 @@ __global__ void __launch_bounds__(LMF_BLOCK, 2) lmce_fused_rows_kernel(T *logits
             for (int i = 0; i < NV; ++i) {
                 const int v = tr + i * tpr;
                 if (v < nvec) {
-                    uint4 a = cur[i];
+                    uint4 a = STAGED ? staged[(set * NV + i) * BLOCK + threadIdx.x] : cur[i];
                     if (bv != nullptr) {
                         const uint4 b = bv[v];
                         a.x = pack2<T>::add(a.x, b.x);
@@ -575,8 +590,11 @@ __global__ void __launch_bounds__(LMF_BLOCK, 2) lmce_fused_rows_kernel(T *logits
                 __syncwarp();
             }
         }
+        if (!STAGED) {
 #pragma unroll
-        for (int i = 0; i < NV; ++i) cur[i] = nxt[i];
+            for (int i = 0; i < NV; ++i) cur[i] = nxt[i];
+        }
+        set ^= 1;
         t = t_next;
     }
 }
@@ -862,33 +880,41 @@ gd_status gd_backend_cross_entropy_backward_stats(gd_backend *be, const gd_backe
 }  // extern "C"
 
 namespace {
-template <typename T, int NV>
-void launch_fused_rows(gd_backend *be, unsigned groups, bool capped, void *lp, const void *bp, const int *tp, const float *gl, const float *cp,
-                       float *rl, size_t rows, int nvec, int wpr, float scale, float cap, float inv_cap, int ignore_index)
+template <typename T, int NV, bool CAP, int BLOCK>
+void launch_fused_rows(gd_backend *be, void *lp, const void *bp, const int *tp, const float *gl, const float *cp, float *rl, size_t rows, int nvec,
+                       float scale, float cap, float inv_cap, int ignore_index)
 {
-    // one wave of resident blocks, each walking over the row groups
-    static int per_sm[2] = {0, 0};
-    int &resident = per_sm[capped ? 1 : 0];
+    auto kern = lmce_fused_rows_kernel<T, NV, CAP, BLOCK>;
+    constexpr size_t smem = BLOCK == LMF_BLOCK ? 0U : (size_t)2 * BLOCK * NV * sizeof(uint4);
+    static int resident = 0;   // one wave of resident blocks, each walking over the row groups
     if (resident == 0) {
         int n = 0;
-        const cudaError_t e = capped ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, lmce_fused_rows_kernel<T, NV, true>, LMF_BLOCK, 0)
-                                     : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, lmce_fused_rows_kernel<T, NV, false>, LMF_BLOCK, 0);
+        cudaError_t e = smem > 0U ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : cudaSuccess;
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, BLOCK, smem);
         resident = (e == cudaSuccess && n > 0) ? n : 1;
     }
+    int wpr = 1;
+    while (wpr * 32 * NV < nvec) wpr <<= 1;
+    const unsigned rpb = (unsigned)((BLOCK / 32) / wpr), groups = (unsigned)((rows + rpb - 1U) / rpb);
     const unsigned wave = (unsigned)(be->sm_count > 0 ? be->sm_count : 1) * (unsigned)resident;
-    const unsigned grid = groups < wave ? groups : wave;
-    if (capped) {
-        gdb_launch(lmce_fused_rows_kernel<T, NV, true>, grid, LMF_BLOCK, 0, be->stream, (T *)lp, (const T *)bp, tp, gl, cp, rl, rows, nvec, wpr, scale, cap, inv_cap, ignore_index);
+    gdb_launch(kern, groups < wave ? groups : wave, BLOCK, smem, be->stream, (T *)lp, (const T *)bp, tp, gl, cp, rl, rows, nvec, wpr, scale, cap, inv_cap, ignore_index);
+}
+template <typename T, bool CAP>
+void launch_fused_rows_of(gd_backend *be, void *lp, const void *bp, const int *tp, const float *gl, const float *cp, float *rl, size_t rows, int nvec,
+                          float scale, float cap, float inv_cap, int ignore_index)
+{
+    if (nvec <= LMF_BLOCK * LMF_VECTORS) {
+        launch_fused_rows<T, LMF_VECTORS, CAP, LMF_BLOCK>(be, lp, bp, tp, gl, cp, rl, rows, nvec, scale, cap, inv_cap, ignore_index);
     } else {
-        gdb_launch(lmce_fused_rows_kernel<T, NV, false>, grid, LMF_BLOCK, 0, be->stream, (T *)lp, (const T *)bp, tp, gl, cp, rl, rows, nvec, wpr, scale, cap, inv_cap, ignore_index);
+        launch_fused_rows<T, LMF_VECTORS, CAP, LMF_BIG_BLOCK>(be, lp, bp, tp, gl, cp, rl, rows, nvec, scale, cap, inv_cap, ignore_index);
     }
 }
 }  // namespace
 
-extern "C" gd_status gdb200_lm_cross_entropy_fused_rows(gd_backend *be, const gd_backend_tensor_view *logits, const gd_backend_tensor_view *bias,
-                                                        const gd_backend_tensor_view *targets, const gd_backend_tensor_view *grad_loss,
-                                                        const gd_backend_tensor_view *counts, const gd_backend_tensor_view *row_loss, float scale,
-                                                        float logits_softcap, int32_t ignore_index)
+gd_status gdb_lm_ce_fused_rows(gd_backend *be, const gd_backend_tensor_view *logits, const gd_backend_tensor_view *bias,
+                               const gd_backend_tensor_view *targets, const gd_backend_tensor_view *grad_loss,
+                               const gd_backend_tensor_view *counts, const gd_backend_tensor_view *row_loss, float scale,
+                               float logits_softcap, int32_t ignore_index)
 {
     chunk_shape cs;
     if (be == NULL || logits == NULL || targets == NULL || grad_loss == NULL || counts == NULL || row_loss == NULL ||
@@ -913,26 +939,29 @@ extern "C" gd_status gdb200_lm_cross_entropy_fused_rows(gd_backend *be, const gd
     if (lp == NULL || tp == NULL || gl == NULL || cp == NULL || rl == NULL) {
         return GD_ERR_INVALID_ARGUMENT;
     }
-    // the whole row sits in the registers of at most 256 threads, LMF_VECTORS 16-byte vectors each; longer or unaligned rows
+    // the whole row sits in the registers of at most LMF_BIG_BLOCK threads, LMF_VECTORS 16-byte vectors each; longer or unaligned rows
     // take the three-entry path
-    if ((cs.classes % 8U) != 0U || (((uintptr_t)lp | (uintptr_t)bp) % 16U) != 0U || cs.classes / 8U > (size_t)(LMF_BLOCK * LMF_VECTORS)) {
+    if ((cs.classes % 8U) != 0U || (((uintptr_t)lp | (uintptr_t)bp) % 16U) != 0U || cs.classes / 8U > (size_t)(LMF_BIG_BLOCK * LMF_VECTORS)) {
         return GD_ERR_UNSUPPORTED;
     }
     const int nvec = (int)(cs.classes / 8U);
-    int wpr = 1;
-    while (wpr * 32 * LMF_VECTORS < nvec) {
-        wpr <<= 1;
-    }
-    const unsigned rpb = (unsigned)((LMF_BLOCK / 32) / wpr);
-    const unsigned groups = (unsigned)((cs.rows + rpb - 1U) / rpb);
     const float inv_cap = logits_softcap > 0.0f ? 1.0f / logits_softcap : 0.0f;
-    const bool capped = logits_softcap > 0.0f;
-    if (dt == GDB_DTYPE_F16) {
-        launch_fused_rows<__half, LMF_VECTORS>(be, groups, capped, lp, bp, tp, gl, cp, rl, cs.rows, nvec, wpr, scale, logits_softcap, inv_cap, (int)ignore_index);
-    } else {
-        launch_fused_rows<__nv_bfloat16, LMF_VECTORS>(be, groups, capped, lp, bp, tp, gl, cp, rl, cs.rows, nvec, wpr, scale, logits_softcap, inv_cap, (int)ignore_index);
-    }
+    auto launch = dt == GDB_DTYPE_F16 ? (logits_softcap > 0.0f ? launch_fused_rows_of<__half, true> : launch_fused_rows_of<__half, false>)
+                                      : (logits_softcap > 0.0f ? launch_fused_rows_of<__nv_bfloat16, true> : launch_fused_rows_of<__nv_bfloat16, false>);
+    launch(be, lp, bp, tp, gl, cp, rl, cs.rows, nvec, scale, logits_softcap, inv_cap, (int)ignore_index);
     return gdb_launched(be, "lm_cross_entropy_fused_rows");
+}
+
+// The additive entry takes up to 8192 classes, as it always has (its callers fall back to the chunked entries beyond).
+extern "C" gd_status gdb200_lm_cross_entropy_fused_rows(gd_backend *be, const gd_backend_tensor_view *logits, const gd_backend_tensor_view *bias,
+                                                        const gd_backend_tensor_view *targets, const gd_backend_tensor_view *grad_loss,
+                                                        const gd_backend_tensor_view *counts, const gd_backend_tensor_view *row_loss, float scale,
+                                                        float logits_softcap, int32_t ignore_index)
+{
+    if (logits != NULL && logits->rank == 2U && logits->shape[1] > (int64_t)LMF_BLOCK * LMF_VECTORS * 8) {
+        return GD_ERR_UNSUPPORTED;
+    }
+    return gdb_lm_ce_fused_rows(be, logits, bias, targets, grad_loss, counts, row_loss, scale, logits_softcap, ignore_index);
 }
 
 gd_status gdb_lm_ce_count_valid(gd_backend *be, const gd_backend_tensor_view *targets, int32_t ignore_index, const gd_backend_tensor_view *counts)
