@@ -457,6 +457,10 @@ __device__ __forceinline__ void decode_split_item(const T *q, const T *kc, const
             for (int c = 0; c < 16; ++c) qr[c] = gdb_io<T>::ld(q, qb + c) * p.scale;
 #pragma unroll 1
             for (int jb = s_lo; jb < s_hi; jb += TILE) {
+                if (DH == 64) {   // the tile after this one on its way to L2: a line of K or V per lane
+                    const int j = jb + TILE + (lane & 15);
+                    if (j < s_hi) asm volatile("prefetch.global.L2 [%0];" ::"l"((lane < 16 ? kc : vc) + (((size_t)b * p.tmax + (size_t)j) * p.hkv + hk) * DH));
+                }
                 uint4 k0[2], k1[2], v0[2], v1[2];
                 bool valid[2];
 #pragma unroll

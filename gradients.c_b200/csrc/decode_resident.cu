@@ -1,4 +1,4 @@
-// The greedy KV-cache decode of decode_mega.cu for at most 16 sequences and a model that fits the shared memory of the GPU:
+// The greedy KV-cache decode of decode_mega.cu for a model that fits the shared memory of the GPU:
 // ONE cooperative launch whose CTAs keep their share of all weights in shared memory for the whole run.
 //
 // What bounds a step of few sequences is the chain of its 5 L + 1 dependent phases, each an exchange of activations through L2.
@@ -18,6 +18,7 @@
 // Waits are bounded: a CTA that gives up stores code 398 in the backend's error word, raises the abort word and returns.
 #include "common.cuh"
 #include "decode_parts.cuh"
+#include "tcgen05.cuh"   // packed FP32 pairs
 
 #include <vector>
 #include <algorithm>
@@ -26,7 +27,8 @@ namespace {
 
 using namespace gdb_dec;
 
-constexpr int DR_THREADS = 512, DR_WARPS = 16, DR_ROWS = 16;
+constexpr int DR_THREADS = 512, DR_WARPS = 16;
+constexpr int DR_ROWS = 16, DR_MAX_ROWS = 64;   // rows of one pass over a phase's units, rows of a batch
 constexpr int DR_MAX_UNITS = 2048, DR_MAX_CTA_UNITS = 96, DR_MAX_PHASES = 4 * GDB_MEGA_MAX_LAYERS + 1;
 constexpr unsigned DR_SPIN_LIMIT = 1U << 22;
 constexpr int DR_ERR_BARRIER = 398;
@@ -55,7 +57,13 @@ __host__ __device__ inline uint32_t dr_phase_units(int kind, uint32_t D, uint32_
     return kind == DR_QKV ? 3U * D / 16U : (kind == DR_OUT || kind == DR_DOWN ? D / 16U : (kind == DR_UP ? F / 8U : V / 16U));
 }
 
+// A unit of this CTA: its weights' place in shared memory and its weight rows (dr_unit_rows).
+struct dr_unit {
+    uint32_t off, lo, hi;
+};
+
 struct dr_ctx {
+    const int *pos;   // positions of the batch at the first step
     unsigned char *sm;
     unsigned *sync;
     int *err_flag, *ok_flag;
@@ -130,21 +138,46 @@ __device__ __forceinline__ void dr_unit_rows(int kind, uint32_t unit, uint32_t D
 // byte offset of a 16-byte piece of the down projection's tile [F][16]: eight consecutive rows hit distinct banks
 __device__ __forceinline__ uint32_t dr_down_off(uint32_t k, uint32_t piece) { return k * 32U + ((piece ^ ((k >> 2) & 1U)) << 4); }
 
-// One projection phase (one body of code for all kinds: a step must not run through much more than the 32 KB instruction cache). GATHER: the normalised rows are the embedding rows of the current ids; otherwise rows of `x` ([B, K]).
+// The id row r is at: given for the first step, else the previous step's maximum.
+__device__ __forceinline__ int dr_current_id(const dr_args &g, int step, int r)
+{
+    return step == 0 ? g.a.tokens[r] : (int)(0xffffffffU - (unsigned)(__ldcg(&g.best[((step - 1) % 3) * DR_MAX_ROWS + r]) & 0xffffffffULL));
+}
+
+// A warp's accumulator tile (16 rows x 8 columns from column c0) of k range kslot, and the sum of the eight ranges in order.
+typedef float (*dr_red_t)[DR_ROWS][SK_COLS + 1];
+__device__ __forceinline__ void dr_store_partial(dr_red_t red, int kslot, int c0, const float (&acc)[4], int lane)
+{
+    const int gr = lane >> 2, cc = c0 + 2 * (lane & 3);
+    red[kslot][gr][cc] = acc[0];
+    red[kslot][gr][cc + 1] = acc[1];
+    red[kslot][gr + 8][cc] = acc[2];
+    red[kslot][gr + 8][cc + 1] = acc[3];
+}
+__device__ __forceinline__ float dr_sum(dr_red_t red, int r, int cc)
+{
+    float v = 0.0f;
+#pragma unroll
+    for (int w = 0; w < SK_WARPS; ++w) v += red[w][r][cc];
+    return v;
+}
+
+// One projection phase with K = D (one body of code for all kinds: a step must not run through much more than the 32 KB instruction
+// cache). GATHER: the normalised rows are the embedding rows of the current ids; otherwise rows of `x` ([B, K]). A pass takes 32
+// rows; its items, a unit and 16 of the rows each, go to the two gangs of eight warps (a CTA has one or two units in a phase).
+// The next pass's rows are read while this one is worked on.
 template <typename T>
-__device__ __forceinline__ bool dr_phase(const dr_ctx &c, const dr_args &g, const int KIND, const bool GATHER, const uint16_t *my_unit, const uint32_t *my_off, int n_my, int phase, int wait_idx,
+__device__ __forceinline__ bool dr_phase(const dr_ctx &c, const dr_args &g, const int KIND, const bool GATHER, const dr_unit *my, int n_my, int phase, int wait_idx,
                                          unsigned wait_target, int layer, int step, const T *x, const T *norm_w, T *out)
 {
     if (n_my == 0) return true;
-    const bool NORM = KIND == DR_QKV || KIND == DR_UP || KIND == DR_LM;
+    const bool NORM = KIND != DR_OUT;
     const gdb_mega_args &a = g.a;
-    const uint32_t D = (uint32_t)a.D, F = (uint32_t)a.F, H = (uint32_t)a.H, K = KIND == DR_DOWN ? F : D, LDA = K + 8U;
-    const uint32_t CH = KIND == DR_DOWN ? ((F % 512U) == 0U ? 512U : ((F % 256U) == 0U ? 256U : 128U)) : D, kw = CH / SK_WARPS;
+    const uint32_t D = (uint32_t)a.D, F = (uint32_t)a.F, LDA = D + 8U, kw = D / SK_WARPS;
+    const float inv_d = 1.0f / (float)(int)D;   // exact: D is a power of two
     const int B = a.B, gang = c.warp >> 3, kslot = c.warp & 7, gt = c.tid & 255;
     T *As = reinterpret_cast<T *>(c.sm + g.work_off);
-    const uint32_t a_bytes = DR_ROWS * LDA * 2U;
-    const bool alias = KIND == DR_DOWN;                       // the down projection's long rows leave no room beside them
-    float(*red)[DR_ROWS][SK_COLS + 1] = reinterpret_cast<float(*)[DR_ROWS][SK_COLS + 1]>(c.sm + g.work_off + (alias ? 0U : a_bytes) + (uint32_t)gang * DR_RED_BYTES);
+    dr_red_t red = reinterpret_cast<dr_red_t>(c.sm + g.work_off + (B > DR_ROWS ? 2U : 1U) * DR_ROWS * LDA * 2U + (uint32_t)gang * DR_RED_BYTES);
 
     // ---- what does not depend on the previous phase ----
     uint4 wraw[2] = {make_uint4(0U, 0U, 0U, 0U), make_uint4(0U, 0U, 0U, 0U)};
@@ -156,204 +189,275 @@ __device__ __forceinline__ bool dr_phase(const dr_ctx &c, const dr_args &g, cons
             if (v < vecs) wraw[i] = __ldg(reinterpret_cast<const uint4 *>(norm_w) + v);
         }
     }
-    float cs = 1.0f, sn = 0.0f;
-    if (KIND == DR_QKV && gang < n_my && gt < DR_ROWS * 8) {
-        const uint32_t unit = my_unit[gang];
-        const int r = gt >> 3, e = gt & 7;
-        if (r < B && unit < 8U * H) rope_cos_sin(a.rope, a.rope_table, (unit & 3U) * 8U + (unsigned)e, a.positions[r] + step, &cs, &sn);
-    }
     if (!dr_wait(c, wait_idx, wait_target)) return false;
-
-    auto current_id = [&](int r) -> int {   // the id row r is at: given for the first step, else the previous step's maximum
-        return step == 0 ? a.tokens[r] : (int)(0xffffffffU - (unsigned)(__ldcg(&g.best[((step - 1) % 3) * DR_ROWS + r]) & 0xffffffffULL));
-    };
-    if (GATHER && my_unit[0] == 0U && c.tid < DR_ROWS && c.tid < B && step > 0) {
+    if (GATHER && my[0].lo == 0U && c.tid < B && step > 0) {
         // the CTA of the first unit records the previous step's ids and clears the maxima that the next step will use
         const int t = *a.step_counter + step - 1;
-        if (t >= 0 && t < a.max_steps) a.out_tokens[(size_t)t * B + c.tid] = current_id(c.tid);
-        g.best[((step + 1) % 3) * DR_ROWS + c.tid] = 0ULL;
+        if (t >= 0 && t < a.max_steps) a.out_tokens[(size_t)t * B + c.tid] = dr_current_id(g, step, c.tid);
+        g.best[((step + 1) % 3) * DR_MAX_ROWS + c.tid] = 0ULL;
     }
 
-#pragma unroll 1
-    for (int it = 0; it < n_my; it += 2) {
-        const int mine = it + gang;
-        const bool have = mine < n_my;
-        const uint32_t unit = have ? my_unit[mine] : 0U;
-        const T *Ws = reinterpret_cast<const T *>(c.sm + (have ? my_off[mine] : 0U));
-        const T *bias = reinterpret_cast<const T *>(c.sm + (have ? my_off[mine] : 0U) + dr_unit_bytes(KIND, D, F) - 32U);
-        uint32_t lo, hi;
-        dr_unit_rows(KIND, unit, D, F, H, &lo, &hi);
-        float res = 0.0f;
-        const int r0 = gt >> 4, c0 = gt & 15;
-        if ((KIND == DR_OUT || KIND == DR_DOWN) && have && r0 < B) {
-            // residual operand of this thread's output: the block's input (layer 0: the embedding row) or the attention branch's sum
-            const T *src = (const T *)(KIND == DR_DOWN ? a.resid : a.xbuf);
-            size_t row = (size_t)r0;
-            bool nan_row = false;
-            if (KIND == DR_OUT && layer == 0) {
-                const int id = current_id(r0);
-                nan_row = id < 0 || id >= a.V;
-                src = (const T *)a.emb;
-                row = nan_row ? 0U : (size_t)id;
-            }
-            const unsigned short bits = __ldcg(reinterpret_cast<const unsigned short *>(src) + row * D + lo + c0);
-            res = nan_row ? __int_as_float(0x7fc00000) : gdb_io<T>::up(bits);
-        }
-        if (NORM && it == 0) {
-            // one warp per row: mean square over the lane's vectors lane, lane + 32, then round(x * w * rsqrt)
-            const int r = c.warp;
-            if (r < B) {
-                const T *row = x + (size_t)r * D;
-                bool nan_row = false;
-                if (GATHER) {
-                    const int id = current_id(r);
-                    nan_row = id < 0 || id >= a.V;
-                    row = x + (size_t)(nan_row ? 0 : id) * D;
-                }
-                uint4 raw[2];
-                float ss = 0.0f;
+    // Rows of the pass that begins at row base: a normalised row is read to registers (a warp has rows warp, warp + 16), other rows
+    // are copied to As.
+    uint4 raw[2][2];
+    bool nan_row[2];
+    auto fetch = [&](int base) {
+        if (NORM) {
 #pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const int v = c.lane + 32 * i;
-                    raw[i] = make_uint4(0U, 0U, 0U, 0U);
-                    if (v < vecs) raw[i] = __ldcg(reinterpret_cast<const uint4 *>(row) + v);
-                }
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    if (c.lane + 32 * i < vecs) {
-                        float f[8];
-                        unpack8<T>(raw[i], f);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) ss += f[e] * f[e];
+            for (int q = 0; q < 2; ++q) {
+                const int r = base + c.warp + q * DR_ROWS;
+                nan_row[q] = false;
+                if (r < B) {
+                    const T *row = x + (size_t)r * D;
+                    if (GATHER) {
+                        const int id = dr_current_id(g, step, r);
+                        nan_row[q] = id < 0 || id >= a.V;
+                        row = x + (size_t)(nan_row[q] ? 0 : id) * D;
                     }
-                }
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffU, ss, o);
-                const float inv = nan_row ? __int_as_float(0x7fc00000) : rsqrtf(ss / (float)(size_t)D + a.eps);
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const int v = c.lane + 32 * i;
-                    if (v < vecs) {
-                        float f[8], w[8];
-                        unpack8<T>(raw[i], f);
-                        unpack8<T>(wraw[i], w);
-                        uint4 o;
-                        o.x = pack2<T>::down(f[0] * w[0] * inv, f[1] * w[1] * inv);
-                        o.y = pack2<T>::down(f[2] * w[2] * inv, f[3] * w[3] * inv);
-                        o.z = pack2<T>::down(f[4] * w[4] * inv, f[5] * w[5] * inv);
-                        o.w = pack2<T>::down(f[6] * w[6] * inv, f[7] * w[7] * inv);
-                        *reinterpret_cast<uint4 *>(As + (size_t)r * LDA + v * 8) = o;
+                    for (int i = 0; i < 2; ++i) {
+                        const int v = c.lane + 32 * i;
+                        raw[q][i] = make_uint4(0U, 0U, 0U, 0U);
+                        if (v < vecs) raw[q][i] = __ldcg(reinterpret_cast<const uint4 *>(row) + v);
                     }
                 }
             }
-            __syncthreads();
-        } else if (!NORM && (it == 0 || alias)) {
-            const uint32_t segs = K / 8U;
+        } else {
+            const uint32_t segs = D / 8U, n = (uint32_t)min(B - base, 2 * DR_ROWS);
             uint32_t r = 0U, sg = (uint32_t)c.tid;
 #pragma unroll 1
             for (;;) {
 #pragma unroll 1
                 for (; sg >= segs; sg -= segs) ++r;
-                if (r >= (uint32_t)B) break;
-                sk_cp16(As + r * LDA + sg * 8U, x + (size_t)r * K + sg * 8U, true);
+                if (r >= n) break;
+                sk_cp16(As + r * LDA + sg * 8U, x + (size_t)(base + (int)r) * D + sg * 8U, true);
                 sg += DR_THREADS;
             }
-            asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
-            __syncthreads();
+            asm volatile("cp.async.commit_group;" ::: "memory");
         }
-        float acc[2][4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[0][e] = acc[1][e] = 0.0f;
-        if (have) {
+    };
+    fetch(0);
 #pragma unroll 1
-            for (uint32_t k0 = (uint32_t)kslot * kw; k0 < K; k0 += CH) {
-#pragma unroll 4
-                for (uint32_t k = k0; k < k0 + kw; k += 16U) {
-                    uint32_t av[4], b4[4];
-                    sk_ldm4(av, As + (c.lane & 15) * LDA + k + (c.lane >> 4) * 8);
-                    if (KIND == DR_DOWN) {
-                        sk_ldm4t(b4, reinterpret_cast<const unsigned char *>(Ws) + dr_down_off(k + (uint32_t)(c.lane & 15), (uint32_t)c.lane >> 4));
-                    } else {
-                        sk_ldm4(b4, Ws + ((c.lane & 7) + ((c.lane >> 4) << 3)) * LDA + k + ((c.lane >> 3) & 1) * 8);
+    for (int base = 0; base < B; base += 2 * DR_ROWS) {
+        const int rows = min(B - base, 2 * DR_ROWS), items = rows > DR_ROWS ? 2 * n_my : n_my;
+        const bool more = base + 2 * DR_ROWS < B;
+        if (NORM) {
+            // mean square over the lane's vectors lane, lane + 32, then round(x * w * rsqrt)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                if (c.warp + q * DR_ROWS < rows) {
+                    float ss = 0.0f;
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        if (c.lane + 32 * i < vecs) {
+                            float f[8];
+                            unpack8<T>(raw[q][i], f);
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) ss += f[e] * f[e];
+                        }
                     }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffU, ss, o);
+                    const float inv = nan_row[q] ? __int_as_float(0x7fc00000) : rsqrtf(ss * inv_d + a.eps);
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const int v = c.lane + 32 * i;
+                        if (v < vecs) {
+                            const uint32_t xr[4] = {raw[q][i].x, raw[q][i].y, raw[q][i].z, raw[q][i].w}, wr[4] = {wraw[i].x, wraw[i].y, wraw[i].z, wraw[i].w};
+                            uint32_t ow[4];
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const float2 xf = pack2<T>::up(xr[e]), wf = pack2<T>::up(wr[e]);
+                                float y0, y1;
+                                gdb_t5::f2_split(gdb_t5::f2_mul(gdb_t5::f2_mul(gdb_t5::f2_make(xf.x, xf.y), gdb_t5::f2_make(wf.x, wf.y)), gdb_t5::f2_make(inv, inv)), y0, y1);
+                                ow[e] = pack2<T>::down(y0, y1);
+                            }
+                            const uint4 o = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+                            *reinterpret_cast<uint4 *>(As + (size_t)(c.warp + q * DR_ROWS) * LDA + v * 8) = o;
+                        }
+                    }
+                }
+            }
+            if (more) fetch(base + 2 * DR_ROWS);
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int it = 0; it < items; it += 2) {
+            const int item = it + gang;
+            const bool have = item < items;
+            const int mine = !have ? 0 : (rows > DR_ROWS ? item >> 1 : item), tile = have && rows > DR_ROWS ? (item & 1) * DR_ROWS : 0;
+            const int row0 = base + tile, n_rows = rows - tile;      // rows of the batch from row0 on; at most 16 count here
+            const uint32_t off = my[mine].off, lo = my[mine].lo;
+            const bool rotated = lo < 2U * D;   // (QKV) 8 rotation pairs of one head, otherwise 16 value columns
+            const T *Ws = reinterpret_cast<const T *>(c.sm + off);
+            const T *bias = reinterpret_cast<const T *>(c.sm + off + dr_unit_bytes(KIND, D, F) - 32U);
+            const int r0 = gt >> 4, c0 = gt & 15, r8 = gt >> 3, e8 = gt & 7;
+            float res = 0.0f;
+            if (KIND == DR_OUT && have && r0 < n_rows) {
+                // residual operand of this thread's output: the block's input (layer 0: the embedding row)
+                const T *src = (const T *)a.xbuf;
+                size_t row = (size_t)(row0 + r0);
+                bool nan_res = false;
+                if (layer == 0) {
+                    const int id = dr_current_id(g, step, row0 + r0);
+                    nan_res = id < 0 || id >= a.V;
+                    src = (const T *)a.emb;
+                    row = nan_res ? 0U : (size_t)id;
+                }
+                const unsigned short bits = __ldcg(reinterpret_cast<const unsigned short *>(src) + row * D + lo + c0);
+                res = nan_res ? __int_as_float(0x7fc00000) : gdb_io<T>::up(bits);
+            }
+            // (QKV) position and, from the table, cos / sin of this thread's pair: on their way during the products
+            const int pos = KIND == DR_QKV && have ? c.pos[min(row0 + (rotated ? r8 & 15 : r0), B - 1)] + step : 0;
+            const unsigned pair = ((lo >> 3) & 3U) * 8U + (unsigned)e8;
+            const bool tabled = KIND == DR_QKV && rotated && a.rope.use_table && pos >= 0 && (unsigned)pos < TABLE_POSITIONS;
+            float2 trig = make_float2(1.0f, 0.0f);
+            if (tabled) trig = __ldg(reinterpret_cast<const float2 *>(a.rope_table) + (size_t)pos * TABLE_PAIRS + pair);
+            float acc[2][4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[0][e] = acc[1][e] = 0.0f;
+            if (have) {
+                const T *at = As + (tile + (c.lane & 15)) * LDA + (c.lane >> 4) * 8;
+                const T *wt = Ws + ((c.lane & 7) + ((c.lane >> 4) << 3)) * LDA + ((c.lane >> 3) & 1) * 8;
+#pragma unroll 4
+                for (uint32_t k = (uint32_t)kslot * kw; k < (uint32_t)(kslot + 1) * kw; k += 16U) {
+                    uint32_t av[4], b4[4];
+                    sk_ldm4(av, at + k);
+                    sk_ldm4(b4, wt + k);
                     const uint32_t b0[2] = {b4[0], b4[1]}, b1[2] = {b4[2], b4[3]};
                     mma16816<T>::run(acc[0], av, b0);
                     mma16816<T>::run(acc[1], av, b1);
                 }
+                dr_store_partial(red, kslot, 0, acc[0], c.lane);
+                dr_store_partial(red, kslot, 8, acc[1], c.lane);
             }
-        }
-        if (alias) __syncthreads();
-        if (have) {
-            const int gr = c.lane >> 2, tc = c.lane & 3;
+            __syncthreads();
+            if (!NORM && more && it + 2 >= items) fetch(base + 2 * DR_ROWS);   // every warp is done with As
+            if (have) {
+                if (KIND == DR_UP) {
+                    if (gt < DR_ROWS * 8 && r8 < n_rows) {
+                        gdb_io<T>::st(out, (size_t)(row0 + r8) * F + lo + e8, sk_swiglu<T>(dr_sum(red, r8, e8), dr_sum(red, r8, e8 + 8), bias, 2, (uint32_t)e8, (uint32_t)e8 + 8U));
+                    }
+                } else if (KIND == DR_OUT) {
+                    if (r0 < n_rows) {
+                        const float y = gdb_io<T>::rnd(sk_bias<T>(dr_sum(red, r0, c0), bias, 2, (uint32_t)c0));
+                        gdb_io<T>::st(out, (size_t)(row0 + r0) * D + lo + c0, res + y);
+                    }
+                } else if (KIND == DR_LM) {
+                    // soft cap, non-finite -> -inf, maximum of the unit's 16 classes (the first of equal ones)
+                    unsigned long long key = 0ULL;
+                    if (r0 < n_rows) {
+                        float v = gdb_io<T>::rnd(sk_bias<T>(dr_sum(red, r0, c0), bias, 2, (uint32_t)c0));
+                        if (a.softcap > 0.0f) v = a.softcap * tanhf(v / a.softcap);
+                        if (!isfinite(v)) v = -INFINITY;
+                        if (v == 0.0f) v = 0.0f;   // -0 and +0 are equal
+                        key = ((unsigned long long)dr_order(v) << 32) | (unsigned long long)(0xffffffffU - (lo + (uint32_t)c0));
+                    }
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
-                red[kslot][gr][nt * 8 + 2 * tc] = acc[nt][0];
-                red[kslot][gr][nt * 8 + 2 * tc + 1] = acc[nt][1];
-                red[kslot][gr + 8][nt * 8 + 2 * tc] = acc[nt][2];
-                red[kslot][gr + 8][nt * 8 + 2 * tc + 1] = acc[nt][3];
-            }
-        }
-        __syncthreads();
-        auto sum = [&](int r, int cc) {
-            float v = 0.0f;
-#pragma unroll
-            for (int w = 0; w < SK_WARPS; ++w) v += red[w][r][cc];
-            return v;
-        };
-        if (have) {
-            if (KIND == DR_UP) {
-                const int r = gt >> 3, cc = gt & 7;
-                if (gt < DR_ROWS * 8 && r < B) {
-                    gdb_io<T>::st(out, (size_t)r * F + lo + cc, sk_swiglu<T>(sum(r, cc), sum(r, cc + 8), bias, 2, (uint32_t)cc, (uint32_t)cc + 8U));
-                }
-            } else if (KIND == DR_OUT || KIND == DR_DOWN) {
-                if (r0 < B) {
-                    const float y = gdb_io<T>::rnd(sk_bias<T>(sum(r0, c0), bias, KIND == DR_OUT ? 2 : 1, (uint32_t)c0));
-                    gdb_io<T>::st(out, (size_t)r0 * D + lo + c0, res + y);
-                }
-            } else if (KIND == DR_LM) {
-                // soft cap, non-finite -> -inf, maximum of the unit's 16 classes (the first of equal ones)
-                unsigned long long key = 0ULL;
-                if (r0 < B) {
-                    float v = gdb_io<T>::rnd(sk_bias<T>(sum(r0, c0), bias, 2, (uint32_t)c0));
-                    if (a.softcap > 0.0f) v = a.softcap * tanhf(v / a.softcap);
-                    if (!isfinite(v)) v = -INFINITY;
-                    if (v == 0.0f) v = 0.0f;   // -0 and +0 are equal
-                    key = ((unsigned long long)dr_order(v) << 32) | (unsigned long long)(0xffffffffU - (lo + (uint32_t)c0));
-                }
-#pragma unroll
-                for (int o = 8; o > 0; o >>= 1) {
-                    const unsigned long long other = __shfl_xor_sync(0xffffffffU, key, o);
-                    key = other > key ? other : key;
-                }
-                if (r0 < B && c0 == 0) atomicMax(&g.best[(step % 3) * DR_ROWS + r0], key);
-            } else {
-                const uint32_t nrope = 8U * H;
-                if (unit < nrope) {
-                    const int r = gt >> 3, e = gt & 7;
-                    if (gt < DR_ROWS * 8 && r < B) {
-                        const int pos = a.positions[r] + step;
-                        const uint32_t region = unit / (H * 4U), hg = unit % (H * 4U), hcol = (hg / 4U) * 64U + (hg % 4U) * 8U;
-                        if (it > 0) rope_cos_sin(a.rope, a.rope_table, (hg % 4U) * 8U + (unsigned)e, pos, &cs, &sn);
-                        const float x0 = gdb_io<T>::rnd(sk_bias<T>(sum(r, e), bias, 2, (uint32_t)e)), x1 = gdb_io<T>::rnd(sk_bias<T>(sum(r, e + 8), bias, 2, (uint32_t)e + 8U));
+                    for (int o = 8; o > 0; o >>= 1) {
+                        const unsigned long long other = __shfl_xor_sync(0xffffffffU, key, o);
+                        key = other > key ? other : key;
+                    }
+                    if (r0 < n_rows && c0 == 0) atomicMax(&g.best[(step % 3) * DR_MAX_ROWS + row0 + r0], key);
+                } else if (rotated) {
+                    if (gt < DR_ROWS * 8 && r8 < n_rows) {
+                        const uint32_t region = lo >= D ? 1U : 0U, hcol = lo - region * D;
+                        float cs = trig.x, sn = trig.y * a.rope.sin_sign;
+                        if (!tabled) rope_cos_sin(a.rope, a.rope_table, pair, pos, &cs, &sn);
+                        const float x0 = gdb_io<T>::rnd(sk_bias<T>(dr_sum(red, r8, e8), bias, 2, (uint32_t)e8)), x1 = gdb_io<T>::rnd(sk_bias<T>(dr_sum(red, r8, e8 + 8), bias, 2, (uint32_t)e8 + 8U));
                         const float y0 = rope_lo(x0, x1, cs, sn), y1 = rope_hi(x0, x1, cs, sn);
                         if (region == 0U) {
-                            gdb_io<T>::st((T *)a.q, (size_t)r * D + hcol + e, y0);
-                            gdb_io<T>::st((T *)a.q, (size_t)r * D + hcol + 32U + e, y1);
+                            gdb_io<T>::st((T *)a.q, (size_t)(row0 + r8) * D + hcol + e8, y0);
+                            gdb_io<T>::st((T *)a.q, (size_t)(row0 + r8) * D + hcol + 32U + e8, y1);
                         } else if (pos >= 0 && pos < a.CAP) {
-                            const size_t kv = ((size_t)r * a.CAP + (size_t)pos) * D + hcol + e;
+                            const size_t kv = ((size_t)(row0 + r8) * a.CAP + (size_t)pos) * D + hcol + e8;
                             gdb_io<T>::st((T *)a.kc[layer], kv, y0);
                             gdb_io<T>::st((T *)a.kc[layer], kv + 32U, y1);
                         }
                     }
-                } else if (r0 < B) {
-                    const int pos = a.positions[r0] + step;
-                    const float y = gdb_io<T>::rnd(sk_bias<T>(sum(r0, c0), bias, 2, (uint32_t)c0));
-                    if (pos >= 0 && pos < a.CAP) gdb_io<T>::st((T *)a.vc[layer], ((size_t)r0 * a.CAP + (size_t)pos) * D + (lo - 2U * D) + c0, y);
+                } else if (r0 < n_rows) {
+                    const float y = gdb_io<T>::rnd(sk_bias<T>(dr_sum(red, r0, c0), bias, 2, (uint32_t)c0));
+                    if (pos >= 0 && pos < a.CAP) gdb_io<T>::st((T *)a.vc[layer], ((size_t)(row0 + r0) * a.CAP + (size_t)pos) * D + (lo - 2U * D) + c0, y);
                 }
             }
+            if (it + 2 < items || more) __syncthreads();   // the partial sums are reused by the next items
         }
-        if (it + 2 < n_my) __syncthreads();   // the partial sums (and an aliased A tile) are reused by the next pair of units
+    }
+    dr_arrive(c, phase);
+    return true;
+}
+
+// The down projection (K = F, rows of act): 16 rows x one chunk of k at a time through a ring of three stages. Its units are few, so
+// the two gangs share one: each forms eight of its columns.
+template <typename T>
+__device__ __forceinline__ bool dr_down(const dr_ctx &c, const dr_args &g, const dr_unit *my, int n_my, int phase, int wait_idx, unsigned wait_target)
+{
+    if (n_my == 0) return true;
+    const gdb_mega_args &a = g.a;
+    const uint32_t D = (uint32_t)a.D, F = (uint32_t)a.F, CH = (F % 512U) == 0U ? 512U : ((F % 256U) == 0U ? 256U : 128U), LDA = CH + 8U, kw = CH / SK_WARPS, segs = CH / 8U;
+    const int B = a.B, gang = c.warp >> 3, kslot = c.warp & 7, n_chunks = (int)(F / CH), stages = (B + DR_ROWS - 1) / DR_ROWS * n_chunks;
+    const uint32_t stage_elems = DR_ROWS * LDA;
+    T *As = reinterpret_cast<T *>(c.sm + g.work_off);
+    dr_red_t red = reinterpret_cast<dr_red_t>(c.sm + g.work_off + 3U * stage_elems * 2U);
+    const int r0 = c.tid >> 4, c0 = c.tid & 15;
+    if (!dr_wait(c, wait_idx, wait_target)) return false;
+#pragma unroll 1
+    for (int u = 0; u < n_my; ++u) {
+        const uint32_t lo = my[u].lo;
+        const unsigned char *Ws = c.sm + my[u].off;
+        const T *bias = reinterpret_cast<const T *>(c.sm + my[u].off + dr_unit_bytes(DR_DOWN, D, F) - 32U);
+        int i_base = 0, i_chunk = 0, i_slot = 0;     // the next stage to be copied
+        auto issue = [&]() {
+            const uint32_t n = (uint32_t)max(0, min(B - i_base, DR_ROWS));
+            uint32_t r = (uint32_t)c.tid / segs, sg = (uint32_t)c.tid % segs;
+            const uint32_t dr = DR_THREADS / segs;   // segs is 16, 32 or 64
+#pragma unroll 1
+            for (; r < n; r += dr) sk_cp16(As + (uint32_t)i_slot * stage_elems + r * LDA + sg * 8U, (const T *)a.act + (size_t)(i_base + (int)r) * F + (uint32_t)i_chunk * CH + sg * 8U, true);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            i_slot = i_slot == 2 ? 0 : i_slot + 1;
+            if (++i_chunk == n_chunks) {
+                i_chunk = 0;
+                i_base += DR_ROWS;
+            }
+        };
+        issue();
+        issue();
+        float acc[4], res = 0.0f;
+        int chunk = 0, base = 0, slot = 0;
+#pragma unroll 1
+        for (int s = 0; s < stages; ++s) {
+            if (chunk == 0) {
+                acc[0] = acc[1] = acc[2] = acc[3] = 0.0f;
+                if (c.tid < 256 && base + r0 < B) res = gdb_io<T>::up(__ldcg(reinterpret_cast<const unsigned short *>(a.resid) + (size_t)(base + r0) * D + lo + c0));
+            }
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads();   // the stage has landed for every thread, and the one before it has been read
+            issue();
+            const T *at = As + (uint32_t)slot * stage_elems + (c.lane & 15) * LDA + (c.lane >> 4) * 8;
+            const uint32_t wk = (uint32_t)chunk * CH;
+#pragma unroll 4
+            for (uint32_t k = (uint32_t)kslot * kw; k < (uint32_t)(kslot + 1) * kw; k += 16U) {
+                uint32_t av[4], b[2];
+                sk_ldm4(av, at + k);
+                asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(b[0]), "=r"(b[1]) : "r"(sk_smem(Ws + dr_down_off(wk + k + (uint32_t)(c.lane & 15), (uint32_t)gang))));
+                mma16816<T>::run(acc, av, b);
+            }
+            slot = slot == 2 ? 0 : slot + 1;
+            if (++chunk == n_chunks) {
+                dr_store_partial(red, kslot, gang * 8, acc, c.lane);
+                __syncthreads();
+                if (c.tid < 256 && base + r0 < B) {
+                    const float y = gdb_io<T>::rnd(sk_bias<T>(dr_sum(red, r0, c0), bias, 1, (uint32_t)c0));
+                    gdb_io<T>::st((T *)a.xbuf, (size_t)(base + r0) * D + lo + c0, res + y);
+                }
+                chunk = 0;
+                base += DR_ROWS;
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
     }
     dr_arrive(c, phase);
     return true;
@@ -364,11 +468,12 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decode_resident_kernel(const __
 {
     extern __shared__ __align__(16) unsigned char dr_sm[];
     __shared__ int ok_flag;
-    __shared__ uint16_t my_unit[DR_MAX_CTA_UNITS];
-    __shared__ uint32_t my_off[DR_MAX_CTA_UNITS];
+    __shared__ dr_unit my[DR_MAX_CTA_UNITS];
+    __shared__ int positions[DR_MAX_ROWS];
     __shared__ uint16_t first[DR_MAX_PHASES + 1];
     const gdb_mega_args &a = g.a;
     dr_ctx c;
+    c.pos = positions;
     c.sm = dr_sm;
     c.sync = a.sync;
     c.err_flag = a.err_flag;
@@ -380,6 +485,7 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decode_resident_kernel(const __
     const int L = a.L, n_phases = 4 * L + 1;
 
     // ---- this CTA's units, in phase order, and their weights ----
+    if (c.tid < a.B) positions[c.tid] = a.positions[c.tid];
     if (c.warp == 0) {
         int n = 0;
         uint32_t off = 0U;
@@ -394,8 +500,10 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decode_resident_kernel(const __
                 const unsigned mask = __ballot_sync(0xffffffffU, mine);
                 const int rank = __popc(mask & ((1U << c.lane) - 1U));
                 if (mine && n + rank < DR_MAX_CTA_UNITS) {
-                    my_unit[n + rank] = (uint16_t)(u - g.phase_unit[ph]);
-                    my_off[n + rank] = off + (uint32_t)rank * bytes;
+                    dr_unit d;
+                    d.off = off + (uint32_t)rank * bytes;
+                    dr_unit_rows(ph == 4 * L ? (int)DR_LM : (ph & 3), u - g.phase_unit[ph], D, F, H, &d.lo, &d.hi);
+                    my[n + rank] = d;
                 }
                 n += __popc(mask);
                 off += (uint32_t)__popc(mask) * bytes;
@@ -412,9 +520,8 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decode_resident_kernel(const __
         const T *bias = (const T *)(kind == DR_LM ? a.b_lm : lw[kind == DR_QKV ? 2 : (kind == DR_OUT ? 4 : (kind == DR_UP ? 7 : 9))]);
 #pragma unroll 1
         for (int i = first[ph]; i < first[ph + 1]; ++i) {
-            uint32_t lo, hi;
-            dr_unit_rows(kind, my_unit[i], D, F, H, &lo, &hi);
-            unsigned char *dst = dr_sm + my_off[i];
+            const uint32_t lo = my[i].lo, hi = my[i].hi;
+            unsigned char *dst = dr_sm + my[i].off;
             if (kind == DR_DOWN) {
 #pragma unroll 1
                 for (uint32_t j = (uint32_t)c.tid; j < F * 2U; j += DR_THREADS) sk_cp16(dst + dr_down_off(j >> 1, j & 1U), w + (size_t)(j >> 1) * D + lo + (j & 1U) * 8U, true);
@@ -461,7 +568,7 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decode_resident_kernel(const __
 #pragma unroll 1
                 for (int unit = blockIdx.x; unit < attn_units; unit += gridDim.x) {
                     const int b = unit / groups, h0 = (unit - b * groups) * hpc, hl = c.warp % hpc, split = c.warp / hpc, item = hl * a.splits + split;
-                    dp.cache_pos = a.positions[b] + step;
+                    dp.cache_pos = positions[b] + step;
                     if (split < a.splits) {
                         decode_split_item<T, 64, false>((const T *)a.q, (const T *)a.kc[layer], (const T *)a.vc[layer], nullptr, sm_ml + item * 2, sm_acc + item * 64, dp,
                                                         a.splits, (long long)b * a.H + h0 + hl, split, c.lane);
@@ -493,17 +600,21 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decode_resident_kernel(const __
             // the counter of the phase in front: the attention for OUT, the previous step's last phase for the first
             const int wait_idx = i == 0 ? 5 * L : i - 1;
             const unsigned wait_n = kind == DR_OUT ? attn_workers : (unsigned)g.workers[i == 0 ? 4 * L : ph - 1], wait_rounds = i == 0 ? (unsigned)step : round;
-            const void *src = kind == DR_OUT ? a.attn : (kind == DR_UP ? a.resid : (kind == DR_DOWN ? a.act : (i == 0 ? a.emb : a.xbuf)));
-            void *dst = kind == DR_OUT ? a.resid : (kind == DR_UP ? a.act : a.xbuf);
+            if (kind == DR_DOWN) {
+                if (!dr_down<T>(c, g, my + first[ph], units_of(ph), i, wait_idx, wait_n * wait_rounds)) return;
+                continue;
+            }
+            const void *src = kind == DR_OUT ? a.attn : (kind == DR_UP ? a.resid : (i == 0 ? a.emb : a.xbuf));
+            void *dst = kind == DR_OUT ? a.resid : a.act;
             const void *nw = kind == DR_LM ? a.w_final : a.lw[layer < L ? layer : 0][kind == DR_UP ? 5 : 0];
-            if (!dr_phase<T>(c, g, kind, i == 0, my_unit + first[ph], my_off + first[ph], units_of(ph), i, wait_idx, wait_n * wait_rounds, layer, step, (const T *)src,
+            if (!dr_phase<T>(c, g, kind, i == 0, my + first[ph], units_of(ph), i, wait_idx, wait_n * wait_rounds, layer, step, (const T *)src,
                              (const T *)nw, (T *)dst)) return;
         }
     }
     if (blockIdx.x == 0) {
         if (!dr_wait(c, 5 * L, g.workers[4 * L] * (unsigned)a.n_steps)) return;
         if (c.tid < a.B) {
-            const int id = (int)(0xffffffffU - (unsigned)(__ldcg(&g.best[((a.n_steps - 1) % 3) * DR_ROWS + c.tid]) & 0xffffffffULL));
+            const int id = (int)(0xffffffffU - (unsigned)(__ldcg(&g.best[((a.n_steps - 1) % 3) * DR_MAX_ROWS + c.tid]) & 0xffffffffULL));
             const int t = *a.step_counter + a.n_steps - 1;
             a.tokens[c.tid] = id;
             a.positions[c.tid] += a.n_steps;
@@ -517,7 +628,7 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decode_resident_kernel(const __
 // Which CTA keeps which unit: per phase every CTA at most one unit more than another, the CTAs that hold least so far first; the
 // down projections, whose units are the largest, before the rest. False when the model does not fit.
 struct dr_plan {
-    uint32_t D, F, V, L, ctas;
+    uint32_t D, F, V, L, ctas, work;
     bool fits;
     uint32_t weight_bytes;
     dr_args tables;   // phase_unit, workers, cta_of, n_units
@@ -555,7 +666,7 @@ bool dr_make_plan(dr_plan *p, uint32_t max_weight_bytes)
 
 }  // namespace
 
-size_t gdb_decode_resident_sync_words(int L) { return (size_t)(2 + 5 * L) * DR_SYNC_STRIDE + 3U * DR_ROWS * 2U; }
+size_t gdb_decode_resident_sync_words(int L) { return (size_t)(2 + 5 * L) * DR_SYNC_STRIDE + 3U * DR_MAX_ROWS * 2U; }
 
 // n_steps greedy decode steps of at most 16 sequences with the weights in shared memory; GD_ERR_UNSUPPORTED when the model does
 // not fit (decode_mega.cu then takes the call). a->sync: gdb_decode_resident_sync_words(L) zeroed words, 8-byte aligned.
@@ -563,21 +674,24 @@ size_t gdb_decode_resident_sync_words(int L) { return (size_t)(2 + 5 * L) * DR_S
 gd_status gdb_decode_resident_launch(gd_backend *be, uint32_t dtype, const gdb_mega_args *a)
 {
     static thread_local dr_plan plan;   // of the last model
-    if (a->B > DR_ROWS || a->L > GDB_MEGA_MAX_LAYERS || be->sm_count > 255) {
+    if (a->B > DR_MAX_ROWS || a->L > GDB_MEGA_MAX_LAYERS || be->sm_count > 255 || (a->D & (a->D - 1)) != 0) {
         return GD_ERR_UNSUPPORTED;
     }
     const uint32_t D = (uint32_t)a->D, F = (uint32_t)a->F, ctas = (uint32_t)be->sm_count;
-    const uint32_t work = std::max({DR_ROWS * (F + 8U) * 2U, DR_ROWS * (D + 8U) * 2U + 2U * DR_RED_BYTES, (uint32_t)(DR_WARPS * 66 * sizeof(float))});
+    const uint32_t ch = (F % 512U) == 0U ? 512U : ((F % 256U) == 0U ? 256U : 128U), row_tiles = a->B > DR_ROWS ? 2U : 1U;
+    const uint32_t work = std::max({3U * DR_ROWS * (ch + 8U) * 2U + DR_RED_BYTES, row_tiles * DR_ROWS * (D + 8U) * 2U + 2U * DR_RED_BYTES,
+                                    (uint32_t)(DR_WARPS * 66 * sizeof(float))});
     constexpr uint32_t smem_limit = 232448U - 2048U;   // dynamic part beside the kernel's static tables
     if (work >= smem_limit) {
         return GD_ERR_UNSUPPORTED;
     }
-    if (plan.ctas != ctas || plan.D != D || plan.F != F || plan.V != (uint32_t)a->V || plan.L != (uint32_t)a->L) {
+    if (plan.ctas != ctas || plan.work != work || plan.D != D || plan.F != F || plan.V != (uint32_t)a->V || plan.L != (uint32_t)a->L) {
         plan.D = D;
         plan.F = F;
         plan.V = (uint32_t)a->V;
         plan.L = (uint32_t)a->L;
         plan.ctas = ctas;
+        plan.work = work;
         plan.fits = dr_make_plan(&plan, smem_limit - work);
     }
     if (!plan.fits) {
