@@ -178,10 +178,14 @@ gd_status gd_backend_create_default(gd_backend **out_backend)
         cudaMalloc((void **)&be->ws, be->ws_bytes) != cudaSuccess ||
         cudaMalloc((void **)&be->err_flag, GDB_FLAG_BYTES) != cudaSuccess ||
         cudaMallocHost((void **)&be->err_flag_host, 256) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&be->side_stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&be->side_fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&be->side_join, cudaEventDisableTiming) != cudaSuccess ||
         cudaMemset(be->err_flag, 0, GDB_FLAG_BYTES) != cudaSuccess) {
         gd_backend_destroy(be);
         return GD_ERR_OUT_OF_MEMORY;
     }
+    be->tickets = (unsigned *)be->err_flag + 64;
     *out_backend = be;
     return GD_OK;
 }
@@ -195,6 +199,9 @@ void gd_backend_destroy(gd_backend *be)
     if (be->stream != NULL) {
         cudaStreamSynchronize(be->stream);
     }
+    if (be->side_stream != NULL) {
+        cudaStreamSynchronize(be->side_stream);
+    }
     gdb_dp_destroy(be);
     gdb_tmap_cache_destroy(be);
     cudaFree(be->ws);
@@ -202,6 +209,9 @@ void gd_backend_destroy(gd_backend *be)
     cudaFreeHost(be->err_flag_host);
     cudaFree(be->rope_table);
     cudaFree(be->l2_flush);
+    if (be->side_fork != NULL) cudaEventDestroy(be->side_fork);
+    if (be->side_join != NULL) cudaEventDestroy(be->side_join);
+    if (be->side_stream != NULL) cudaStreamDestroy(be->side_stream);
     if (be->stream != NULL) {
         cudaStreamDestroy(be->stream);
     }

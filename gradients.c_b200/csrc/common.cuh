@@ -20,8 +20,8 @@
 #define GDB_SM_COUNT_DEFAULT 148
 // gd_backend::err_flag points at GDB_FLAG_BYTES of zeroed device words: word 0 is the error code of
 // bounded waits; words 64.. are arrival tickets of multi-block reductions (each user leaves them zero).
-#define GDB_FLAG_BYTES 16384
-#define GDB_TICKET_WORDS ((GDB_FLAG_BYTES / 4) - 64)
+#define GDB_FLAG_BYTES 32512
+#define GDB_TICKET_WORDS (4096 - 64)   // of each of the two streams
 
 struct gdb_tmap_cache;  // tcgen05 GEMM tensor-map cache (gemm_tcgen05.cu)
 struct gdb_dp_state;    // NCCL state (dp.cu)
@@ -46,6 +46,11 @@ struct gd_backend {
     size_t l2_flush_bytes;
     gdb_tmap_cache *tmaps;
     gdb_dp_state *dp;
+    // A second stream for work that nothing on `stream` waits for soon (gdb_side); its kernels use the upper half of the workspace
+    // and the upper half of the tickets.
+    cudaStream_t side_stream;
+    cudaEvent_t side_fork, side_join;
+    unsigned *tickets;
     // scratch offsets of the parameter gradients of the last gdb200_gpt_train_step (valid until the arena is reused)
     int32_t last_grad_count;
     size_t last_grad_offset[GDB200_GPT_MAX_PARAMS];
@@ -62,7 +67,23 @@ struct gd_backend_buffer {
     int kind;
 };
 
-static inline unsigned *gdb_tickets(const struct gd_backend *be) { return (unsigned *)be->err_flag + 64; }
+static inline unsigned *gdb_tickets(const struct gd_backend *be) { return be->tickets; }
+
+// While it lives, what is enqueued through `be` goes to the side stream. Only contractions and reductions that keep to half of the
+// workspace (split-K partials do: ws_bytes / 2 is their limit) may be enqueued there; the caller orders the streams with the
+// two events.
+struct gdb_side {
+    gd_backend *be;
+    explicit gdb_side(gd_backend *b) : be(b) { swap(b->ws_bytes / 2U, GDB_TICKET_WORDS); }
+    ~gdb_side() { swap((size_t)0 - be->ws_bytes / 2U, -(ptrdiff_t)GDB_TICKET_WORDS); }
+    gdb_side(const gdb_side &) = delete;
+    void swap(size_t ws, ptrdiff_t tickets)
+    {
+        std::swap(be->stream, be->side_stream);
+        be->ws += ws;
+        be->tickets += tickets;
+    }
+};
 
 static inline gd_status gdb_fail(gd_backend *be, cudaError_t e, const char *what)
 {
