@@ -57,13 +57,14 @@ constexpr int P_SMEM_TOTAL_SWIGLU = (P_STAGES_DEFAULT - 1) * P_STAGE_BYTES + P_E
 // x w^T contraction with N = F): the epilogue does not write dact but the gradient of the up / gate projection's output,
 // d_x1 = dact x2 sigmoid(x2) and d_x2 = dact x1 sigmoid(x2) (1 + x2 (1 - sigmoid(x2))) with dact rounded to storage first
 // (the rounding point of the separate swiglu_split_backward call, src/ops/swiglu_split_linear/core_swiglu_split_linear.c:303-420).
-// x1 / x2 come from `aux` = the saved [M, 2F] x12 matrix (16-byte loads, a row per thread); tma_c maps d_x12 [M, 2F].
+// x1 / x2 come from the saved [M, 2F] x12 matrix, which tma_act maps, 32 x 64 tiles at a time into the staging buffers the results leave
+// from; tma_c maps d_x12 [M, 2F].
 template <typename T, bool A_MN, bool B_MN, bool SPLITK, bool COLSUM, bool SWIGLU = false, bool SWIGLU_BWD = false>
 __global__ void __launch_bounds__(P_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  const __grid_constant__ CUtensorMap tma_c, const T *__restrict__ bias, uint32_t M, uint32_t N, uint32_t K,
                  uint32_t tiles_m, uint32_t tiles_n, uint32_t splits, uint32_t k_iters_per_split, int bias_mode, int *err_flag,
-                 float *__restrict__ colsum_partial, const __grid_constant__ CUtensorMap tma_act, const T *__restrict__ aux, size_t ld_aux)
+                 float *__restrict__ colsum_partial, const __grid_constant__ CUtensorMap tma_act)
 {
     static_assert(!COLSUM || SPLITK, "column sums ride on the split-K (FP32 partial) output path");
     static_assert(!SWIGLU || (!SPLITK && !A_MN && !B_MN), "the SwiGLU epilogue belongs to y = x w^T with direct output");
@@ -77,8 +78,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023U) & ~(uintptr_t)1023U);
     unsigned char *staging = smem + PSTAGES * P_STAGE_BYTES;
     uint64_t *bars = reinterpret_cast<uint64_t *>(staging + P_STAGING_BYTES);
-    // bars: [0, S) full, [S, 2S) empty, [2S, 2S+2) accumulator full, [2S+2, 2S+4) accumulator empty
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * PSTAGES + 4);
+    // bars: [0, S) full, [S, 2S) empty, [2S, 2S+2) accumulator full, [2S+2, 2S+4) accumulator empty, then one per epilogue warp (SWIGLU_BWD)
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * PSTAGES + 4 + P_EPI_WARPS);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
@@ -102,6 +103,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         for (int b = 0; b < 2; ++b) {
             mbar_init(tfull0 + 8 * b, 1);
             mbar_init(tempty0 + 8 * b, 2 * P_EPI_WARPS);   // the epilogue warps of the two CTAs
+        }
+        if (SWIGLU_BWD) {
+            for (int w = 0; w < P_EPI_WARPS; ++w) mbar_init(smem_u32(&bars[2 * PSTAGES + 4 + w]), 1);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -213,6 +217,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         const uint32_t tempty_leader = mapa_shared(tempty0, 0);
         uint32_t unit_idx = 0, store_cnt = 0;
         constexpr int CHUNK_COLS = SPLITK ? 32 : 64;   // 128 bytes of output per row
+        // SWIGLU_BWD: this warp's x1 / x2 tiles of chunk c of unit u, 32 rows x 64 columns each, on their way to its staging buffers
+        const uint32_t xbar = smem_u32(&bars[2 * PSTAGES + 4 + (warp - 2)]);
+        uint32_t x_phase = 0;
+        auto load_x12 = [&](uint32_t u, int c) {
+            const uint32_t x_col = (u % tiles_n) * PBN + c * 64, x_row = ((u / tiles_n) % tiles_m) * 2 * BM + rank * BM + quad * 32;
+            if (u >= units || x_row >= M || x_col >= N) return;
+            mbar_expect_tx(xbar, 8192);
+            tma_load_2d(smem_u32(my_stage), &tma_act, (int)x_col, (int)x_row, xbar);
+            tma_load_2d(smem_u32(my_stage + 4096), &tma_act, (int)(N + x_col), (int)x_row, xbar);
+        };
+        if (SWIGLU_BWD && lane == 0) load_x12(cluster_id, chalf * 2);
         for (uint32_t u = cluster_id; u < units; u += n_clusters, ++unit_idx) {
             const uint32_t tn = u % tiles_n, tm = (u / tiles_n) % tiles_m, z = u / (tiles_n * tiles_m);
             const uint32_t buf = COLSUM ? 0U : (unit_idx & 1U), acc_ph = COLSUM ? (unit_idx & 1U) : ((unit_idx >> 1) & 1U);
@@ -297,25 +312,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                 continue;
             }
             if (SWIGLU_BWD) {
-                const uint32_t row = row0 + lane;
+                // two chunks of 64 columns per warp: x1 / x2 tiles arrive in the staging buffers (the first one while the products
+                // were formed), are replaced there by d_x1 / d_x2 and stored
 #pragma unroll 1
-                for (int c = chalf * 2; c < chalf * 2 + 2; ++c) {          // two chunks of 64 columns per warp
+                for (int c = chalf * 2; c < chalf * 2 + 2; ++c) {
                     const uint32_t col0 = tn * PBN + c * 64;
-                    if (lane == 0) bulk_wait_group_read<0>();               // the two staged tiles of the previous chunk have been read
-                    __syncwarp();
+                    const bool in = row0 < M && col0 < N;
+                    if (in && !mbar_wait(xbar, x_phase++ & 1U)) {
+                        if (lane == 0) atomicExch(err_flag, 205);
+                        break;
+                    }
                     unsigned char *r1 = my_stage + lane * 128, *r2 = r1 + 4096;
 #pragma unroll 1
                     for (int pc = 0; pc < 2; ++pc) {                        // 32 columns at a time
-                        const uint32_t cc0 = col0 + pc * 32;
-                        uint4 xa[4], xb[4];
-                        const bool in = row < M && cc0 < N;
-                        const uint4 *p1 = reinterpret_cast<const uint4 *>(aux + (size_t)row * ld_aux + cc0);
-                        const uint4 *p2 = reinterpret_cast<const uint4 *>(aux + (size_t)row * ld_aux + N + cc0);
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            xa[j] = in ? p1[j] : make_uint4(0U, 0U, 0U, 0U);
-                            xb[j] = in ? p2[j] : make_uint4(0U, 0U, 0U, 0U);
-                        }
                         uint32_t v[32];
                         tmem_ld_32x32b_x32(tbase + c * 64 + pc * 32, v);
                         if (c == chalf * 2 + 1 && pc == 1) {
@@ -325,17 +334,25 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                         }
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
-                            gdb_vec8<T> a, b, d1, d2;
-                            a.raw = xa[j];
-                            b.raw = xb[j];
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) {
-                                const float gv = gdb_io<T>::rnd(__uint_as_float(v[j * 8 + e]));
-                                const float z = b.get(e), sg = gdb_swiglu_sigmoid(z);
-                                d1.set(e, gv * (z * sg));
-                                d2.set(e, gv * a.get(e) * (sg * (1.0f + z * (1.0f - sg))));
-                            }
                             const int chunk = ((pc * 4 + j) ^ (lane & 7)) << 4;
+                            gdb_vec8<T> a, b, d1, d2;
+                            a.raw = *reinterpret_cast<const uint4 *>(r1 + chunk);
+                            b.raw = *reinterpret_cast<const uint4 *>(r2 + chunk);
+#pragma unroll
+                            for (int e = 0; e < 8; e += 2) {
+                                // d_x1 = g (z sg), d_x2 = (g x1) (sg (1 + z (1 - sg))), two columns per instruction
+                                const f32x2 gv = f2_make(gdb_io<T>::rnd(__uint_as_float(v[j * 8 + e])), gdb_io<T>::rnd(__uint_as_float(v[j * 8 + e + 1])));
+                                const float z0 = b.get(e), z1 = b.get(e + 1);
+                                const f32x2 z = f2_make(z0, z1), sg = f2_make(gdb_swiglu_sigmoid(z0), gdb_swiglu_sigmoid(z1)), one = f2_make(1.0f, 1.0f);
+                                const f32x2 t = f2_mul(sg, f2_fma(z, f2_fma(sg, f2_make(-1.0f, -1.0f), one), one));
+                                float u0, u1;
+                                f2_split(f2_mul(gv, f2_mul(z, sg)), u0, u1);
+                                d1.set(e, u0);
+                                d1.set(e + 1, u1);
+                                f2_split(f2_mul(f2_mul(gv, f2_make(a.get(e), a.get(e + 1))), t), u0, u1);
+                                d2.set(e, u0);
+                                d2.set(e + 1, u1);
+                            }
                             *reinterpret_cast<uint4 *>(r1 + chunk) = d1.raw;
                             *reinterpret_cast<uint4 *>(r2 + chunk) = d2.raw;
                         }
@@ -343,11 +360,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) {
-                        if (row0 < M && col0 < N) {
+                        if (in) {
                             tma_store_2d(&tma_c, (int)col0, (int)row0, smem_u32(my_stage));
                             tma_store_2d(&tma_c, (int)(N + col0), (int)row0, smem_u32(my_stage + 4096));
                         }
                         bulk_commit_group();
+                        bulk_wait_group_read<0>();
+                        // the next chunk's x1 / x2: of this unit, or of the next one
+                        if (c == chalf * 2) load_x12(u, c + 1); else load_x12(u + n_clusters, c - 1);
                     }
                 }
                 continue;
@@ -449,7 +469,7 @@ int max_clusters(gd_backend *be, const void *kern, int smem_bytes)
 template <typename T, bool A_MN, bool B_MN, bool SPLITK, bool COLSUM = false, bool SWIGLU = false, bool SWIGLU_BWD = false>
 gd_status launch_pair(gd_backend *be, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &tc, const void *bias, uint32_t M,
                       uint32_t N, uint32_t K, uint32_t tiles_m, uint32_t tiles_n, uint32_t splits, uint32_t kps, int bias_mode, int *clusters_out,
-                      float *colsum_partial = nullptr, const CUtensorMap *tact = nullptr, const void *aux = nullptr, size_t ld_aux = 0)
+                      float *colsum_partial = nullptr, const CUtensorMap *tact = nullptr)
 {
     constexpr int SMEM = SWIGLU ? P_SMEM_TOTAL_SWIGLU : (COLSUM ? P_SMEM_TOTAL_COLSUM : P_SMEM_TOTAL);
     auto kern = gemm_pair_kernel<T, A_MN, B_MN, SPLITK, COLSUM, SWIGLU, SWIGLU_BWD>;
@@ -485,7 +505,7 @@ gd_status launch_pair(gd_backend *be, const CUtensorMap &ta, const CUtensorMap &
     cfg.attrs = attr;
     cfg.numAttrs = 2;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, (const T *)bias, M, N, K, tiles_m, tiles_n, splits, kps, bias_mode, be->err_flag, colsum_partial,
-                                       tact != nullptr ? *tact : tc, (const T *)aux, ld_aux);
+                                       tact != nullptr ? *tact : tc);
     if (e != cudaSuccess) {
         be->launches += 1U;
         return gdb_fail(be, e, "gemm_tcgen05_pair");
@@ -617,15 +637,13 @@ gd_status gdb_gemm_tcgen05_pair_swiglu_bwd(gd_backend *be, uint32_t dtype, const
         (ldg_bytes % 16U) != 0U || (ldw_bytes % 16U) != 0U || (ld12_bytes % 16U) != 0U || (ldd_bytes % 16U) != 0U) {
         return GD_ERR_UNSUPPORTED;
     }
-    CUtensorMap ma, mb, md;
+    CUtensorMap ma, mb, mx, md;
     if (!make_tmap(&ma, dtype, g, M, K, ldg_bytes, BK, BM) || !make_tmap(&mb, dtype, w, F, K, ldw_bytes, BK, PBN / 2) ||
-        !make_tmap(&md, dtype, d_x12, M, 2ULL * F, ldd_bytes, 64, 32)) {
+        !make_tmap(&mx, dtype, x12, M, 2ULL * F, ld12_bytes, 64, 32) || !make_tmap(&md, dtype, d_x12, M, 2ULL * F, ldd_bytes, 64, 32)) {
         return GD_ERR_UNSUPPORTED;
     }
     const uint32_t tiles_m = (M + 2 * BM - 1) / (2 * BM), tiles_n = (F + PBN - 1) / PBN, kps = (K + BK - 1) / BK;
     return dtype == GDB_DTYPE_F16
-               ? launch_pair<__half, false, false, false, false, false, true>(be, ma, mb, md, nullptr, M, F, K, tiles_m, tiles_n, 1, kps, 0, nullptr, nullptr,
-                                                                              nullptr, x12, ld12_bytes / 2U)
-               : launch_pair<__nv_bfloat16, false, false, false, false, false, true>(be, ma, mb, md, nullptr, M, F, K, tiles_m, tiles_n, 1, kps, 0, nullptr,
-                                                                                     nullptr, nullptr, x12, ld12_bytes / 2U);
+               ? launch_pair<__half, false, false, false, false, false, true>(be, ma, mb, md, nullptr, M, F, K, tiles_m, tiles_n, 1, kps, 0, nullptr, nullptr, &mx)
+               : launch_pair<__nv_bfloat16, false, false, false, false, false, true>(be, ma, mb, md, nullptr, M, F, K, tiles_m, tiles_n, 1, kps, 0, nullptr, nullptr, &mx);
 }

@@ -768,15 +768,11 @@ extern "C" gd_status gdb200_gpt_train_step(gd_backend *be, const gdb200_gpt_spec
             // d_act = g w^T and the SwiGLU backward in its epilogue; the two separate calls when the fused kernel declines
             Ten d_up = c.alloc(dt, {T, 2 * F});
             gd_backend_matrix_view ugm = mv(sv.up_gate, (uint32_t)T, (uint32_t)(2 * F)), dum = mv(d_up, (uint32_t)T, (uint32_t)(2 * F));
-            // (measured on the benchmark step: the fused launch takes as long as the two it replaces, 3.114 against 3.109 ms per
-            // step, because the epilogue then carries two special-function evaluations and two 16-byte loads per element; it
-            // saves the [T, F] scratch, so it is what GDB200_FUSE_SWIGLU_BWD=1 selects)
-            static int fuse_bwd = -1;
-            if (fuse_bwd < 0) {
-                const char *env = getenv("GDB200_FUSE_SWIGLU_BWD");
-                fuse_bwd = (env != NULL && env[0] == '1') ? 1 : 0;
-            }
-            gd_status fst = (c.st == GD_OK && fuse_bwd) ? gdb200_matmul_nt_swiglu_backward(be, &gm, &wm, &ugm, &dum) : GD_ERR_UNSUPPORTED;
+            // (GDB200_FUSE_SWIGLU_BWD=0: two calls everywhere)
+            static const bool fuse_bwd = !(getenv("GDB200_FUSE_SWIGLU_BWD") != NULL && getenv("GDB200_FUSE_SWIGLU_BWD")[0] == '0');
+            // one launch where its 256 x 256 tiles give every pair of SMs work; below that the separate ones spread further
+            const bool fills = ((T + 255) / 256) * ((F + 255) / 256) >= be->sm_count / 2;
+            gd_status fst = (c.st == GD_OK && fuse_bwd && fills) ? gdb200_matmul_nt_swiglu_backward(be, &gm, &wm, &ugm, &dum) : GD_ERR_UNSUPPORTED;
             if (fst == GD_ERR_UNSUPPORTED) {
                 Ten dact = c.alloc(dt, {T, F});
                 gd_backend_matrix_view dam = mv(dact, (uint32_t)T, (uint32_t)F);
