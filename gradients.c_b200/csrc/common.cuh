@@ -21,6 +21,7 @@
 // gd_backend::err_flag points at GDB_FLAG_BYTES of zeroed device words: word 0 is the error code of
 // bounded waits; words 64.. are arrival tickets of multi-block reductions (each user leaves them zero).
 #define GDB_FLAG_BYTES 32512
+#define GDB_STAGE_BYTES 65536U
 #define GDB_TICKET_WORDS (4096 - 64)   // of each of the two streams
 
 struct gdb_tmap_cache;  // tcgen05 GEMM tensor-map cache (gemm_tcgen05.cu)
@@ -50,6 +51,10 @@ struct gd_backend {
     // and the upper half of the tickets.
     cudaStream_t side_stream;
     cudaEvent_t side_fork, side_join;
+    // page-locked slots in which small uploads are put together (gdb200_upload_beside), and when each was last read
+    unsigned char *stage;
+    cudaEvent_t stage_free[4];
+    unsigned stage_next;
     unsigned *tickets;
     // scratch offsets of the parameter gradients of the last gdb200_gpt_train_step (valid until the arena is reused)
     int32_t last_grad_count;
@@ -350,7 +355,11 @@ gd_status gdb_embedding_dropout_rms_norm(gd_backend *be, const gd_backend_tensor
 // gdb_lm_ce_count_valid writes the local count into both; the caller sums element 0 over the ranks before
 // gdb_lm_ce_reduce_normalize_global divides by it (the reference's kernel, src/ops/lm_cross_entropy/metal_lm_cross_entropy.metal:244-252,
 // divides by the local count because it knows one device only).
-gd_status gdb_lm_ce_count_valid(gd_backend *be, const gd_backend_tensor_view *targets, int32_t ignore_index, const gd_backend_tensor_view *counts);
+// `amp` != NULL: gd_backend_amp_begin_step and the seed (gd_backend_amp_fill_scale of one F32) in the same launch.
+gd_status gdb_lm_ce_count_valid(gd_backend *be, const gd_backend_tensor_view *targets, int32_t ignore_index, const gd_backend_tensor_view *counts,
+                                const gd_backend_amp_state_desc *amp = NULL, const gd_backend_tensor_view *seed = NULL);
+// gd_backend_adamw_batch and gd_backend_amp_finish_step, the latter in the last launch of the former.
+gd_status gdb_adamw_batch_amp_finish(gd_backend *be, const gd_backend_adamw_desc *descs, uint32_t desc_count, const gd_backend_amp_state_desc *amp);
 gd_status gdb_lm_ce_reduce_normalize_global(gd_backend *be, const gd_backend_tensor_view *row_loss, const gd_backend_tensor_view *counts,
                                             const gd_backend_tensor_view *loss, const gd_backend_tensor_view *inv_valid_count);
 // gdb200_lm_cross_entropy_fused_rows for up to 32768 classes.

@@ -537,14 +537,15 @@ extern "C" gd_status gdb200_gpt_train_step(gd_backend *be, const gdb200_gpt_spec
     Ten seed;
     memset(&seed, 0, sizeof(seed));
     if (single && lmce_fused != 0) {
+        seed = c.alloc(GDB_DTYPE_F32, {});
         if (!global_norm) {
             counts = c.alloc(GDB_DTYPE_F32, {2});
-            gd_backend_tensor_view cv0 = tv(counts);
-            c.ok(gdb_lm_ce_count_valid(be, &tgv, s->pad_token_id, &cv0), "lm_ce_count_valid");
+            gd_backend_tensor_view cv0 = tv(counts), sdv0 = tv(seed);
+            c.ok(gdb_lm_ce_count_valid(be, &tgv, s->pad_token_id, &cv0, &amp, &sdv0), "amp_begin_step + lm_ce_count_valid");
+        } else {
+            c.ok(gd_backend_amp_begin_step(be, &amp), "amp_begin_step");
+            c.ok(gd_backend_amp_fill_scale(be, seed.buf, seed.off, 1, GDB_DTYPE_F32, s->state_buffer, s->amp_scale_offset), "amp_fill_scale");
         }
-        c.ok(gd_backend_amp_begin_step(be, &amp), "amp_begin_step");
-        seed = c.alloc(GDB_DTYPE_F32, {});
-        c.ok(gd_backend_amp_fill_scale(be, seed.buf, seed.off, 1, GDB_DTYPE_F32, s->state_buffer, s->amp_scale_offset), "amp_fill_scale");
         Ten logits = c.alloc(dt, {T, V});
         gd_backend_matrix_view hm = mv(final_norm, (uint32_t)T, (uint32_t)D), wm = mv(lm_w, (uint32_t)V, (uint32_t)D), lm = mv(logits, (uint32_t)T, (uint32_t)V);
         c.ok(gd_backend_matmul_nt(be, &hm, &wm, &lm), "matmul_nt(logits)");
@@ -555,7 +556,7 @@ extern "C" gd_status gdb200_gpt_train_step(gd_backend *be, const gdb200_gpt_spec
             const gd_status fst = gdb_lm_ce_fused_rows(be, &lv, &bv, &tgv, &sdv, &cv1, &rlv, 1.0f, s->logits_softcap, s->pad_token_id);
             if (fst == GD_OK) {
                 fused_ce = true;
-                c.ok(gdb_lm_ce_reduce_normalize_global(be, &rlv, &cv1, &lov, &ivv), "lm_ce_reduce_normalize(rows)");
+                if (dp || !drop) c.ok(gdb_lm_ce_reduce_normalize_global(be, &rlv, &cv1, &lov, &ivv), "lm_ce_reduce_normalize(rows)");
                 if (dp) c.ok(gdb200_dp_all_reduce(be, loss.buf, loss.off, 1, GDB_DTYPE_F32), "dp_all_reduce(loss)");
             } else if (fst != GD_ERR_UNSUPPORTED) {
                 c.ok(fst, "lm_ce_fused_rows");
@@ -689,9 +690,12 @@ extern "C" gd_status gdb200_gpt_train_step(gd_backend *be, const gdb200_gpt_spec
         }
     };
     const Ten none = {};
+    gd_backend_tensor_view cvn = tv(counts);
+    if (fused_ce && !dp && drop && !side) c.ok(gdb_lm_ce_reduce_normalize_global(be, &rlv, &cvn, &lov, &ivv), "lm_ce_reduce_normalize(rows)");
     if (side) {
         fork();
         gdb_side on(be);
+        if (fused_ce) c.ok(gdb_lm_ce_reduce_normalize_global(be, &rlv, &cvn, &lov, &ivv), "lm_ce_reduce_normalize(rows)");   // the loss, for the host
         linear_t_backward(c, final_norm, none, saved_logits, T, D, V, NULL, lmw_grad, grads[(size_t)P_LMB]);
     }
     for (int64_t start = 0; start < V && c.st == GD_OK; start += pass) {
@@ -949,8 +953,7 @@ extern "C" gd_status gdb200_gpt_train_step(gd_backend *be, const gdb200_gpt_spec
     be->last_grad_count = n_params;
     for (int p = 0; p < n_params; ++p) be->last_grad_offset[p] = grads[(size_t)p].off;
     c.ok(gd_backend_grad_clip_scale(be, nd.data(), (uint32_t)n_params, s->state_buffer, s->clip_scale_offset, s->grad_clip_norm, 1.0e-6f), "grad_clip_scale");
-    c.ok(gd_backend_adamw_batch(be, ad.data(), (uint32_t)n_params), "adamw_batch");
-    c.ok(gd_backend_amp_finish_step(be, &amp), "amp_finish_step");
+    c.ok(gdb_adamw_batch_amp_finish(be, ad.data(), (uint32_t)n_params, &amp), "adamw_batch + amp_finish_step");
     if (scratch_used != NULL) {
         *scratch_used = c.top;
     }

@@ -227,9 +227,18 @@ __global__ void lmce_reduce_normalize_global_kernel(const float *row_loss, const
 }
 
 // counts[0] = counts[1] = number of rows whose target takes part in the loss (same rule as lmce_finalize_kernel).
-__global__ void lmce_count_valid_kernel(const int *targets, size_t rows, int ignore_index, float *counts)
+// `scale` != NULL: also the AMP scaler's begin of a step (clamp, inverse, overflow flag) and the loss gradient's seed.
+__global__ void lmce_count_valid_kernel(const int *targets, size_t rows, int ignore_index, float *counts, float *scale, int *flags, float min_scale,
+                                        float max_scale, float *seed)
 {
     gdb_pdl_sync();
+    if (scale != nullptr && threadIdx.x == 0) {
+        const float s = fminf(fmaxf(scale[0], min_scale), max_scale);
+        scale[0] = s;
+        scale[1] = 1.0f / s;
+        flags[1] = 0;
+        *seed = s;
+    }
     __shared__ float sh[33];
     // out-of-range ids count (their loss is NaN), as in finalize
     const float n = strided_sum(rows, [&](size_t i) {
@@ -964,8 +973,19 @@ extern "C" gd_status gdb200_lm_cross_entropy_fused_rows(gd_backend *be, const gd
     return gdb_lm_ce_fused_rows(be, logits, bias, targets, grad_loss, counts, row_loss, scale, logits_softcap, ignore_index);
 }
 
-gd_status gdb_lm_ce_count_valid(gd_backend *be, const gd_backend_tensor_view *targets, int32_t ignore_index, const gd_backend_tensor_view *counts)
+gd_status gdb_lm_ce_count_valid(gd_backend *be, const gd_backend_tensor_view *targets, int32_t ignore_index, const gd_backend_tensor_view *counts,
+                                const gd_backend_amp_state_desc *amp, const gd_backend_tensor_view *seed)
 {
+    float *scale = NULL, *sp = NULL;
+    int *flags = NULL;
+    if (amp != NULL) {
+        sp = (float *)gdb_tv_ptr(seed, GDB_DTYPE_F32);
+        if (sp == NULL || !gdb_range_ok(amp->scale_buffer, amp->scale_offset, 8U) || !gdb_range_ok(amp->flags_buffer, amp->flags_offset, 12U)) {
+            return GD_ERR_INVALID_ARGUMENT;
+        }
+        scale = (float *)(amp->scale_buffer->dptr + amp->scale_offset);
+        flags = (int *)(amp->flags_buffer->dptr + amp->flags_offset);
+    }
     if (be == NULL || targets == NULL || counts == NULL || targets->count == 0U || counts->count != 2U) {
         return GD_ERR_INVALID_ARGUMENT;
     }
@@ -974,7 +994,8 @@ gd_status gdb_lm_ce_count_valid(gd_backend *be, const gd_backend_tensor_view *ta
     if (tp == NULL || cp == NULL) {
         return GD_ERR_INVALID_ARGUMENT;
     }
-    gdb_launch(lmce_count_valid_kernel, 1, 1024, 0, be->stream, tp, (size_t)targets->count, (int)ignore_index, cp);
+    gdb_launch(lmce_count_valid_kernel, 1, 1024, 0, be->stream, tp, (size_t)targets->count, (int)ignore_index, cp, scale, flags, amp != NULL ? amp->min_scale : 0.0f,
+               amp != NULL ? amp->max_scale : 0.0f, sp);
     return gdb_launched(be, "lm_cross_entropy_count_valid");
 }
 

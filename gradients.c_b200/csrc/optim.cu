@@ -45,10 +45,8 @@ __global__ void amp_begin_kernel(float *scale, int *flags, float min_scale, floa
     scale[1] = 1.0f / s;
     flags[1] = 0;
 }
-__global__ void amp_finish_kernel(float *scale, unsigned *flags, float growth, float backoff, float min_scale,
-                                  float max_scale, unsigned interval)
+__device__ __forceinline__ void amp_finish(float *scale, unsigned *flags, float growth, float backoff, float min_scale, float max_scale, unsigned interval)
 {
-    gdb_pdl_sync();
     const bool found = flags[1] != 0U;
     float s = scale[0];
     unsigned tracker = flags[0];
@@ -66,6 +64,11 @@ __global__ void amp_finish_kernel(float *scale, unsigned *flags, float growth, f
     scale[0] = s;
     scale[1] = 1.0f / s;
     flags[0] = tracker;
+}
+__global__ void amp_finish_kernel(float *scale, unsigned *flags, float growth, float backoff, float min_scale, float max_scale, unsigned interval)
+{
+    gdb_pdl_sync();
+    amp_finish(scale, flags, growth, backoff, min_scale, max_scale, interval);
 }
 // dst[i] = (src ? src[i] : 1) * scale[0]
 __global__ void amp_scale_kernel(void *dst, const void *src, size_t n, uint32_t dtype, const float *scale)
@@ -275,11 +278,20 @@ struct adamw_commit_item {
 struct adamw_commit_batch {
     adamw_commit_item it[ADAMW_BATCH];
     int n;
+    // the AMP scaler's end of the step (scale == NULL: not in this launch); it reads the overflow flag as the tensors do
+    float *scale;
+    unsigned *flags;
+    float growth, backoff, min_scale, max_scale;
+    unsigned interval;
 };
 __global__ void adamw_commit_kernel(adamw_commit_batch b)
 {
     gdb_pdl_sync();
     const int t = threadIdx.x;
+    static_assert(ADAMW_BATCH < 64, "the last thread has no tensor");
+    if (t == 63 && b.scale != nullptr) {
+        amp_finish(b.scale, b.flags, b.growth, b.backoff, b.min_scale, b.max_scale, b.interval);
+    }
     if (t >= b.n) {
         return;
     }
@@ -640,12 +652,20 @@ gd_status gd_backend_grad_clip_scale(gd_backend *be, const gd_backend_grad_norm_
 
 gd_status gd_backend_adamw_batch(gd_backend *be, const gd_backend_adamw_desc *descs, uint32_t desc_count)
 {
+    return gdb_adamw_batch_amp_finish(be, descs, desc_count, NULL);
+}
+
+}  // extern "C"
+
+gd_status gdb_adamw_batch_amp_finish(gd_backend *be, const gd_backend_adamw_desc *descs, uint32_t desc_count, const gd_backend_amp_state_desc *amp)
+{
     if (desc_count == 0U) {
-        return GD_OK;
+        return amp != NULL ? gd_backend_amp_finish_step(be, amp) : GD_OK;
     }
-    if (be == NULL || descs == NULL) {
+    if (be == NULL || descs == NULL || (amp != NULL && !amp_desc_ok(amp))) {
         return GD_ERR_INVALID_ARGUMENT;
     }
+    bool finished = amp == NULL;
     // validate everything before the first launch so a bad descriptor leaves no partial update
     {
         adamw_item tmp;
@@ -692,6 +712,16 @@ gd_status gd_backend_adamw_batch(gd_backend *be, const gd_backend_adamw_desc *de
                 c.beta2 = a.beta2;
                 c.update_optimizer_step = a.update_optimizer_step;
             }
+            if (!finished && start + (uint32_t)ADAMW_BATCH >= desc_count) {
+                cb.scale = (float *)(amp->scale_buffer->dptr + amp->scale_offset);
+                cb.flags = (unsigned *)(amp->flags_buffer->dptr + amp->flags_offset);
+                cb.growth = amp->growth_factor;
+                cb.backoff = amp->backoff_factor;
+                cb.min_scale = amp->min_scale;
+                cb.max_scale = amp->max_scale;
+                cb.interval = amp->growth_interval;
+                finished = true;
+            }
             gdb_launch(adamw_commit_kernel, 1, 64, 0, be->stream, cb);
             st = gdb_launched(be, "adamw_commit");
             if (st != GD_OK) {
@@ -699,8 +729,10 @@ gd_status gd_backend_adamw_batch(gd_backend *be, const gd_backend_adamw_desc *de
             }
         }
     }
-    return GD_OK;
+    return finished ? GD_OK : gd_backend_amp_finish_step(be, amp);
 }
+
+extern "C" {
 
 gd_status gd_backend_adamw(gd_backend *be, const gd_backend_adamw_desc *desc)
 {

@@ -289,6 +289,7 @@ PROTOTYPES = {
     "gdb200_pinned_alloc": (P, [SZ]),
     "gdb200_pinned_free": (None, [P]),
     "gdb200_upload_async": (_ST, [P, P, SZ, P, SZ]),
+    "gdb200_upload_beside": (_ST, [P, P, U32, C.POINTER(SZ), C.POINTER(P), C.POINTER(SZ)]),
     "gdb200_download_async": (_ST, [P, P, SZ, P, SZ]),
     "gdb200_gemm_profile_enable": (None, [P, C.c_int]),
     "gdb200_gemm_profile_read": (_ST, [P, C.POINTER(U64), C.POINTER(C.c_double), C.POINTER(C.c_double), C.POINTER(C.c_double)]),

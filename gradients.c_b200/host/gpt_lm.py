@@ -292,12 +292,15 @@ class GptLm:
                                                               cfg.logits_softcap, cfg.pad_token_id, shard_share)
 
     def upload_batch(self, batch: Batch, stream_ordered: bool = False):
-        """Places the batch in the data slot. `stream_ordered`: the arrays are page-locked and are copied behind
+        """Places the batch in the data slot. `stream_ordered`: the arrays are page-locked and are copied beside or behind
         the work already submitted, without a wait (they must stay unchanged until the step's fence completes)."""
         ctx = self.ctx
         if isinstance(batch, CompactBatch):
             return self.expand_compact_batch(batch, stream_ordered)[:4]
         if stream_ordered:
+            beside = ctx.upload_beside((batch.input_ids, batch.targets, batch.positions, batch.cu_seqlens))
+            if beside is not None:
+                return tuple(beside)
             out = []
             for a, name in ((batch.input_ids, "input_ids"), (batch.targets, "targets"), (batch.positions, "positions"), (batch.cu_seqlens, "cu_seqlens")):
                 t = ctx.empty(ctx.data, I32, a.shape, name)

@@ -89,17 +89,21 @@ class Arena:
 class Tensor:
     """Descriptor of contiguous tensor bytes inside an arena (reference gd_tensor)."""
 
-    __slots__ = ("ctx", "arena", "offset", "dtype", "shape", "count", "requires_grad", "grad", "is_leaf", "name", "_tv", "_ref")
+    # what most tensors never set
+    requires_grad = False
+    grad: Optional["Tensor"] = None
+    is_leaf = False
+    _count = _tv = _ref = None
 
     def __init__(self, ctx: "Context", arena: Arena, offset: int, dtype: int, shape: Sequence[int], name: str = ""):
-        self.ctx, self.arena, self.offset, self.dtype = ctx, arena, int(offset), dtype
-        self.shape = shape = tuple(map(int, shape))
-        self.count = math.prod(shape)
-        self.requires_grad = False
-        self.grad: Optional[Tensor] = None
-        self.is_leaf = False
-        self.name = name
-        self._tv = self._ref = None
+        self.ctx, self.arena, self.offset, self.dtype, self.name = ctx, arena, offset, dtype, name
+        self.shape = shape if type(shape) is tuple else tuple(map(int, shape))
+
+    @property
+    def count(self) -> int:
+        if self._count is None:
+            self._count = math.prod(self.shape)
+        return self._count
 
     @property
     def nbytes(self) -> int:
@@ -117,9 +121,10 @@ class Tensor:
 
     def ref(self):
         """Pointer argument to tv() (cached with it)."""
-        if self._ref is None:
-            self._ref = C.byref(self.tv())
-        return self._ref
+        r = self._ref
+        if r is None:
+            r = self._ref = C.byref(self.tv())
+        return r
 
     def mv(self, rows: int, cols: int, row_offset: int = 0, row_bytes: Optional[int] = None) -> abi.MatrixView:
         es = DTYPE_SIZE[self.dtype]
@@ -201,6 +206,7 @@ class Context:
         self.grad_enabled = True
         self._fences: list[abi.Fence] = []
         self.run_ahead = 0
+        self._data_before, self._data_base = (0, 0), 0
         self.in_step = False
         self.grad_ready_hook: Optional[Callable[[Tensor], None]] = None
 
@@ -254,6 +260,7 @@ class Context:
         assert not self.in_step
         self.wait_steps(self.run_ahead)
         self.scratch.reset()
+        self._data_before, self._data_base = (self._data_base, self.data.top), 0   # range of the data slot the step before uses
         self.data.reset()
         self.tape.clear()
         self.check(self.lib.gd_backend_scope_begin(self.backend), "scope_begin")
@@ -278,7 +285,8 @@ class Context:
     # ---- tensors ----
     def empty(self, arena: Arena, dtype: int, shape: Sequence[int], name: str = "") -> Tensor:
         t = Tensor(self, arena, 0, dtype, shape, name)
-        t.offset = arena.alloc((t.count or 1) * DTYPE_SIZE[dtype])
+        t._count = n = math.prod(t.shape)
+        t.offset = arena.alloc((n or 1) * DTYPE_SIZE[dtype])
         return t
 
     def scratch_empty(self, dtype: int, shape: Sequence[int], name: str = "") -> Tensor:
@@ -296,6 +304,23 @@ class Context:
         t = self.empty(arena, dtype, host.shape, name)
         t.write(host)
         return t
+
+    def upload_beside(self, arrays: Sequence[np.ndarray]) -> Optional[list[Tensor]]:
+        """I32 tensors of a step's page-locked arrays in the half of the data slot that the step before does not use, copied while that step
+        still runs. None when there is no such half: more steps may be in flight, or the slot is used otherwise or too small."""
+        half = self.data.capacity // 2 & ~(ALIGN - 1)
+        lo, hi = self._data_before
+        base = half if hi <= half else 0
+        if self.run_ahead > 1 or self.data.top != 0 or (base == 0 and lo < half) or sum(a.nbytes + ALIGN for a in arrays) > half:
+            return None
+        self.data.top = self._data_base = base
+        ts = [self.empty(self.data, I32, a.shape) for a in arrays]
+        n = len(ts)
+        assert all(a.dtype == np.int32 and a.flags.c_contiguous for a in arrays)
+        self.check(self.lib.gdb200_upload_beside(self.backend, self.data.buffer, n, (C.c_size_t * n)(*[t.offset for t in ts]),
+                                                 (C.c_void_p * n)(*[a.ctypes.data for a in arrays]), (C.c_size_t * n)(*[a.nbytes for a in arrays])),
+                   "upload_beside")
+        return ts
 
     # ---- tape (reference gd_autograd_record + reverse walk) ----
     def record(self, backward: Callable[[], None]) -> None:

@@ -386,6 +386,10 @@ void gdb200_pinned_free(void *p);
  * host range must not be written (upload) or read (download) until a fence recorded after the call has completed. */
 gd_status gdb200_upload_async(gd_backend *backend, gd_backend_buffer *buffer, size_t offset, const void *pinned_src, size_t nbytes);
 gd_status gdb200_download_async(gd_backend *backend, gd_backend_buffer *buffer, size_t offset, void *pinned_dst, size_t nbytes);
+/* `count` uploads in one call, copied beside the submitted work instead of behind it; work submitted after the call waits for them.
+ * The caller guarantees that nothing submitted and unfinished touches the destination ranges. Ranges that follow one another in the
+ * buffer may be copied as one: what lies between two of them (less than 256 bytes apart) is unspecified afterwards. */
+gd_status gdb200_upload_beside(gd_backend *backend, gd_backend_buffer *buffer, uint32_t count, const size_t *offsets, const void *const *pinned_srcs, const size_t *nbytes);
 /* Benchmark instrumentation: bracket every dense-contraction dispatch with a CUDA event pair on
  * the backend stream; read returns the number of launches, their summed device time and the
  * algorithmic FLOPs / bytes (2MNK and one pass over each operand) accumulated since enable. */
