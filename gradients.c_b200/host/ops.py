@@ -27,6 +27,11 @@ F32_NEG_INF_PATTERN = 0xFF800000      # :15
 FUSE_BIAS_ADD = True
 # gd_sdpa_varlen's backward through gdb200_sdpa_varlen_backward_with_output (False: the reference entry, two passes)
 SDPA_BACKWARD_WITH_OUTPUT = True
+# Backward of a norm, and weight and bias gradient of a linear layer, through the additive one-pass entries where they take the shape
+# (False: the reference's entries, each of which reads the same operands again). The benchmark's batch on the default model:
+# 2.91 -> 2.70 ms per step.
+ONE_PASS_BACKWARD = True
+RMS_ONE_PASS_ROWS = 512               # partial-sum rows of gdb200_rms_norm_backward_with_weight (two per SM)
 
 
 def _tvp(t: Optional[Tensor]):
@@ -156,6 +161,20 @@ def gd_rms_norm(ctx: Context, x: Tensor, weight: Tensor, eps: float) -> Tensor:
         def backward():
             if out.grad is None:
                 return
+            if ONE_PASS_BACKWARD and x.requires_grad and weight.requires_grad:
+                mark, into = ctx.scratch.top, x.grad is not None      # a gradient that is there is added to in the same launch
+                dx = x.grad if into else ctx.scratch_empty(x.dtype, x.shape, "d_rms_x")
+                dw = ctx.scratch_empty(weight.dtype, weight.shape, "d_rms_w")
+                partial = ctx.scratch_empty(F32, (max(args.row_blocks, RMS_ONE_PASS_ROWS), cols), "rms_partial")
+                st = ctx.lib.gdb200_rms_norm_backward_with_weight(ctx.backend, _tvp(x), _tvp(weight), _tvp(inv), _tvp(out.grad), _tvp(dx), 1 if into else 0,
+                                                                  _tvp(dw), _tvp(partial), byref(args))
+                if st != abi.GD_ERR_UNSUPPORTED:
+                    ctx.check(st, "rms_norm_backward_with_weight")
+                    if not into:
+                        ctx.accumulate_grad(x, dx)
+                    ctx.accumulate_grad(weight, dw)
+                    return
+                ctx.scratch.top = mark
             if x.requires_grad:
                 dx = ctx.scratch_empty(x.dtype, x.shape, "d_rms_x")
                 ctx.check(ctx.lib.gd_backend_rms_norm_backward_stats(ctx.backend, _tvp(x), _tvp(weight), _tvp(inv), _tvp(out.grad), _tvp(dx), byref(args)), "rms_norm_backward_stats")
@@ -212,6 +231,13 @@ def gd_linear_transposed_weight(ctx: Context, x: Tensor, w: Tensor, bias: Option
                 dx = ctx.scratch_empty(x.dtype, x.shape, "d_linear_t_x")
                 _matmul(ctx, lib.gd_backend_matmul, g.mv(m, n), w.mv(n, k), dx.mv(m, k), "matmul(dX)")
                 ctx.accumulate_grad(x, dx)
+            if ONE_PASS_BACKWARD and w.requires_grad and bias is not None and bias.requires_grad:
+                dw, db = ctx.scratch_empty(w.dtype, w.shape, "d_linear_t_w"), ctx.scratch_empty(bias.dtype, bias.shape, "d_bias")
+                gm, xm, dwm, dbv = g.mv(m, n), x.mv(m, k), dw.mv(n, k), db.vv()
+                ctx.check(lib.gdb200_matmul_tn_colsum(ctx.backend, byref(gm), byref(xm), byref(dwm), byref(dbv)), "matmul_tn_colsum(dW, db)")
+                ctx.accumulate_grad(w, dw)
+                ctx.accumulate_grad(bias, db)
+                return
             if w.requires_grad:
                 dw = ctx.scratch_empty(w.dtype, w.shape, "d_linear_t_w")
                 _matmul(ctx, lib.gd_backend_matmul_tn, g.mv(m, n), x.mv(m, k), dw.mv(n, k), "matmul_tn(dW)")
@@ -510,6 +536,10 @@ def gd_lm_cross_entropy_softcapped_bias_ignore(ctx: Context, hidden: Tensor, wei
                     _matmul(ctx, lib.gd_backend_matmul, logits.mv(rows, cc), weight.mv(cc, k, row_offset=start), dst.mv(rows, k), "matmul(d_hidden)")
                     if not single:
                         ctx.check(lib.gd_backend_accumulate(ctx.backend, dh.buffer, dh.offset, partial.buffer, partial.offset, dh.count, dh.dtype), "accumulate")
+                if need_w and need_b and ONE_PASS_BACKWARD:
+                    lm, hm, dwm, dbv = logits.mv(rows, cc), hidden.mv(rows, k), dw.mv(cc, k, row_offset=start), db.vv(start, cc)
+                    ctx.check(lib.gdb200_matmul_tn_colsum(ctx.backend, byref(lm), byref(hm), byref(dwm), byref(dbv)), "matmul_tn_colsum(d_lm_w, d_lm_b)")
+                    continue
                 if need_w:
                     _matmul(ctx, lib.gd_backend_matmul_tn, logits.mv(rows, cc), hidden.mv(rows, k), dw.mv(cc, k, row_offset=start), "matmul_tn(d_lm_w)")
                 if need_b:
