@@ -434,8 +434,8 @@ gd_status gdb_gemm_tcgen05_tn_colsum(gd_backend *be, uint32_t dtype, const void 
     }
     uint32_t splits = 1;
     float *cs = nullptr;
-    gd_status st = gdb_gemm_tcgen05_pair(be, 1, 0, dtype, a, lda_bytes, b, ldb_bytes, c, ldc_bytes, NULL, 1, M, N, K, &splits, &cs);
-    if (st != GD_OK) {
+    gd_status st = gdb_gemm_tcgen05_pair(be, 1, 0, dtype, a, lda_bytes, b, ldb_bytes, c, ldc_bytes, NULL, 1, M, N, K, &splits, &cs, colsum);
+    if (st != GD_OK || splits == 1U) {
         return st;
     }
     return reduce_partials(be, dtype, (const float *)be->ws, c, ldc_bytes / 2U, NULL, M, N, splits, 1, cs, colsum);

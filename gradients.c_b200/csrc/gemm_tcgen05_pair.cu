@@ -38,9 +38,9 @@ constexpr int P_SMEM_TOTAL = P_STAGES_DEFAULT * P_STAGE_BYTES + P_EPI_WARPS * 2 
 constexpr int P_SMEM_TOTAL_COLSUM = P_STAGES_DEFAULT * P_STAGE_BYTES + P_EPI_WARPS * 2 * 4096 + 1024 + 1024 + 1024;   // barriers padded to 1 KB, ones tile, alignment slack
 constexpr int P_SMEM_TOTAL_SWIGLU = (P_STAGES_DEFAULT - 1) * P_STAGE_BYTES + P_EPI_WARPS * 3 * 4096 + 256 + 1024;
 
-// COLSUM (split-K output only): the units of the first tile column also accumulate the sums of A over the
+// COLSUM: the units of the first tile column also accumulate the sums of A over the
 // contraction, colsum[m] = sum_k A[m, k], by one more MMA per k-step against a tile of ones (N = 16; every output
-// column holds the sum), and write them per k-slice to colsum_partial[splits, M]. This is the bias gradient of a
+// column holds the sum), and write them per k-slice to colsum_partial[splits, M], or, with direct output, rounded to colsum_out[M]. This is the bias gradient of a
 // linear layer for free while its weight gradient dW = dY^T X is computed (A = dY^T). Tensor memory then holds ONE
 // accumulator (256 columns) plus the 16 column-sum columns, so units are not overlapped (split-K launches run about one
 // unit per CTA pair anyway).
@@ -64,9 +64,8 @@ __global__ void __launch_bounds__(P_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  const __grid_constant__ CUtensorMap tma_c, const T *__restrict__ bias, uint32_t M, uint32_t N, uint32_t K,
                  uint32_t tiles_m, uint32_t tiles_n, uint32_t splits, uint32_t k_iters_per_split, int bias_mode, int *err_flag,
-                 float *__restrict__ colsum_partial, const __grid_constant__ CUtensorMap tma_act)
+                 float *__restrict__ colsum_partial, const __grid_constant__ CUtensorMap tma_act, T *__restrict__ colsum_out)
 {
-    static_assert(!COLSUM || SPLITK, "column sums ride on the split-K (FP32 partial) output path");
     static_assert(!SWIGLU || (!SPLITK && !A_MN && !B_MN), "the SwiGLU epilogue belongs to y = x w^T with direct output");
     static_assert(!SWIGLU_BWD || (!SPLITK && !A_MN && !B_MN && !SWIGLU), "the SwiGLU backward epilogue belongs to dact = g w^T with direct output");
     // The SwiGLU epilogue stages three output tiles per warp (x1, x2, act) instead of two alternating ones: it runs with
@@ -243,7 +242,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                 uint32_t cs[32];
                 tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(quad * 32) << 16) + PBN, cs);   // every column holds the row's sum
                 const uint32_t row = row0 + lane;
-                if (row < M) colsum_partial[(size_t)z * M + row] = __uint_as_float(cs[0]);
+                if (row < M && SPLITK) colsum_partial[(size_t)z * M + row] = __uint_as_float(cs[0]);
+                if (row < M && !SPLITK) gdb_io<T>::st(colsum_out, row, __uint_as_float(cs[0]));
             }
             if (SWIGLU) {
                 // this warp: 32 rows x 64 activation columns, 32 at a time (x1 and x2 values of the same columns); the three
@@ -469,7 +469,7 @@ int max_clusters(gd_backend *be, const void *kern, int smem_bytes)
 template <typename T, bool A_MN, bool B_MN, bool SPLITK, bool COLSUM = false, bool SWIGLU = false, bool SWIGLU_BWD = false>
 gd_status launch_pair(gd_backend *be, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &tc, const void *bias, uint32_t M,
                       uint32_t N, uint32_t K, uint32_t tiles_m, uint32_t tiles_n, uint32_t splits, uint32_t kps, int bias_mode, int *clusters_out,
-                      float *colsum_partial = nullptr, const CUtensorMap *tact = nullptr)
+                      float *colsum_partial = nullptr, const CUtensorMap *tact = nullptr, void *colsum_out = nullptr)
 {
     constexpr int SMEM = SWIGLU ? P_SMEM_TOTAL_SWIGLU : (COLSUM ? P_SMEM_TOTAL_COLSUM : P_SMEM_TOTAL);
     auto kern = gemm_pair_kernel<T, A_MN, B_MN, SPLITK, COLSUM, SWIGLU, SWIGLU_BWD>;
@@ -505,7 +505,7 @@ gd_status launch_pair(gd_backend *be, const CUtensorMap &ta, const CUtensorMap &
     cfg.attrs = attr;
     cfg.numAttrs = 2;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, (const T *)bias, M, N, K, tiles_m, tiles_n, splits, kps, bias_mode, be->err_flag, colsum_partial,
-                                       tact != nullptr ? *tact : tc);
+                                       tact != nullptr ? *tact : tc, (T *)colsum_out);
     if (e != cudaSuccess) {
         be->launches += 1U;
         return gdb_fail(be, e, "gemm_tcgen05_pair");
@@ -533,14 +533,15 @@ gd_status dispatch_pair(gd_backend *be, int ta, int tb, bool sk, const CUtensorM
 // Same contract as gdb_gemm_tcgen05 (which calls this first). Returns GD_ERR_UNSUPPORTED when the
 // problem is too small for 256-row tiles or clusters of two cannot be scheduled; `*splits_out`
 // receives the number of FP32 partial slices written to the workspace (1 = C was written directly).
-// `colsum_partial_out` != NULL (only for ta = 1, tb = 0, the weight-gradient layout): the FP32 partial path is taken even
-// for a single k-slice, and *colsum_partial_out receives the workspace address of colsum partials [*splits_out, M].
+// `colsum_out` != NULL (only for ta = 1, tb = 0, the weight-gradient layout): the sums of A's columns too. With a single k-slice
+// both results are written directly (two layers of d2048, vocabulary 32768: six FP32 round trips of 20 us and a column reduction of
+// 150 us less per step); else *colsum_partial_out receives the workspace address of partial sums [*splits_out, M].
 gd_status gdb_gemm_tcgen05_pair(gd_backend *be, int ta, int tb, uint32_t dtype, const void *a, size_t lda_bytes, const void *b,
                                 size_t ldb_bytes, void *c, size_t ldc_bytes, const void *bias, int bias_mode, uint32_t M, uint32_t N,
-                                uint32_t K, uint32_t *splits_out, float **colsum_partial_out)
+                                uint32_t K, uint32_t *splits_out, float **colsum_partial_out, void *colsum_out)
 {
     *splits_out = 1;
-    const bool want_colsum = colsum_partial_out != nullptr;
+    const bool want_colsum = colsum_out != nullptr;
     if (M < 256U || N < 128U || K < 64U || (want_colsum && !(ta && !tb))) {
         return GD_ERR_UNSUPPORTED;
     }
@@ -571,6 +572,15 @@ gd_status gdb_gemm_tcgen05_pair(gd_backend *be, int ta, int tb, uint32_t dtype, 
     }
     uint32_t kps = (total_k + splits - 1U) / splits;
     splits = (total_k + kps - 1U) / kps;
+    if (want_colsum && splits == 1U) {
+        if (!make_tmap(&mc, dtype, c, M, N, ldc_bytes, 64, 32)) {
+            return GD_ERR_UNSUPPORTED;
+        }
+        return dtype == GDB_DTYPE_F16
+                   ? launch_pair<__half, true, true, false, true>(be, ma, mb, mc, bias, M, N, K, tiles_m, tiles_n, 1, kps, bias_mode, nullptr, nullptr, nullptr, colsum_out)
+                   : launch_pair<__nv_bfloat16, true, true, false, true>(be, ma, mb, mc, bias, M, N, K, tiles_m, tiles_n, 1, kps, bias_mode, nullptr, nullptr, nullptr,
+                                                                         colsum_out);
+    }
     if (want_colsum) {
         const size_t dw_bytes = ((size_t)splits * M * N * sizeof(float) + 255U) & ~(size_t)255U;
         if (dw_bytes + (size_t)splits * M * sizeof(float) > be->ws_bytes / 2U) {

@@ -130,3 +130,20 @@ def test_greedy_generation_batch_edges(dtype, batch, vocab, window, prompt):
         for a, b in zip(caches, model.k_cache + model.v_cache):
             close(host(b), a, dtype, scale=2)
     assert np.array_equal(got, want)
+
+
+# enough tiles for one k-slice (both results written directly), with ragged edges in all three extents; one tile fewer than that takes slices
+@pytest.mark.parametrize("dtype", [F16, BF16])
+@pytest.mark.parametrize("m,n,k", [(2560, 1024, 200), (2568, 1032, 72), (4096, 776, 1096), (1024, 1024, 2048)])
+def test_weight_gradient_with_column_sums(ctx, dtype, m, n, k):
+    r, sd = np.random.default_rng(m + k), storage_name(dtype)
+    a, b = (rnd_np(r.standard_normal(s).astype(np.float32), dtype) for s in ((k, m), (k, n)))
+    ctx.begin_step()
+    y, s = ctx.scratch_empty(dtype, (m, n)), ctx.scratch_empty(dtype, (m,))
+    am, bm, ym, sv = dev(ctx, a, dtype).mv(k, m), dev(ctx, b, dtype).mv(k, n), y.mv(m, n), s.vv()
+    ctx.check(ctx.lib.gdb200_matmul_tn_colsum(ctx.backend, C.byref(am), C.byref(bm), C.byref(ym), C.byref(sv)), "tn_colsum")
+    ctx.flush()
+    scale = np.sqrt(k) / 8
+    close(host(y), O.rnd(torch.from_numpy(a).t() @ torch.from_numpy(b), sd), dtype, scale=scale, what="dW")
+    close(host(s), O.rnd(torch.from_numpy(a).sum(dim=0), sd), dtype, scale=scale, what="db")
+    ctx.end_step()
