@@ -287,9 +287,10 @@ __global__ void rms_bwd_kernel(const T *x, const T *w, const float *inv_in, cons
 // gradient is accumulated) with cp.async and reads them back itself, so two rows per warp (96 KB per SM) are in flight
 // while one is consumed, with no register cost and no synchronisation between lanes. The lane accumulates g * x * inv of
 // its 16 columns over its rows; the warps of a block are summed through shared memory into partial[blockIdx.x, cols]
-// (FP32), and the block that arrives last (ticket) sums the blocks' partials in block order and rounds dw once, so the
-// result does not depend on which block was last. dx is computed exactly as rms_bwd_kernel does.
+// (FP32), which are merged in a fixed order by the blocks that arrive last (tickets) and rounded once, so the result does not depend
+// on which block was last. 18.4 k rows of 512 with mask and its column sums: 31 -> 27 us (2304 rows: 14.4 -> 11.7). dx is computed exactly as rms_bwd_kernel does.
 constexpr int RBW_WARPS = 16, RBW_MAX_COLS = 512, RBW_DEPTH = 3;
+constexpr unsigned RBW_GROUP = 16;   // rows of partial sums a thread adds at a time; 256 blocks at most
 constexpr int RBW_ROW_BYTES = RBW_MAX_COLS * 2;                          // one 16-bit row
 constexpr int RBW_MASK_BYTES = RBW_MAX_COLS;                             // one byte per element of a dropout mask row
 constexpr int RBW_SLOT_BYTES = 3 * RBW_ROW_BYTES + RBW_MASK_BYTES;       // x, g, dx, mask
@@ -433,30 +434,41 @@ rms_bwd_wgrad_kernel(const T *__restrict__ x, const T *__restrict__ w, const flo
         __syncthreads();
         publish(csacc, (size_t)gridDim.x + blockIdx.x);
     }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(ticket, 1U) == gridDim.x - 1U;
-    __syncthreads();
-    if (last) {
+    // Merge in two levels: the last block of a group of at most RBW_GROUP adds the group's rows in block order, the last group adds the
+    // groups' sums in order. One thread per column and all its loads in flight: one block that walked over the 148 rows of both
+    // slabs with eight loads in flight took 3-4 us more, behind which the next launch waited.
+    // (up to RBW_GROUP blocks: every block a group)
+    const unsigned per = (gridDim.x + RBW_GROUP - 1U) / RBW_GROUP, group = blockIdx.x / per, groups = (gridDim.x + per - 1U) / per;
+    const unsigned members = min(per, gridDim.x - group * per), slabs = masked_colsum != nullptr ? 2U : 1U;
+    auto arrive = [&](unsigned *word, unsigned n) {
         __threadfence();
-        auto merge = [&](const float *slab, T *out) {
-            for (size_t c = threadIdx.x; c < cols; c += blockDim.x) {
-                float s = 0.0f;
-                unsigned b = 0;
-                for (; b + 8U <= gridDim.x; b += 8U) {   // eight loads in flight, summed in block order
-                    float t[8];
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            last = atomicAdd(word, 1U) == n - 1U;
+            if (last) *word = 0U;
+        }
+        __syncthreads();
+        if (last) __threadfence();
+        return last;
+    };
+    // sum of n rows of a slab, `step` rows apart from row `first` on
+    auto row_sum = [&](const float *slab, unsigned first, unsigned n, unsigned step, size_t c) {
+        float t[RBW_GROUP], sum = 0.0f;
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) t[u] = __ldcg(&slab[(size_t)(b + u) * cols + c]);
+        for (unsigned u = 0; u < RBW_GROUP; ++u) t[u] = u < n ? __ldcg(&slab[(size_t)(first + u * step) * cols + c]) : 0.0f;
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) s += t[u];
-                }
-                for (; b < gridDim.x; ++b) s += __ldcg(&slab[(size_t)b * cols + c]);
-                gdb_io<T>::st(out, c, s);
-            }
-        };
-        merge(partial, dw);
-        if (masked_colsum != nullptr) merge(partial + (size_t)gridDim.x * cols, masked_colsum);
-        if (threadIdx.x == 0) *ticket = 0U;
+        for (unsigned u = 0; u < RBW_GROUP; ++u) sum += t[u];
+        return sum;
+    };
+    if (per > 1U && !arrive(ticket + 1U + group, members)) return;
+    for (unsigned k = 0; per > 1U && k < slabs; ++k) {
+        float *slab = partial + (size_t)k * gridDim.x * cols;
+        for (size_t c = threadIdx.x; c < cols; c += blockDim.x) slab[(size_t)group * per * cols + c] = row_sum(slab, group * per, members, 1U, c);
+    }
+    if (!arrive(ticket, groups)) return;
+    for (unsigned k = 0; k < slabs; ++k) {
+        const float *slab = partial + (size_t)k * gridDim.x * cols;
+        for (size_t c = threadIdx.x; c < cols; c += blockDim.x) gdb_io<T>::st(k == 0U ? dw : masked_colsum, c, row_sum(slab, 0U, groups, per, c));
     }
 }
 
@@ -787,6 +799,7 @@ gd_status gdb_rms_norm_backward_with_weight(gd_backend *be, const gd_backend_ten
     }
     if (blocks > need) blocks = need;
     if (blocks > room) blocks = room;   // one FP32 row of partial sums per block
+    if (blocks > RBW_GROUP * RBW_GROUP) blocks = RBW_GROUP * RBW_GROUP;
     unsigned *ticket = gdb_tickets(be);
     {
         static bool configured = false;   // one device per process
