@@ -59,13 +59,15 @@ constexpr int P_SMEM_TOTAL_SWIGLU = (P_STAGES_DEFAULT - 1) * P_STAGE_BYTES + P_E
 // (the rounding point of the separate swiglu_split_backward call, src/ops/swiglu_split_linear/core_swiglu_split_linear.c:303-420).
 // x1 / x2 come from the saved [M, 2F] x12 matrix, which tma_act maps, 32 x 64 tiles at a time into the staging buffers the results leave
 // from; tma_c maps d_x12 [M, 2F].
-template <typename T, bool A_MN, bool B_MN, bool SPLITK, bool COLSUM, bool SWIGLU = false, bool SWIGLU_BWD = false>
+// HALVES: a unit is 128 columns of a tile (two units per tile), for launches of few tiles.
+template <typename T, bool A_MN, bool B_MN, bool SPLITK, bool COLSUM, bool SWIGLU = false, bool SWIGLU_BWD = false, bool HALVES = false>
 __global__ void __launch_bounds__(P_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  const __grid_constant__ CUtensorMap tma_c, const T *__restrict__ bias, uint32_t M, uint32_t N, uint32_t K,
                  uint32_t tiles_m, uint32_t tiles_n, uint32_t splits, uint32_t k_iters_per_split, int bias_mode, int *err_flag,
                  float *__restrict__ colsum_partial, const __grid_constant__ CUtensorMap tma_act, T *__restrict__ colsum_out)
 {
+    static_assert(!HALVES || (!SPLITK && !COLSUM && !SWIGLU && !SWIGLU_BWD), "half tiles belong to the plain direct output");
     static_assert(!SWIGLU || (!SPLITK && !A_MN && !B_MN), "the SwiGLU epilogue belongs to y = x w^T with direct output");
     static_assert(!SWIGLU_BWD || (!SPLITK && !A_MN && !B_MN && !SWIGLU), "the SwiGLU backward epilogue belongs to dact = g w^T with direct output");
     // The SwiGLU epilogue stages three output tiles per warp (x1, x2, act) instead of two alternating ones: it runs with
@@ -84,7 +86,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     const uint32_t rank = cluster_ctarank();
     const uint32_t cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
     const uint32_t total_k_iters = (K + BK - 1) / BK;
-    const uint32_t units = tiles_m * tiles_n * splits;
+    const uint32_t units = HALVES ? 2U * tiles_m * tiles_n : tiles_m * tiles_n * splits;
+    constexpr int UN = HALVES ? PBN / 2 : PBN;   // columns of a unit
 
     const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[PSTAGES]);
     const uint32_t tfull0 = smem_u32(&bars[2 * PSTAGES]), tempty0 = smem_u32(&bars[2 * PSTAGES + 2]);
@@ -126,8 +129,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             uint32_t it = 0;
             bool ok = true;
             for (uint32_t u = cluster_id; u < units && ok; u += n_clusters) {
-                const uint32_t tn = u % tiles_n, tm = (u / tiles_n) % tiles_m, z = u / (tiles_n * tiles_m);
-                const int am = (int)(tm * 2 * BM + rank * BM), bn = SWIGLU ? (int)(tn * (PBN / 2) + rank * N) : (int)(tn * PBN + rank * (PBN / 2));
+                const uint32_t tile = HALVES ? u >> 1 : u, tn = tile % tiles_n, tm = (tile / tiles_n) % tiles_m, z = tile / (tiles_n * tiles_m);
+                const int am = (int)(tm * 2 * BM + rank * BM);
+                const int bn = SWIGLU ? (int)(tn * (PBN / 2) + rank * N) : (int)(tn * PBN + (HALVES ? (u & 1U) * UN : 0U) + rank * (UN / 2));
                 const uint32_t k_begin = z * k_iters_per_split;
                 const uint32_t k_end = min(total_k_iters, k_begin + k_iters_per_split);
                 for (uint32_t kb = k_begin; kb < k_end; ++kb, ++it) {
@@ -138,7 +142,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                         break;
                     }
                     if (rank == 0) {
-                        mbar_expect_tx(full0 + 8 * s, 2 * P_STAGE_BYTES);
+                        mbar_expect_tx(full0 + 8 * s, HALVES ? 2 * P_STAGE_BYTES - P_B_BYTES : 2 * P_STAGE_BYTES);
                     }
                     const uint32_t a_dst = smem_u32(smem + s * P_STAGE_BYTES), b_dst = a_dst + P_A_BYTES;
                     const uint32_t bar = full_leader + 8 * s;
@@ -151,9 +155,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                     }
                     if (B_MN) {
                         tma_load_2d_pair(b_dst, &tma_b, bn, k0, bar);
-                        tma_load_2d_pair(b_dst + BK * 128, &tma_b, bn + 64, k0, bar);
+                        if (!HALVES) tma_load_2d_pair(b_dst + BK * 128, &tma_b, bn + 64, k0, bar);
                     } else {
-                        tma_load_2d_pair(b_dst, &tma_b, k0, bn, bar);
+                        tma_load_2d_pair(b_dst, &tma_b, k0, bn, bar);   // (HALVES: the map's box has 64 rows)
                     }
                 }
             }
@@ -163,11 +167,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         if (lane == 0 && rank == 0) {
             constexpr uint32_t FMT = std::is_same<T, __nv_bfloat16>::value ? 1U : 0U;
             constexpr uint32_t IDESC = (1U << 4) | (FMT << 7) | (FMT << 10) | ((A_MN ? 1U : 0U) << 15) | ((B_MN ? 1U : 0U) << 16) |
-                                       ((uint32_t)(PBN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
+                                       ((uint32_t)(UN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
             uint32_t it = 0, unit_idx = 0;
             bool ok = true;
             for (uint32_t u = cluster_id; u < units && ok; u += n_clusters, ++unit_idx) {
-                const uint32_t z = u / (tiles_n * tiles_m);
+                const uint32_t z = HALVES ? 0U : u / (tiles_n * tiles_m);
                 const uint32_t k_begin = z * k_iters_per_split;
                 const uint32_t k_end = min(total_k_iters, k_begin + k_iters_per_split);
                 const uint32_t buf = COLSUM ? 0U : (unit_idx & 1U), acc_ph = COLSUM ? (unit_idx & 1U) : ((unit_idx >> 1) & 1U);
@@ -228,7 +232,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         };
         if (SWIGLU_BWD && lane == 0) load_x12(cluster_id, chalf * 2);
         for (uint32_t u = cluster_id; u < units; u += n_clusters, ++unit_idx) {
-            const uint32_t tn = u % tiles_n, tm = (u / tiles_n) % tiles_m, z = u / (tiles_n * tiles_m);
+            const uint32_t tile = HALVES ? u >> 1 : u, tn = tile % tiles_n, tm = (tile / tiles_n) % tiles_m, z = tile / (tiles_n * tiles_m);
             const uint32_t buf = COLSUM ? 0U : (unit_idx & 1U), acc_ph = COLSUM ? (unit_idx & 1U) : ((unit_idx >> 1) & 1U);
             const bool got = mbar_wait(tfull0 + 8 * buf, acc_ph);
             if (!got) {
@@ -372,7 +376,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                 }
                 continue;
             }
-            constexpr int NCH = PBN / CHUNK_COLS / 2;   // chunks per warp
+            constexpr int NCH = UN / CHUNK_COLS / 2;   // chunks per warp
 #pragma unroll 1
             for (int c = chalf * NCH; c < (chalf + 1) * NCH; ++c) {
                 uint32_t v0[32], v1[32];
@@ -390,7 +394,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                 unsigned char *sb = my_stage + (store_cnt & 1U) * 4096;
                 if (lane == 0) bulk_wait_group_read<1>();   // the store that last used this buffer has read it
                 __syncwarp();
-                const uint32_t col0 = tn * PBN + c * CHUNK_COLS;
+                const uint32_t col0 = tn * PBN + (HALVES ? (u & 1U) * UN : 0U) + c * CHUNK_COLS;
                 unsigned char *rowp = sb + lane * 128;
                 if (SPLITK) {
 #pragma unroll
@@ -466,13 +470,13 @@ int max_clusters(gd_backend *be, const void *kern, int smem_bytes)
     return n < be->sm_count / 2 ? n : be->sm_count / 2;
 }
 
-template <typename T, bool A_MN, bool B_MN, bool SPLITK, bool COLSUM = false, bool SWIGLU = false, bool SWIGLU_BWD = false>
+template <typename T, bool A_MN, bool B_MN, bool SPLITK, bool COLSUM = false, bool SWIGLU = false, bool SWIGLU_BWD = false, bool HALVES = false>
 gd_status launch_pair(gd_backend *be, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &tc, const void *bias, uint32_t M,
                       uint32_t N, uint32_t K, uint32_t tiles_m, uint32_t tiles_n, uint32_t splits, uint32_t kps, int bias_mode, int *clusters_out,
                       float *colsum_partial = nullptr, const CUtensorMap *tact = nullptr, void *colsum_out = nullptr)
 {
     constexpr int SMEM = SWIGLU ? P_SMEM_TOTAL_SWIGLU : (COLSUM ? P_SMEM_TOTAL_COLSUM : P_SMEM_TOTAL);
-    auto kern = gemm_pair_kernel<T, A_MN, B_MN, SPLITK, COLSUM, SWIGLU, SWIGLU_BWD>;
+    auto kern = gemm_pair_kernel<T, A_MN, B_MN, SPLITK, COLSUM, SWIGLU, SWIGLU_BWD, HALVES>;
     static int clusters = -1;
     if (clusters < 0) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
@@ -488,8 +492,8 @@ gd_status launch_pair(gd_backend *be, const CUtensorMap &ta, const CUtensorMap &
     if (clusters <= 0) {
         return GD_ERR_UNSUPPORTED;
     }
-    const uint32_t units = tiles_m * tiles_n * splits;
     const int usable = clusters - (be->sm_reserve + 1) / 2 > 0 ? clusters - (be->sm_reserve + 1) / 2 : 1;
+    const uint32_t units = (HALVES ? 2U : 1U) * tiles_m * tiles_n * splits;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -516,11 +520,12 @@ gd_status launch_pair(gd_backend *be, const CUtensorMap &ta, const CUtensorMap &
 template <typename T>
 gd_status dispatch_pair(gd_backend *be, int ta, int tb, bool sk, const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc,
                         const void *bias, uint32_t M, uint32_t N, uint32_t K, uint32_t tiles_m, uint32_t tiles_n, uint32_t splits,
-                        uint32_t kps, int bias_mode, int *clusters_out)
+                        uint32_t kps, int bias_mode, int *clusters_out, bool halves = false)
 {
-#define GDB_GO(AM, BMJ)                                                                                                         \
-    (sk ? launch_pair<T, AM, BMJ, true>(be, ma, mb, mc, bias, M, N, K, tiles_m, tiles_n, splits, kps, bias_mode, clusters_out) \
-        : launch_pair<T, AM, BMJ, false>(be, ma, mb, mc, bias, M, N, K, tiles_m, tiles_n, splits, kps, bias_mode, clusters_out))
+#define GDB_GO(AM, BMJ)                                                                                                                               \
+    (halves ? launch_pair<T, AM, BMJ, false, false, false, false, true>(be, ma, mb, mc, bias, M, N, K, tiles_m, tiles_n, 1, kps, bias_mode, clusters_out) \
+     : sk   ? launch_pair<T, AM, BMJ, true>(be, ma, mb, mc, bias, M, N, K, tiles_m, tiles_n, splits, kps, bias_mode, clusters_out)                         \
+            : launch_pair<T, AM, BMJ, false>(be, ma, mb, mc, bias, M, N, K, tiles_m, tiles_n, splits, kps, bias_mode, clusters_out))
     if (ta) {
         return tb ? GDB_GO(true, false) : GDB_GO(true, true);
     }
@@ -600,13 +605,17 @@ gd_status gdb_gemm_tcgen05_pair(gd_backend *be, int ta, int tb, uint32_t dtype, 
         return st;
     }
     const bool sk = splits > 1U;
+    // Few tiles: two units of 128 columns each, twice the SMs at work (an output element is the same chain of products either way). Behind
+    // whole waves the same split of the last one gained nothing: its idle SMs leave the others the bandwidth (57600 x 512 x 512: 34.2 us
+    // against 35.7 with a last wave of halves). 2560 x 512 x 512: 10.4 -> 8.8 us, 4096 x 512 x 512: 10.6 -> 8.5 us.
+    const bool halves = !sk && tiles * 2U <= (uint32_t)clusters;
     const bool okc = sk ? make_tmap_f32_3d(&mc, be->ws, splits, M, N, 32) : make_tmap(&mc, dtype, c, M, N, ldc_bytes, 64, 32);
-    if (!okc) {
+    if (!okc || (halves && tb && !make_tmap(&mb, dtype, b, N, K, ldb_bytes, BK, PBN / 4))) {
         return GD_ERR_UNSUPPORTED;
     }
     st = dtype == GDB_DTYPE_F16
-             ? dispatch_pair<__half>(be, ta, tb, sk, ma, mb, mc, bias, M, N, K, tiles_m, tiles_n, splits, kps, bias_mode, nullptr)
-             : dispatch_pair<__nv_bfloat16>(be, ta, tb, sk, ma, mb, mc, bias, M, N, K, tiles_m, tiles_n, splits, kps, bias_mode, nullptr);
+             ? dispatch_pair<__half>(be, ta, tb, sk, ma, mb, mc, bias, M, N, K, tiles_m, tiles_n, splits, kps, bias_mode, nullptr, halves)
+             : dispatch_pair<__nv_bfloat16>(be, ta, tb, sk, ma, mb, mc, bias, M, N, K, tiles_m, tiles_n, splits, kps, bias_mode, nullptr, halves);
     if (st == GD_OK) {
         *splits_out = splits;
     }

@@ -147,3 +147,20 @@ def test_weight_gradient_with_column_sums(ctx, dtype, m, n, k):
     close(host(y), O.rnd(torch.from_numpy(a).t() @ torch.from_numpy(b), sd), dtype, scale=scale, what="dW")
     close(host(s), O.rnd(torch.from_numpy(a).sum(dim=0), sd), dtype, scale=scale, what="db")
     ctx.end_step()
+
+
+# a last wave of tiles in halves: the only wave, behind whole waves, with a half that lies behind the last column, ragged k and rows
+@pytest.mark.parametrize("dtype", [F16, BF16])
+@pytest.mark.parametrize("m,n,k", [(2560, 512, 264), (2600, 392, 72), (19200, 264, 128), (9728, 512, 520)])
+def test_contractions_with_half_tiles_in_the_last_wave(ctx, dtype, m, n, k):
+    r, sd, lib = np.random.default_rng(m + n), storage_name(dtype), ctx.lib
+    a, b = (rnd_np(r.standard_normal(s).astype(np.float32), dtype) for s in ((m, k), (k, n)))
+    want = O.rnd(torch.from_numpy(a) @ torch.from_numpy(b), sd)
+    ctx.begin_step()
+    for fn, x, w in ((lib.gd_backend_matmul, a, b), (lib.gd_backend_matmul_nt, a, b.T.copy()), (lib.gd_backend_matmul_tn, a.T.copy(), b)):
+        y = ctx.scratch_empty(dtype, (m, n))
+        xm, wm, ym = dev(ctx, x, dtype).mv(*x.shape), dev(ctx, w, dtype).mv(*w.shape), y.mv(m, n)
+        ctx.check(fn(ctx.backend, C.byref(xm), C.byref(wm), C.byref(ym)), "matmul")
+        ctx.flush()
+        close(host(y), want, dtype, scale=np.sqrt(k) / 8)
+    ctx.end_step()
