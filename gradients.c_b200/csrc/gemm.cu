@@ -247,7 +247,9 @@ gd_status gdb_gemm_dispatch(gd_backend *be, int ta, int tb, const gd_backend_mat
     const void *wp = w->buffer->dptr + w->offset;
     void *cp = y->buffer->dptr + y->offset;
     profile_scope scope(be, 2.0 * M * N * K, (double)es * ((double)M * K + (double)K * N + (double)M * N));
-    if (be->gemm_mode != 1 && be->gemm_mode != 2 && !ta && M <= 64U) {
+    // up to 64 rows: the staged kernel (K in chunks of 128), else the tensor path, else the direct kernel, whose loads wait for one another
+    const bool skinny = be->gemm_mode != 1 && be->gemm_mode != 2 && !ta && M <= 64U;
+    if (skinny && ((K % 128U) == 0U || be->gemm_mode == 3)) {
         gd_status st = gdb_gemm_skinny(be, tb, dt, ap, x->row_bytes, wp, w->row_bytes, cp, y->row_bytes, bp, bias_mode, M, N, K);
         if (st != GD_ERR_UNSUPPORTED) {
             return st;
@@ -263,6 +265,12 @@ gd_status gdb_gemm_dispatch(gd_backend *be, int ta, int tb, const gd_backend_mat
         }
     } else if (be->gemm_mode == 2) {
         return GD_ERR_UNSUPPORTED;
+    }
+    if (skinny) {
+        gd_status st = gdb_gemm_skinny(be, tb, dt, ap, x->row_bytes, wp, w->row_bytes, cp, y->row_bytes, bp, bias_mode, M, N, K);
+        if (st != GD_ERR_UNSUPPORTED) {
+            return st;
+        }
     }
     if (dt == GDB_DTYPE_F16) {
         launch_portable<__half>(be, ta, tb, ap, x->row_bytes / es, wp, w->row_bytes / es, cp, y->row_bytes / es, bp, M, N, K, 1, 0, 0, 0, bias_mode);

@@ -393,10 +393,13 @@ gd_status gdb_gemm_tcgen05(gd_backend *be, int ta, int tb, uint32_t dtype, const
     if (dtype != GDB_DTYPE_F16 && dtype != GDB_DTYPE_BF16) {
         return GD_ERR_UNSUPPORTED;
     }
-    // TMA needs 16-byte aligned bases and pitches; vector stores need N % 8 == 0; tiny problems are
-    // cheaper on the portable kernel than a 128-row tile with bounded-wait pipeline set-up.
+    // TMA needs 16-byte aligned bases and pitches; vector stores need N % 8 == 0. Rows and the contraction are clipped by the tensor maps
+    // and may have any length: a weight gradient over 1500 tokens, not a multiple of eight, took 230 us on the portable kernel (12.5 now),
+    // 33 rows times [1000, 3000] 411 us (7 now). Short contractions of small results (weight gradients of a few tokens) are
+    // cheaper there than a 128-row tile with its pipeline's set-up.
+    const bool small = (ta && M < 64U) || N < 64U || (K < 64U && (!ta || (uint64_t)M * N * K < ((uint64_t)1 << 24)));
     if ((((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) % 16U) != 0U || (lda_bytes % 16U) != 0U || (ldb_bytes % 16U) != 0U ||
-        (ldc_bytes % 16U) != 0U || (N % 8U) != 0U || (K % 8U) != 0U || M < 64U || N < 64U || K < 64U) {
+        (ldc_bytes % 16U) != 0U || (N % 8U) != 0U || small) {
         return GD_ERR_UNSUPPORTED;
     }
     if (bias != NULL && ((uintptr_t)bias % 2U) != 0U) {
@@ -455,7 +458,7 @@ gd_status gdb_gemm_tcgen05_tn_colsum(gd_backend *be, uint32_t dtype, const void 
 {
     if ((dtype != GDB_DTYPE_F16 && dtype != GDB_DTYPE_BF16) || be->gemm_mode == 1 || be->gemm_mode == 3 || colsum == NULL ||
         (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) % 16U) != 0U || (lda_bytes % 16U) != 0U || (ldb_bytes % 16U) != 0U ||
-        (ldc_bytes % 16U) != 0U || (N % 8U) != 0U || (K % 8U) != 0U) {
+        (ldc_bytes % 16U) != 0U || (N % 8U) != 0U) {
         return GD_ERR_UNSUPPORTED;
     }
     uint32_t splits = 1;

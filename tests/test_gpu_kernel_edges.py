@@ -134,7 +134,8 @@ def test_greedy_generation_batch_edges(dtype, batch, vocab, window, prompt):
 
 # enough tiles for one k-slice (both results written directly), with ragged edges in all three extents; one tile fewer than that takes slices
 @pytest.mark.parametrize("dtype", [F16, BF16])
-@pytest.mark.parametrize("m,n,k", [(2560, 1024, 200), (2568, 1032, 72), (4096, 776, 1096), (1024, 1024, 2048)])
+@pytest.mark.parametrize("m,n,k", [(2560, 1024, 200), (2568, 1032, 72), (4096, 776, 1096), (1024, 1024, 2048), (1536, 512, 1501),
+                                   (3000, 1000, 33), (136, 72, 65)])
 def test_weight_gradient_with_column_sums(ctx, dtype, m, n, k):
     r, sd = np.random.default_rng(m + k), storage_name(dtype)
     a, b = (rnd_np(r.standard_normal(s).astype(np.float32), dtype) for s in ((k, m), (k, n)))
@@ -163,4 +164,23 @@ def test_contractions_with_half_tiles_in_the_last_wave(ctx, dtype, m, n, k):
         ctx.check(fn(ctx.backend, C.byref(xm), C.byref(wm), C.byref(ym)), "matmul")
         ctx.flush()
         close(host(y), want, dtype, scale=np.sqrt(k) / 8)
+    ctx.end_step()
+
+
+# few rows with contractions that are no multiple of the staged kernel's chunk, or of eight; a last tile of one row
+@pytest.mark.parametrize("dtype", [F16, BF16])
+@pytest.mark.parametrize("m,n,k", [(1, 176, 312), (33, 3000, 1000), (64, 128, 136), (65, 264, 72), (129, 1000, 128)])
+def test_contractions_of_few_rows(ctx, dtype, m, n, k):
+    r, sd, lib = np.random.default_rng(m + n), storage_name(dtype), ctx.lib
+    a, w, b = (rnd_np(r.standard_normal(s).astype(np.float32), dtype) for s in ((m, k), (n, k), (n,)))
+    ta, tw = torch.from_numpy(a), torch.from_numpy(w)
+    ctx.begin_step()
+    y, dx, wt = ctx.scratch_empty(dtype, (m, n)), ctx.scratch_empty(dtype, (m, n)), dev(ctx, w.T.copy(), dtype)
+    am, wm, ym, xm, tm, bv = dev(ctx, a, dtype).mv(m, k), dev(ctx, w, dtype).mv(n, k), y.mv(m, n), dx.mv(m, n), wt.mv(k, n), dev(ctx, b, dtype).vv()
+    ctx.check(lib.gdb200_matmul_nt_bias(ctx.backend, C.byref(am), C.byref(wm), C.byref(bv), C.byref(ym)), "nt_bias")
+    ctx.check(lib.gd_backend_matmul(ctx.backend, C.byref(am), C.byref(tm), C.byref(xm)), "matmul")
+    ctx.flush()
+    product = O.rnd(ta @ tw.t(), sd)
+    close(host(dx), product, dtype, scale=np.sqrt(k) / 8)
+    close(host(y), O.rnd(product + torch.from_numpy(b), sd), dtype, scale=np.sqrt(k) / 8)
     ctx.end_step()
