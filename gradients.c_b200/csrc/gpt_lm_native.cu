@@ -674,7 +674,7 @@ extern "C" gd_status gdb200_gpt_train_step(gd_backend *be, const gdb200_gpt_spec
     // Weight gradients feed nothing before the optimizer: they go to the side stream, forked behind the loss, the MLP branch and the
     // attention branch of every block, and run beside the chain of input gradients, whose kernels leave SMs idle (most of them on a
     // small batch, their last waves on a large one). What they read must then stay: scratch is not reused from block to block, and with
-    // dropout, whose branch gradients are buffers of their own, nothing they read is added to in place. Same kernels, same bits.
+    // dropout, whose branch gradients are buffers of their own, nothing they read is added to in place (the head's logits: see side_head). Same kernels, same bits.
     // Two-layer model of the smoke test: 336 -> 275 us per step; reference-default model, 8 / 32 sequences: 1015 -> 929 / 1632 -> 1492 us;
     // benchmark model, 64 / 200 sequences: 2945 -> 2923 / 8022 -> 7916 us.
     const size_t block_scratch = (size_t)T * es * (size_t)(3 * F + 16 * D) + ((size_t)4 * (size_t)be->sm_count * (size_t)D + 4096U) * 4U;
@@ -691,11 +691,14 @@ extern "C" gd_status gdb200_gpt_train_step(gd_backend *be, const gdb200_gpt_spec
     };
     const Ten none = {};
     gd_backend_tensor_view cvn = tv(counts);
+    // The head's weight gradient may leave `stream` here only when `saved_logits` holds the gradient already. Without the one-pass kernel
+    // the backward chunk below still has to turn the logits into it, in place, and the contraction stays behind that chunk.
+    const bool side_head = side && fused_ce;
     if (fused_ce && !dp && drop && !side) c.ok(gdb_lm_ce_reduce_normalize_global(be, &rlv, &cvn, &lov, &ivv), "lm_ce_reduce_normalize(rows)");
-    if (side) {
+    if (side_head) {
         fork();
         gdb_side on(be);
-        if (fused_ce) c.ok(gdb_lm_ce_reduce_normalize_global(be, &rlv, &cvn, &lov, &ivv), "lm_ce_reduce_normalize(rows)");   // the loss, for the host
+        c.ok(gdb_lm_ce_reduce_normalize_global(be, &rlv, &cvn, &lov, &ivv), "lm_ce_reduce_normalize(rows)");   // the loss, for the host
         linear_t_backward(c, final_norm, none, saved_logits, T, D, V, NULL, lmw_grad, grads[(size_t)P_LMB]);
     }
     for (int64_t start = 0; start < V && c.st == GD_OK; start += pass) {
@@ -729,7 +732,7 @@ extern "C" gd_status gdb200_gpt_train_step(gd_backend *be, const gdb200_gpt_spec
         }
         gd_backend_matrix_view dwm = mv(lmw_grad, (uint32_t)cc, (uint32_t)D, (size_t)start);
         gd_backend_vector_view dbv = vv(grads[(size_t)P_LMB], (size_t)start, (uint32_t)cc);
-        if (!side) c.ok(gdb200_matmul_tn_colsum(be, &lm, &hm, &dwm, &dbv), "matmul_tn_colsum(d_lm_w, d_lm_b)");
+        if (!side_head) c.ok(gdb200_matmul_tn_colsum(be, &lm, &hm, &dwm, &dbv), "matmul_tn_colsum(d_lm_w, d_lm_b)");
     }
     // Every RMSNorm backward below feeds the residual gradient, whose next consumer is the backward of the dropout in front of
     // the residual add (the MLP branch, the attention branch, the embedding): that gradient comes out of the same launch.
