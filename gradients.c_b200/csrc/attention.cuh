@@ -32,6 +32,8 @@ struct gdb_attn_bwd_meta {
     int *row_hi;       // [N]  last query that may see this key (-1: none)
     int *tile_nqt;     // [ceil(N / 128)]  64-row query tiles, from the key tile's own first row on, that may see one of its keys
 };
+// Workspace that the tensor-memory backward's preparation needs (it runs the general kernels with less).
+size_t gdb_attn_bwd_ws_bytes(int n_tokens, int hq);
 // tcgen05 / tensor-memory key-stationary backward (attention_tcgen05_bwd.cu): dK, dV and the FP32 dQ accumulator dq32
 // [N, Hq, Dh] (zero on entry). GD_ERR_UNSUPPORTED outside its fast path.
 gd_status gdb_attn5_backward(gd_backend *be, const gdb_flash_args *a, float *dq32, const gdb_attn_bwd_meta *m);

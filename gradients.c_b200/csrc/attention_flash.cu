@@ -771,8 +771,8 @@ gd_status backward_single_pass(gd_backend *be, const gdb_flash_args *a, const fl
     gdb_attn_bwd_meta m;
     memset(&m, 0, sizeof(m));
     m.n_pad = (a->n_tokens + 63) & ~63;
-    const size_t per_head = (size_t)m.n_pad * a->hq, tiles = (size_t)(a->n_tokens + 127) / 128U;
-    const bool tensor = be->attn_mode == 0 && a->n_tokens >= 128 && (2U * per_head + (size_t)m.n_pad + tiles) * sizeof(float) <= be->ws_bytes;
+    const size_t per_head = (size_t)m.n_pad * a->hq;
+    const bool tensor = be->attn_mode == 0 && a->n_tokens >= 128 && gdb_attn_bwd_ws_bytes(a->n_tokens, a->hq) <= be->ws_bytes;
     if (!tensor && DH != 64) {
         return GD_ERR_UNSUPPORTED;
     }
@@ -835,6 +835,12 @@ gd_status gdb_flash_varlen_backward(gd_backend *be, const gdb_flash_args *a, boo
     const flash_params p = make_params(a);
     return a->dtype == GDB_DTYPE_F16 ? backward_typed<__half>(be, a, p, have_forward_stats)
                                      : backward_typed<__nv_bfloat16>(be, a, p, have_forward_stats);
+}
+
+size_t gdb_attn_bwd_ws_bytes(int n_tokens, int hq)
+{
+    const size_t n_pad = ((size_t)n_tokens + 63U) & ~(size_t)63U, tiles = ((size_t)n_tokens + 127U) / 128U;
+    return (2U * n_pad * (size_t)hq + n_pad + tiles) * sizeof(float);
 }
 
 // Backward with the forward output at hand (not part of the reference's entry, src/core/backend.h:699-709): D = rowsum(dO o O)

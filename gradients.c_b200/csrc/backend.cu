@@ -173,6 +173,7 @@ gd_status gd_backend_create_default(gd_backend **out_backend)
     }
     be->sm_count = prop.multiProcessorCount;
     be->ws_bytes = env_size("GD_CUDA_WORKSPACE_MB", 512U) << 20;
+    be->split_bytes = be->ws_bytes / 2U;
     be->l2_flush_bytes = (size_t)256U << 20;
     if (cudaStreamCreateWithFlags(&be->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaMalloc((void **)&be->ws, be->ws_bytes) != cudaSuccess ||

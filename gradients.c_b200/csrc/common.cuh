@@ -39,7 +39,8 @@ struct gd_backend {
     // private workspace (split-K partials, reductions, attention scratch); created once at
     // create_default so no allocation happens while a step is being enqueued.
     unsigned char *ws;
-    size_t ws_bytes;
+    size_t ws_bytes;      // what the work enqueued now may use (half of the workspace while two streams share it)
+    size_t split_bytes;   // half of the workspace: limit of a contraction's partial slices, and the second stream's share
     int *err_flag;            // device int: set by kernels whose bounded waits gave up
     int *err_flag_host;       // pinned mirror
     float *rope_table;        // cos/sin table [512][32][2] for head_dim 64, theta 10000
@@ -74,20 +75,39 @@ struct gd_backend_buffer {
 
 static inline unsigned *gdb_tickets(const struct gd_backend *be) { return be->tickets; }
 
-// While it lives, what is enqueued through `be` goes to the side stream. Only contractions and reductions that keep to half of the
-// workspace (split-K partials do: ws_bytes / 2 is their limit) may be enqueued there; the caller orders the streams with the
-// two events.
+// From the first fork of the side stream to its join: what is enqueued on `stream` keeps to the lower half of the workspace.
+struct gdb_shared_ws {
+    gd_backend *be;
+    size_t whole;
+    gdb_shared_ws(gd_backend *b, bool shared) : be(b), whole(b->ws_bytes)
+    {
+        if (shared) be->ws_bytes = be->split_bytes;
+    }
+    ~gdb_shared_ws() { end(); }
+    gdb_shared_ws(const gdb_shared_ws &) = delete;
+    void end() { be->ws_bytes = whole; }
+};
+
+// While it lives, what is enqueued through `be` goes to the side stream, with the upper half of the workspace and the upper half of
+// the tickets (within a gdb_shared_ws, so that `stream` has the lower ones). The caller orders the streams with the two events.
 struct gdb_side {
     gd_backend *be;
-    explicit gdb_side(gd_backend *b) : be(b) { swap(b->ws_bytes / 2U, GDB_TICKET_WORDS); }
-    ~gdb_side() { swap((size_t)0 - be->ws_bytes / 2U, -(ptrdiff_t)GDB_TICKET_WORDS); }
-    gdb_side(const gdb_side &) = delete;
-    void swap(size_t ws, ptrdiff_t tickets)
+    size_t before;
+    explicit gdb_side(gd_backend *b) : be(b), before(b->ws_bytes)
     {
         std::swap(be->stream, be->side_stream);
-        be->ws += ws;
-        be->tickets += tickets;
+        be->ws += be->split_bytes;
+        be->ws_bytes = be->split_bytes;
+        be->tickets += GDB_TICKET_WORDS;
     }
+    ~gdb_side()
+    {
+        std::swap(be->stream, be->side_stream);
+        be->ws -= be->split_bytes;
+        be->ws_bytes = before;
+        be->tickets -= GDB_TICKET_WORDS;
+    }
+    gdb_side(const gdb_side &) = delete;
 };
 
 static inline gd_status gdb_fail(gd_backend *be, cudaError_t e, const char *what)

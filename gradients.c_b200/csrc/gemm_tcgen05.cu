@@ -432,7 +432,7 @@ gd_status gdb_gemm_tcgen05(gd_backend *be, int ta, int tb, uint32_t dtype, const
         splits = ((uint32_t)be->sm_count * 2U + tiles - 1U) / tiles;
         if (splits > total_k / 4U) splits = total_k / 4U;
         if (splits > 32U) splits = 32U;
-        while (splits > 1U && (size_t)splits * M * N * sizeof(float) > be->ws_bytes / 2U) --splits;
+        while (splits > 1U && (size_t)splits * M * N * sizeof(float) > be->split_bytes) --splits;
         if (splits < 1U) splits = 1U;
     }
     uint32_t kps = (total_k + splits - 1U) / splits;

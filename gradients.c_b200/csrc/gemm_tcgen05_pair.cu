@@ -569,7 +569,7 @@ gd_status gdb_gemm_tcgen05_pair(gd_backend *be, int ta, int tb, uint32_t dtype, 
     if (tiles * 2U <= (uint32_t)clusters && total_k >= 16U) {
         splits = (uint32_t)clusters / tiles;
         if (splits > total_k / 4U) splits = total_k / 4U;
-        while (splits > 1U && (size_t)splits * M * N * sizeof(float) > be->ws_bytes / 2U) --splits;
+        while (splits > 1U && (size_t)splits * M * N * sizeof(float) > be->split_bytes) --splits;
         if (splits < 1U) splits = 1U;
     }
     if (splits == 1U && tiles * 4U < (uint32_t)clusters) {
@@ -588,7 +588,7 @@ gd_status gdb_gemm_tcgen05_pair(gd_backend *be, int ta, int tb, uint32_t dtype, 
     }
     if (want_colsum) {
         const size_t dw_bytes = ((size_t)splits * M * N * sizeof(float) + 255U) & ~(size_t)255U;
-        if (dw_bytes + (size_t)splits * M * sizeof(float) > be->ws_bytes / 2U) {
+        if (dw_bytes + (size_t)splits * M * sizeof(float) > be->split_bytes) {
             return GD_ERR_UNSUPPORTED;
         }
         float *cs = reinterpret_cast<float *>(be->ws + dw_bytes);

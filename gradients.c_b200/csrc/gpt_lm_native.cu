@@ -15,6 +15,7 @@
 // normalised by the number of valid target rows of ALL ranks (counted and all-reduced at the start of
 // the step), so the summed gradients are those of the global batch without a division by the world size.
 #include "common.cuh"
+#include "attention.cuh"
 #include "decode_parts.cuh"
 
 #include <math.h>
@@ -678,7 +679,12 @@ extern "C" gd_status gdb200_gpt_train_step(gd_backend *be, const gdb200_gpt_spec
     // Two-layer model of the smoke test: 336 -> 275 us per step; reference-default model, 8 / 32 sequences: 1015 -> 929 / 1632 -> 1492 us;
     // benchmark model, 64 / 200 sequences: 2945 -> 2923 / 8022 -> 7916 us.
     const size_t block_scratch = (size_t)T * es * (size_t)(3 * F + 16 * D) + ((size_t)4 * (size_t)be->sm_count * (size_t)D + 4096U) * 4U;
-    const bool side = drop && !dp && single && c.top + (size_t)(L + 1) * block_scratch + (size_t)V * (size_t)D * 6U <= s->scratch_bytes;
+    // The streams share the workspace by halves: not where half of it is too little for the attention's preparation (all of it being
+    // enough) or for one row of column sums.
+    const size_t attn_ws = gdb_attn_bwd_ws_bytes((int)T, (int)H), widest = (size_t)std::max({V, 3 * D, 2 * F});
+    const bool halves = (attn_ws <= be->split_bytes || attn_ws > be->ws_bytes) && widest * sizeof(float) <= be->split_bytes;
+    const bool side = drop && !dp && single && halves && c.top + (size_t)(L + 1) * block_scratch + (size_t)V * (size_t)D * 6U <= s->scratch_bytes;
+    gdb_shared_ws shared_ws(be, side);
     auto fork = [&]() {
         if (c.st == GD_OK && (cudaEventRecord(be->side_fork, be->stream) != cudaSuccess || cudaStreamWaitEvent(be->side_stream, be->side_fork, 0) != cudaSuccess)) {
             c.ok(GD_ERR_INTERNAL, "side stream fork");
@@ -873,6 +879,7 @@ extern "C" gd_status gdb200_gpt_train_step(gd_backend *be, const gdb200_gpt_spec
         gd_backend_tensor_view gv = tv(gx), iv = tv(ids), tvw = tv(t2), sv2 = tv(scratch);
         c.ok(gd_backend_embedding_backward(be, &gv, &iv, &tvw, &sv2, &ea), "embedding_backward");
         if (side) join();   // (also with a step that failed half way: nothing is left running beside `stream`)
+        shared_ws.end();
         if (s->tied_lm_head) c.accumulate(emb_grad, target);
         reduce_range(emb_grad.off, (size_t)V * (size_t)D);
     }

@@ -84,3 +84,14 @@ def test_gradients_with_scratch_too_small_for_the_second_stream():
     narrow = step_gradients(g.NativeTrainer, *p, scratch=used[0], used=used)
     assert used[1] < used[0]      # scratch is reused from block to block
     agree(narrow, wide, F16)
+
+
+@pytest.mark.parametrize("mib,n_seqs", [(1, 64), (1, 192), (2, 64)])
+def test_gradients_with_a_small_workspace(monkeypatch, mib, n_seqs):
+    """Two streams share the workspace by halves. 64 sequences (2 k tokens of 16 heads): 0.26 MiB of attention statistics fit a half of either
+    workspace; 192: 0.81 MiB fit one MiB but not its half, and the step keeps to one stream. Column sums and partial sums get
+    half a MiB (256 MiB by default): other slices, FP32 rounding only."""
+    p = problem(vocab_size=2040, d_model=1024, n_heads=16, mlp_hidden=512, n_seqs=n_seqs)
+    want = step_gradients(g.NativeTrainer, *p, scratch=3 << 30)
+    monkeypatch.setenv("GD_CUDA_WORKSPACE_MB", str(mib))
+    agree(step_gradients(g.NativeTrainer, *p, scratch=3 << 30), want, F16)
