@@ -572,12 +572,7 @@ def greedy_generate(model: GptLm, prompts: np.ndarray, new_tokens: int, capacity
 def model_spec(model: GptLm) -> "abi.GptSpec":
     """gdb200_gpt_spec with the model fields and parameter locations only (what the decode driver reads)."""
     mc, ctx = model.cfg, model.ctx
-    # a model's parameters do not move: the description is kept until the arenas or the configuration change
-    key = (ctx.params, ctx.state, ctx.scratch, tuple(vars(mc).values()))
-    if getattr(model, "_spec_key", None) == key:
-        return model._spec
     s = abi.GptSpec()
-    model._spec_key, model._spec = key, s
     s.params_buffer, s.state_buffer, s.scratch_buffer = ctx.params.buffer, ctx.state.buffer, ctx.scratch.buffer
     s.scratch_bytes = ctx.scratch.capacity
     s.vocab_size, s.context_length, s.d_model, s.n_layers = mc.vocab_size, mc.context_length, mc.d_model, mc.n_layers
@@ -586,8 +581,8 @@ def model_spec(model: GptLm) -> "abi.GptSpec":
     s.logits_softcap, s.rms_eps, s.rope_theta, s.dropout_seed = mc.logits_softcap, mc.rms_eps, mc.rope_theta, mc.dropout_seed
     plist = model.param_list()
     s.n_params, s.dp_world = len(plist), 1
-    for i, t in enumerate(plist):
-        s.param_offset[i], s.param_count[i] = t.offset, t.count
+    s.param_offset[:len(plist)] = [t.offset for t in plist]
+    s.param_count[:len(plist)] = [t.count for t in plist]
     return s
 
 
