@@ -96,8 +96,8 @@ class Tensor:
     _count = _tv = _ref = None
 
     def __init__(self, ctx: "Context", arena: Arena, offset: int, dtype: int, shape: Sequence[int], name: str = ""):
-        self.ctx, self.arena, self.offset, self.dtype, self.name = ctx, arena, offset, dtype, name
-        self.shape = shape if type(shape) is tuple else tuple(map(int, shape))
+        self.ctx, self.arena, self.offset, self.dtype, self.name = ctx, arena, int(offset), dtype, name
+        self.shape = tuple(map(int, shape))
 
     @property
     def count(self) -> int:

@@ -3,6 +3,9 @@ from __future__ import annotations
 
 from types import SimpleNamespace
 
+import numpy as np
+import pytest
+
 from conftest import graft
 
 pkg = graft.load_package()
@@ -35,3 +38,13 @@ def test_model_description_follows_the_parameters():
     assert first.param_offset[names.index(moved)] == old.offset
     second.scratch_bytes = 1
     assert g.model_spec(model).scratch_bytes == model.ctx.scratch.capacity
+
+
+@pytest.mark.parametrize("offset,shape", [(np.int64(512), (np.int64(3), np.int32(4))), (512, [3, 4]), (np.uint32(512), np.array([3, 4])), (512, (3.0, 4))])
+def test_tensor_of_any_whole_numbers(offset, shape):
+    ctx = host_context()
+    t = runtime.Tensor(ctx, ctx.params, offset, abi.F16, shape)
+    assert t.shape == (3, 4) and all(type(v) is int for v in (t.offset, t.count, t.nbytes) + t.shape)
+    v = t.tv()
+    assert (v.offset, v.count, v.rank, list(v.shape[:2]), list(v.strides[:2])) == (512, 12, 2, [3, 4], [4, 1])
+    assert ctx.empty(ctx.params, abi.F16, shape).shape == (3, 4)
