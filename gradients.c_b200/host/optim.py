@@ -195,13 +195,15 @@ class AdamW:
                                                  self.grad_clip_scale.offset, max_grad_norm, GRAD_CLIP_SCALE_EPS), "grad_clip_scale")
         cfg = self.config
         bias_correction = 1 if cfg.bias_correction else 0
+        shared = (self.state_f32, self.state_i32, self.grad_clip_scale)   # a program may put others in their place
         for j, i in enumerate(active):
             s = self.slots[i]
             g = s.param.grad
             d = self._adamw_descs[j]
-            if self._laid_out[j] != (i, s.param, s.master, s.m, s.v):
+            written_for = (i, s.param, s.master, s.m, s.v) + shared
+            if self._laid_out[j] != written_for:
                 self._lay_out(d, i, s, first=j == 0)
-                self._laid_out[j] = (i, s.param, s.master, s.m, s.v)
+                self._laid_out[j] = written_for
             d.grad_buffer, d.grad_offset, d.grad_dtype = g.arena.buffer, g.offset, g.dtype
             d.found_inf_buffer, d.found_inf_offset = found_buf, found_off
             d.bias_correction = bias_correction

@@ -9,7 +9,7 @@ import pytest
 from conftest import graft
 
 pkg = graft.load_package()
-abi, g, runtime = pkg.abi, pkg.gpt_lm, pkg.runtime
+abi, g, optim, runtime = pkg.abi, pkg.gpt_lm, pkg.optim, pkg.runtime
 
 
 def host_context():
@@ -48,3 +48,31 @@ def test_tensor_of_any_whole_numbers(offset, shape):
     v = t.tv()
     assert (v.offset, v.count, v.rank, list(v.shape[:2]), list(v.strides[:2])) == (512, 12, 2, [3, 4], [4, 1])
     assert ctx.empty(ctx.params, abi.F16, shape).shape == (3, 4)
+
+
+def test_optimizer_descriptors_follow_replaced_state():
+    ctx, seen = host_context(), []
+    ctx.check = lambda st, what: None
+    ctx.lib = SimpleNamespace(gd_backend_grad_clip_scale=lambda *a: seen.append([("clip", a[4])]),
+                              gd_backend_adamw_batch=lambda be, d, n: seen[-1].extend((x.grad_scale_offset, x.beta1_power_offset, x.param_step_offset, x.m_offset)
+                                                                                      for x in d[:n]))
+    place = lambda count, dtype=abi.F32: ctx.empty(ctx.state, dtype, (count,))
+    opt = optim.AdamW.__new__(optim.AdamW)
+    opt.ctx, opt.config, opt.n = ctx, optim.AdamwConfig(1e-3, 0.9, 0.95, 1e-8, 0.0, True), 2
+    opt.slots = [optim.ParamSlot(ctx.empty(ctx.params, abi.F16, (8,)), 0.0, 1.0, place(8), place(8), place(8)) for _ in range(2)]
+    opt.state_f32, opt.state_i32, opt.partials, opt.grad_clip_scale = place(10), place(3, abi.I32), place(2), place(2)
+    opt._norm_descs, opt._adamw_descs, opt._laid_out = (abi.GradNormDesc * 2)(), (abi.AdamwDesc * 2)(), [None] * 2
+    scaler = SimpleNamespace(begin_step=lambda: None, finish_step=lambda: None, scale_state=place(2), flag_state=place(3, abi.I32))
+
+    def step():
+        for s in opt.slots:
+            s.param.grad = ctx.empty(ctx.scratch, abi.F16, (8,))
+        opt.step_amp_clip_lr(scaler, 1e-3, 1.0)
+        return seen[-1][1:]
+
+    want = lambda: [(opt.grad_clip_scale.offset, opt._f32_off(0, i), opt.state_i32.offset + 4 * i, opt.slots[i].m.offset) for i in range(2)]
+    assert step() == want() == step()
+    for replace in (lambda: setattr(opt, "state_f32", place(10)), lambda: setattr(opt, "state_i32", place(3, abi.I32)),
+                    lambda: setattr(opt, "grad_clip_scale", place(2)), lambda: setattr(opt.slots[1], "m", place(8))):
+        replace()
+        assert step() == want()
