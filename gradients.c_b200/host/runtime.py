@@ -185,9 +185,10 @@ class Context:
     reuse (memory.c:701); with one slot that is a wait for the previous step's fence at
     begin_step, which is what this class does by default (`run_ahead` 0). With `run_ahead` = n the
     host may enqueue up to n steps beyond the one the device is executing: begin_step then waits
-    only for the fence of step k - n. The device arenas need no ring for that, because every
-    kernel and every stream-ordered copy of step k + 1 is queued behind step k on the one in-order
-    stream; only host memory handed to write_async / read_async must be rotated by the caller.
+    only for the fence of step k - n. Of the device arenas only the data slot needs two places for
+    that (upload_beside copies a batch while the step before it runs): every kernel and every other
+    copy of step k + 1 is queued behind step k; host memory handed to write_async / read_async must
+    be rotated by the caller.
     """
 
     def __init__(self, params_bytes: int = 256 << 20, state_bytes: int = 512 << 20,
@@ -201,14 +202,18 @@ class Context:
         self.params = Arena(self, "params", params_bytes)
         self.state = Arena(self, "state", state_bytes)
         self.scratch = Arena(self, "scratch", scratch_bytes)
-        self.data = Arena(self, "data", data_bytes)
+        self._make_data_slot(data_bytes)
         self.tape: list[Callable[[], None]] = []
         self.grad_enabled = True
         self._fences: list[abi.Fence] = []
         self.run_ahead = 0
-        self._data_before, self._data_base = (0, 0), 0
         self.in_step = False
         self.grad_ready_hook: Optional[Callable[[Tensor], None]] = None
+
+    def _make_data_slot(self, nbytes: int) -> None:
+        """The data arena: twice what was asked for, because batches copied beside the running step alternate between its halves."""
+        self.data = Arena(self, "data", 2 * ((nbytes + ALIGN - 1) & ~(ALIGN - 1)))
+        self._data_before, self._data_base = (0, 0), 0
 
     # ---- plumbing ----
     def last_error(self) -> str:

@@ -76,3 +76,26 @@ def test_optimizer_descriptors_follow_replaced_state():
                     lambda: setattr(opt, "grad_clip_scale", place(2)), lambda: setattr(opt.slots[1], "m", place(8))):
         replace()
         assert step() == want()
+
+
+def test_data_slot_takes_what_it_was_asked_for_beside_a_running_step():
+    """Batches copied beside the running step alternate between two places; what a step adds to its batch has the asked-for size in both."""
+    def no_device(be, size, out):
+        out._obj.value = 0x9000
+        return abi.GD_OK
+    copies = []
+    lib = SimpleNamespace(gd_backend_buffer_create=no_device, gdb200_upload_beside=lambda be, buf, n, offs, src, sizes: copies.append((offs[0], offs[n - 1] + sizes[n - 1])) or 0)
+    ctx = runtime.Context.__new__(runtime.Context)
+    ctx.lib, ctx.backend, ctx.run_ahead, ctx.tape, ctx.in_step = lib, 1, 1, [], False
+    ctx.check, ctx.wait_steps = (lambda st, what: None), (lambda n: None)
+    lib.gd_backend_scope_begin = lambda be: 0
+    ctx.scratch = host_context().scratch
+    ctx._make_data_slot(10000)
+    batch = [np.zeros(n, dtype=np.int32) for n in (1100, 1100, 60)]
+    for step in range(4):
+        ctx.begin_step()
+        ts = ctx.upload_beside(batch)
+        assert ts is not None and copies[-1] == (ts[0].offset, ts[-1].offset + ts[-1].nbytes)
+        assert step == 0 or copies[-1][0] >= copies[-2][1] or copies[-2][0] >= copies[-1][1]
+        ctx.empty(ctx.data, abi.I32, (130,))    # 9992 bytes in use with it
+        ctx.in_step = False
