@@ -617,7 +617,7 @@ def greedy_generate_native(model: GptLm, prompts: np.ndarray, new_tokens: int, c
     words[at[4]:at[5]] = np.arange(1, b + 1, dtype=np.int32) * plen - 1
     words[at[6]:at[7]] = plen - 1
     ctx.begin_step()
-    io = ctx.from_numpy(ctx.data, I32, words)
+    io = ctx.from_numpy(ctx.data if words.nbytes <= ctx.data.capacity else ctx.state, I32, words)
     off = [io.offset + 4 * int(i) for i in at]
     batch = abi.GptBatch(io.buffer, off[0], 0, off[1], off[2], n, b + 1)
     d = abi.GptDecodeState()
