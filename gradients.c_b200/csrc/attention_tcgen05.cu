@@ -26,9 +26,12 @@
 // at the price of a second read of S: 83 us for 32768 tokens in sequences of 16-512, 8 heads, against 72 with O in tensor memory and
 // a maximum that may lag (124 with 128-key tiles one at a time, P through shared memory). Also measured: the product added before
 // the next exponentials instead of after them 89 us, two warps per row 95 us, skipping masked halves of a step by a branch 88 us.
-// head_dim 128: O (128 columns) does not fit the registers. It stays in tensor memory for the whole item and is rescaled there only
-// when a row's maximum has grown by more than 2^8 since the last rescale (the sum is kept relative to the same stale maximum);
-// after the first tile that is rare. 8191 tokens in sequences of 256-2048, 16 heads, window 1024: 78 us (mma.sync kernel: 286 us).
+// head_dim 128: O (128 columns) does not fit the registers. It stays in tensor memory for the whole item and is multiplied there by
+// alpha whenever the maximum of one of a warp's rows has grown (most of an item's first steps), behind the step's exponentials, so that
+// the product of the step before has finished by then. P is relative to the exact running maximum of every 64 keys: the largest
+// probability is then exactly 1 and takes no rounding. With a maximum that may lag by 2^8 (rescaling is rare) forward and backward of 8191
+// tokens in sequences of 256-2048, 16 heads, window 1024, took 414 us instead of 424, and the output's error against 64-bit arithmetic
+// was 2.06e-3 (bf16) and 2.59e-4 (f16, no window) instead of 1.99e-3 and 2.48e-4, as with the mma.sync kernel (forward alone 286 us).
 // Tensor memory per CTA (256 columns): S / P 3 x 64 or 2 x 64, O head_dim.
 //
 // Statistics written for the backward pass: (row max in natural-log units, sum of exp, 0).
@@ -61,8 +64,7 @@ struct attn5_plan {
     static constexpr int TMEM_COLS = 256;
     static constexpr uint32_t SBUF = DH == 64 ? 3 : 2;            // S / P buffers of A_BKV columns
     static constexpr uint32_t COL_S = 0, COL_O = SBUF * A_BKV;
-    static constexpr bool PAIRED = DH == 64;                      // O in registers, one maximum per 128 keys
-    static constexpr float RESCALE = 8.0f;                        // (otherwise) log2 of the growth of a row maximum that triggers a rescale of O
+    static constexpr bool PAIRED = DH == 64;                      // O in registers, one maximum per 128 keys; else in tensor memory, one per 64
 };
 
 __device__ __forceinline__ float ex2_approx(float x)
@@ -508,8 +510,7 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                     }
                 }
             } else {
-                // m: the maximum O and l are relative to (log2 units, may lag the true maximum by up to RESCALE); m_true: the maximum
-                float m_true = -INFINITY;
+                // m: the running maximum, exact after every step (log2 units); O in tensor memory and l are relative to it
                 l = 0.0f;
 #pragma unroll 1
                 for (int t = 0; t < n_tiles; ++t, ++g) {
@@ -532,28 +533,10 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                         float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
                         max_keys(v[0], mx);
                         max_keys(v[1], mx);
-                        const float m_cand = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl2;
-                        m_true = fmaxf(m_true, m_cand);
-                        const bool bump = m_cand > m + plan::RESCALE || (m == -INFINITY && m_cand != -INFINITY);
-                        if (__any_sync(0xffffffffU, bump)) {
-                            const float alpha = bump ? ex2_approx(m - m_cand) : 1.0f;   // m = -inf: 0
-                            if (__any_sync(0xffffffffU, bump && m != -INFINITY)) {
-                                wait_or_die(PV_DONE + (g - 1U) % NS, ((g - 1U) / NS) & 1U, 309);   // O holds every step before this one
-                                if (dead) break;
-                                tcgen05_fence_after();
-#pragma unroll 1
-                                for (int c = 0; c < DH / 16; ++c) {
-                                    uint32_t o[16];
-                                    tmem_ld_32x32b_x16_nowait(lane_base + plan::COL_O + c * 16, o);
-                                    tmem_ld_wait();
-#pragma unroll
-                                    for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                                    tmem_st_32x32b_x16(lane_base + plan::COL_O + c * 16, o);
-                                }
-                            }
-                            l *= alpha;
-                            if (bump) m = m_cand;
-                        }
+                        const float m_new = fmaxf(m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl2);
+                        const float alpha = m == m_new ? 1.0f : ex2_approx(m - m_new);   // (m = -inf: 0)
+                        const bool grown = __any_sync(0xffffffffU, m != m_new && m != -INFINITY);
+                        m = m_new;
                         const f32x2 scale2 = f2_make(sl2, sl2), shift2 = m == -INFINITY ? f2_make(0.0f, 0.0f) : f2_make(-m, -m);
                         f32x2 sum0 = f2_make(0.0f, 0.0f), sum1 = sum0;
 #pragma unroll
@@ -573,7 +556,27 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                         }
                         float a0, a1;
                         f2_split(f2_add(sum0, sum1), a0, a1);
-                        l += a0 + a1;
+                        l = fmaf(l, alpha, a0 + a1);
+                        if (grown) {   // behind the exponentials, so that the product of the step before is rarely waited for
+                            wait_or_die(PV_DONE + (g - 1U) % NS, ((g - 1U) / NS) & 1U, 309);
+                            if (dead) break;
+                            tcgen05_fence_after();
+                            const f32x2 alpha2 = f2_make(alpha, alpha);
+#pragma unroll 1
+                            for (int c = 0; c < DH / 32; ++c) {
+                                uint32_t o[32];
+                                tmem_ld_32x32b_x32(lane_base + plan::COL_O + c * 32, o);
+#pragma unroll
+                                for (int i = 0; i < 32; i += 2) {
+                                    float o0, o1;
+                                    f2_split(f2_mul(f2_make(__uint_as_float(o[i]), __uint_as_float(o[i + 1])), alpha2), o0, o1);
+                                    o[i] = __float_as_uint(o0);
+                                    o[i + 1] = __float_as_uint(o1);
+                                }
+                                tmem_st_32x32b_x16(lane_base + plan::COL_O + c * 32, o);
+                                tmem_st_32x32b_x16(lane_base + plan::COL_O + c * 32 + 16, o + 16);
+                            }
+                        }
                     } else {
                         const uint32_t zero[16] = {0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U, 0U};
                         tmem_st_32x32b_x16(s_col, zero);
@@ -610,8 +613,6 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
 #pragma unroll
                     for (int j = 0; j < DH / 8; ++j) *reinterpret_cast<uint4 *>(dst + 8 * j) = make_uint4(0U, 0U, 0U, 0U);
                 }
-                l = m_true == -INFINITY ? l : l * ex2_approx(m - m_true);
-                m = m_true;
             }
             if (stats != nullptr && valid) {
                 float *s = stats + ((size_t)qi * p.hq + h) * 3;

@@ -1,0 +1,54 @@
+"""Attention on the tensor path: what the order of sums, the choice of the row maximum and the rows behind the last sequence may not change."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from conftest import graft
+from gpu_util import BF16, F16, I32, close, dev, host, rnd_np, storage_name
+
+pkg = graft.load_package()
+ops = pkg.ops
+from oracle import ops as O  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = pkg.runtime.Context(params_bytes=64 << 20, state_bytes=64 << 20, scratch_bytes=2 << 30)
+    yield c
+    c.destroy()
+
+
+@pytest.mark.parametrize("dtype", [F16, BF16])
+@pytest.mark.parametrize("dh", [64, 128])
+def test_largest_probability_is_not_rounded(ctx, dtype, dh):
+    """Probabilities are rounded to 16 bits relative to the row's maximum, so the largest one is exactly 1. Every 64 keys bring a record, 3.3
+    above the one before in powers of two; columns of V that only the record names then come out as V / sum with the output's rounding alone
+    (half a unit in the last place; 1e-5 for the FP32 sum and exponentials). Relative to an older maximum they carry a second rounding."""
+    n, blocks, width = 384, 6, dh // 8
+    a, v = np.zeros(n, np.float32), np.zeros((n, 1, dh), np.float32)
+    records = np.arange(1, blocks) * 64 + 3
+    a[records] = np.arange(1, blocks) * 3.3 / np.log2(np.e) * np.sqrt(dh) / 4.0
+    rng = np.random.default_rng(dh)
+    for t, r in enumerate(records, 1):
+        v[r, 0, t * width:(t + 1) * width] = rng.uniform(1.0, 2.0, width)
+    q, k = np.zeros((2, n, 1, dh), np.float32)
+    q[:, 0, 0], k[:, 0, 0] = 4.0, a
+    k, v = rnd_np(k, dtype), rnd_np(v, dtype)
+    ctx.begin_step()
+    out = ops.gd_sdpa_varlen(ctx, dev(ctx, q, dtype), dev(ctx, k, dtype), dev(ctx, v, dtype), dev(ctx, np.array([0, n], np.int32), I32), causal=True,
+                             sliding_window=0, max_seqlen=n)
+    got = host(out).astype(np.float64)
+    ctx.end_step()
+    s = 4.0 * k[:, 0, 0].astype(np.float64) / np.sqrt(dh)
+    half_unit = 2.0 ** (-11 if dtype == F16 else -8)   # of a value just above a power of two, relative
+    for t, r in enumerate(records, 1):
+        cols = slice(t * width, (t + 1) * width)
+        for row in range(r, (t + 1) * 64):
+            want = v[r, 0, cols].astype(np.float64) / np.exp(s[:row + 1] - s[r]).sum()
+            # spacing of the storage type at each value
+            spacing = 2.0 ** np.floor(np.log2(want)) * 2.0 * half_unit
+            assert np.all(np.abs(got[row, 0, cols] - want) <= 0.5 * spacing + 1e-5 * want), (t, row)
