@@ -31,7 +31,8 @@
 // the product of the step before has finished by then. P is relative to the exact running maximum of every 64 keys: the largest
 // probability is then exactly 1 and takes no rounding. With a maximum that may lag by 2^8 (rescaling is rare) forward and backward of 8191
 // tokens in sequences of 256-2048, 16 heads, window 1024, took 414 us instead of 424, and the output's error against 64-bit arithmetic
-// was 2.06e-3 (bf16) and 2.59e-4 (f16, no window) instead of 1.99e-3 and 2.48e-4, as with the mma.sync kernel (forward alone 286 us).
+// was 2.06e-3 (bf16) and 2.59e-4 (f16, no window) instead of 2.00e-3 and 2.48e-4 (mma.sync kernel, 32 keys at a time: 1.99e-3 and 2.48e-4, 286 us
+// for the forward alone).
 // Tensor memory per CTA (256 columns): S / P 3 x 64 or 2 x 64, O head_dim.
 //
 // Statistics written for the backward pass: (row max in natural-log units, sum of exp, 0).
@@ -250,8 +251,9 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
             constexpr uint64_t QBLOCK16 = plan::QBLOCK >> 4, BLOCK16 = plan::BLOCK >> 4, TILE16 = plan::TILE >> 4, QTILE16 = plan::QTILE >> 4;
             // Two cursors over the same sequence of steps: `s_*` issues S, NS - 1 steps ahead (across items), `g` issues P V.
             uint32_t s_g = 0, s_item = 0, s_si = 0, s_tile = 0;
-            int s_tiles = 0;
-            int ahead[3] = {0, 0, 0}, n_ahead = 0;   // key tiles of the items S has moved on to, which P V has not reached
+            int s_tiles = 0, s_behind = 0;   // key tiles of the item, rows of its last tile behind the last sequence
+            // the same (tiles + behind << 24) for the items S has moved on to, which P V has not reached
+            int ahead[3] = {0, 0, 0}, n_ahead = 0;
             bool ok = true;
             auto fail = [&](int code) {
                 atomicExch(err_flag, code);
@@ -273,6 +275,8 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                     if (item < 0) return;
                     int kb;
                     item_range(cu_s, p, n_valid, (item / p.hq) * A_BQ, &kb, &s_tiles);
+                    // (behind the last token TMA fills zeros itself)
+                    s_behind = n_valid < p.n_tokens ? max(kb + s_tiles * A_BKV - n_valid, 0) : 0;
                     if (s_tiles > 0) return;
                 }
             };
@@ -295,16 +299,18 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                     tcgen05_commit(bar(Q_EMPTY + qs));
                     ++s_item;
                     seek();
-                    ahead[0] = n_ahead == 0 ? s_tiles : ahead[0];
-                    ahead[1] = n_ahead == 1 ? s_tiles : ahead[1];
-                    ahead[2] = n_ahead == 2 ? s_tiles : ahead[2];
+                    const int next = s_tiles | (s_behind << 24);
+                    ahead[0] = n_ahead == 0 ? next : ahead[0];
+                    ahead[1] = n_ahead == 1 ? next : ahead[1];
+                    ahead[2] = n_ahead == 2 ? next : ahead[2];
                     ++n_ahead;
                 }
             };
             uint32_t n_item = 0;
-            int tiles = 0, t = 0;
+            int tiles = 0, behind = 0, t = 0;
             seek();
             tiles = s_tiles;
+            behind = s_behind;
 #pragma unroll 1
             for (uint32_t i = 1; i < NS && ok && s_tiles > 0; ++i) issue_s();
 #pragma unroll 1
@@ -320,6 +326,16 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                     fail(306);
                     break;
                 }
+                if (behind > 0 && t + 1 == tiles) {
+                    // Rows behind the last sequence are not read: their probabilities are zero, but zero times what may lie there is not.
+                    // They are cleared in V (2 us by this one thread, once per head).
+#pragma unroll 1
+                    for (int i = 0; i < behind * 8 * (DH / 64); ++i) {
+                        unsigned char *end = smem + plan::OFF_V + s * plan::TILE + (i / (behind * 8) + 1) * plan::BLOCK;
+                        *reinterpret_cast<uint4 *>(end - (i % (behind * 8) + 1) * 16) = make_uint4(0U, 0U, 0U, 0U);
+                    }
+                    fence_proxy_async_smem();
+                }
                 tcgen05_fence_after();
 #pragma unroll
                 for (int kk = 0; kk < A_BKV / UMMA_K; ++kk) {
@@ -332,7 +348,8 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                     // the S cursor is ahead, so it already stands in the next item
                     t = 0;
                     ++n_item;
-                    tiles = ahead[0];
+                    tiles = ahead[0] & 0xffffff;
+                    behind = ahead[0] >> 24;
                     ahead[0] = ahead[1];
                     ahead[1] = ahead[2];
                     --n_ahead;

@@ -238,6 +238,21 @@ attn5_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                         atomicExch(err_flag, 322);
                         break;
                     }
+                    // Rows behind the last sequence are not read: their P and dS are zero, but zero times what may lie there is not. All four tiles
+                    // are cleared there before the first product that meets them. (Behind the last token TMA fills zeros itself.) One
+                    // thread: 3 us at the most, in the few steps that reach behind the last row.
+                    auto clear_behind = [&](int row0, int rows, unsigned char *blocks, int n_blocks) {
+                        const int first = n_valid - row0;
+                        if (first >= rows || n_valid == p.n_tokens) return;
+                        for (int b = 0; b < n_blocks; ++b) {
+#pragma unroll 1
+                            for (int i = first * 8; i < rows * 8; ++i) reinterpret_cast<uint4 *>(blocks + b * rows * 128)[i] = make_uint4(0U, 0U, 0U, 0U);
+                        }
+                        fence_proxy_async_smem();
+                    };
+                    const int k0 = (item / p.hkv) * B_K;
+                    clear_behind(k0, B_K, smem + plan::OFF_K + ks * plan::KTILE, plan::NB);
+                    clear_behind(k0, B_K, smem + plan::OFF_V + vs * plan::KTILE, plan::NB);
                     const uint64_t kd = k_d + ks * KT, vd = v_d + vs * KT;
                     const int steps = nqt * group;
 #pragma unroll 1
@@ -248,6 +263,7 @@ attn5_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                             ok = false;
                             break;
                         }
+                        clear_behind(k0 + (t % nqt) * B_Q, B_Q, smem + plan::OFF_QG + qs * 2 * plan::QTILE, 2 * plan::NB);
                         if (!mbar_wait(bar(REG_FREE + b), ((g / NR) & 1U) ^ 1U)) {   // dQ^T of the region's previous step has been read back
                             atomicExch(err_flag, 324);
                             ok = false;

@@ -52,3 +52,33 @@ def test_largest_probability_is_not_rounded(ctx, dtype, dh):
             # spacing of the storage type at each value
             spacing = 2.0 ** np.floor(np.log2(want)) * 2.0 * half_unit
             assert np.all(np.abs(got[row, 0, cols] - want) <= 0.5 * spacing + 1e-5 * want), (t, row)
+
+
+# behind the last sequence: inside its last tile, a whole tile and more; one key step only; a last row that begins a tile; grouped heads
+@pytest.mark.parametrize("dtype,dh", [(F16, 64), (BF16, 64), (F16, 128), (BF16, 128)])
+@pytest.mark.parametrize("lengths,behind,hq,hkv,window", [([150, 43], 7, 2, 2, 0), ([130, 63], 200, 4, 2, 40), ([64, 65], 63, 2, 1, 0), ([20], 120, 2, 2, 0),
+                                                          ([300, 1], 19, 2, 2, 128)])
+def test_rows_behind_the_last_sequence_are_not_read(ctx, dtype, dh, lengths, behind, hq, hkv, window):
+    """They may hold anything (scratch memory is not cleared): with NaN and infinities there every result is that of zeros there, bit for bit
+    but for dQ, whose contributions are added in no fixed order."""
+    rng, nv = np.random.default_rng(7), sum(lengths)
+    cu = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    shapes = [(nv + behind, h, dh) for h in (hq, hkv, hkv, hq)]
+    clean = [rnd_np(rng.standard_normal(s).astype(np.float32), dtype) for s in shapes]
+    results = []
+    for fill in (0.0, np.nan, np.inf):
+        arrays = [a.copy() for a in clean]
+        for a in arrays:
+            a[nv:] = fill
+        ctx.begin_step()
+        q, k, v, go = (dev(ctx, a, dtype) for a in arrays)
+        q.requires_grad = k.requires_grad = v.requires_grad = True
+        out = ops.gd_sdpa_varlen(ctx, q, k, v, dev(ctx, cu, I32), causal=True, sliding_window=window, max_seqlen=max(lengths))
+        out.grad = go
+        ctx.run_backward()
+        results.append([host(t) for t in (out, k.grad, v.grad, q.grad)])
+        ctx.end_step()
+    for got in results[1:]:
+        for name, a, b in zip(("out", "dk", "dv"), got, results[0]):
+            assert np.array_equal(a, b), name
+        close(got[3], results[0][3], dtype, what="dq")
