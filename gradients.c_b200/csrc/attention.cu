@@ -669,7 +669,7 @@ gd_status gd_backend_sdpa_varlen(gd_backend *be, const gd_backend_tensor_view *q
 }
 
 // `out` (the forward output) and `dq_accum` (FP32 scratch of q's element count) are optional: with both, forward
-// statistics and head_dim 64 or 128 the backward runs as one attention pass.
+// statistics and head_dim 64 or 128 the backward runs on the tensor-memory kernels (head_dim 64: as one attention pass).
 static gd_status sdpa_varlen_backward_impl(gd_backend *be, const gd_backend_tensor_view *grad_out, const gd_backend_tensor_view *q, const gd_backend_tensor_view *k, const gd_backend_tensor_view *v, const gd_backend_tensor_view *cu_seqlens, const gd_backend_tensor_view *grad_q, const gd_backend_tensor_view *grad_k, const gd_backend_tensor_view *grad_v, const gd_backend_tensor_view *stats, const gd_backend_sdpa_varlen_args *args, const gd_backend_tensor_view *out, const gd_backend_tensor_view *dq_accum,
                                            int32_t *query_grad_in_accum = NULL)
 {

@@ -702,7 +702,7 @@ __global__ void bwd_prep_kernel(const uint4 *__restrict__ go, const uint4 *__res
     constexpr int PIECES = DH / 8;                      // 16-byte pieces of a (row, head)
     extern __shared__ float d_s[];                      // [PREP_ROWS][hq]
     const int row0 = (int)blockIdx.x * PREP_ROWS, rows = min(PREP_ROWS, n_tokens - row0);
-    const int n_vec = max(rows, 0) * hq * PIECES;
+    const int n_vec = DH == 64 ? max(rows, 0) * hq * PIECES : 0;   // (head_dim 128: D and dQ come from a kernel of their own)
     const size_t base = (size_t)row0 * hq * PIECES;
     for (int i = threadIdx.x; i < ((n_vec + 31) & ~31); i += blockDim.x) {
         float s = 0.0f;
@@ -727,11 +727,11 @@ __global__ void bwd_prep_kernel(const uint4 *__restrict__ go, const uint4 *__res
         if (row < n_tokens) {
             float *st = stats + ((size_t)row0 * hq + i) * 3U;
             const float mx = st[0], l = st[1];
-            st[2] = d_s[i];
+            if (DH == 64) st[2] = d_s[i];
             if (row < n_valid) {
                 // P = exp(s scale - max) / sum = exp2(s scale log2e - m2); a row without keys has no products either
                 m2 = l > 0.0f && mx != -INFINITY ? -fmaf(mx, 1.4426950408889634f, __log2f(l)) : -INFINITY;
-                d = -d_s[i] * scale;
+                if (DH == 64) d = -d_s[i] * scale;
             }
         }
         if (m.neg_m2 != nullptr && row < m.n_pad) {
@@ -744,8 +744,10 @@ __global__ void bwd_prep_kernel(const uint4 *__restrict__ go, const uint4 *__res
         const int row = row0 + (int)threadIdx.x;
         int hi = -1;
         if (row < n_valid) {
-            hi = min(cu[seg_of(cu, batch, row) + 1], n_valid) - 1;
+            const int seg = seg_of(cu, batch, row);
+            hi = min(cu[seg + 1], n_valid) - 1;
             if (window > 0) hi = min(hi, row + window - 1);
+            m.row_lo[row] = window > 0 ? max(cu[seg], row - window + 1) : cu[seg];
         }
         m.row_hi[row] = hi;
         if ((row & 127) == 0) {
@@ -761,10 +763,11 @@ __global__ void bwd_prep_kernel(const uint4 *__restrict__ go, const uint4 *__res
     }
 }
 
-// Backward in one attention pass (statistics (max, sum) saved by the forward): D from dO and the forward output, then the
-// key-stationary kernel forms dK, dV and accumulates dQ in FP32, then dQ is rounded. head_dim 128 has the tensor-memory kernel only.
+// Backward with the statistics (max, sum) saved by the forward. head_dim 64, one attention pass: D from dO and the forward output, then
+// the key-stationary kernel forms dK, dV and accumulates dQ in FP32, then dQ is rounded. head_dim 128, tensor-memory kernels only: a
+// query-stationary pass for D and dQ, then the key-stationary one.
 template <typename T, int DH>
-gd_status backward_single_pass(gd_backend *be, const gdb_flash_args *a, const flash_params &p, const void *out, float *dq32)
+gd_status backward_with_out(gd_backend *be, const gdb_flash_args *a, const flash_params &p, const void *out, float *dq32)
 {
     const size_t n = (size_t)a->n_tokens * a->hq * DH, n_vec = n / 8U;
     // statistics by head and mask bounds live at the start of the backend workspace between the two launches
@@ -780,7 +783,8 @@ gd_status backward_single_pass(gd_backend *be, const gdb_flash_args *a, const fl
         m.neg_m2 = (float *)be->ws;
         m.neg_d = m.neg_m2 + per_head;
         m.row_hi = (int *)(m.neg_d + per_head);
-        m.tile_nqt = m.row_hi + m.n_pad;
+        m.row_lo = m.row_hi + m.n_pad;
+        m.tile_nqt = m.row_lo + m.n_pad;
     }
     gdb_launch(bwd_prep_kernel<T, DH>, (unsigned)((m.n_pad + PREP_ROWS - 1) / PREP_ROWS), 256, (size_t)PREP_ROWS * a->hq * sizeof(float), be->stream,
                (const uint4 *)a->grad_out, (const uint4 *)out, a->stats, (float4 *)dq32, a->cu, a->batch, a->n_tokens, a->hq, a->window, a->scale, m);
@@ -789,8 +793,8 @@ gd_status backward_single_pass(gd_backend *be, const gdb_flash_args *a, const fl
     st = tensor ? gdb_attn5_backward(be, a, dq32, &m) : GD_ERR_UNSUPPORTED;   // tensor-memory kernel where the shape allows
     if (st == GD_ERR_UNSUPPORTED && DH == 64) st = launch_kv<T, 64, 64, true>(be, a, p, dq32);
     if (st != GD_OK) return st;
-    if (a->keep_dq32 != 0) {
-        return GD_OK;   // the caller's next kernel reads the accumulator and rounds on load
+    if (DH != 64 || a->keep_dq32 != 0) {
+        return GD_OK;   // written already, or the caller's next kernel reads the accumulator and rounds on load
     }
     gdb_launch(dq_convert_kernel<T>, gdb_grid_for(n_vec, 256, be, 8), 256, 0, be->stream, (const float4 *)dq32, (uint4 *)a->out_or_dq, n_vec);
     return gdb_launched(be, "flash_backward_dq_convert");
@@ -840,10 +844,10 @@ gd_status gdb_flash_varlen_backward(gd_backend *be, const gdb_flash_args *a, boo
 size_t gdb_attn_bwd_ws_bytes(int n_tokens, int hq)
 {
     const size_t n_pad = ((size_t)n_tokens + 63U) & ~(size_t)63U, tiles = ((size_t)n_tokens + 127U) / 128U;
-    return (2U * n_pad * (size_t)hq + n_pad + tiles) * sizeof(float);
+    return (2U * n_pad * (size_t)hq + 2U * n_pad + tiles) * sizeof(float);
 }
 
-// Backward with the forward output at hand (not part of the reference's entry, src/core/backend.h:699-709): D = rowsum(dO o O)
+// Backward with the forward output at hand (not part of the reference's entry, src/core/backend.h:699-709): at head_dim 64 D = rowsum(dO o O)
 // replaces the query-stationary pass. `dq32`: FP32 scratch [N, Hq, Dh]. GD_ERR_UNSUPPORTED outside the fast path.
 gd_status gdb_flash_varlen_backward_with_out(gd_backend *be, const gdb_flash_args *a, const void *out, float *dq32)
 {
@@ -854,7 +858,7 @@ gd_status gdb_flash_varlen_backward_with_out(gd_backend *be, const gdb_flash_arg
     }
     const flash_params p = make_params(a);
     if (a->dh == 64) {
-        return a->dtype == GDB_DTYPE_F16 ? backward_single_pass<__half, 64>(be, a, p, out, dq32) : backward_single_pass<__nv_bfloat16, 64>(be, a, p, out, dq32);
+        return a->dtype == GDB_DTYPE_F16 ? backward_with_out<__half, 64>(be, a, p, out, dq32) : backward_with_out<__nv_bfloat16, 64>(be, a, p, out, dq32);
     }
-    return a->dtype == GDB_DTYPE_F16 ? backward_single_pass<__half, 128>(be, a, p, out, dq32) : backward_single_pass<__nv_bfloat16, 128>(be, a, p, out, dq32);
+    return a->dtype == GDB_DTYPE_F16 ? backward_with_out<__half, 128>(be, a, p, out, dq32) : backward_with_out<__nv_bfloat16, 128>(be, a, p, out, dq32);
 }

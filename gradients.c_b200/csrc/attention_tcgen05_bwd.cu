@@ -4,7 +4,7 @@
 //     S^T  = K Q^T            dP^T = V dO^T                       (128 keys x 64 queries each)
 //     P    = exp(S scale - m) / l,   dS = P o (dP - D) scale      (softmax warps, one thread per key row and 32 queries)
 //     dV  += P^T dO           dK  += dS^T Q                       (128 keys x head_dim, accumulated over the query tiles)
-//     dQ^T = K^T dS^T                                             (head_dim x 64 queries, added to an FP32 accumulator in memory)
+//     dQ^T = K^T dS^T                                             (head_dim 64 only: 64 x 64 queries, added to an FP32 accumulator in memory)
 // (reference semantics: src/ops/sdpa_varlen/metal_sdpa_varlen.metal:30-55 for the mask, :1138-1909 for the backward;
 // CPU restatement tests/test_sdpa_varlen.c:232-371). Fast path: 16-bit storage, head_dim 64 or 128, causal (+ window), prefix 0;
 // row statistics and mask bounds come from the preparation kernel in attention_flash.cu. The mask is evaluated in packed
@@ -12,9 +12,9 @@
 //
 // Why transposed: with keys as rows, P^T and dS^T are the A operands of dV and dK, and an A operand may lie in tensor memory.
 // They are written with tcgen05.st over the S^T columns they came from; only dS goes to shared memory (16 KB per step, the B
-// operand of dQ^T). dQ^T overwrites the dP^T columns of its step. A step thus owns one 128-column region of tensor memory; two
-// (head_dim 128) or three regions take turns, and while the softmax warps work on one step the products of the step before and S / dP of the step after
-// run. At head_dim 64 the M = 128 rows of dQ^T are 64 dimensions of K and 64 of whatever lies behind it (not read back).
+// operand of dQ^T). dQ^T overwrites the dP^T columns of its step. (head_dim 128 has its dQ and D from attention_tcgen05_dq.cu.) A step
+// thus owns one 128-column region of tensor memory; two (head_dim 128) or three regions take turns, and while the softmax warps work
+// on one step the products of the step before and S / dP of the step after run. At head_dim 64 the M = 128 rows of dQ^T are 64 dimensions of K and 64 of whatever lies behind it (not read back).
 //
 // One persistent CTA per SM, 512 threads: warp 0 TMA producer (draws key tiles from a launch-wide ticket counter and publishes
 // them), warp 1 issues S^T / dP^T, warp 2 issues dV / dK / dQ^T (one thread cannot issue an MMA more often than every ~61 cycles,
@@ -44,12 +44,13 @@ struct attn5b_plan {
     static constexpr int KBLOCK = B_K * 128, QBLOCK = B_Q * 128;    // one 128-byte-swizzled block of keys / queries
     static constexpr int KTILE = KBLOCK * NB, QTILE = QBLOCK * NB;
     static constexpr int REGIONS = DH == 64 ? 3 : 2;                // steps in flight (tensor memory: 128 columns each)
-    static constexpr int KST = 2, VST = DH == 64 ? 2 : 1, QST = DH == 64 ? 4 : 2;
+    static constexpr bool WITH_DQ = DH == 64;                       // (head_dim 128: attention_tcgen05_dq.cu)
+    static constexpr int KST = 2, VST = DH == 64 ? 2 : 1, QST = DH == 64 ? 4 : 3;
     static constexpr int OFF_K = 0, OFF_V = OFF_K + KST * KTILE, OFF_QG = OFF_V + VST * KTILE;   // [QST][Q, dO]
     static constexpr int OFF_DS = OFF_QG + QST * 2 * QTILE;         // [REGIONS] tiles of [128 keys][64 queries]
-    static constexpr int STG = DH == 64 ? 2 : 1, STG_BYTES = B_Q * 128;   // FP32 [64 queries][32 dims] per draining warp: dQ on its way to memory
-    static constexpr int OFF_DQ = OFF_DS + REGIONS * KBLOCK;
-    static constexpr int OFF_ST = OFF_DQ + STG * (DH / 32) * STG_BYTES;            // [QST][-(m log2e + log2 l) x 64, -D scale x 64]
+    static constexpr int STG = 2, STG_BYTES = B_Q * 128;            // FP32 [64 queries][32 dims] per draining warp: dQ on its way to memory
+    static constexpr int OFF_DQ = OFF_DS + (WITH_DQ ? REGIONS * KBLOCK : 0);
+    static constexpr int OFF_ST = OFF_DQ + (WITH_DQ ? STG * (DH / 32) * STG_BYTES : 0);   // [QST][-(m log2e + log2 l) x 64, -D scale x 64]
     static constexpr int OFF_BAR = OFF_ST + QST * 512;
     static constexpr int TOTAL = OFF_BAR + 512 + 1024;
     static constexpr uint32_t COL_DK = REGIONS * 128, COL_DV = COL_DK + DH;
@@ -104,7 +105,7 @@ attn5_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
         for (int i = 0; i < N_BARS; ++i) {
             uint32_t count = 1U;
             if (i >= PD_FULL && i < PD_FULL + 3) count = 8U;                     // softmax warps
-            if (i >= REG_FREE && i < REG_FREE + 3) count = (uint32_t)(DH / 32);  // warps that drain dQ^T
+            if (i >= REG_FREE && i < REG_FREE + 3) count = plan::WITH_DQ ? (uint32_t)(DH / 32) : 1U;  // warps that drain dQ^T, or a commit
             if (i == ACC_FREE) count = 8U;
             if (i >= SCHED_EMPTY) count = 14U;                                   // two issuers, four drain and eight softmax warps
             mbar_init(bar(i), count);
@@ -320,11 +321,15 @@ attn5_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                             tcgen05_mma_f16_ts(tmem_base + plan::COL_DK, reg + 16 + (kk >> 1) * 32 + (kk & 1) * 8, qd + kk * 128, IDESC_ACC, (t != 0 || kk != 0) ? 1U : 0U);
                         }
                         tcgen05_commit(bar(QG_EMPTY + qs));
+                        if constexpr (plan::WITH_DQ) {
 #pragma unroll
-                        for (int kk = 0; kk < B_K / UMMA_K; ++kk) {
-                            tcgen05_mma_f16(reg + B_Q, k_d + ks * KT + kk * 128, ds_d + b * KB + kk * 128, IDESC_DQ, kk != 0 ? 1U : 0U);
+                            for (int kk = 0; kk < B_K / UMMA_K; ++kk) {
+                                tcgen05_mma_f16(reg + B_Q, k_d + ks * KT + kk * 128, ds_d + b * KB + kk * 128, IDESC_DQ, kk != 0 ? 1U : 0U);
+                            }
+                            tcgen05_commit(bar(DQ_FULL + b));
+                        } else {
+                            tcgen05_commit(bar(REG_FREE + b));
                         }
-                        tcgen05_commit(bar(DQ_FULL + b));
                     }
                     tcgen05_commit(bar(ACC_FULL));
                     tcgen05_commit(bar(K_EMPTY + ks));
@@ -445,7 +450,7 @@ attn5_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                     tmem_st_32x32b_x16(reg, pk);
                     tmem_st_32x32b_x16(reg + 16, sk);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
+                    for (int j = 0; plan::WITH_DQ && j < 4; ++j) {
                         *reinterpret_cast<uint4 *>(ds_row + b * plan::KBLOCK + (((half * 4 + j) ^ (r & 7)) << 4)) = make_uint4(sk[4 * j], sk[4 * j + 1], sk[4 * j + 2], sk[4 * j + 3]);
                     }
                     tmem_st_wait();
@@ -492,7 +497,7 @@ attn5_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                 }
                 continue;
             }
-            if (quad * 32 < DH) {
+            if (plan::WITH_DQ && quad * 32 < DH) {
 #pragma unroll 1
                 for (int h = hk * group; !dead && h < (hk + 1) * group; ++h) {
 #pragma unroll 1
@@ -558,9 +563,14 @@ gd_status launch_bwd(gd_backend *be, const gdb_flash_args *a, float *dq32, const
     const uint64_t n = (uint64_t)a->n_tokens, qc = (uint64_t)a->hq * DH, kc = (uint64_t)a->hkv * DH;
     const bool ok = make_tmap(&mq, a->dtype, a->q, n, qc, qc * 2U, 64, B_Q) && make_tmap(&mk, a->dtype, a->k, n, kc, kc * 2U, 64, B_K) &&
                     make_tmap(&mv, a->dtype, a->v, n, kc, kc * 2U, 64, B_K) && make_tmap(&mg, a->dtype, a->grad_out, n, qc, qc * 2U, 64, B_Q) &&
-                    make_tmap_f32_2d(&md, dq32, n, qc, 32, B_Q);
+                    (!plan::WITH_DQ || make_tmap_f32_2d(&md, dq32, n, qc, 32, B_Q));
     if (!ok) {
         return GD_ERR_UNSUPPORTED;
+    }
+    if (!plan::WITH_DQ) {
+        md = mq;   // not used
+        const gd_status st = gdb_attn5_query_gradient(be, a, m);
+        if (st != GD_OK) return st;
     }
     attn5b_params p = {a->n_tokens, m->n_pad, a->hq, a->hkv, a->window, ((a->n_tokens + B_K - 1) / B_K) * a->hkv, a->scale};
     const int resident = be->sm_count - be->sm_reserve;

@@ -485,8 +485,9 @@ gd_status gdb200_lm_cross_entropy_fused_rows(gd_backend *backend, const gd_backe
 /* gd_backend_sdpa_varlen_backward (src/core/backend.h:699-709) for a caller that still holds the forward output `out`
  * [N, Hq, Dh] and can lend FP32 scratch `dq_accum` of q's element count: D = rowsum(grad_out o out) replaces the
  * query-stationary recomputation, and dK, dV and dQ come from one key-stationary pass (dQ accumulated in dq_accum, then
- * rounded). Needs the forward's statistics (args->use_forward_stats) and head_dim 64; every other case runs exactly
- * as gd_backend_sdpa_varlen_backward. Results agree with it to FP32 rounding of D (out is a rounded tensor). */
+ * rounded). Needs the forward's statistics (args->use_forward_stats) and head_dim 64. Results agree with
+ * gd_backend_sdpa_varlen_backward to FP32 rounding of D (out is a rounded tensor). At head_dim 128 the same sums as there run on the
+ * tensor-memory kernels (D from P and dP; out and dq_accum are not read); every other case runs exactly as there. */
 gd_status gdb200_sdpa_varlen_backward_with_output(gd_backend *backend, const gd_backend_tensor_view *grad_out, const gd_backend_tensor_view *q,
                                                   const gd_backend_tensor_view *k, const gd_backend_tensor_view *v,
                                                   const gd_backend_tensor_view *cu_seqlens, const gd_backend_tensor_view *out,
