@@ -408,6 +408,7 @@ gd_status gdb_gemm_tcgen05_pair_swiglu(gd_backend *be, uint32_t dtype, const voi
 gd_status gdb_gemm_tcgen05_pair_swiglu_bwd(gd_backend *be, uint32_t dtype, const void *g, size_t ldg_bytes, const void *w, size_t ldw_bytes,
                                            const void *x12, size_t ld12_bytes, void *d_x12, size_t ldd_bytes, uint32_t M, uint32_t F, uint32_t K);
 // CTA-pair persistent variant; *splits_out > 1 means FP32 partials were left in the workspace.
+bool gdb_gemm_profiling();   // contractions are being bracketed with event pairs: nothing else may run beside them
 gd_status gdb_gemm_tcgen05_pair(gd_backend *be, int ta, int tb, uint32_t dtype,
                                 const void *a, size_t lda_bytes, const void *b, size_t ldb_bytes,
                                 void *c, size_t ldc_bytes, const void *bias, int bias_mode,

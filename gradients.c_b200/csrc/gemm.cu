@@ -20,6 +20,7 @@ struct gdb_gemm_profile {
     bool enabled;
 };
 static gdb_gemm_profile *g_profile = nullptr;
+bool gdb_gemm_profiling() { return g_profile != nullptr && g_profile->enabled; }
 
 namespace {
 

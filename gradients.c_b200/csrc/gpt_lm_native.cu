@@ -683,7 +683,7 @@ extern "C" gd_status gdb200_gpt_train_step(gd_backend *be, const gdb200_gpt_spec
     // enough) or for one row of column sums.
     const size_t attn_ws = gdb_attn_bwd_ws_bytes((int)T, (int)H), widest = (size_t)std::max({V, 3 * D, 2 * F});
     const bool halves = (attn_ws <= be->split_bytes || attn_ws > be->ws_bytes) && widest * sizeof(float) <= be->split_bytes;
-    const bool side = drop && !dp && single && halves && c.top + (size_t)(L + 1) * block_scratch + (size_t)V * (size_t)D * 6U <= s->scratch_bytes;
+    const bool side = drop && !dp && single && halves && !gdb_gemm_profiling() && c.top + (size_t)(L + 1) * block_scratch + (size_t)V * (size_t)D * 6U <= s->scratch_bytes;
     gdb_shared_ws shared_ws(be, side);
     auto fork = [&]() {
         if (c.st == GD_OK && (cudaEventRecord(be->side_fork, be->stream) != cudaSuccess || cudaStreamWaitEvent(be->side_stream, be->side_fork, 0) != cudaSuccess)) {

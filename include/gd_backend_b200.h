@@ -392,7 +392,8 @@ gd_status gdb200_download_async(gd_backend *backend, gd_backend_buffer *buffer, 
 gd_status gdb200_upload_beside(gd_backend *backend, gd_backend_buffer *buffer, uint32_t count, const size_t *offsets, const void *const *pinned_srcs, const size_t *nbytes);
 /* Benchmark instrumentation: bracket every dense-contraction dispatch with a CUDA event pair on
  * the backend stream; read returns the number of launches, their summed device time and the
- * algorithmic FLOPs / bytes (2MNK and one pass over each operand) accumulated since enable. */
+ * algorithmic FLOPs / bytes (2MNK and one pass over each operand) accumulated since enable. While enabled, training steps keep to one
+ * stream, so that a pair holds its own contraction only. */
 void gdb200_gemm_profile_enable(gd_backend *backend, int enable);
 gd_status gdb200_gemm_profile_read(gd_backend *backend, uint64_t *launches, double *total_ms, double *flops, double *bytes);
 /* Overwrite a private buffer larger than L2 so that the next kernel starts with a cold L2. */

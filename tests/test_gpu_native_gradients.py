@@ -95,3 +95,16 @@ def test_gradients_with_a_small_workspace(monkeypatch, mib, n_seqs):
     want = step_gradients(g.NativeTrainer, *p, scratch=3 << 30)
     monkeypatch.setenv("GD_CUDA_WORKSPACE_MB", str(mib))
     agree(step_gradients(g.NativeTrainer, *p, scratch=3 << 30), want, F16)
+
+
+def test_profiled_step_keeps_to_one_stream():
+    """A pair of events around a contraction must not hold the work of another stream. With one stream scratch is reused from block to block."""
+    cfg, hp, batch = problem(vocab_size=328)
+    with pkg.runtime.Context(params_bytes=64 << 20, state_bytes=256 << 20, scratch_bytes=1 << 30) as c:
+        trainer, used = g.NativeTrainer(g.GptLm(c, cfg, hp), g.TrainConfig.baseline()), []
+        for enabled in (0, 1, 0):
+            c.lib.gdb200_gemm_profile_enable(c.backend, enabled)
+            trainer.train_batch(batch)
+            used.append(c.scratch.top)
+        c.flush()
+    assert used[1] < used[0] == used[2]
