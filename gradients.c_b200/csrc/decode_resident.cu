@@ -12,7 +12,8 @@
 //     it with a 64-bit atomic maximum whose low half orders equal values by first index, so sampling is no phase of its own;
 //   * norm weights, biases, residuals and cos / sin values are read ahead of the wait.
 // Every sum is formed as in decode_parts.cuh (eight k ranges, k16 products in order, ranges added in order; attention over the
-// same key splits), so the generated ids are those of decode_mega.cu and of the per-operation path.
+// same key splits, merged with the same roundings), so ids and caches are those of decode_mega.cu and of the per-operation path, bit
+// for bit.
 // One sequence, 31 steps of the benchmark model: see the figures at gdb_decode_resident_launch.
 //
 // Waits are bounded: a CTA that gives up stores code 398 in the backend's error word, raises the abort word and returns.
@@ -35,7 +36,7 @@ constexpr int DR_ERR_BARRIER = 398;
 constexpr uint32_t DR_RED_BYTES = SK_WARPS * DR_ROWS * (SK_COLS + 1) * 4U;   // partial sums of one unit
 constexpr uint32_t DR_SYNC_STRIDE = 8U;                                      // counter words are 32 bytes apart
 
-// Counters: [0] abort, then one per phase (5 L + 1, in the order of a step); behind them the running maxima [3][16].
+// Counters: [0] abort, then one per phase (5 L + 1, in the order of a step); behind them the running maxima [3][DR_MAX_ROWS].
 struct dr_args {
     gdb_mega_args a;
     unsigned long long *best;
@@ -586,7 +587,7 @@ __global__ void __launch_bounds__(DR_THREADS, 1) decode_resident_kernel(const __
                         for (int s = 0; s < a.splits; ++s) {
                             const float2 p = ml[s];
                             const float w = p.x == -INFINITY ? 0.0f : __expf(p.x - m);
-                            l = fmaf(p.y, w, l);
+                            l += __fmul_rn(p.y, w);   // (rounded as in decode_combine_query)
                             if (p.x != -INFINITY) o = fmaf(acc[s * 64], w, o);
                         }
                         gdb_io<T>::st((T *)a.attn, ((size_t)b * a.H + h0 + hh) * 64 + col, o * (l > 0.0f ? 1.0f / l : 0.0f));
@@ -668,9 +669,9 @@ bool dr_make_plan(dr_plan *p, uint32_t max_weight_bytes)
 
 size_t gdb_decode_resident_sync_words(int L) { return (size_t)(2 + 5 * L) * DR_SYNC_STRIDE + 3U * DR_MAX_ROWS * 2U; }
 
-// n_steps greedy decode steps of at most 16 sequences with the weights in shared memory; GD_ERR_UNSUPPORTED when the model does
+// n_steps greedy decode steps of at most 64 sequences with the weights in shared memory; GD_ERR_UNSUPPORTED when the model does
 // not fit (decode_mega.cu then takes the call). a->sync: gdb_decode_resident_sync_words(L) zeroed words, 8-byte aligned.
-// The benchmark model on one B200, per step: 104 -> 53.5 us per step (1 sequence), 110 -> 59 us (13 sequences)
+// The benchmark model on one B200, per step: 104 -> 53.5 us per step (1 sequence), 110 -> 59 us (13), 118 -> 80 us (32), 150 -> 148 us (64)
 gd_status gdb_decode_resident_launch(gd_backend *be, uint32_t dtype, const gdb_mega_args *a)
 {
     static thread_local dr_plan plan;   // of the last model

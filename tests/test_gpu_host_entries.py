@@ -7,7 +7,7 @@ import pytest
 from conftest import graft
 
 pkg = graft.load_package()
-g = pkg.gpt_lm
+abi, g = pkg.abi, pkg.gpt_lm
 from test_gpu_gpt_lm import small_cfg  # noqa: E402
 
 pytestmark = pytest.mark.gpu
@@ -25,3 +25,27 @@ def test_generation_with_a_data_slot_for_the_prompts_only():
             model.training = False
             out.append(g.greedy_generate_native(model, prompts, new_tokens=40, capacity=48))
     assert np.array_equal(*out)
+
+
+# one pass of rows and its edges (16 rows to a tile, 32 to a pass), a window, the largest batch
+@pytest.mark.parametrize("dtype", [abi.F16, abi.BF16])
+@pytest.mark.parametrize("batch,prompt,new,window", [(1, 16, 32, 0), (13, 77, 45, 64), (16, 40, 24, 0), (17, 40, 24, 0), (32, 30, 24, 0), (33, 100, 40, 0), (64, 200, 48, 0)])
+def test_decode_forms_agree_bit_for_bit(monkeypatch, dtype, batch, prompt, new, window):
+    """One launch for all steps and one launch per operation form every sum alike: a difference in the last bit of a cache is enough to turn
+    a greedy choice between two nearly equal logits, as those of an untrained model are."""
+    cfg = g.GptConfig.baseline()
+    cfg.dropout_p, cfg.sdpa_window, cfg.dtype = 0.0, window, dtype
+    hp = g.init_params(cfg, seed=12, residual_scaled=False)
+    prompts = np.random.default_rng(batch).integers(0, cfg.vocab_size, size=(batch, prompt)).astype(np.int32)
+    forms = []
+    with pkg.runtime.Context(params_bytes=128 << 20, state_bytes=1 << 30, scratch_bytes=2 << 30) as c:
+        model = g.GptLm(c, cfg, hp)
+        model.training = False
+        for persistent in ("1", "0"):
+            monkeypatch.setenv("GDB200_DECODE_MEGA", persistent)
+            mark, timing = c.state.top, {}
+            ids = g.greedy_generate_native(model, prompts, new, prompt + new, timing=timing)
+            forms.append([ids] + [t.read() for t in model.k_cache + model.v_cache])
+            c.state.top = mark
+            assert (timing["decode_launches"] <= 2) == (persistent == "1")
+    assert all(np.array_equal(a, b) for a, b in zip(*forms))
