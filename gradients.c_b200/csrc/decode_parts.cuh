@@ -574,7 +574,7 @@ struct gdb_mega_args {
 bool gdb_decode_mega_supported(const gd_backend *be, uint32_t dtype, int B, int D, int F, int V, int H, int Dh, int L);
 // n_steps decode steps in ONE cooperative launch. a->sync must be zeroed by the caller (stream-ordered) before the launch.
 gd_status gdb_decode_mega_launch(gd_backend *be, uint32_t dtype, const gdb_mega_args *a);
-// The same for at most 16 sequences and a model whose weights fit the GPU's shared memory (decode_resident.cu);
+// The same for a model whose weights fit the GPU's shared memory (decode_resident.cu);
 // GD_ERR_UNSUPPORTED otherwise. a->sync then holds gdb_decode_resident_sync_words(L) zeroed words.
 size_t gdb_decode_resident_sync_words(int L);
 gd_status gdb_decode_resident_launch(gd_backend *be, uint32_t dtype, const gdb_mega_args *a);

@@ -205,6 +205,21 @@ Ten rms_forward(Step &c, const Ten &x, const Ten &w, int64_t rows, int64_t cols,
     return out;
 }
 
+// sum = x + y and normed = rms_norm(sum, w) (no statistics kept) in one launch when the vector path applies, else the two calls
+void add_then_rms(Step &c, const Ten &x, const Ten &y, const Ten &w, int64_t rows, int64_t cols, Ten *sum, Ten *normed)
+{
+    *sum = c.alloc(x.dt, {rows, cols});
+    *normed = c.alloc(x.dt, {rows, cols});
+    gd_backend_tensor_view xv = tv(x), yv = tv(y), wv = tv(w), sv = tv(*sum), nv = tv(*normed);
+    gd_status r = gdb_add_rms_norm(c.be, &xv, &yv, &wv, &sv, &nv, (size_t)rows, (size_t)cols, c.s->rms_eps);
+    if (r == GD_ERR_UNSUPPORTED) {
+        c.ok(gd_backend_add(c.be, &xv, &yv, &sv), "add");
+        gd_backend_rms_norm_args a = rms_args(rows, cols, c.s->rms_eps);
+        r = gd_backend_rms_norm_forward(c.be, &sv, &wv, &nv, &a);
+    }
+    c.ok(r, "add + rms_norm");
+}
+
 // `accum` != NULL: the input gradient is added into *accum (rounded, then added, then rounded: the two calls
 // rms_norm_backward_stats + accumulate in one launch) and *accum is returned.
 Ten dropout_mask_backward(Step &c, const Ten &mask, const Ten &g, float scale);
@@ -1091,19 +1106,6 @@ gd_status decode_step_body(gd_backend *be, const gdb200_gpt_spec *s, const gdb20
     da.scale = (float)(1.0 / sqrt((double)Dh));
     da.sliding_window = (uint32_t)s->sdpa_window;
     gd_backend_kv_cache_append_args ka = {0};
-    // out = x + y and normed = rms_norm(out, w) in one launch when the vector path applies, else the two calls
-    auto add_then_rms = [&](const Ten &xa, const Ten &ya, const Ten &w, Ten *sum, Ten *normed) {
-        *sum = c.alloc(dt, {B, D});
-        *normed = c.alloc(dt, {B, D});
-        gd_backend_tensor_view xv = tv(xa), yv = tv(ya), wv = tv(w), sv = tv(*sum), nv = tv(*normed);
-        gd_status r = gdb_add_rms_norm(be, &xv, &yv, &wv, &sv, &nv, (size_t)B, (size_t)D, s->rms_eps);
-        if (r == GD_ERR_UNSUPPORTED) {
-            c.ok(gd_backend_add(be, &xv, &yv, &sv), "add");
-            gd_backend_rms_norm_args a = rms_args(B, D, s->rms_eps);
-            r = gd_backend_rms_norm_forward(be, &sv, &wv, &nv, &a);
-        }
-        c.ok(r, "add + rms_norm");
-    };
     Ten inv0;
     Ten normed = rms_forward(c, x, c.param(1, {D}), B, D, &inv0);
     for (int i = 0; i < L && c.st == GD_OK; ++i) {
@@ -1150,7 +1152,7 @@ gd_status decode_step_body(gd_backend *be, const gdb200_gpt_spec *s, const gdb20
         }
         Ten proj = linear_t(c, attn, c.param(pb + 3, {D, D}), c.param(pb + 4, {D}), B, D, D);
         Ten resid, normed2;
-        add_then_rms(x, proj, c.param(pb + 5, {D}), &resid, &normed2);
+        add_then_rms(c, x, proj, c.param(pb + 5, {D}), B, D, &resid, &normed2);
         Ten act = c.alloc(dt, {B, F});
         {
             // up / gate projection and the gate in one launch when the 64-row kernel takes the shape, else the two calls
@@ -1177,7 +1179,7 @@ gd_status decode_step_body(gd_backend *be, const gdb200_gpt_spec *s, const gdb20
         }
         // residual add fused with the norm that consumes it: the next block's attention norm, or the final norm
         Ten out;
-        add_then_rms(resid, mlp, i + 1 < L ? c.param(1 + 10 * (i + 1), {D}) : c.param(P_FINAL, {D}), &out, &normed);
+        add_then_rms(c, resid, mlp, i + 1 < L ? c.param(1 + 10 * (i + 1), {D}) : c.param(P_FINAL, {D}), B, D, &out, &normed);
         x = out;
     }
     Ten final_norm = normed;
@@ -1379,18 +1381,6 @@ extern "C" gd_status gdb200_gpt_prefill(gd_backend *be, const gdb200_gpt_spec *s
         c.ok(gd_backend_rms_norm_forward(be, &xv, &wv, &ov, &a), "rms_norm_forward");
         return out;
     };
-    auto add_then_rms = [&](const Ten &xa, const Ten &ya, const Ten &w, Ten *sum, Ten *normed) {
-        *sum = c.alloc(dt, {T, D});
-        *normed = c.alloc(dt, {T, D});
-        gd_backend_tensor_view xv = tv(xa), yv = tv(ya), wv = tv(w), sv = tv(*sum), nv = tv(*normed);
-        gd_status r = gdb_add_rms_norm(be, &xv, &yv, &wv, &sv, &nv, (size_t)T, (size_t)D, s->rms_eps);
-        if (r == GD_ERR_UNSUPPORTED) {
-            c.ok(gd_backend_add(be, &xv, &yv, &sv), "add");
-            gd_backend_rms_norm_args a = rms_args(T, D, s->rms_eps);
-            r = gd_backend_rms_norm_forward(be, &sv, &wv, &nv, &a);
-        }
-        c.ok(r, "add + rms_norm");
-    };
     gd_backend_rope_args rope = {s->rope_theta, (uint32_t)Dh, 0U};
     gd_backend_sdpa_varlen_args sa;
     memset(&sa, 0, sizeof(sa));
@@ -1422,7 +1412,7 @@ extern "C" gd_status gdb200_gpt_prefill(gd_backend *be, const gdb200_gpt_spec *s
             c.ok(gd_backend_sdpa_varlen(be, &qv, &kv, &vv_, &cuv, &ov, NULL, &sa), "sdpa_varlen");
         }
         Ten proj = linear_t(c, attn, c.param(pb + 3, {D, D}), c.param(pb + 4, {D}), T, D, D), resid, normed2;
-        add_then_rms(x, proj, c.param(pb + 5, {D}), &resid, &normed2);
+        add_then_rms(c, x, proj, c.param(pb + 5, {D}), T, D, &resid, &normed2);
         Ten up_gate = c.alloc(dt, {T, 2 * F}), act = c.alloc(dt, {T, F}), mlp = c.alloc(dt, {T, D});
         {
             const Ten w = c.param(pb + 6, {2 * F, D}), b = c.param(pb + 7, {2 * F}), wd = c.param(pb + 8, {F, D}), bd = c.param(pb + 9, {D});
@@ -1436,7 +1426,7 @@ extern "C" gd_status gdb200_gpt_prefill(gd_backend *be, const gdb200_gpt_spec *s
         }
         if (i + 1 < L) {
             Ten out;
-            add_then_rms(resid, mlp, c.param(1 + 10 * (i + 1), {D}), &out, &normed);
+            add_then_rms(c, resid, mlp, c.param(1 + 10 * (i + 1), {D}), T, D, &out, &normed);
             x = out;
         } else {
             x = c.alloc(dt, {T, D});

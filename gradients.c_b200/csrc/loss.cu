@@ -9,6 +9,7 @@
 //   dlogit = (p - 1[target]) * max(0, 1 - (logit/cap)^2) * grad * scale * inv_valid (:294-310)
 // and src/ops/cross_entropy/metal_cross_entropy.metal for the materialised path.
 #include "common.cuh"
+#include "tcgen05.cuh"   // packed FP32 pairs
 #include "decode_parts.cuh"
 
 namespace {
@@ -342,37 +343,13 @@ __device__ __forceinline__ float rcp_ftz(float x)
 }
 constexpr float LOG2E = 1.4426950408889634f;
 
-// Two FP32 values in one 64-bit register pair: sm_100 multiplies, adds and fuses both halves in one instruction, which
-// halves the issue slots of the arithmetic between the special-function calls (each half rounds as the scalar instruction does).
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 f2_make(float lo, float hi)
-{
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void f2_split(f32x2 p, float &lo, float &hi)
-{
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p));
-}
-__device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b)
-{
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b)
-{
-    f32x2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c)
-{
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
+// (pairs of FP32 values in one instruction, for the arithmetic between the special-function calls)
+using gdb_t5::f2_add;
+using gdb_t5::f2_fma;
+using gdb_t5::f2_make;
+using gdb_t5::f2_mul;
+using gdb_t5::f2_split;
+using gdb_t5::f32x2;
 // tanh(raw / cap) = 1 - 2 / (1 + E), E = exp(2 raw / cap) = 2^(raw * arg_scale): one form for both signs (E = inf gives 1,
 // E = 0 gives -1), absolute error about 2e-7, i.e. 6e-6 on a logit capped at 30 - far below the spacing of the 16-bit logits
 // it is computed from. (The reference's form, metal_lm_cross_entropy.metal:13-31, takes |y|, divides and restores the sign,
