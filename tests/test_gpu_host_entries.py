@@ -27,18 +27,13 @@ def test_generation_with_a_data_slot_for_the_prompts_only():
     assert np.array_equal(*out)
 
 
-# one pass of rows and its edges (16 rows to a tile, 32 to a pass), a window, the largest batch
-@pytest.mark.parametrize("dtype", [abi.F16, abi.BF16])
-@pytest.mark.parametrize("batch,prompt,new,window", [(1, 16, 32, 0), (13, 77, 45, 64), (16, 40, 24, 0), (17, 40, 24, 0), (32, 30, 24, 0), (33, 100, 40, 0), (64, 200, 48, 0)])
-def test_decode_forms_agree_bit_for_bit(monkeypatch, dtype, batch, prompt, new, window):
-    """One launch for all steps and one launch per operation form every sum alike: a difference in the last bit of a cache is enough to turn
-    a greedy choice between two nearly equal logits, as those of an untrained model are."""
-    cfg = g.GptConfig.baseline()
-    cfg.dropout_p, cfg.sdpa_window, cfg.dtype = 0.0, window, dtype
+def compare_decode_forms(monkeypatch, cfg, batch, prompt, new):
+    """Ids and caches of one launch for all steps against one launch per operation. Every sum is formed alike: a difference in the last bit of
+    a cache is enough to turn a greedy choice between two nearly equal logits, as those of an untrained model are."""
     hp = g.init_params(cfg, seed=12, residual_scaled=False)
     prompts = np.random.default_rng(batch).integers(0, cfg.vocab_size, size=(batch, prompt)).astype(np.int32)
     forms = []
-    with pkg.runtime.Context(params_bytes=128 << 20, state_bytes=1 << 30, scratch_bytes=2 << 30) as c:
+    with pkg.runtime.Context(params_bytes=256 << 20, state_bytes=1 << 30, scratch_bytes=2 << 30) as c:
         model = g.GptLm(c, cfg, hp)
         model.training = False
         for persistent in ("1", "0"):
@@ -49,3 +44,23 @@ def test_decode_forms_agree_bit_for_bit(monkeypatch, dtype, batch, prompt, new, 
             c.state.top = mark
             assert (timing["decode_launches"] <= 2) == (persistent == "1")
     assert all(np.array_equal(a, b) for a, b in zip(*forms))
+
+
+# weights resident in shared memory: one pass of rows and its edges (16 rows to a tile, 32 to a pass), a window, the largest batch
+@pytest.mark.parametrize("dtype", [abi.F16, abi.BF16])
+@pytest.mark.parametrize("batch,prompt,new,window", [(1, 16, 32, 0), (13, 77, 45, 64), (16, 40, 24, 0), (17, 40, 24, 0), (32, 30, 24, 0), (33, 100, 40, 0), (64, 200, 48, 0)])
+def test_resident_decode_agrees_bit_for_bit(monkeypatch, dtype, batch, prompt, new, window):
+    cfg = g.GptConfig.baseline()
+    cfg.dropout_p, cfg.sdpa_window, cfg.dtype = 0.0, window, dtype
+    compare_decode_forms(monkeypatch, cfg, batch, prompt, new)
+
+
+# a model whose weights do not fit the GPU's shared memory: one row, an odd count, both halves of the 64-row tile, a window, a tied head
+@pytest.mark.parametrize("dtype", [abi.F16, abi.BF16])
+@pytest.mark.parametrize("batch,prompt,new,window,tied", [(1, 5, 20, 0, False), (7, 70, 20, 48, True), (33, 20, 12, 0, False), (64, 60, 16, 0, False)])
+def test_persistent_decode_of_a_larger_model_agrees_bit_for_bit(monkeypatch, dtype, batch, prompt, new, window, tied):
+    cfg = g.GptConfig.baseline()
+    cfg.dropout_p, cfg.sdpa_window, cfg.dtype, cfg.n_layers, cfg.tied_lm_head = 0.0, window, dtype, 6, tied
+    weights = 2 * (cfg.n_layers * (4 * cfg.d_model ** 2 + 3 * cfg.d_model * cfg.mlp_hidden) + cfg.vocab_size * cfg.d_model)
+    assert weights > 160 * 232448      # more SMs than there are, all of a block's shared memory
+    compare_decode_forms(monkeypatch, cfg, batch, prompt, new)

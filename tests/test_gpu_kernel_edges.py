@@ -114,7 +114,7 @@ def test_native_step_with_a_chunked_vocabulary(vocab, dtype):
         assert off <= (4e-3 if dtype == F16 else 2e-2), (name, off)
 
 
-# one sequence, the most that one tile of rows takes, one more (the other kernel), a head of classes that ends inside a unit
+# one sequence, the most that one tile of rows takes, one more; a head that ends inside a unit of 16 classes (one launch per operation)
 @pytest.mark.parametrize("dtype", [F16, BF16])
 @pytest.mark.parametrize("batch,vocab,window,prompt", [(1, 512, 0, 1), (2, 520, 0, 5), (16, 512, 24, 30), (17, 512, 0, 7)])
 def test_greedy_generation_batch_edges(dtype, batch, vocab, window, prompt):
