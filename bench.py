@@ -377,7 +377,8 @@ def run_b200(args) -> None:
                 "traffic": None, "traffic_note": "DRAM bytes per launch are not measured by this run; the ncu capture of these kernels is summarised "
                                                  "under profiles/ (outputs of this size stay in the 126 MB L2, so DRAM traffic is below the algorithmic bytes)",
                 "peak_source": peak_src,
-                "kernel": "dense contractions (matmul / matmul_nt / matmul_tn / linear), each bracketed by its own CUDA event pair",
+                "kernel": "dense contractions (matmul / matmul_nt / matmul_tn / linear), each bracketed by its own CUDA event pair, the step on one stream "
+                          "meanwhile (the timed step runs weight gradients beside the main stream, so share_of_step is of work, not of time)",
                 "launches_per_step": n_l.value / prof_steps, "avg_launch_us": 1000.0 * ms.value / max(1, n_l.value),
                 "share_of_step": (ms.value / prof_steps) / step_ms_prof, "algorithmic_gb_per_step": by.value / prof_steps / 1e9,
                 "algorithmic_bytes_per_launch": by.value / max(1, n_l.value)}
