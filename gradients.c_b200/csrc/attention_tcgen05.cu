@@ -31,8 +31,8 @@
 // the product of the step before has finished by then. P is relative to the exact running maximum of every 64 keys: the largest
 // probability is then exactly 1 and takes no rounding. With a maximum that may lag by 2^8 (rescaling is rare) forward and backward of 8191
 // tokens in sequences of 256-2048, 16 heads, window 1024, took 414 us instead of 424, and the output's error against 64-bit arithmetic
-// was 2.06e-3 (bf16) and 2.59e-4 (f16, no window) instead of 2.00e-3 and 2.48e-4 (mma.sync kernel, 32 keys at a time: 1.99e-3 and 2.48e-4, 286 us
-// for the forward alone).
+// was 2.06e-3 (bf16) and 2.59e-4 (f16, no window) instead of 2.00e-3 and 2.48e-4 (mma.sync kernel, tiles at other offsets: 1.99e-3 and 2.48e-4,
+// 286 us for the forward alone).
 // Tensor memory per CTA (256 columns): S / P 3 x 64 or 2 x 64, O head_dim.
 //
 // Statistics written for the backward pass: (row max in natural-log units, sum of exp, 0).

@@ -96,8 +96,15 @@ class Tensor:
     _count = _tv = _ref = None
 
     def __init__(self, ctx: "Context", arena: Arena, offset: int, dtype: int, shape: Sequence[int], name: str = ""):
-        self.ctx, self.arena, self.offset, self.dtype, self.name = ctx, arena, int(offset), dtype, name
-        self.shape = tuple(map(int, shape))
+        self.ctx, self.arena, self.dtype, self.name = ctx, arena, dtype, name
+        self.offset = offset if type(offset) is int else int(offset)
+        if type(shape) is not tuple:
+            shape = tuple(map(int, shape))
+        for d in shape:   # (a copy of every shape would cost as much as the rest of this)
+            if type(d) is not int:
+                shape = tuple(map(int, shape))
+                break
+        self.shape = shape
 
     @property
     def count(self) -> int:
