@@ -3,14 +3,12 @@ from __future__ import annotations
 
 import numpy as np
 import pytest
-import torch
 
 from conftest import graft
-from gpu_util import BF16, F16, I32, close, dev, host, rnd_np, storage_name
+from gpu_util import BF16, F16, I32, close, dev, host, rnd_np
 
 pkg = graft.load_package()
 ops = pkg.ops
-from oracle import ops as O  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
