@@ -256,13 +256,15 @@ __global__ void decode_split_kernel(const T *q, const T *kc, const T *vc, const 
                                     float *part_acc, decode_params p, int splits, T *out, unsigned *tickets)
 {
     gdb_pdl_sync();
+    __shared__ __align__(128) unsigned char tiles[DH == 64 ? 4 : 1][gdb_dec::DECODE_TILES_BYTES];   // (DH 128 keeps its keys in registers)
     const int lane = threadIdx.x & 31;
     const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const long long total = (long long)p.batch * p.tq * p.hq;
     const bool active = w < total;
     if (active) {
         const size_t item = (size_t)w * splits + blockIdx.y;
-        gdb_dec::decode_split_item<T, DH, false>(q, kc, vc, pos_buf, part_ml + item * 2U, part_acc + item * DH, p, splits, w, (int)blockIdx.y, lane);
+        gdb_dec::decode_split_item<T, DH>(q, kc, vc, pos_buf, part_ml + item * 2U, part_acc + item * DH, p, splits, w, (int)blockIdx.y, lane,
+                                          tiles[DH == 64 ? threadIdx.x >> 5 : 0]);
     }   // active
     if (tickets == nullptr) {
         return;

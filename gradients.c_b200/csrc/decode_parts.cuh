@@ -1,6 +1,6 @@
 // Device-side building blocks of one KV-cache decode step, shared by the stand-alone kernels (one
 // launch per operation: gemm_skinny.cu, embedding_rope.cu, attention.cu, the argmax of gpt_lm_native.cu)
-// and by the persistent whole-step kernel of decode_mega.cu. Both sides call the same functions, so a
+// and by the kernel of all steps (decode_cluster.cu). Both sides call the same functions, so a
 // step computed by one launch per operation and a step computed by the persistent kernel perform the
 // same floating-point operations in the same order and produce the same bits.
 #ifndef GDB200_DECODE_PARTS_CUH
@@ -50,11 +50,10 @@ __device__ __forceinline__ void sk_ldm4t(uint32_t (&r)[4], const void *p)
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(sk_smem(p)));
 }
 
-template <int MTN>
-__device__ __forceinline__ void sk_zero(float (&acc)[MTN][2][4])
+__device__ __forceinline__ void sk_zero(float (&acc)[4][2][4])
 {
 #pragma unroll
-    for (int i = 0; i < MTN; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
@@ -62,16 +61,15 @@ __device__ __forceinline__ void sk_zero(float (&acc)[MTN][2][4])
 }
 
 // One warp's share [k_begin, k_end) of a staged chunk: As [64][LDA] row-major activations, Ws either [16][LDW]
-// (B_KMAJOR: one row per output column) or [chunk][LDW = 24] (one row per k). The warp multiplies the 16-row tiles
-// MT0 .. MT0 + MTN - 1 (all four, or two when two warps share a k range); acc is indexed by tile - MT0.
-template <typename T, bool B_KMAJOR, int MT0 = 0, int MTN = 4>
-__device__ __forceinline__ void sk_mma_chunk(float (&acc)[MTN][2][4], const T *As, const T *Ws, uint32_t LDA, uint32_t LDW,
+// (B_KMAJOR: one row per output column) or [chunk][LDW = 24] (one row per k).
+template <typename T, bool B_KMAJOR>
+__device__ __forceinline__ void sk_mma_chunk(float (&acc)[4][2][4], const T *As, const T *Ws, uint32_t LDA, uint32_t LDW,
                                              uint32_t k_begin, uint32_t k_end, int lane)
 {
     for (uint32_t k = k_begin; k < k_end; k += 16U) {
-        uint32_t a[MTN][4], b4[4];
+        uint32_t a[4][4], b4[4];
 #pragma unroll
-        for (int mt = 0; mt < MTN; ++mt) sk_ldm4(a[mt], As + ((MT0 + mt) * 16 + (lane & 15)) * LDA + k + (lane >> 4) * 8);
+        for (int mt = 0; mt < 4; ++mt) sk_ldm4(a[mt], As + (mt * 16 + (lane & 15)) * LDA + k + (lane >> 4) * 8);
         if (B_KMAJOR) {
             sk_ldm4(b4, Ws + ((lane & 7) + ((lane >> 4) << 3)) * LDW + k + ((lane >> 3) & 1) * 8);
         } else {
@@ -79,23 +77,22 @@ __device__ __forceinline__ void sk_mma_chunk(float (&acc)[MTN][2][4], const T *A
         }
         const uint32_t b0[2] = {b4[0], b4[1]}, b1[2] = {b4[2], b4[3]};
 #pragma unroll
-        for (int mt = 0; mt < MTN; ++mt) {
+        for (int mt = 0; mt < 4; ++mt) {
             mma16816<T>::run(acc[mt][0], a[mt], b0);
             mma16816<T>::run(acc[mt][1], a[mt], b1);
         }
     }
 }
 
-// A warp's partial tile (row tiles MT0 .. MT0 + MTN - 1 of the 64 x 16 unit) into slot `kslot` of the reduction buffer.
-template <int MT0 = 0, int MTN = 4>
-__device__ __forceinline__ void sk_store_partials(sk_red_t red, const float (&acc)[MTN][2][4], int kslot, int lane)
+// A warp's partial tile of the 64 x 16 unit into slot `kslot` of the reduction buffer.
+__device__ __forceinline__ void sk_store_partials(sk_red_t red, const float (&acc)[4][2][4], int kslot, int lane)
 {
     const int g = lane >> 2, t = lane & 3;
 #pragma unroll
-    for (int mt = 0; mt < MTN; ++mt)
+    for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
-            const int r = (MT0 + mt) * 16 + g, c = nt * 8 + 2 * t;
+            const int r = mt * 16 + g, c = nt * 8 + 2 * t;
             red[kslot][r][c] = acc[mt][nt][0];
             red[kslot][r][c + 1] = acc[mt][nt][1];
             red[kslot][r + 8][c] = acc[mt][nt][2];
@@ -251,18 +248,19 @@ __device__ __forceinline__ bool decode_allowed(int qpos, int j, int window, int 
     return mask_allowed(qpos, j, 1, window, prefix);
 }
 
-// Number of key splits per query. One new token per sequence, head_dim 64 and at most 64 sequences (the shapes the
-// persistent decode kernel takes): the 16 warps of a CTA are `heads_per_cta` heads x `splits` key ranges of ONE sequence,
-// merged through shared memory; heads_per_cta is the smallest power of two (dividing hq, at most 16) that still gives every
-// CTA a unit, batch * hq / heads_per_cta <= sm_count, else the largest. Other shapes: as many splits as keep
+// Number of key splits per query. One new token per sequence, head_dim 64 and at most 64 sequences (the shapes the kernel of all
+// steps takes): the 16 warps of a CTA are `heads_per_cta` heads x `splits` key ranges of ONE sequence, merged through shared memory;
+// heads_per_cta is the smallest power of two (dividing hq, at most 16) that keeps the units within sm_count, or within twice
+// sm_count when the cache has 256 positions and more (a unit is then long enough for a finer deal to pay: 64 sequences of 256-512
+// tokens over seven clusters, two rounds of four heads or three of two), else the largest. Other shapes: as many splits as keep
 // `warps_per_sm` warps per SM busy, at least 32 keys of the cache per split, at most 16.
-static inline int decode_heads_per_cta(int sm_count, int batch, int hq)
+static inline int decode_heads_per_cta(int sm_count, int batch, int hq, int tmax)
 {
     int largest = 0, chosen = 0;
     for (int hg = 16; hg >= 1; hg >>= 1) {
         if (hg > hq || (hq % hg) != 0) continue;
         if (largest == 0) largest = hg;
-        if ((long long)batch * (hq / hg) > sm_count) break;
+        if ((long long)batch * (hq / hg) > (long long)sm_count * (tmax >= 256 ? 2 : 1)) break;
         chosen = hg;
     }
     return chosen != 0 ? chosen : largest;
@@ -270,7 +268,7 @@ static inline int decode_heads_per_cta(int sm_count, int batch, int hq)
 static inline int decode_choose_splits(int sm_count, int batch, int tq, int hq, int dh, int tmax, int warps_per_sm)
 {
     if (tq == 1 && dh == 64 && batch <= 64) {
-        return 16 / decode_heads_per_cta(sm_count, batch, hq);
+        return 16 / decode_heads_per_cta(sm_count, batch, hq, tmax);
     }
     const long long total_queries = (long long)batch * tq * hq;
     int splits = (int)(((long long)sm_count * warps_per_sm) / total_queries);
@@ -306,47 +304,36 @@ __device__ __forceinline__ void decode_combine_query(const float *ml, const floa
     }
 }
 
-// One warp: query w = (b, t, hq) against the keys of split `split` of its live range. A key is handled by DH / 16
-// adjacent lanes (16 head dims = two 16-byte pieces each of K and V), so a warp takes 32 / (DH / 16) keys per group and
-// two groups per tile, folded into the running (max, sum, acc) with one rescale per tile; the partial goes to
-// ml_item [2] = (max, sum) and acc_item [DH] (global or shared memory).
-// RING = false: a tile's loads go to registers and are consumed at once. RING = true (DH = 64): `ring` is 12 KB of
-// shared memory owned by this warp, three tiles of 16 keys deep; the warp copies a tile with cp.async, 4 keys x 128
-// contiguous bytes per instruction (full sectors), the 16-byte pieces of key k stored at piece ^ (k & 7) so that the
-// lanes' reads hit distinct banks, and up to three tiles (48 keys) are in flight per warp with no register cost. Both
-// variants fold the keys into (m, l, acc) with the same operations in the same order.
-template <typename T, int DH, bool RING>
-__device__ __forceinline__ void decode_split_item(const T *q, const T *kc, const T *vc, const int *pos_buf, float *ml_item, float *acc_item,
-                                                  const decode_params &p, int splits, long long w, int split, int lane,
-                                                  unsigned char *ring = nullptr)
-{
-    static_assert(!RING || DH == 64, "the shared-memory ring is laid out for head_dim 64");
-    constexpr int LPK = DH / 16, KPW = 32 / LPK, TILE = 2 * KPW;
-    const int sub = lane % LPK, kg = lane / LPK;
-    const int h = (int)(w % p.hq);
-    const int t = (int)((w / p.hq) % p.tq);
-    const int b = (int)(w / ((long long)p.hq * p.tq));
-    const int hk = h / (p.hq / p.hkv);
-    const int pos = p.pos_mode == 0 ? p.cache_pos : pos_buf[p.pos_mode == 2 ? b : 0];
-    float m = -INFINITY, l = 0.0f;
-    float acc[16], qr[16];
+// One warp's state while it folds keys into the output of one query. A key is handled by DH / 16 adjacent lanes (16 head dims = two
+// 16-byte pieces each of K and V), so a warp takes 32 / (DH / 16) keys per group; two groups are a tile, folded into the running
+// (max, sum, acc) with one rescale.
+template <typename T, int DH>
+struct decode_fold {
+    static constexpr int LPK = DH / 16, KPW = 32 / LPK, TILE = 2 * KPW;
+    float m, l, acc[16], qr[16];
+
+    __device__ __forceinline__ void init()
+    {
+        m = -INFINITY;
+        l = 0.0f;
 #pragma unroll
-    for (int c = 0; c < 16; ++c) acc[c] = 0.0f;
-    // one tile = two groups of keys: both scores, ONE running-max update, both keys folded into (l, acc)
-    auto fold2 = [&](const bool (&valid)[2], const uint4 (&k0)[2], const uint4 (&k1)[2], const uint4 (&v0)[2], const uint4 (&v1)[2]) {
+        for (int c = 0; c < 16; ++c) acc[c] = 0.0f;
+    }
+    // Both scores, ONE running-max update, both keys folded into (l, acc). No branches: a key that is not valid counts with
+    // probability 0 and value 0.
+    __device__ __forceinline__ void fold2(const bool (&valid)[2], const uint4 (&k0)[2], const uint4 (&k1)[2], const uint4 (&v0)[2], const uint4 (&v1)[2])
+    {
         float s[2];
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
+            float ka[8], kb[8];
+            unpack8<T>(k0[u], ka);
+            unpack8<T>(k1[u], kb);
             s[u] = 0.0f;
-            if (valid[u]) {
-                float ka[8], kb[8];
-                unpack8<T>(k0[u], ka);
-                unpack8<T>(k1[u], kb);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) s[u] = fmaf(qr[e], ka[e], s[u]);
+            for (int e = 0; e < 8; ++e) s[u] = fmaf(qr[e], ka[e], s[u]);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) s[u] = fmaf(qr[8 + e], kb[e], s[u]);
-            }
+            for (int e = 0; e < 8; ++e) s[u] = fmaf(qr[8 + e], kb[e], s[u]);
         }
 #pragma unroll
         for (int o = 1; o < LPK; o <<= 1) {
@@ -354,150 +341,229 @@ __device__ __forceinline__ void decode_split_item(const T *q, const T *kc, const
             s[1] += __shfl_xor_sync(0xffffffffU, s[1], o);
         }
         const float s0 = valid[0] ? s[0] : -INFINITY, s1 = valid[1] ? s[1] : -INFINITY;
-        const float mnew = fmaxf(m, fmaxf(s0, s1));
-        if (mnew != -INFINITY) {
-            const float corr = __expf(m - mnew), e0 = __expf(s0 - mnew), e1 = __expf(s1 - mnew);   // exp(-inf) = 0
-            l = l * corr + e0 + e1;
+        const float mnew = fmaxf(m, fmaxf(s0, s1)), base = mnew == -INFINITY ? 0.0f : mnew;
+        const float corr = __expf(m - base), e0 = __expf(s0 - base), e1 = __expf(s1 - base);   // exp(-inf) = 0
+        l = l * corr + e0 + e1;
+        m = mnew;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
             float va[8], vb[8];
-            if (valid[0]) {
-                unpack8<T>(v0[0], va);
-                unpack8<T>(v1[0], vb);
+            unpack8<T>(only(half == 0 ? v0[0] : v1[0], valid[0]), va);
+            unpack8<T>(only(half == 0 ? v0[1] : v1[1], valid[1]), vb);
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    acc[c] = fmaf(e0, va[c], acc[c] * corr);
-                    acc[8 + c] = fmaf(e0, vb[c], acc[8 + c] * corr);
-                }
-            } else {
-#pragma unroll
-                for (int c = 0; c < 16; ++c) acc[c] *= corr;
-            }
-            if (valid[1]) {
-                unpack8<T>(v0[1], va);
-                unpack8<T>(v1[1], vb);
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    acc[c] = fmaf(e1, va[c], acc[c]);
-                    acc[8 + c] = fmaf(e1, vb[c], acc[8 + c]);
-                }
-            }
-            m = mnew;
+            for (int c = 0; c < 8; ++c) acc[half * 8 + c] = fmaf(e1, vb[c], fmaf(e0, va[c], acc[half * 8 + c] * corr));
         }
-    };
-    if (pos >= 0) {
-        int live = pos + p.tq;
-        if (live > p.tmax) live = p.tmax;
-        const int qpos = pos + t;
-        int j_hi = qpos + 1;
-        if (p.prefix > 0 && qpos < p.prefix) j_hi = p.prefix;
-        if (j_hi > live) j_hi = live;
-        int j_lo = 0;
-        if (p.window > 0 && p.prefix <= 0 && qpos - p.window + 1 > 0) j_lo = qpos - p.window + 1;
-        const int span = j_hi > j_lo ? j_hi - j_lo : 0;
-        const int chunk = (span + splits - 1) / splits;
-        const int s_lo = j_lo + split * chunk;
-        int s_hi = s_lo + chunk;
-        if (s_hi > j_hi) s_hi = j_hi;
-        const size_t qb = (((size_t)b * p.tq + t) * p.hq + h) * DH + sub * 16;
-        auto key_valid = [&](int j) { return j < s_hi && decode_allowed(qpos, j, p.window, p.prefix); };
-        if (RING) {
-            const int n_tiles = s_hi > s_lo ? (s_hi - s_lo + TILE - 1) / TILE : 0;
-            const size_t head_base = ((size_t)b * p.tmax * p.hkv + hk) * DH;    // + j * hkv * DH per key
-            const int piece = lane & 7, krow = lane >> 3;                       // copy: lane -> (key within a group of 4, 16-byte piece)
-            auto issue = [&](int tile, int slot) {
-                if (tile < n_tiles) {
-                    unsigned char *base = ring + (size_t)slot * 4096U;
+    }
+    static __device__ __forceinline__ uint4 only(const uint4 &v, bool valid) { return make_uint4(valid ? v.x : 0U, valid ? v.y : 0U, valid ? v.z : 0U, valid ? v.w : 0U); }
+    template <int N>
+    static __device__ __forceinline__ int give_half(float (&a)[16], int lane, int o)
+    {
+        const bool upper = (lane & o) != 0;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int kl = i * 4 + krow, j = s_lo + tile * TILE + kl;
-                        if (j < s_hi) {
-                            const size_t src = head_base + (size_t)j * p.hkv * DH + (size_t)piece * 8U;
-                            unsigned char *dst = base + kl * 128 + ((piece ^ (kl & 7)) << 4);
-                            sk_cp16(dst, kc + src, true);
-                            sk_cp16(dst + 2048, vc + src, true);
-                        }
-                    }
-                }
-                asm volatile("cp.async.commit_group;" ::: "memory");
-            };
-            issue(0, 0);
-            issue(1, 1);
-            issue(2, 2);
+        for (int c = 0; c < N; ++c) {
+            const float give = upper ? a[c] : a[c + N], keep = upper ? a[c + N] : a[c];
+            a[c] = keep + __shfl_xor_sync(0xffffffffU, give, o);
+        }
+        return upper ? N : 0;
+    }
+    // The key groups of the warp (lanes with equal lane % LPK) merged: (max, sum) to ml_item [2], the weighted sums to acc_item [DH]
+    // (global or shared memory). Every addition is between lanes that differ in one bit of the group, low bits first; the lanes give
+    // away half of their sums at each, so a group ends with 16 / (32 / LPK) of them.
+    __device__ __forceinline__ void merge_groups(float *ml_item, float *acc_item, int lane)
+    {
+        const int sub = lane % LPK;
+        float wm = m;
 #pragma unroll
-            for (int c = 0; c < 16; ++c) qr[c] = gdb_io<T>::ld(q, qb + c) * p.scale;
-            int slot = 0;
-            for (int tile = 0; tile < n_tiles; ++tile) {
-                asm volatile("cp.async.wait_group 2;" ::: "memory");
-                __syncwarp();   // every lane's copies of this tile have landed
-                const int jb = s_lo + tile * TILE;
-                const unsigned char *base = ring + (size_t)slot * 4096U;
-                bool valid[2];
-                uint4 k0[2], k1[2], v0[2], v1[2];
+        for (int o = LPK; o < 32; o <<= 1) wm = fmaxf(wm, __shfl_xor_sync(0xffffffffU, wm, o));
+        const float f = (m == -INFINITY) ? 0.0f : __expf(m - wm);
+        l *= f;
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int kl = u * KPW + kg;
-                    valid[u] = key_valid(jb + kl);
-                    if (valid[u]) {
-                        const unsigned char *row = base + kl * 128;
-                        const int p0 = ((sub * 2) ^ (kl & 7)) << 4, p1 = ((sub * 2 + 1) ^ (kl & 7)) << 4;
-                        k0[u] = *reinterpret_cast<const uint4 *>(row + p0);
-                        k1[u] = *reinterpret_cast<const uint4 *>(row + p1);
-                        v0[u] = *reinterpret_cast<const uint4 *>(row + 2048 + p0);
-                        v1[u] = *reinterpret_cast<const uint4 *>(row + 2048 + p1);
-                    }
-                }
-                fold2(valid, k0, k1, v0, v1);
-                __syncwarp();   // every lane is done with the slot before it is refilled
-                issue(tile + 3, slot);
-                slot = slot == 2 ? 0 : slot + 1;
-            }
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        for (int o = LPK; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffU, l, o);
+        float a[16];
+#pragma unroll
+        for (int c = 0; c < 16; ++c) a[c] = acc[c] * f;
+        int first = 0;
+        if (LPK == 4) {
+            first = give_half<8>(a, lane, 4);
+            first += give_half<4>(a, lane, 8);
+            first += give_half<2>(a, lane, 16);
         } else {
-            auto key_base = [&](int j) { return (((size_t)b * p.tmax + (size_t)j) * p.hkv + hk) * DH + sub * 16; };
+            first = give_half<8>(a, lane, 8);
+            first += give_half<4>(a, lane, 16);
+        }
+        constexpr int LEFT = 16 / (32 / LPK);
 #pragma unroll
-            for (int c = 0; c < 16; ++c) qr[c] = gdb_io<T>::ld(q, qb + c) * p.scale;
-#pragma unroll 1
-            for (int jb = s_lo; jb < s_hi; jb += TILE) {
-                if (DH == 64) {   // the tile after this one on its way to L2: a line of K or V per lane
-                    const int j = jb + TILE + (lane & 15);
-                    if (j < s_hi) asm volatile("prefetch.global.L2 [%0];" ::"l"((lane < 16 ? kc : vc) + (((size_t)b * p.tmax + (size_t)j) * p.hkv + hk) * DH));
-                }
-                uint4 k0[2], k1[2], v0[2], v1[2];
-                bool valid[2];
+        for (int c = 0; c < LEFT; ++c) acc_item[sub * 16 + first + c] = a[c];
+        if (lane == 0) {
+            ml_item[0] = wm;
+            ml_item[1] = l;
+        }
+    }
+};
+
+// The same for head_dim 64 with the keys in shared memory: a tile is 16 keys and 16 values of 128 bytes, the 16-byte pieces of row r at
+// piece ^ (r & 7) (as a copy with the 128-byte swizzle leaves them). Scores are products of the tensor cores (the keys are the 16-row
+// operand, the query is column 0; 16-bit factors, FP32 sums), which takes a third of the instructions of converting and multiplying
+// them; the probabilities and their products with the values stay FP32: lane (row r, quarter) folds keys r and r + 8 into 16 columns.
+template <typename T>
+struct decode_fold64 {
+    decode_fold<T, 64> s;        // (max, sum, acc); its query registers are not used
+    uint32_t q[4][2];            // the query as the products' second operand: lanes 0 .. 3, zero elsewhere
+
+    // two consecutive elements of the query for k16 product i and half h: word(i, h) is called on lanes 0 .. 3
+    template <typename F>
+    __device__ __forceinline__ void init(int lane, F word)
+    {
+        s.init();
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int j = jb + u * KPW + kg;
-                    valid[u] = key_valid(j);
-                    if (valid[u]) {
-                        const size_t kb = key_base(j);
-                        k0[u] = *reinterpret_cast<const uint4 *>(kc + kb);
-                        k1[u] = *reinterpret_cast<const uint4 *>(kc + kb + 8);
-                        v0[u] = *reinterpret_cast<const uint4 *>(vc + kb);
-                        v1[u] = *reinterpret_cast<const uint4 *>(vc + kb + 8);
-                    }
-                }
-                fold2(valid, k0, k1, v0, v1);
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) q[i][h] = lane < 4 ? word(i, h) : 0U;
+    }
+    // ok0, ok1: whether this lane's rows lane / 4 and lane / 4 + 8 count; the values of rows that do not must be zero
+    __device__ __forceinline__ void fold(uint32_t keys, uint32_t values, bool ok0, bool ok1, float scale, int lane)
+    {
+        const uint32_t r = (uint32_t)lane & 7U, half = ((uint32_t)lane >> 3) & 1U, kc = (uint32_t)lane >> 4, row = keys + (half * 8U + r) * 128U;
+        float sc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+            uint32_t a[4];
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(row + (((i * 2U + kc) ^ r) << 4)));
+            mma16816<T>::run(sc, a, q[i]);
+        }
+        // column 0 lies in the lanes with lane % 4 == 0: keys g and g + 8 of lane 4 g
+        const int g = lane >> 2, quarter = lane & 3;
+        const float s0 = quarter == 0 && ok0 ? sc[0] * scale : -INFINITY, s1 = quarter == 0 && ok1 ? sc[2] * scale : -INFINITY;
+        float top;
+        asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(top) : "f"(fmaxf(s0, s1)));
+        const float mnew = fmaxf(s.m, top), base = mnew == -INFINITY ? 0.0f : mnew;
+        const float corr = __expf(s.m - base), p0 = __expf(s0 - base), p1 = __expf(s1 - base);   // exp(-inf) = 0
+        s.l = s.l * corr + p0 + p1;
+        s.m = mnew;
+        const float e0 = __shfl_sync(0xffffffffU, p0, lane & ~3), e1 = __shfl_sync(0xffffffffU, p1, lane & ~3);
+        const uint32_t at = values + (uint32_t)g * 128U;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t off = (((uint32_t)(quarter * 2 + h)) ^ (uint32_t)g) << 4;   // (rows g and g + 8 share g & 7)
+            uint4 v0, v1;
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v0.x), "=r"(v0.y), "=r"(v0.z), "=r"(v0.w) : "r"(at + off) : "memory");
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v1.x), "=r"(v1.y), "=r"(v1.z), "=r"(v1.w) : "r"(at + 1024U + off) : "memory");
+            const uint32_t w0[4] = {v0.x, v0.y, v0.z, v0.w}, w1[4] = {v1.x, v1.y, v1.z, v1.w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float2 a = pack2<T>::up(w0[c]), b = pack2<T>::up(w1[c]);
+                float &x = s.acc[h * 8 + c * 2], &y = s.acc[h * 8 + c * 2 + 1];
+                x = fmaf(e1, b.x, fmaf(e0, a.x, x * corr));
+                y = fmaf(e1, b.y, fmaf(e0, a.y, y * corr));
             }
         }
     }
-    // merge the key groups of the warp (lanes with equal `sub`)
-    float wm = m;
+    // the rows' sums merged as in decode_fold (the maximum is the warp's already; the probabilities were summed by lanes 0, 4, ...)
+    __device__ __forceinline__ void merge_groups(float *ml_item, float *acc_item, int lane)
+    {
+        float l = s.l;
 #pragma unroll
-    for (int o = LPK; o < 32; o <<= 1) wm = fmaxf(wm, __shfl_xor_sync(0xffffffffU, wm, o));
-    const float f = (m == -INFINITY) ? 0.0f : __expf(m - wm);
-    l *= f;
-#pragma unroll
-    for (int o = LPK; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffU, l, o);
-    float *pa = acc_item + sub * 16;
-#pragma unroll
-    for (int c = 0; c < 16; ++c) {
-        float a = acc[c] * f;
-#pragma unroll
-        for (int o = LPK; o < 32; o <<= 1) a += __shfl_xor_sync(0xffffffffU, a, o);
-        if (kg == 0) pa[c] = a;
+        for (int o = 4; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffU, l, o);
+        int first = decode_fold<T, 64>::template give_half<8>(s.acc, lane, 4);
+        first += decode_fold<T, 64>::template give_half<4>(s.acc, lane, 8);
+        first += decode_fold<T, 64>::template give_half<2>(s.acc, lane, 16);
+        *reinterpret_cast<float2 *>(acc_item + (lane & 3) * 16 + first) = make_float2(s.acc[0], s.acc[1]);
+        if (lane == 0) *reinterpret_cast<float2 *>(ml_item) = make_float2(s.m, l);
     }
-    if (lane == 0) {
-        ml_item[0] = wm;
-        ml_item[1] = l;
+};
+
+// One warp: query w = (b, t, hq) against the keys of split `split` of its live range; the partial goes to ml_item and acc_item
+// (8-byte aligned). DH 64: `tiles` is shared memory of this warp, DECODE_TILES_BYTES, 128-byte aligned.
+constexpr int DECODE_TILES_BYTES = 2 * 4096;   // two tiles of 16 keys and values, one on its way while the other is folded
+template <typename T, int DH>
+__device__ __forceinline__ void decode_split_item(const T *q, const T *kc, const T *vc, const int *pos_buf, float *ml_item, float *acc_item,
+                                                  const decode_params &p, int splits, long long w, int split, int lane, unsigned char *tiles)
+{
+    const int h = (int)(w % p.hq);
+    const int t = (int)((w / p.hq) % p.tq);
+    const int b = (int)(w / ((long long)p.hq * p.tq));
+    const int hk = h / (p.hq / p.hkv);
+    const int pos = p.pos_mode == 0 ? p.cache_pos : pos_buf[p.pos_mode == 2 ? b : 0];
+    int live = pos + p.tq;
+    if (live > p.tmax) live = p.tmax;
+    const int qpos = pos + t;
+    int j_hi = qpos + 1;
+    if (p.prefix > 0 && qpos < p.prefix) j_hi = p.prefix;
+    if (j_hi > live) j_hi = live;
+    int j_lo = 0;
+    if (p.window > 0 && p.prefix <= 0 && qpos - p.window + 1 > 0) j_lo = qpos - p.window + 1;
+    const int span = pos >= 0 && j_hi > j_lo ? j_hi - j_lo : 0;
+    const int chunk = (span + splits - 1) / splits;
+    const int s_lo = j_lo + split * chunk;
+    int s_hi = s_lo + chunk;
+    if (s_hi > j_hi) s_hi = j_hi;
+    if (span == 0) s_hi = s_lo;
+    const T *qh = q + (((size_t)b * p.tq + t) * p.hq + h) * DH;
+    const size_t head = ((size_t)b * p.tmax * p.hkv + hk) * DH, pitch = (size_t)p.hkv * DH;   // key j at head + j * pitch
+    auto key_valid = [&](int j) { return j < s_hi && decode_allowed(qpos, j, p.window, p.prefix); };
+    if constexpr (DH == 64) {
+        decode_fold64<T> state;
+        state.init(lane, [&](int i, int hh) {
+            const unsigned short *e = reinterpret_cast<const unsigned short *>(qh) + i * 16 + hh * 8 + lane * 2;
+            return (uint32_t)e[0] | ((uint32_t)e[1] << 16);
+        });
+        const int piece = lane & 7, krow = lane >> 3;   // copy: lane -> (key within a group of 4, 16-byte piece)
+        auto issue = [&](int jb, int slot) {
+            if (jb < s_hi) {
+                unsigned char *base = tiles + slot * 4096;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int kl = i * 4 + krow, j = jb + kl;
+                    const bool ok = key_valid(j);
+                    const size_t src = head + (size_t)(ok ? j : s_lo) * pitch + (size_t)piece * 8U;
+                    unsigned char *dst = base + kl * 128 + ((piece ^ (kl & 7)) << 4);
+                    sk_cp16(dst, kc + src, ok);
+                    sk_cp16(dst + 2048, vc + src, ok);
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        issue(s_lo, 0);
+        int slot = 0;
+#pragma unroll 1
+        for (int jb = s_lo; jb < s_hi; jb += 16) {
+            issue(jb + 16, slot ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncwarp();   // every lane's copies of this tile have landed
+            const uint32_t tile = sk_smem(tiles + slot * 4096);
+            state.fold(tile, tile + 2048U, key_valid(jb + (lane >> 2)), key_valid(jb + 8 + (lane >> 2)), p.scale, lane);
+            __syncwarp();   // every lane is done with the slot before it is refilled
+            slot ^= 1;
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        state.merge_groups(ml_item, acc_item, lane);
+    } else {
+        typedef decode_fold<T, DH> fold;
+        constexpr int LPK = fold::LPK, KPW = fold::KPW, TILE = fold::TILE;
+        const int sub = lane % LPK, kg = lane / LPK;
+        fold state;
+        state.init();
+#pragma unroll
+        for (int c = 0; c < 16; ++c) state.qr[c] = gdb_io<T>::ld(qh, (size_t)(sub * 16 + c)) * p.scale;
+#pragma unroll 1
+        for (int jb = s_lo; jb < s_hi; jb += TILE) {
+            uint4 k0[2] = {}, k1[2] = {}, v0[2] = {}, v1[2] = {};
+            bool valid[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int j = jb + u * KPW + kg;
+                valid[u] = key_valid(j);
+                if (valid[u]) {
+                    const size_t kb = head + (size_t)j * pitch + (size_t)(sub * 16);
+                    k0[u] = *reinterpret_cast<const uint4 *>(kc + kb);
+                    k1[u] = *reinterpret_cast<const uint4 *>(kc + kb + 8);
+                    v0[u] = *reinterpret_cast<const uint4 *>(vc + kb);
+                    v1[u] = *reinterpret_cast<const uint4 *>(vc + kb + 8);
+                }
+            }
+            state.fold2(valid, k0, k1, v0, v1);
+        }
+        state.merge_groups(ml_item, acc_item, lane);
     }
 }
 
@@ -552,32 +618,28 @@ __device__ __forceinline__ int32_t argmax_row(const T *x, uint32_t classes, floa
 
 }  // namespace gdb_dec
 
-// ------------------------------------------------------------------ persistent whole-step decode kernel (decode_mega.cu)
-constexpr int GDB_MEGA_MAX_LAYERS = 16;
+// ------------------------------------------------------------------ all decode steps in one launch (decode_cluster.cu)
+constexpr int GDB_DECODE_MAX_LAYERS = 16;
 // Per-layer weights in the order of the model's parameter list: norm1 w, Wqkv [3D, D], bqkv, Wo [D, D], bo, norm2 w,
 // Wupgate [2F, D], bupgate, Wdown [F, D], bdown.
-struct gdb_mega_args {
+struct gdb_decode_args {
     const void *emb, *w_final, *w_lm, *b_lm;
-    const void *lw[GDB_MEGA_MAX_LAYERS][10];
-    void *kc[GDB_MEGA_MAX_LAYERS], *vc[GDB_MEGA_MAX_LAYERS];
+    const void *lw[GDB_DECODE_MAX_LAYERS][10];
+    void *kc[GDB_DECODE_MAX_LAYERS], *vc[GDB_DECODE_MAX_LAYERS];
     int B, D, F, V, H, L, CAP, window, splits, max_steps, n_steps;
     float eps, scale, softcap;
     gdb_dec::rope_params rope;
     const float *rope_table;
-    void *xbuf, *resid, *q, *attn, *act, *logits;                // activations of one step, [B, D | F | V]
-    unsigned *sync;                                               // [0] barrier counter (bit 31: abort)
+    unsigned *sync;                                               // one zeroed word: clusters that are done
     int32_t *tokens, *positions, *out_tokens, *step_counter;
     int *err_flag;
-    unsigned long long *timeline;   // diagnostic (NULL = off): global timer of CTA 0 after every barrier, [n_steps, 5 L + 2]
+    unsigned long long *timeline;   // diagnostic (NULL = off): global timer of CTA 0 after every exchange, [n_steps, 5 L + 1]
 };
-// Shapes the persistent kernel takes (everything else runs as one launch per operation).
-bool gdb_decode_mega_supported(const gd_backend *be, uint32_t dtype, int B, int D, int F, int V, int H, int Dh, int L);
-// n_steps decode steps in ONE cooperative launch. a->sync must be zeroed by the caller (stream-ordered) before the launch.
-gd_status gdb_decode_mega_launch(gd_backend *be, uint32_t dtype, const gdb_mega_args *a);
-// The same for a model whose weights fit the GPU's shared memory (decode_resident.cu);
-// GD_ERR_UNSUPPORTED otherwise. a->sync then holds gdb_decode_resident_sync_words(L) zeroed words.
-size_t gdb_decode_resident_sync_words(int L);
-gd_status gdb_decode_resident_launch(gd_backend *be, uint32_t dtype, const gdb_mega_args *a);
+// Shapes the kernel takes (everything else runs as one launch per operation).
+bool gdb_decode_cluster_supported(const gd_backend *be, uint32_t dtype, int B, int D, int F, int V, int H, int Dh, int L);
+// n_steps decode steps in one launch; GD_ERR_UNSUPPORTED where the device has no room for such clusters. a->sync must be zeroed
+// by the caller (stream-ordered) before the launch.
+gd_status gdb_decode_cluster_launch(gd_backend *be, uint32_t dtype, const gdb_decode_args *a);
 gd_status gdb_rope_params_for_decode(gd_backend *be, uint32_t n_heads, uint32_t head_dim, const gd_backend_rope_args *args, size_t tokens,
                                      gdb_dec::rope_params *out);
 

@@ -1203,18 +1203,15 @@ gd_status decode_step_body(gd_backend *be, const gdb200_gpt_spec *s, const gdb20
     return c.st;
 }
 
-// The whole run of decode steps in one persistent kernel (decode_mega.cu) where its shapes allow; GD_ERR_UNSUPPORTED
+// The whole run of decode steps in one launch (decode_cluster.cu) where its shapes allow; GD_ERR_UNSUPPORTED
 // otherwise (the caller then enqueues one launch per operation).
 gd_status decode_steps_persistent(gd_backend *be, const gdb200_gpt_spec *s, const gdb200_gpt_decode_state *d, int32_t n_steps, size_t *scratch_used)
 {
     const int64_t B = d->batch, D = s->d_model, F = s->mlp_hidden, V = s->vocab_size, H = s->n_heads, Dh = s->head_dim, CAP = d->capacity;
     const int L = s->n_layers;
     const uint32_t dt = s->dtype;
-    if (!gdb_decode_mega_supported(be, dt, (int)B, (int)D, (int)F, (int)V, (int)H, (int)Dh, L)) {
+    if (!gdb_decode_cluster_supported(be, dt, (int)B, (int)D, (int)F, (int)V, (int)H, (int)Dh, L)) {
         return GD_ERR_UNSUPPORTED;
-    }
-    if ((long long)n_steps * (5 * L + 2) * be->sm_count >= (1LL << 30)) {
-        return GD_ERR_UNSUPPORTED;   // the barrier counter of one launch has 31 bits
     }
     const size_t es = gdb_dtype_size(dt);
     Step c;
@@ -1223,7 +1220,7 @@ gd_status decode_steps_persistent(gd_backend *be, const gdb200_gpt_spec *s, cons
     c.top = 0;
     c.st = GD_OK;
     c.where = "";
-    gdb_mega_args a;
+    gdb_decode_args a;
     memset(&a, 0, sizeof(a));
     bool aligned = true;
     auto pptr = [&](int idx, size_t count) -> const void * {
@@ -1269,17 +1266,7 @@ gd_status decode_steps_persistent(gd_backend *be, const gdb200_gpt_spec *s, cons
     a.eps = s->rms_eps;
     a.scale = (float)(1.0 / sqrt((double)Dh));
     a.softcap = s->logits_softcap;
-    auto act = [&](int64_t cols) -> void * {
-        Ten t = c.alloc(dt, {B, cols});
-        return t.buf != NULL ? (void *)(t.buf->dptr + t.off) : NULL;
-    };
-    a.xbuf = act(D);
-    a.resid = act(D);
-    a.q = act(D);
-    a.attn = act(D);
-    a.act = act(F);
-    a.logits = act(V);
-    Ten sync = c.alloc(GDB_DTYPE_I32, {(int64_t)gdb_decode_resident_sync_words(L)});
+    Ten sync = c.alloc(GDB_DTYPE_I32, {1});
     if (c.st != GD_OK) {
         snprintf(be->last_error, sizeof(be->last_error), "gpt decode steps: %s", c.where);
         return c.st;
@@ -1298,8 +1285,8 @@ gd_status decode_steps_persistent(gd_backend *be, const gdb200_gpt_spec *s, cons
     if (st != GD_OK) {
         return st;
     }
-    // GDB200_DECODE_TIMELINE=1 (diagnostic): time stamps after every grid barrier, printed per phase as a mean over the steps
-    const int per_step = 5 * L + 2;
+    // GDB200_DECODE_TIMELINE=1 (diagnostic): time stamps after every exchange, printed per phase as a mean over the steps
+    const int per_step = 5 * L + 1;
     Ten tl;
     const bool want_tl = getenv("GDB200_DECODE_TIMELINE") != NULL;
     if (want_tl) {
@@ -1309,8 +1296,7 @@ gd_status decode_steps_persistent(gd_backend *be, const gdb200_gpt_spec *s, cons
     if (scratch_used != NULL) {
         *scratch_used = c.top;
     }
-    st = a.timeline == NULL ? gdb_decode_resident_launch(be, dt, &a) : GD_ERR_UNSUPPORTED;
-    if (st == GD_ERR_UNSUPPORTED) st = gdb_decode_mega_launch(be, dt, &a);
+    st = gdb_decode_cluster_launch(be, dt, &a);
     if (st == GD_OK && a.timeline != NULL && n_steps > 2) {
         std::vector<unsigned long long> h((size_t)n_steps * per_step);
         if (cudaStreamSynchronize(be->stream) == cudaSuccess &&
@@ -1327,7 +1313,7 @@ gd_status decode_steps_persistent(gd_backend *be, const gdb200_gpt_spec *s, cons
                 if (k < 5 * L) {
                     fprintf(stderr, "  layer %d %-12s %8.0f\n", k / 5, names[k % 5], sum / (n_steps - 1));
                 } else {
-                    fprintf(stderr, "  %-20s %8.0f\n", k == 5 * L ? "F logits" : "G argmax", sum / (n_steps - 1));
+                    fprintf(stderr, "  %-20s %8.0f\n", "F logits, argmax", sum / (n_steps - 1));
                 }
             }
         }

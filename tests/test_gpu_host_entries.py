@@ -64,3 +64,15 @@ def test_persistent_decode_of_a_larger_model_agrees_bit_for_bit(monkeypatch, dty
     weights = 2 * (cfg.n_layers * (4 * cfg.d_model ** 2 + 3 * cfg.d_model * cfg.mlp_hidden) + cfg.vocab_size * cfg.d_model)
     assert weights > 160 * 232448      # more SMs than there are, all of a block's shared memory
     compare_decode_forms(monkeypatch, cfg, batch, prompt, new)
+
+
+# clusters of four and eight CTAs; more than 16 units of a phase to a CTA (rounds), a CTA with one unit more than another, k ranges of 16 and
+# 32, one 128-wide tile of the down projection; positions behind the cos / sin table (512) and more than 32 keys to a warp
+@pytest.mark.parametrize("d_model,mlp_hidden,vocab,layers,batch,prompt,new,window", [
+    (128, 128, 4096, 2, 5, 6, 12, 0), (128, 2560, 272, 1, 64, 4, 9, 3), (256, 640, 272, 2, 20, 30, 20, 0), (256, 768, 4112, 1, 3, 17, 8, 5),
+    (512, 1536, 2048, 1, 3, 490, 40, 0), (512, 512, 16, 1, 59, 250, 12, 200)])
+def test_decode_of_other_shapes_agrees_bit_for_bit(monkeypatch, d_model, mlp_hidden, vocab, layers, batch, prompt, new, window):
+    cfg = g.GptConfig.baseline()
+    cfg.dropout_p, cfg.sdpa_window, cfg.n_layers, cfg.vocab_size = 0.0, window, layers, vocab
+    cfg.d_model, cfg.n_heads, cfg.mlp_hidden, cfg.context_length = d_model, d_model // 64, mlp_hidden, 1024
+    compare_decode_forms(monkeypatch, cfg, batch, prompt, new)

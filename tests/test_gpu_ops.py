@@ -385,6 +385,24 @@ def test_sdpa_varlen_forward_backward(step, dtype, lengths, hq, hkv, dh, window,
     close(host(vt.grad), wdv, dtype, scale=6, what="dv")
 
 
+# the keys of a warp are multiplied 16 at a time: ranges that end on, before and behind a tile's edge, caches that hold NaN wherever no live key lies
+@pytest.mark.parametrize("dtype", [F16, BF16])
+@pytest.mark.parametrize("tq,hq,hkv,window,prefix", [(1, 8, 8, 0, 0), (1, 4, 2, 20, 0), (2, 4, 4, 0, 0), (1, 2, 2, 9, 24)])
+def test_decode_attention_reads_live_keys_only(step, dtype, tq, hq, hkv, window, prefix):
+    ctx, sd = step, storage_name(dtype)
+    pos = np.array([0, 1, 14, 15, 16, 17, 30, 31, 32, 33, 255, 256, 257, 511, 509 - tq], dtype=np.int32)
+    b, tmax, dh = len(pos), 512 + tq - 1, 64
+    kc, vc, q = (rnd_np(rng(50 + i).standard_normal(shape).astype(np.float32), dtype) for i, shape in enumerate(((b, tmax, hkv, dh), (b, tmax, hkv, dh), (b, tq, hq, dh))))
+    dirty = [c.copy() for c in (kc, vc)]
+    for c in dirty:
+        for i, p in enumerate(pos):
+            c[i, p + tq:] = np.nan
+            if window > 0 and prefix == 0 and p - window + 1 > 0:
+                c[i, :p - window + 1] = np.nan
+    out = ops.gd_sdpa_decode_positions(ctx, dev(ctx, q, dtype), dev(ctx, dirty[0], dtype), dev(ctx, dirty[1], dtype), dev(ctx, pos, I32), sliding_window=window, prefix_len=prefix)
+    close(host(out), O.sdpa_decode(t32(q), t32(kc), t32(vc), pos, 0.0, window, prefix, sd), dtype, scale=2)
+
+
 @pytest.mark.parametrize("dtype,b,tq,tmax,hq,hkv,dh,window", [(F16, 5, 1, 512, 8, 8, 64, 256), (F16, 3, 2, 40, 4, 2, 64, 0),
                                                               (BF16, 2, 1, 300, 16, 16, 128, 0), (F16, 2, 3, 11, 2, 1, 8, 4)])
 def test_kv_append_and_decode(step, dtype, b, tq, tmax, hq, hkv, dh, window):
