@@ -609,7 +609,7 @@ def measure_decode(args, with_cpu: bool = True) -> dict:
     bytes_per_step = 2.0 * n_mm + 2.0 * layers * batch * kv_rows * d * 2.0
     res = {"metric": "gpt_lm_kv_decode_tokens_per_s", "unit": "tokens/s", "higher_is_better": True, "dtype": "f16",
            "config": {"workload": f"greedy KV decode, {batch} prompts x {plen}, {new_tokens} new tokens, cache {cap}, gpt_lm baseline model",
-                      "host": "native: all decode steps in one persistent cooperative kernel (grid barriers between the phases of a step), device argmax, ids / positions fed back on the device" if native
+                      "host": "native: all decode steps in one kernel of independent thread-block clusters (exchanges through distributed shared memory between the phases of a step), device argmax, ids / positions fed back on the device" if native
                       else "python: host argmax and three small uploads per step"},
            "checksum": int(out.astype(np.int64).sum()), "gpu_launches": launches}
     if native and timing:

@@ -231,12 +231,14 @@ __device__ __forceinline__ dc_keys dc_key_range(int pos, int window, int cap, ui
 }
 
 // ------------------------------------------------------------------------------------------------------- producer warps
-// Every tile of every step in the order of use; warp `which` of the producers issues tiles which, which + DC_PRODUCERS, ...
+// Every tile of every step in the order of use; warp `which` of the producers issues tiles which, which + DC_PRODUCERS, ... of a phase,
+// and of the attention the tiles of consumer warps 4 which .. 4 which + 3, one per lane (a warp that shares its scheduler with working
+// ones takes some five cycles per instruction: one tile at a time, keys and values came at 19 bytes per cycle and SM).
 template <typename T, int D>
 __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, int rows, const int *positions, uint32_t lm_bar)
 {
+    static_assert(DC_WARPS == 4 * DC_PRODUCERS, "four consumer warps to a producer");
     constexpr uint32_t CS = D / 32U;
-    enum { ATTN = 5 };
     const gdb_decode_args &a = g.a;
     const uint32_t F = (uint32_t)a.F, splits_log = 31U - (uint32_t)__clz(a.splits), hpc_log = 4U - splits_log;
     const int groups = a.H >> hpc_log, attn_units = rows * groups;
@@ -244,64 +246,81 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
     dc_share(F / 8U, c.rank, CS, &up_first, &up_n);
     dc_share((uint32_t)a.V / 16U, c.rank, CS, &lm_first, &lm_n);
     uint32_t n = 0U, slot = 0U;
+    auto claim = [&](uint32_t tile) {   // the tile's slot is free
+        if (tile >= c.slots) dc_wait(c, c.empty + ((tile - c.slots) % DC_TILE_BARS) * 8U, ((tile - c.slots) / DC_TILE_BARS) & 1U);
+    };
+    auto wrap = [&](uint32_t s) {
+#pragma unroll 1
+        while (s >= c.slots) s -= c.slots;
+        return s;
+    };
 #pragma unroll 1
     for (int step = 0; step < a.n_steps; ++step) {
-        int layer = 0, kind = DC_QKV, unit = (int)c.rank;   // the phases of a layer: QKV, attention (a round per unit), OUT, UP, DOWN
 #pragma unroll 1
-        for (;;) {
-            uint32_t tiles, units = 0U, first = 0U;
-            int row = 0, h0 = 0;
-            dc_keys kr = {0, 0, 0, 0};
-            if (kind == ATTN) {
-                // keys and values of an attention unit: tile (i, w) for the i-th 32 keys of warp w's (head, split)
-                if (layer == 0 && step > 0 && unit == (int)c.rank) {
+        for (int ph = 0; ph <= 4 * a.L; ++ph) {
+            const int kind = ph == 4 * a.L ? (int)DC_LM : (ph & 3), layer = ph >> 2;
+            if (kind == DC_OUT) {
+                // keys and values of this CTA's attention units: tile (i, w) for the i-th 32 keys of warp w's (head, split)
+                if (layer == 0 && step > 0 && attn_units > (int)c.rank) {
                     // the rows that the step before has written: acquired with its last exchange, then ordered for the copies
                     dc_wait(c, lm_bar, (uint32_t)(step - 1) & 1U);
                     asm volatile("fence.proxy.async.global;" ::: "memory");
                 }
-                row = unit / groups;
-                h0 = (unit - row * groups) << hpc_log;
-                kr = dc_key_range(positions[row] + step, a.window, a.CAP, splits_log);
-                tiles = (uint32_t)(kr.iters * DC_WARPS);
-                // The next attention's keys and values on their way from DRAM to L2 while the phases in between leave DRAM idle (64
-                // sequences, 256 + 256 tokens: all clusters fetch them in the same phases, 38 MB a layer)
-                if (kr.span >= 64 && c.lane == 0) {
-                    const int ahead = layer + 1 == a.L ? 0 : layer + 1;
+                const int w = (int)which * 4 + (c.lane & 3), split = w >> hpc_log;
 #pragma unroll 1
-                    for (int i = (int)which; i < (kr.span + 63) / 64; i += DC_PRODUCERS) {
-                        gdb_t5::tma_prefetch_3d(&g.kv_ahead[ahead][0], h0 * 64, kr.lo + i * 64, b0 + row);
-                        gdb_t5::tma_prefetch_3d(&g.kv_ahead[ahead][1], h0 * 64, kr.lo + i * 64, b0 + row);
-                    }
-                }
-                __syncwarp();
-            } else if (kind == DC_DOWN) {
-                tiles = F / 128U;
-            } else {
-                units = kind == DC_QKV ? 6U : (kind == DC_OUT ? 2U : (kind == DC_UP ? up_n : lm_n));
-                first = kind == DC_UP ? up_first : lm_first;
-                tiles = 2U * units;
-            }
-            const CUtensorMap *map = kind == DC_LM ? &g.lm : &g.w[layer][kind & 3];
+                for (int unit = (int)c.rank; unit < attn_units; unit += (int)CS) {
+                    const int row = unit / groups, h0 = (unit - row * groups) << hpc_log;
+                    const dc_keys kr = dc_key_range(positions[row] + step, a.window, a.CAP, splits_log);
+                    const int x = (h0 + (w & ((1 << hpc_log) - 1))) * 64, end = kr.lo + min((split + 1) * kr.chunk, kr.span);
+                    uint32_t tile = n + (uint32_t)w, s = wrap(slot + (uint32_t)w);
+                    int j = kr.lo + split * kr.chunk;
 #pragma unroll 1
-            for (uint32_t i = 0; i < tiles; ++i, ++n, slot = slot + 1U == c.slots ? 0U : slot + 1U) {
-                if ((n & (DC_PRODUCERS - 1U)) != which) continue;
-                if (n >= c.slots) dc_wait(c, c.empty + ((n - c.slots) % DC_TILE_BARS) * 8U, ((n - c.slots) / DC_TILE_BARS) & 1U);   // the slot is free
-                if (c.alive && c.lane == 0) {
-                    const uint32_t full = c.full + (n % DC_TILE_BARS) * 8U, dst = c.sm + slot * DC_TILE;
-                    if (kind == ATTN) {
-                        const int w = (int)(i % DC_WARPS), split = w >> hpc_log, h = h0 + (w & ((1 << hpc_log) - 1)), j = kr.lo + split * kr.chunk + (int)(i / DC_WARPS) * 32;
-                        const int left = kr.lo + min((split + 1) * kr.chunk, kr.span) - j, box = left > 16 ? 0 : 1;   // keys of this tile (32 at most)
-                        gdb_t5::mbar_expect_tx(full, left <= 0 ? 0U : (box == 0 ? 8192U : 4096U));
-                        if (left > 0) {
-                            gdb_t5::tma_load_3d(dst, &g.kv[layer][0][box], h * 64, j, b0 + row, full);
-                            gdb_t5::tma_load_3d(dst + 4096U, &g.kv[layer][1][box], h * 64, j, b0 + row, full);
+                    for (int i = 0; i < kr.iters; ++i, j += 32, tile += DC_WARPS, s = wrap(s + DC_WARPS)) {
+                        if (c.lane < 4) {
+                            claim(tile);
+                            if (c.alive) {
+                                const uint32_t full = c.full + (tile % DC_TILE_BARS) * 8U, dst = c.sm + s * DC_TILE;
+                                const int box = end - j > 16 ? 0 : 1;   // 32 keys, or 16
+                                gdb_t5::mbar_expect_tx(full, j >= end ? 0U : (box == 0 ? 8192U : 4096U));
+                                if (j < end) {
+                                    gdb_t5::tma_load_3d(dst, &g.kv[layer][0][box], x, j, b0 + row, full);
+                                    gdb_t5::tma_load_3d(dst + 4096U, &g.kv[layer][1][box], x, j, b0 + row, full);
+                                }
+                            }
                         }
-                    } else if (kind == DC_DOWN) {
+                        __syncwarp();
+                    }
+                    n += (uint32_t)(kr.iters * DC_WARPS);
+                    slot = wrap(slot + (uint32_t)(kr.iters * DC_WARPS));
+                    // The next attention's keys and values on their way from DRAM to L2 while the phases in between leave DRAM idle (64
+                    // sequences, 256 + 256 tokens: all clusters fetch them in the same phases, 38 MB a layer)
+                    if (kr.span >= 64 && c.lane == 0) {
+                        const int ahead = layer + 1 == a.L ? 0 : layer + 1;
+#pragma unroll 1
+                        for (int i = (int)which; i < (kr.span + 63) / 64; i += DC_PRODUCERS) {
+                            gdb_t5::tma_prefetch_3d(&g.kv_ahead[ahead][0], h0 * 64, kr.lo + i * 64, b0 + row);
+                            gdb_t5::tma_prefetch_3d(&g.kv_ahead[ahead][1], h0 * 64, kr.lo + i * 64, b0 + row);
+                        }
+                    }
+                    __syncwarp();
+                }
+            }
+            const CUtensorMap *map = kind == DC_LM ? &g.lm : &g.w[layer][kind];
+            const uint32_t units = kind == DC_QKV ? 6U : (kind == DC_OUT ? 2U : (kind == DC_UP ? up_n : lm_n)), first = kind == DC_UP ? up_first : lm_first;
+            const uint32_t tiles = kind == DC_DOWN ? F / 128U : 2U * units;
+            const bool whole = (kind == DC_UP || kind == DC_LM) && units > 8U;   // a warp to a unit: the first halves of 16 units, then the second
+            uint32_t s = wrap(slot + which);
+#pragma unroll 1
+            for (uint32_t i = which; i < tiles; i += DC_PRODUCERS, s = wrap(s + DC_PRODUCERS)) {
+                claim(n + i);
+                if (c.alive && c.lane == 0) {
+                    const uint32_t full = c.full + ((n + i) % DC_TILE_BARS) * 8U, dst = c.sm + s * DC_TILE;
+                    if (kind == DC_DOWN) {
                         gdb_t5::mbar_expect_tx(full, DC_TILE);
                         gdb_t5::tma_load_2d(dst, map, (int)(c.rank * 32U), (int)(i * 128U), full);
                     } else {
                         uint32_t u = i >> 1, half = i & 1U, lo, hi;
-                        if (kind != DC_QKV && units > 8U) {   // a warp to a unit: the first halves of 16 units, then the second
+                        if (whole) {
                             const uint32_t u0 = i / 32U * 16U, in = i % 32U, nr = min(units - u0, 16U);
                             half = in >= nr ? 1U : 0U;
                             u = u0 + in - half * nr;
@@ -314,17 +333,8 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
                 }
                 __syncwarp();
             }
-            if (kind == DC_LM) break;
-            if (kind == ATTN) unit += (int)CS;
-            if (kind == DC_QKV) unit = (int)c.rank;
-            if (kind == DC_DOWN) {
-                ++layer;
-                kind = layer == a.L ? (int)DC_LM : (int)DC_QKV;
-            } else if (kind == DC_QKV || kind == ATTN) {
-                kind = unit < attn_units ? (int)ATTN : (int)DC_OUT;
-            } else {
-                ++kind;   // OUT -> UP -> DOWN
-            }
+            n += tiles;
+            slot = wrap(slot + tiles);
         }
     }
 }
@@ -753,39 +763,39 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                 }
 
                 if (!up && my_attn != 0U) {
-                    // ---- attention: head hl of the unit, key range `split`; the ranges are merged in shared memory ----
+                    // ---- attention: head hl of each of the CTA's units, key range `split`; the ranges are merged in shared memory ----
+                    const uint32_t s_part = c.sm + g.lay.scratch;
                     uint32_t at = 0U;
+                    int turn = 0;   // tiles of 32 keys this warp has folded in this phase
 #pragma unroll 1
                     for (int unit = (int)c.rank; unit < attn_units; unit += (int)CS, ++at) {
-                        const int row = unit >> groups_log, h0 = (unit - (row << groups_log)) << hpc_log, pos = positions[row] + step;
+                        const int row = unit >> groups_log, pos = positions[row] + step;
                         const dc_keys kr = dc_key_range(pos, a.window, a.CAP, 4U - hpc_log);
                         const int s_lo = kr.lo + split * kr.chunk, s_hi = kr.lo + min((split + 1) * kr.chunk, kr.span);
                         const uint32_t fresh = s_qkv + (at * 3U * (uint32_t)hpc + (uint32_t)hl) * 128U;   // q, then k and v hpc and 2 hpc rows on
                         uint32_t em = 0U, tile = 0U;
-                        if (kr.iters > 0) tile = wait_tile((uint32_t)c.warp, &em);
-                        if (at == 0U) receive(DX_QKV, qkv_bytes);
+                        if (at == 0U) {
+                            if (kr.iters > 0) tile = wait_tile((uint32_t)c.warp, &em);
+                            receive(DX_QKV, qkv_bytes);
+                        }
                         decode_fold64<T> state;
                         state.init(c.lane, [&](int i, int hh) { return dc_lds4(fresh + (uint32_t)(i * 32 + hh * 16 + c.lane * 4)); });
 #pragma unroll 1
-                        for (int it = 0; it < kr.iters; ++it) {
-                            if (it != 0) {
-                                if ((it & 1) == 0) dc_sync();
-                                tile = wait_tile((uint32_t)(it * DC_WARPS + c.warp), &em);
-                            }
+                        for (int it = 0; it < kr.iters; ++it, ++turn) {
+                            if (turn != 0 && (turn & 1) == 0) dc_sync();
+                            if (at != 0U || it != 0) tile = wait_tile((uint32_t)(it * DC_WARPS + c.warp), &em);
                             bool written = false;
 #pragma unroll 1
                             for (int k0 = 0; k0 < 32; k0 += 16) {
-                                const int j = s_lo + it * 32 + k0, left = s_hi - j, newest = pos - j;
+                                const int key = s_lo + it * 32 + k0, left = s_hi - key, newest = pos - key;
                                 if (left <= 0) break;
                                 const uint32_t keys = tile + (uint32_t)k0 * 128U, values = keys + 4096U;
-                                if (left < 16 || (newest >= 0 && newest < 16)) {
-                                    // the newest key and value in their rows; no values behind the range's end
-                                    if (newest >= 0 && newest < min(left, 16) && c.lane < 16) {
+                                if (newest >= 0 && newest < min(left, 16)) {   // the newest key and value in their rows
+                                    if (c.lane < 16) {
                                         const uint32_t piece = (uint32_t)c.lane & 7U, kind_of = (uint32_t)c.lane >> 3;
                                         dc_sts16((kind_of == 0U ? keys : values) + (uint32_t)newest * 128U + ((piece ^ ((uint32_t)newest & 7U)) << 4),
                                                  dc_lds16(fresh + (kind_of + 1U) * (uint32_t)hpc * 128U + piece * 16U));
                                     }
-                                    for (int i = c.lane + left * 8; i < 128; i += 32) dc_sts16(values + (uint32_t)i * 16U, make_uint4(0U, 0U, 0U, 0U));
                                     __syncwarp();
                                     written = true;
                                 }
@@ -795,41 +805,44 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                             dc_release<16>(em, c.lane);
                         }
                         advance((uint32_t)(kr.iters * DC_WARPS));
-                        // two sets of partials: the next unit's are written while this one's may still be read
-                        float *sm_ml = reinterpret_cast<float *>(generic + g.lay.scratch) + (at & 1U) * DC_PARTIALS, *sm_acc = sm_ml + DC_WARPS * 2;
+                        float *ml = reinterpret_cast<float *>(generic + g.lay.scratch) + at * DC_PARTIALS;
                         const int item = (hl << (4U - hpc_log)) + split;
-                        state.merge_groups(sm_ml + item * 2, sm_acc + item * 64, c.lane);
-                        dc_sync();
-                        // merge of the splits (decode_combine_query), one thread per output: weights, sum and output over the splits in order
-                        if (c.tid < hpc * 64) {
-                            const int head = c.tid >> 6;
-                            const uint32_t s_ml = smem_u32(sm_ml) + (uint32_t)(head * a.splits) * 8U, s_acc = smem_u32(sm_acc) + (uint32_t)(head * a.splits * 64 + (c.tid & 63)) * 4U;
-                            float m = -INFINITY, l = 0.0f, o = 0.0f;
-                            // (reads behind the head's splits: another's, or no split's)
-                            float pm[16], pl[16], x[16];
+                        state.merge_groups(ml + item * 2, ml + DC_WARPS * 2 + item * 64, c.lane);
+                    }
+                    dc_sync();
+                    // Merge of the splits of all units at once (decode_combine_query), one thread per output: weights, sum and output over the
+                    // splits in order. (Unit by unit, by the warps of that unit's outputs: 64 sequences 122 us per step.)
+#pragma unroll 1
+                    for (uint32_t out = (uint32_t)c.tid; out < at * ((uint32_t)hpc * 64U); out += DC_WARPS * 32U) {
+                        const uint32_t of = (out >> 6) >> hpc_log, head = (out >> 6) & ((uint32_t)hpc - 1U), unit = c.rank + of * CS;
+                        const uint32_t row = unit >> groups_log, col = ((unit - (row << groups_log)) << hpc_log) * 64U + head * 64U + (out & 63U);
+                        const uint32_t s_ml = s_part + of * (DC_PARTIALS * 4U) + head * (uint32_t)a.splits * 8U;
+                        const uint32_t s_acc = s_part + of * (DC_PARTIALS * 4U) + DC_WARPS * 8U + (head * (uint32_t)a.splits * 64U + (out & 63U)) * 4U;
+                        float m = -INFINITY, l = 0.0f, o = 0.0f;
+                        // (reads behind the head's splits: another's, or no split's)
+                        float pm[16], pl[16], x[16];
 #pragma unroll
-                            for (int s = 0; s < 16; ++s) {
-                                const unsigned long long p = dc_lds8(s_ml + (uint32_t)s * 8U);
-                                asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x[s]) : "r"(s_acc + (uint32_t)s * 256U) : "memory");
-                                pm[s] = s < a.splits ? __uint_as_float((uint32_t)p) : -INFINITY;
-                                pl[s] = __uint_as_float((uint32_t)(p >> 32));
-                            }
+                        for (int s = 0; s < 16; ++s) {
+                            const unsigned long long p = dc_lds8(s_ml + (uint32_t)s * 8U);
+                            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x[s]) : "r"(s_acc + (uint32_t)s * 256U) : "memory");
+                            pm[s] = s < a.splits ? __uint_as_float((uint32_t)p) : -INFINITY;
+                            pl[s] = __uint_as_float((uint32_t)(p >> 32));
+                        }
 #pragma unroll
-                            for (int s = 0; s < 16; ++s) m = fmaxf(m, pm[s]);
+                        for (int s = 0; s < 16; ++s) m = fmaxf(m, pm[s]);
 #pragma unroll
-                            for (int s = 0; s < 16; ++s) {
-                                const bool some = pm[s] != -INFINITY;
-                                const float w = some ? __expf(pm[s] - m) : 0.0f;
-                                l += __fmul_rn(some ? pl[s] : 0.0f, w);   // (rounded as in decode_combine_query)
-                                o = some ? fmaf(x[s], w, o) : o;
-                            }
-                            const uint4 vec = gather8(o * (l > 0.0f ? 1.0f / l : 0.0f));
-                            if (c.alive) {
+                        for (int s = 0; s < 16; ++s) {
+                            const bool some = pm[s] != -INFINITY;
+                            const float w = some ? __expf(pm[s] - m) : 0.0f;
+                            l += __fmul_rn(some ? pl[s] : 0.0f, w);   // (rounded as in decode_combine_query)
+                            o = some ? fmaf(x[s], w, o) : o;
+                        }
+                        const uint4 vec = gather8(o * (l > 0.0f ? 1.0f / l : 0.0f));
+                        if (c.alive) {
 #pragma unroll
-                                for (uint32_t i = 0; i < (CS + 7U) / 8U; ++i) {
-                                    const uint32_t to = i * 8U + ((uint32_t)c.lane & 7U);
-                                    if (to < CS) dc_send(mapa_shared(s_attn + (uint32_t)row * LDA + (uint32_t)h0 * 128U + (uint32_t)(c.tid >> 3) * 16U, to), vec, mapa_shared(bar(DX_ATTN), to));
-                                }
+                            for (uint32_t i = 0; i < (CS + 7U) / 8U; ++i) {
+                                const uint32_t to = i * 8U + ((uint32_t)c.lane & 7U);
+                                if (to < CS) dc_send(mapa_shared(s_attn + row * LDA + (col & ~7U) * 2U, to), vec, mapa_shared(bar(DX_ATTN), to));
                             }
                         }
                     }
@@ -1002,7 +1015,7 @@ bool dc_make_layout(dc_layout *l, uint32_t rows, uint32_t D, uint32_t F, uint32_
     // CTAs have sent before any can be in the next attention, and attention rows are multiplied before any residual row leaves.
     const uint32_t attn_bytes = (rows * (D + 8U) * 2U + 127U) & ~127U;
     // (the merge of a head's splits reads 16 items' worth of words from its first one on)
-    l->act = take(std::max(rows * (F + 8U) * 2U, attn_bytes + (2U * DC_PARTIALS + 16U * 64U) * 4U));
+    l->act = take(std::max(rows * (F + 8U) * 2U, attn_bytes + (units * DC_PARTIALS + 16U * 64U) * 4U));
     l->attn = l->act;
     l->scratch = l->act + attn_bytes;
     l->qkv = take(units * hpc * 384U);

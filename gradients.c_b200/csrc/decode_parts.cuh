@@ -250,17 +250,18 @@ __device__ __forceinline__ bool decode_allowed(int qpos, int j, int window, int 
 
 // Number of key splits per query. One new token per sequence, head_dim 64 and at most 64 sequences (the shapes the kernel of all
 // steps takes): the 16 warps of a CTA are `heads_per_cta` heads x `splits` key ranges of ONE sequence, merged through shared memory;
-// heads_per_cta is the smallest power of two (dividing hq, at most 16) that keeps the units within sm_count, or within twice
-// sm_count when the cache has 256 positions and more (a unit is then long enough for a finer deal to pay: 64 sequences of 256-512
-// tokens over seven clusters, two rounds of four heads or three of two), else the largest. Other shapes: as many splits as keep
-// `warps_per_sm` warps per SM busy, at least 32 keys of the cache per split, at most 16.
-static inline int decode_heads_per_cta(int sm_count, int batch, int hq, int tmax)
+// heads_per_cta is the smallest power of two (dividing hq, at most 16) that leaves at most DECODE_UNITS units, one for every CTA of the
+// seven clusters of 16 that a B200 holds, else the largest: a second unit per CTA costs its latency in every layer (us per step, units
+// within 112 / within twice the SMs: 20 sequences 42.9 / 49.4, 32 52.9 / 59.9, 64 of 20-84 tokens 71 / 81, 64 of 256-512 123.2 / 122.7).
+// Other shapes: as many splits as keep `warps_per_sm` warps per SM busy, at least 32 keys of the cache per split, at most 16.
+constexpr int DECODE_UNITS = 112;
+static inline int decode_heads_per_cta(int batch, int hq)
 {
     int largest = 0, chosen = 0;
     for (int hg = 16; hg >= 1; hg >>= 1) {
         if (hg > hq || (hq % hg) != 0) continue;
         if (largest == 0) largest = hg;
-        if ((long long)batch * (hq / hg) > (long long)sm_count * (tmax >= 256 ? 2 : 1)) break;
+        if ((long long)batch * (hq / hg) > DECODE_UNITS) break;
         chosen = hg;
     }
     return chosen != 0 ? chosen : largest;
@@ -268,7 +269,7 @@ static inline int decode_heads_per_cta(int sm_count, int batch, int hq, int tmax
 static inline int decode_choose_splits(int sm_count, int batch, int tq, int hq, int dh, int tmax, int warps_per_sm)
 {
     if (tq == 1 && dh == 64 && batch <= 64) {
-        return 16 / decode_heads_per_cta(sm_count, batch, hq, tmax);
+        return 16 / decode_heads_per_cta(batch, hq);
     }
     const long long total_queries = (long long)batch * tq * hq;
     int splits = (int)(((long long)sm_count * warps_per_sm) / total_queries);
@@ -420,7 +421,7 @@ struct decode_fold64 {
 #pragma unroll
             for (int h = 0; h < 2; ++h) q[i][h] = lane < 4 ? word(i, h) : 0U;
     }
-    // ok0, ok1: whether this lane's rows lane / 4 and lane / 4 + 8 count; the values of rows that do not must be zero
+    // ok0, ok1: whether this lane's rows lane / 4 and lane / 4 + 8 count (what lies in rows that do not is not used)
     __device__ __forceinline__ void fold(uint32_t keys, uint32_t values, bool ok0, bool ok1, float scale, int lane)
     {
         const uint32_t r = (uint32_t)lane & 7U, half = ((uint32_t)lane >> 3) & 1U, kc = (uint32_t)lane >> 4, row = keys + (half * 8U + r) * 128U;
@@ -448,7 +449,7 @@ struct decode_fold64 {
             uint4 v0, v1;
             asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v0.x), "=r"(v0.y), "=r"(v0.z), "=r"(v0.w) : "r"(at + off) : "memory");
             asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v1.x), "=r"(v1.y), "=r"(v1.z), "=r"(v1.w) : "r"(at + 1024U + off) : "memory");
-            const uint32_t w0[4] = {v0.x, v0.y, v0.z, v0.w}, w1[4] = {v1.x, v1.y, v1.z, v1.w};
+            const uint32_t w0[4] = {ok0 ? v0.x : 0U, ok0 ? v0.y : 0U, ok0 ? v0.z : 0U, ok0 ? v0.w : 0U}, w1[4] = {ok1 ? v1.x : 0U, ok1 ? v1.y : 0U, ok1 ? v1.z : 0U, ok1 ? v1.w : 0U};
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const float2 a = pack2<T>::up(w0[c]), b = pack2<T>::up(w1[c]);

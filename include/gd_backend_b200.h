@@ -643,9 +643,9 @@ gd_status gdb200_gpt_prefill(gd_backend *backend, const gdb200_gpt_spec *spec, c
                              size_t last_rows_offset, const gdb200_gpt_decode_state *state, size_t *scratch_used);
 /* Enqueues n_steps decode steps without any host synchronisation. use_graph == 0: one launch per operation, step after
  * step. use_graph != 0: where the shapes allow (16-bit storage, at most 64 sequences, head_dim 64, d_model 128 / 256 / 512,
- * mlp_hidden a multiple of 128, the cos / sin table of the rotation in use) ALL steps run in one persistent cooperative
- * kernel (one CTA per SM; the weights stay in shared memory where they fit, else they are read from L2; a phase that is not reached
- * within its bounded wait stores code 398 in the error word and ends the kernel); otherwise the first step runs eagerly, the second is
+ * mlp_hidden a multiple of 128 and what of it fits shared memory, vocab_size a multiple of 16) ALL steps run in one kernel of
+ * independent thread-block clusters (d_model / 32 CTAs each, a few sequences each, the weights read from L2; a wait that gives up
+ * stores code 398 in the error word); otherwise the first step runs eagerly, the second is
  * recorded as a CUDA graph and the rest replay it. All forms generate the same ids and caches. */
 gd_status gdb200_gpt_decode_steps(gd_backend *backend, const gdb200_gpt_spec *spec, const gdb200_gpt_decode_state *state,
                                   int32_t n_steps, int32_t use_graph, size_t *scratch_used);
