@@ -34,15 +34,17 @@ using gdb_t5::mapa_shared;
 constexpr int DC_WARPS = 16, DC_PRODUCERS = 4, DC_THREADS = (DC_WARPS + DC_PRODUCERS) * 32;
 constexpr int DC_MAX_ROWS = 16;              // sequences of a cluster
 constexpr int DC_PARTIALS = DC_WARPS * 2 + DC_WARPS * 64;   // (max, sum) and weighted sums of the 16 (head, split) items of an attention unit
-constexpr uint32_t DC_TILE = 8192U;          // ring slot: 16 weight rows x half of k (d_model 512), 128 k x 32 columns of the down
-                                             // projection, or 32 keys and values of a head
-constexpr uint32_t DC_MAX_SLOTS = 24U, DC_MIN_SLOTS = 8U;
-// Tile n of the run has barriers n % 128 of its own (full: its bytes have landed; empty: its readers are done), not its slot's: a warp
-// may wait for a tile whose slot is still to be used once or twice before, and a parity cannot tell those phases apart. A barrier's use
-// before, tile n - 128, is over by then: the warps lie at most 44 tiles apart (a block barrier ends every 16 units of two tiles and every
-// two tiles per warp of the attention, whose warps may start while others have their part of the 12 QKV tiles to do; an exchange that
-// needs all warps ends the other phases), and at most 24 more are in flight.
-constexpr uint32_t DC_TILE_BARS = 128U;
+// The ring is used in places of 4 KB: a weight tile takes two (16 rows x half of k for d_model 512, or 128 k x 32 columns of the down
+// projection), 16 keys and values of a head take one. (Tiles of 32 keys in places of 8 KB: with 14 places and 16 warps the copy of a
+// warp's next tile began when it was done with this one, 27 bytes per cycle and SM for 64 sequences.)
+constexpr uint32_t DC_PLACE = 4096U, DC_TILE = 2U * DC_PLACE;
+constexpr uint32_t DC_MAX_PLACES = 48U, DC_MIN_PLACES = 16U;
+// Use n of a place has barriers n % 256 of its own (full: its bytes have landed; empty: its readers are done), not the place's: a warp
+// may wait for a tile whose place is still to be used once or twice before, and a parity cannot tell those phases apart. A barrier's use
+// before, n - 256, is over by then: the warps lie at most 88 places apart (a block barrier ends every 16 units of two tiles and every
+// four tiles per warp of the attention, whose warps may start while others have their part of the 12 QKV tiles to do; an exchange that
+// needs all warps ends the other phases), and at most 48 more are in flight.
+constexpr uint32_t DC_BARS = 256U;
 constexpr unsigned DC_SPIN_LIMIT = 1U << 21;
 constexpr int DC_ERR_WAIT = 398;
 
@@ -52,7 +54,7 @@ enum { DC_QKV = 0, DC_OUT = 1, DC_UP = 2, DC_DOWN = 3, DC_LM = 4 };
 enum { DX_QKV = 0, DX_ATTN = 1, DX_RESID = 2, DX_ACT = 3, DX_X = 4, DX_LM = 5, DX_COUNT = 6 };
 
 struct dc_layout {
-    uint32_t slots;
+    uint32_t places;
     uint32_t x, resid, normed, act, attn, scratch, qkv, red, staging, keys, total;   // byte offsets from the ring's start
 };
 
@@ -61,17 +63,17 @@ struct dc_args {
     dc_layout lay;
     int rows;                 // sequences per cluster
     CUtensorMap lm, w[GDB_DECODE_MAX_LAYERS][4];
-    CUtensorMap kv[GDB_DECODE_MAX_LAYERS][2][2];   // keys, values; in boxes of 32 and of 16 positions
+    CUtensorMap kv[GDB_DECODE_MAX_LAYERS][2];         // keys, values; a head x 16 positions
     CUtensorMap kv_ahead[GDB_DECODE_MAX_LAYERS][2];   // the heads of an attention unit x 64 positions, for prefetches
 };
 
 // One CTA's side of the exchanges and of the ring.
 struct dc_ctx {
     uint32_t sm;                  // shared-memory address of the ring; everything else lies behind it
-    uint32_t full, empty;         // addresses of the tiles' barriers
+    uint32_t full, empty;         // addresses of the uses' barriers
     volatile int *dead;
     int *err_flag;
-    uint32_t rank, slots, n, slot;   // ring cursor: number and slot of the next phase's first tile
+    uint32_t rank, places, n, place;   // ring cursor: use and place of the next phase's first tile
     int tid, warp, lane;
     bool alive;
 };
@@ -217,7 +219,7 @@ __device__ __forceinline__ void dc_unit_rows(int kind, uint32_t u, uint32_t firs
 
 // Live keys [lo, lo + span) of a query at `pos` and the keys of each of its splits (decode_split_item).
 struct dc_keys {
-    int lo, span, chunk, iters;   // iters: tiles of 32 keys per split
+    int lo, span, chunk, iters;   // iters: tiles of 16 keys per split
 };
 __device__ __forceinline__ dc_keys dc_key_range(int pos, int window, int cap, uint32_t splits_log)
 {
@@ -226,7 +228,7 @@ __device__ __forceinline__ dc_keys dc_key_range(int pos, int window, int cap, ui
     k.lo = window > 0 && pos - window + 1 > 0 ? pos - window + 1 : 0;
     k.span = pos >= 0 && hi > k.lo ? hi - k.lo : 0;
     k.chunk = (k.span + (1 << splits_log) - 1) >> splits_log;
-    k.iters = (k.chunk + 31) >> 5;
+    k.iters = (k.chunk + 15) >> 4;
     return k;
 }
 
@@ -245,13 +247,13 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
     uint32_t up_first, up_n, lm_first, lm_n;
     dc_share(F / 8U, c.rank, CS, &up_first, &up_n);
     dc_share((uint32_t)a.V / 16U, c.rank, CS, &lm_first, &lm_n);
-    uint32_t n = 0U, slot = 0U;
-    auto claim = [&](uint32_t tile) {   // the tile's slot is free
-        if (tile >= c.slots) dc_wait(c, c.empty + ((tile - c.slots) % DC_TILE_BARS) * 8U, ((tile - c.slots) / DC_TILE_BARS) & 1U);
+    uint32_t n = 0U, place = 0U;
+    auto claim = [&](uint32_t use) {   // its place is free
+        if (use >= c.places) dc_wait(c, c.empty + ((use - c.places) % DC_BARS) * 8U, ((use - c.places) / DC_BARS) & 1U);
     };
     auto wrap = [&](uint32_t s) {
 #pragma unroll 1
-        while (s >= c.slots) s -= c.slots;
+        while (s >= c.places) s -= c.places;
         return s;
     };
 #pragma unroll 1
@@ -260,7 +262,7 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
         for (int ph = 0; ph <= 4 * a.L; ++ph) {
             const int kind = ph == 4 * a.L ? (int)DC_LM : (ph & 3), layer = ph >> 2;
             if (kind == DC_OUT) {
-                // keys and values of this CTA's attention units: tile (i, w) for the i-th 32 keys of warp w's (head, split)
+                // keys and values of this CTA's attention units: use (i, w) for the i-th 16 keys of warp w's (head, split)
                 if (layer == 0 && step > 0 && attn_units > (int)c.rank) {
                     // the rows that the step before has written: acquired with its last exchange, then ordered for the copies
                     dc_wait(c, lm_bar, (uint32_t)(step - 1) & 1U);
@@ -272,26 +274,25 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
                     const int row = unit / groups, h0 = (unit - row * groups) << hpc_log;
                     const dc_keys kr = dc_key_range(positions[row] + step, a.window, a.CAP, splits_log);
                     const int x = (h0 + (w & ((1 << hpc_log) - 1))) * 64, end = kr.lo + min((split + 1) * kr.chunk, kr.span);
-                    uint32_t tile = n + (uint32_t)w, s = wrap(slot + (uint32_t)w);
+                    uint32_t use = n + (uint32_t)w, s = wrap(place + (uint32_t)w);
                     int j = kr.lo + split * kr.chunk;
 #pragma unroll 1
-                    for (int i = 0; i < kr.iters; ++i, j += 32, tile += DC_WARPS, s = wrap(s + DC_WARPS)) {
+                    for (int i = 0; i < kr.iters; ++i, j += 16, use += DC_WARPS, s = wrap(s + DC_WARPS)) {
                         if (c.lane < 4) {
-                            claim(tile);
+                            claim(use);
                             if (c.alive) {
-                                const uint32_t full = c.full + (tile % DC_TILE_BARS) * 8U, dst = c.sm + s * DC_TILE;
-                                const int box = end - j > 16 ? 0 : 1;   // 32 keys, or 16
-                                gdb_t5::mbar_expect_tx(full, j >= end ? 0U : (box == 0 ? 8192U : 4096U));
+                                const uint32_t full = c.full + (use % DC_BARS) * 8U, dst = c.sm + s * DC_PLACE;
+                                gdb_t5::mbar_expect_tx(full, j >= end ? 0U : DC_PLACE);
                                 if (j < end) {
-                                    gdb_t5::tma_load_3d(dst, &g.kv[layer][0][box], x, j, b0 + row, full);
-                                    gdb_t5::tma_load_3d(dst + 4096U, &g.kv[layer][1][box], x, j, b0 + row, full);
+                                    gdb_t5::tma_load_3d(dst, &g.kv[layer][0], x, j, b0 + row, full);
+                                    gdb_t5::tma_load_3d(dst + 2048U, &g.kv[layer][1], x, j, b0 + row, full);
                                 }
                             }
                         }
                         __syncwarp();
                     }
                     n += (uint32_t)(kr.iters * DC_WARPS);
-                    slot = wrap(slot + (uint32_t)(kr.iters * DC_WARPS));
+                    place = wrap(place + (uint32_t)(kr.iters * DC_WARPS));
                     // The next attention's keys and values on their way from DRAM to L2 while the phases in between leave DRAM idle (64
                     // sequences, 256 + 256 tokens: all clusters fetch them in the same phases, 38 MB a layer)
                     if (kr.span >= 64 && c.lane == 0) {
@@ -309,12 +310,15 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
             const uint32_t units = kind == DC_QKV ? 6U : (kind == DC_OUT ? 2U : (kind == DC_UP ? up_n : lm_n)), first = kind == DC_UP ? up_first : lm_first;
             const uint32_t tiles = kind == DC_DOWN ? F / 128U : 2U * units;
             const bool whole = (kind == DC_UP || kind == DC_LM) && units > 8U;   // a warp to a unit: the first halves of 16 units, then the second
-            uint32_t s = wrap(slot + which);
+            uint32_t s = wrap(place + 2U * which);
 #pragma unroll 1
-            for (uint32_t i = which; i < tiles; i += DC_PRODUCERS, s = wrap(s + DC_PRODUCERS)) {
-                claim(n + i);
+            for (uint32_t i = which; i < tiles; i += DC_PRODUCERS, s = wrap(s + 2U * DC_PRODUCERS)) {
+                const uint32_t use = n + 2U * i;   // (even: a phase of the attention uses a multiple of 16 places, and their number is even)
+                claim(use);
+                claim(use + 1U);
                 if (c.alive && c.lane == 0) {
-                    const uint32_t full = c.full + ((n + i) % DC_TILE_BARS) * 8U, dst = c.sm + s * DC_TILE;
+                    const uint32_t full = c.full + (use % DC_BARS) * 8U, dst = c.sm + s * DC_PLACE;
+                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full + 8U) : "memory");   // (nobody waits for the second place's use)
                     if (kind == DC_DOWN) {
                         gdb_t5::mbar_expect_tx(full, DC_TILE);
                         gdb_t5::tma_load_2d(dst, map, (int)(c.rank * 32U), (int)(i * 128U), full);
@@ -333,8 +337,8 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
                 }
                 __syncwarp();
             }
-            n += tiles;
-            slot = wrap(slot + tiles);
+            n += 2U * tiles;
+            place = wrap(place + 2U * tiles);
         }
     }
 }
@@ -380,10 +384,12 @@ __device__ __forceinline__ void dc_ranges(float (&acc)[G][NT][4], uint32_t tile,
             }
         }
 }
-template <int N> __device__ __forceinline__ void dc_release(uint32_t empty, int lane)   // N of the tile's 16 reader shares are done
+// `shares` of the 16 reader shares of a tile of one or two places are done.
+template <int PLACES>
+__device__ __forceinline__ void dc_release(uint32_t empty, uint32_t shares, int lane)
 {
     __syncwarp();
-    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(empty), "n"(N) : "memory");
+    if (lane < PLACES) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(empty + (uint32_t)lane * 8U), "r"(shares) : "memory");
 }
 
 template <typename T, int D, int NT>
@@ -393,7 +399,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
     constexpr uint32_t LDA = (D + 8U) * 2U;      // bytes between normalised rows
     constexpr int VECS = D / 8;                  // 16-byte vectors of a row
     extern __shared__ unsigned char dc_raw[];
-    __shared__ __align__(8) unsigned long long full[DC_TILE_BARS], empty[DC_TILE_BARS], xch[DX_COUNT];
+    __shared__ __align__(8) unsigned long long full[DC_BARS], empty[DC_BARS], xch[DX_COUNT];
     __shared__ int dead, positions[DC_MAX_ROWS];
     const gdb_decode_args &a = g.a;
     dc_ctx c;
@@ -403,9 +409,9 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
     c.dead = &dead;
     c.err_flag = a.err_flag;
     c.rank = gdb_t5::cluster_ctarank();
-    c.slots = g.lay.slots;
+    c.places = g.lay.places;
     c.n = 0U;
-    c.slot = 0U;
+    c.place = 0U;
     c.tid = threadIdx.x;
     c.warp = threadIdx.x >> 5;
     c.lane = threadIdx.x & 31;
@@ -423,7 +429,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
 
     if (c.tid < rows) positions[c.tid] = a.positions[b0 + c.tid];
     const int t0 = *a.step_counter;
-    if (c.tid < (int)DC_TILE_BARS) {
+    if (c.tid < (int)DC_BARS) {
         gdb_t5::mbar_init(c.full + (uint32_t)c.tid * 8U, 1U);
         gdb_t5::mbar_init(c.empty + (uint32_t)c.tid * 8U, 16U);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -468,20 +474,21 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
         const int hl = c.warp % hpc, split = c.warp / hpc;
         const uint32_t hpc_log = 31U - (uint32_t)__clz(hpc), groups_log = 31U - (uint32_t)__clz(groups);   // (both divide the head count, a power of two)
 
-        auto wait_tile = [&](uint32_t i, uint32_t *empty_bar) {   // tile i of this phase: its shared-memory address
-            uint32_t slot = c.slot + i;
+        auto wait_use = [&](uint32_t i, uint32_t *empty_bar) {   // use i of this phase: its shared-memory address
+            uint32_t place = c.place + i;
 #pragma unroll 1
-            while (slot >= c.slots) slot -= c.slots;
-            const uint32_t n = c.n + i, which = (n % DC_TILE_BARS) * 8U;
+            while (place >= c.places) place -= c.places;
+            const uint32_t n = c.n + i, which = (n % DC_BARS) * 8U;
             *empty_bar = c.empty + which;
-            dc_wait(c, c.full + which, (n / DC_TILE_BARS) & 1U);
-            return c.sm + slot * DC_TILE;
+            dc_wait(c, c.full + which, (n / DC_BARS) & 1U);
+            return c.sm + place * DC_PLACE;
         };
-        auto advance = [&](uint32_t tiles) {
-            c.n += tiles;
-            c.slot += tiles;
+        auto wait_tile = [&](uint32_t i, uint32_t *empty_bar) { return wait_use(2U * i, empty_bar); };   // weight tile i of this phase
+        auto advance = [&](uint32_t uses) {
+            c.n += uses;
+            c.place += uses;
 #pragma unroll 1
-            while (c.slot >= c.slots) c.slot -= c.slots;
+            while (c.place >= c.places) c.place -= c.places;
         };
         // The id that sequence r is at: the best of the CTAs' classes. CTA 0 records it as the choice of step `step`.
         auto best_id = [&](int r, int step) {
@@ -553,11 +560,11 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                                 }
                             }
                     }
-                    // The weights are there before the rows are, as a rule: their wait is not behind the rows'. (A tile whose slot another
+                    // The weights are there before the rows are, as a rule: their wait is not behind the rows'. (A tile whose place another
                     // tile of this phase must leave first is waited for behind the block barrier that the other's readers need.)
                     uint32_t em0 = 0U, tile0 = 0U;
                     const uint32_t i_first = whole ? u_first : (uint32_t)c.warp;
-                    if (u_first < n && i_first < c.slots) tile0 = wait_tile(i_first, &em0);
+                    if (u_first < n && 2U * i_first + 1U < c.places) tile0 = wait_tile(i_first, &em0);
                     if (j != 0 || step > 0) receive(j == 0 ? DX_LM : (up ? DX_RESID : DX_X), j == 0 ? key_bytes : row_bytes);
                     if (c.warp < rows) {
                         const uint32_t at = (up ? s_resid : s_x) + (uint32_t)c.warp * (D * 2U) + (uint32_t)c.lane * 16U;
@@ -636,9 +643,9 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                             float acc[4][NT][4];
                             uint32_t em = em0, tile = tile0;
                             if (u0 != 0U || (whole && half != 0U)) tile = wait_tile(2U * u0 + half * min(n - u0, 16U) + (u - u0), &em);
-                            else if (i_first >= c.slots) tile = wait_tile(i_first, &em);
+                            else if (2U * i_first + 1U >= c.places) tile = wait_tile(i_first, &em);
                             dc_ranges<T, D, NT, 4>(acc, tile, acts + half * D, 0U, c.lane);
-                            dc_release<16>(em, c.lane);
+                            dc_release<2>(em, 16U, c.lane);
                             if (whole || half == 0U) {
 #pragma unroll
                                 for (int t = 0; t < NT; ++t)
@@ -729,7 +736,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                             __syncwarp();
                         }
                     }
-                    advance(2U * n);
+                    advance(4U * n);
                     if (kind == DC_LM) {
                         // over the eight weight rows of the fragment, then over the warps, then to every CTA
 #pragma unroll
@@ -766,7 +773,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                     // ---- attention: head hl of each of the CTA's units, key range `split`; the ranges are merged in shared memory ----
                     const uint32_t s_part = c.sm + g.lay.scratch;
                     uint32_t at = 0U;
-                    int turn = 0;   // tiles of 32 keys this warp has folded in this phase
+                    int turn = 0;   // tiles of 16 keys this warp has folded in this phase
 #pragma unroll 1
                     for (int unit = (int)c.rank; unit < attn_units; unit += (int)CS, ++at) {
                         const int row = unit >> groups_log, pos = positions[row] + step;
@@ -775,34 +782,30 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                         const uint32_t fresh = s_qkv + (at * 3U * (uint32_t)hpc + (uint32_t)hl) * 128U;   // q, then k and v hpc and 2 hpc rows on
                         uint32_t em = 0U, tile = 0U;
                         if (at == 0U) {
-                            if (kr.iters > 0) tile = wait_tile((uint32_t)c.warp, &em);
+                            if (kr.iters > 0) tile = wait_use((uint32_t)c.warp, &em);
                             receive(DX_QKV, qkv_bytes);
                         }
                         decode_fold64<T> state;
                         state.init(c.lane, [&](int i, int hh) { return dc_lds4(fresh + (uint32_t)(i * 32 + hh * 16 + c.lane * 4)); });
 #pragma unroll 1
                         for (int it = 0; it < kr.iters; ++it, ++turn) {
-                            if (turn != 0 && (turn & 1) == 0) dc_sync();
-                            if (at != 0U || it != 0) tile = wait_tile((uint32_t)(it * DC_WARPS + c.warp), &em);
-                            bool written = false;
-#pragma unroll 1
-                            for (int k0 = 0; k0 < 32; k0 += 16) {
-                                const int key = s_lo + it * 32 + k0, left = s_hi - key, newest = pos - key;
-                                if (left <= 0) break;
-                                const uint32_t keys = tile + (uint32_t)k0 * 128U, values = keys + 4096U;
-                                if (newest >= 0 && newest < min(left, 16)) {   // the newest key and value in their rows
+                            if (turn != 0 && (turn & 3) == 0) dc_sync();
+                            if (at != 0U || it != 0) tile = wait_use((uint32_t)(it * DC_WARPS + c.warp), &em);
+                            const int key = s_lo + it * 16, left = s_hi - key, newest = pos - key;
+                            if (left > 0) {
+                                const bool here = newest >= 0 && newest < min(left, 16);   // the newest key and value: put in their rows
+                                if (here) {
                                     if (c.lane < 16) {
                                         const uint32_t piece = (uint32_t)c.lane & 7U, kind_of = (uint32_t)c.lane >> 3;
-                                        dc_sts16((kind_of == 0U ? keys : values) + (uint32_t)newest * 128U + ((piece ^ ((uint32_t)newest & 7U)) << 4),
+                                        dc_sts16(tile + kind_of * 2048U + (uint32_t)newest * 128U + ((piece ^ ((uint32_t)newest & 7U)) << 4),
                                                  dc_lds16(fresh + (kind_of + 1U) * (uint32_t)hpc * 128U + piece * 16U));
                                     }
                                     __syncwarp();
-                                    written = true;
                                 }
-                                state.fold(keys, values, (c.lane >> 2) < left, (c.lane >> 2) + 8 < left, a.scale, c.lane);
+                                state.fold(tile, tile + 2048U, (c.lane >> 2) < left, (c.lane >> 2) + 8 < left, a.scale, c.lane);
+                                if (here) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // before the place's next copy
                             }
-                            if (written) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // before the slot's next copy
-                            dc_release<16>(em, c.lane);
+                            dc_release<1>(em, 16U, c.lane);
                         }
                         advance((uint32_t)(kr.iters * DC_WARPS));
                         float *ml = reinterpret_cast<float *>(generic + g.lay.scratch) + at * DC_PARTIALS;
@@ -858,8 +861,8 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                     float acc[1][NT][4];
                     if (!up) {
                         dc_ranges<T, D, NT, 1>(acc, tile, s_attn + brow * LDA + bcol + (((uint32_t)c.warp >> 2) & 1U) * D, (uint32_t)c.warp & 3U, c.lane);
-                        dc_release<4>(em, c.lane);
-                        advance(4U);
+                        dc_release<2>(em, 4U, c.lane);
+                        advance(8U);
                     } else {
 #pragma unroll
                         for (int t = 0; t < NT; ++t)
@@ -894,10 +897,9 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
 #pragma unroll 1
                                 for (uint32_t i = 0; i < kw / 16U; ++i) k16(w + i * 1024U, x + i * 32U);
                             }
-                            __syncwarp();
-                            if (c.lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(em), "r"(kw / 16U) : "memory");   // (of 256 / kw warps)
+                            dc_release<2>(em, kw / 16U, c.lane);   // (of 256 / kw warps)
                         }
-                        advance(F / 128U);
+                        advance(F / 64U);
                     }
                     // the ranges' sums through shared memory, then a thread per output; the new rows go to every CTA
                     dc_leave_range<NT>(acc[0], s_red + (uint32_t)c.warp * (NT * 512U) + (uint32_t)c.lane * 16U);
@@ -997,10 +999,10 @@ dc_kernel dc_pick(uint32_t D, int tiles)
     return D == 256U ? decode_cluster_kernel<T, 256, 1> : decode_cluster_kernel<T, 128, 1>;   // (of these enough clusters are resident)
 }
 
-// Shared memory of a CTA whose cluster has `rows` sequences; false when fewer than DC_MIN_SLOTS tiles fit beside it.
+// Shared memory of a CTA whose cluster has `rows` sequences; false when fewer than DC_MIN_PLACES places fit beside it.
 bool dc_make_layout(dc_layout *l, uint32_t rows, uint32_t D, uint32_t F, uint32_t H, uint32_t splits)
 {
-    constexpr uint32_t limit = 232448U - 4096U;   // dynamic part: static tables and the alignment of the ring taken off
+    constexpr uint32_t limit = 232448U - 6144U;   // dynamic part: static tables and the alignment of the ring taken off
     const uint32_t tiles = rows > 8U ? 2U : 1U, CS = D / 32U, hpc = 16U / splits, units = (rows * (H / hpc) + CS - 1U) / CS;
     uint32_t top = 0U;
     auto take = [&](uint32_t bytes) {
@@ -1022,9 +1024,9 @@ bool dc_make_layout(dc_layout *l, uint32_t rows, uint32_t D, uint32_t F, uint32_
     l->red = take(16U * tiles * 1024U);   // eight units of four k ranges, or two of eight
     l->staging = take(16U * std::max(tiles * 256U, (uint32_t)DC_MAX_ROWS * 8U));
     l->keys = take(CS * DC_MAX_ROWS * 8U);
-    if (top + DC_MIN_SLOTS * DC_TILE > limit) return false;
-    l->slots = std::min((limit - top) / DC_TILE, DC_MAX_SLOTS);
-    const uint32_t ring = l->slots * DC_TILE;
+    if (top + DC_MIN_PLACES * DC_PLACE > limit) return false;
+    l->places = std::min((limit - top) / DC_PLACE & ~1U, DC_MAX_PLACES);
+    const uint32_t ring = l->places * DC_PLACE;
     for (uint32_t *o : {&l->x, &l->resid, &l->normed, &l->act, &l->attn, &l->scratch, &l->qkv, &l->red, &l->staging, &l->keys}) *o += ring;
     l->total = top + ring;
     return true;
@@ -1090,8 +1092,8 @@ gd_status gdb_decode_cluster_launch(gd_backend *be, uint32_t dtype, const gdb_de
         mapped = dc_map_rows(&g.w[i][DC_QKV], dtype, a->lw[i][1], 32U, 32U, 3U * D / 32U, D) && dc_map_rows(&g.w[i][DC_OUT], dtype, a->lw[i][3], 8U, 8U, D / 8U, D) &&
                  dc_map_rows(&g.w[i][DC_UP], dtype, a->lw[i][6], F, F, 2U, D) && dc_map_down(&g.w[i][DC_DOWN], dtype, a->lw[i][8], F, D);
         for (int j = 0; j < 2 && mapped; ++j) mapped = dc_map_ahead(&g.kv_ahead[i][j], dtype, j == 0 ? a->kc[i] : a->vc[i], (uint64_t)a->B, cap, D, 64U * (16U / (uint32_t)a->splits));
-        for (int j = 0; j < 4 && mapped; ++j)
-            mapped = gdb_t5::make_tmap_batched(&g.kv[i][j >> 1][j & 1], dtype, j < 2 ? a->kc[i] : a->vc[i], (uint64_t)a->B, cap, D, D * 2U, cap * D * 2U, 64U, (j & 1) != 0 ? 16U : 32U);
+        for (int j = 0; j < 2 && mapped; ++j)
+            mapped = gdb_t5::make_tmap_batched(&g.kv[i][j], dtype, j == 0 ? a->kc[i] : a->vc[i], (uint64_t)a->B, cap, D, D * 2U, cap * D * 2U, 64U, 16U);
     }
     if (!mapped) {
         return GD_ERR_UNSUPPORTED;
