@@ -51,6 +51,12 @@ constexpr uint32_t DC_MAX_PLACES = 48U, DC_MIN_PLACES = 16U;
 // four tiles per warp of the attention, whose warps may start while others have their part of the 12 QKV tiles to do; an exchange that
 // needs all warps ends the other phases), and at most 48 more are in flight.
 constexpr uint32_t DC_BARS = 256U;
+// Hardware barriers of the consumer warps: all of them; the two warps of a unit whose halves of k are formed apart (up to eight units);
+// the eight warps of one of the two units of a residual projection. A barrier has ONE number of threads: only the exchanges keep the
+// last two uses apart, and a CTA that gave a wait up skips those, so they share no barrier.
+constexpr uint32_t DC_BAR_ALL = 1U, DC_BAR_PAIR = 2U, DC_PAIRS = 8U, DC_BAR_SUM = DC_BAR_PAIR + DC_PAIRS, DC_SUMS = 2U;
+static_assert(DC_BAR_ALL > 0U && DC_BAR_PAIR > DC_BAR_ALL && DC_BAR_SUM >= DC_BAR_PAIR + DC_PAIRS && DC_BAR_SUM + DC_SUMS <= 16U,
+              "barrier 0 is __syncthreads, a block has 16, and no barrier is used with two numbers of threads");
 constexpr unsigned DC_SPIN_LIMIT = 1U << 21;
 constexpr int DC_ERR_WAIT = 398;
 
@@ -95,7 +101,7 @@ __device__ __forceinline__ void dc_send8(uint32_t addr, unsigned long long v, ui
 {
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr), "l"(v), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void dc_sync() { asm volatile("bar.sync 1, %0;" ::"n"(DC_WARPS * 32) : "memory"); }
+__device__ __forceinline__ void dc_sync() { asm volatile("bar.sync %0, %1;" ::"n"(DC_BAR_ALL), "n"(DC_WARPS * 32) : "memory"); }
 __device__ __forceinline__ uint4 dc_lds16(uint32_t addr)
 {
     uint4 v;
@@ -315,7 +321,7 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
             const CUtensorMap *map = kind == DC_LM ? &g.lm : &g.w[layer][kind];
             const uint32_t units = kind == DC_QKV ? 6U : (kind == DC_OUT ? 2U : (kind == DC_UP ? up_n : lm_n)), first = kind == DC_UP ? up_first : lm_first;
             const uint32_t tiles = kind == DC_DOWN ? F / 128U : 2U * units;
-            const bool whole = (kind == DC_UP || kind == DC_LM) && units > 8U;   // a warp to a unit: the first halves of 16 units, then the second
+            const bool whole = (kind == DC_UP || kind == DC_LM) && units > DC_PAIRS;   // a warp to a unit: the first halves of 16 units, then the second
             uint32_t s = wrap(place + 2U * which);
 #pragma unroll 1
             for (uint32_t i = which; i < tiles; i += DC_PRODUCERS, s = wrap(s + 2U * DC_PRODUCERS)) {
@@ -533,7 +539,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                 const bool up = (j & 1) != 0;
                 const uint32_t n = kind == DC_QKV ? 6U : (kind == DC_UP ? up_n : lm_n), first = kind == DC_UP ? up_first : lm_first;
                 // Two warps to a unit (a half of k each) when there are up to eight units, else one, in rounds of 16.
-                const bool whole = n > 8U;
+                const bool whole = n > DC_PAIRS;
                 const T *bias = (const T *)(kind == DC_LM ? a.b_lm : lw[kind == DC_QKV ? 2 : 7]);
                 {
                     // ---- the rows' norm; what depends on no exchange is read ahead of it ----
@@ -662,13 +668,13 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                             } else {
 #pragma unroll
                                 for (int s = 0; s < 4; ++s) dc_leave_range<NT>(acc[s], slot0 + (uint32_t)s * (NT * 512U));
-                                asm volatile("bar.arrive %0, 64;" ::"r"(u + 2U) : "memory");
+                                asm volatile("bar.arrive %0, 64;" ::"r"(DC_BAR_PAIR + u) : "memory");
                                 mine = false;
                             }
                         }
                         if (!mine) continue;
                         if (!whole) {
-                            asm volatile("bar.sync %0, 64;" ::"r"(u + 2U) : "memory");
+                            asm volatile("bar.sync %0, 64;" ::"r"(DC_BAR_PAIR + u) : "memory");
 #pragma unroll
                             for (int s = 0; s < 4; ++s)
 #pragma unroll
@@ -909,7 +915,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                     }
                     // the ranges' sums through shared memory, then a thread per output; the new rows go to every CTA
                     dc_leave_range<NT>(acc[0], s_red + (uint32_t)c.warp * (NT * 512U) + (uint32_t)c.lane * 16U);
-                    asm volatile("bar.sync %0, 256;" ::"r"(ou + 2) : "memory");
+                    asm volatile("bar.sync %0, 256;" ::"r"(DC_BAR_SUM + (uint32_t)ou) : "memory");
                     const uint32_t src = s_red + (uint32_t)ou * (NT * 4096U) + (NT == 2 ? (uint32_t)(oi >> 7) * 512U : 0U) + (uint32_t)((oi & 7) * 4 + ((oi >> 3) & 7) / 2) * 16U +
                                          (uint32_t)(ohalf * 2 + ((oi >> 3) & 1)) * 4U;
                     float v = 0.0f;
