@@ -192,6 +192,7 @@ gd_status gd_backend_create_default(gd_backend **out_backend)
         return GD_ERR_OUT_OF_MEMORY;
     }
     be->tickets = (unsigned *)be->err_flag + 64;
+    be->decode_mute = -1;
     *out_backend = be;
     return GD_OK;
 }

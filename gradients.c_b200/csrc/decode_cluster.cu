@@ -23,8 +23,10 @@
 // 148 -> 117.4. A phase of one sequence is some 5 k cycles, of which the exchange 1.0-1.4 k; an all-to-all of 8 KB in a cluster of 16 took
 // 1345 cycles by st.async, 1550 by bulk copies, 2400 by remote stores and a releasing arrive.
 //
-// Waits are bounded: a wait that gives up stores code 398 in the backend's error word and raises the CTA's flag, after which its
-// threads run through the remaining phases without waiting and without sending, up to the cluster barrier at the end.
+// Waits are bounded. One that gives up stores code 398 in the backend's error word and raises the CTA's flag; from then on its thread
+// neither waits nor sends nor releases a place of the ring, nor does a thread that shares a block barrier with it. An exchange that
+// completes therefore carries rows that were formed from complete ones only, the other CTAs of the cluster give up at the next one, and
+// each leaves at the vote its consumer warps take once per norm: their sequences keep the ids, positions and step counter they had.
 #include "common.cuh"
 #include "decode_parts.cuh"
 #include "tcgen05.cuh"
@@ -57,7 +59,7 @@ constexpr uint32_t DC_BARS = 256U;
 constexpr uint32_t DC_BAR_ALL = 1U, DC_BAR_PAIR = 2U, DC_PAIRS = 8U, DC_BAR_SUM = DC_BAR_PAIR + DC_PAIRS, DC_SUMS = 2U;
 static_assert(DC_BAR_ALL > 0U && DC_BAR_PAIR > DC_BAR_ALL && DC_BAR_SUM >= DC_BAR_PAIR + DC_PAIRS && DC_BAR_SUM + DC_SUMS <= 16U,
               "barrier 0 is __syncthreads, a block has 16, and no barrier is used with two numbers of threads");
-constexpr unsigned DC_SPIN_LIMIT = 1U << 21;
+constexpr unsigned DC_WAIT_POLLS = 1U << 21;
 constexpr int DC_ERR_WAIT = 398;
 
 enum { DC_QKV = 0, DC_OUT = 1, DC_UP = 2, DC_DOWN = 3, DC_LM = 4 };
@@ -77,13 +79,15 @@ struct dc_args {
     CUtensorMap lm, w[GDB_DECODE_MAX_LAYERS][4];
     CUtensorMap kv[GDB_DECODE_MAX_LAYERS][2];         // keys, values; a head x 16 positions
     CUtensorMap kv_ahead[GDB_DECODE_MAX_LAYERS][2];   // the heads of an attention unit x 64 positions, for prefetches
+    int mute, mute_step;      // for tests: consumer warps of CTA `mute` of every cluster give up at that step (mute < 0: none)
+    unsigned wait_polls;      // of a wait before it gives up
 };
 
 // One CTA's side of the exchanges and of the ring.
 struct dc_ctx {
     uint32_t sm;                  // shared-memory address of the ring; everything else lies behind it
     uint32_t full, empty;         // addresses of the uses' barriers
-    volatile int *dead;
+    volatile int *dead;           // [0] a wait of this CTA gave up, [1] polls before one does, [2] another CTA of the cluster gave up
     int *err_flag;
     uint32_t rank, places, n, place;   // ring cursor: use and place of the next phase's first tile
     int tid, warp, lane;
@@ -102,6 +106,16 @@ __device__ __forceinline__ void dc_send8(uint32_t addr, unsigned long long v, ui
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr), "l"(v), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void dc_sync() { asm volatile("bar.sync %0, %1;" ::"n"(DC_BAR_ALL), "n"(DC_WARPS * 32) : "memory"); }
+// The same, and whether no consumer thread has given up: one answer for all of them.
+__device__ __forceinline__ bool dc_sync_vote(bool alive)
+{
+    uint32_t all;
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbar.red.and.pred q, %2, %3, p;\nselp.u32 %0, 1, 0, q;\n}"
+                 : "=r"(all)
+                 : "r"((uint32_t)alive), "n"(DC_BAR_ALL), "n"(DC_WARPS * 32)
+                 : "memory");
+    return all != 0U;
+}
 __device__ __forceinline__ uint4 dc_lds16(uint32_t addr)
 {
     uint4 v;
@@ -194,7 +208,7 @@ __device__ __forceinline__ bool dc_try_wait(uint32_t bar, uint32_t parity)
 __device__ __noinline__ bool dc_wait_more(uint32_t bar, uint32_t parity, volatile int *dead, int *err_flag)
 {
 #pragma unroll 1
-    for (unsigned it = 0; it < DC_SPIN_LIMIT; ++it) {
+    for (unsigned it = (unsigned)dead[1]; it > 0U; --it) {
         if (dc_try_wait(bar, parity)) return true;
         if (*dead != 0) return false;
     }
@@ -206,6 +220,8 @@ __device__ __forceinline__ void dc_wait(dc_ctx &c, uint32_t bar, uint32_t parity
 {
     if (c.alive && !dc_try_wait(bar, parity)) c.alive = dc_wait_more(bar, parity, c.dead, c.err_flag);
 }
+// Behind a block barrier: what the others left in shared memory is complete if none of them had given up before it.
+__device__ __forceinline__ void dc_check(dc_ctx &c) { c.alive = c.alive && *c.dead == 0; }
 
 // First unit and number of units of this CTA in a phase of `n` units shared by the cluster.
 __device__ __forceinline__ void dc_share(uint32_t n, uint32_t rank, uint32_t ctas, uint32_t *first, uint32_t *count)
@@ -272,6 +288,7 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
     for (int step = 0; step < a.n_steps; ++step) {
 #pragma unroll 1
         for (int ph = 0; ph <= 4 * a.L; ++ph) {
+            if (!__all_sync(0xffffffffU, c.alive)) return;
             const int kind = ph == 4 * a.L ? (int)DC_LM : (ph & 3), layer = ph >> 2;
             if (kind == DC_OUT) {
                 // keys and values of this CTA's attention units: use (i, w) for the i-th 16 keys of warp w's (head, split)
@@ -398,10 +415,10 @@ __device__ __forceinline__ void dc_ranges(float (&acc)[G][NT][4], uint32_t tile,
 }
 // `shares` of the 16 reader shares of a tile of one or two places are done.
 template <int PLACES>
-__device__ __forceinline__ void dc_release(uint32_t empty, uint32_t shares, int lane)
+__device__ __forceinline__ void dc_release(const dc_ctx &c, uint32_t empty, uint32_t shares)
 {
     __syncwarp();
-    if (lane < PLACES) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(empty + (uint32_t)lane * 8U), "r"(shares) : "memory");
+    if (c.lane < PLACES && c.alive) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(empty + (uint32_t)c.lane * 8U), "r"(shares) : "memory");
 }
 
 template <typename T, int D, int NT>
@@ -412,13 +429,13 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
     constexpr int VECS = D / 8;                  // 16-byte vectors of a row
     extern __shared__ unsigned char dc_raw[];
     __shared__ __align__(8) unsigned long long full[DC_BARS], empty[DC_BARS], xch[DX_COUNT];
-    __shared__ int dead, positions[DC_MAX_ROWS];
+    __shared__ int dead[3], positions[DC_MAX_ROWS];
     const gdb_decode_args &a = g.a;
     dc_ctx c;
     c.sm = (smem_u32(dc_raw) + 1023U) & ~1023U;
     c.full = smem_u32(full);
     c.empty = smem_u32(empty);
-    c.dead = &dead;
+    c.dead = dead;
     c.err_flag = a.err_flag;
     c.rank = gdb_t5::cluster_ctarank();
     c.places = g.lay.places;
@@ -447,7 +464,8 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (c.tid == 0) {
-        dead = 0;
+        dead[0] = dead[2] = 0;
+        dead[1] = (int)g.wait_polls;
         for (int i = 0; i < DX_COUNT; ++i) gdb_t5::mbar_init(bar(i), i == DX_LM ? CS + 1U : 1U);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         gdb_t5::mbar_expect_tx(bar(DX_QKV), qkv_bytes);
@@ -511,7 +529,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                 key = other > key ? other : key;
             }
             const int id = (int)(0xffffffffU - (unsigned)(key & 0xffffffffULL)), t = t0 + step;
-            if (c.rank == 0U && c.lane == 0 && t >= 0 && t < a.max_steps) a.out_tokens[(size_t)t * a.B + b0 + r] = id;
+            if (c.rank == 0U && c.lane == 0 && c.alive && t >= 0 && t < a.max_steps) a.out_tokens[(size_t)t * a.B + b0 + r] = id;
             return id;
         };
         // Eight lanes' neighbouring outputs as one vector, which every one of them gets.
@@ -527,8 +545,10 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
             return v;
         };
 
+        bool going = true;   // no consumer thread has given up at the last vote
 #pragma unroll 1
-        for (int step = 0; step < a.n_steps; ++step) {
+        for (int step = 0; step < a.n_steps && going; ++step) {
+            if (step == g.mute_step && g.mute == (int)c.rank) c.alive = false;
             // Pairs of a normed projection and what follows it: QKV, attention, output projection; up / gate, down projection; at last the LM
             // head. One body of code for all of them (with a copy per kind, 100 KB of code instead of 70, a step of one sequence took
             // 45.0 us instead of 44.4).
@@ -626,7 +646,8 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                             }
                         }
                     }
-                    dc_sync();
+                    going = dc_sync_vote(c.alive);
+                    if (!going) break;
 
                     // ---- QKV, up / gate or LM head ----
                     const uint32_t acts = s_normed + brow * LDA + bcol;
@@ -657,7 +678,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                             if (u0 != 0U || (whole && half != 0U)) tile = wait_tile(2U * u0 + half * min(n - u0, 16U) + (u - u0), &em);
                             else if (2U * i_first + 1U >= c.places) tile = wait_tile(i_first, &em);
                             dc_ranges<T, D, NT, 4>(acc, tile, acts + half * D, 0U, c.lane);
-                            dc_release<2>(em, 16U, c.lane);
+                            dc_release<2>(c, em, 16U);
                             if (whole || half == 0U) {
 #pragma unroll
                                 for (int t = 0; t < NT; ++t)
@@ -675,6 +696,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                         if (!mine) continue;
                         if (!whole) {
                             asm volatile("bar.sync %0, 64;" ::"r"(DC_BAR_PAIR + u) : "memory");
+                            dc_check(c);
 #pragma unroll
                             for (int s = 0; s < 4; ++s)
 #pragma unroll
@@ -742,7 +764,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                                 const uint32_t dst = s_qkv + ((at * 3U + what) * (uint32_t)hpc + (head & ((uint32_t)hpc - 1U))) * 128U + (col & 63U) * 2U;
                                 if (c.alive) dc_send(mapa_shared(dst, to), val, mapa_shared(bar(DX_QKV), to));
                                 const int pos = positions[row] + step;
-                                if (what != 0U && pos >= 0 && pos < a.CAP)
+                                if (c.alive && what != 0U && pos >= 0 && pos < a.CAP)
                                     *reinterpret_cast<uint4 *>((T *)(what == 1U ? a.kc[j >> 1] : a.vc[j >> 1]) + ((size_t)(b0 + row) * a.CAP + (size_t)pos) * D + col) = val;
                             }
                             __syncwarp();
@@ -763,6 +785,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                                 if (c.lane < 4) asm volatile("st.shared.b64 [%0], %1;" ::"r"(s_wkeys + (uint32_t)(c.warp * DC_MAX_ROWS + t * 8 + t2 + e) * 8U), "l"(best[t][e]) : "memory");
                             }
                         dc_sync();
+                        dc_check(c);
                         const uint32_t row = (uint32_t)c.tid & 15U, to = (uint32_t)c.tid >> 4;
                         if (to < CS) {
                             if ((int)row < rows) {
@@ -817,7 +840,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                                 state.fold(tile, tile + 2048U, (c.lane >> 2) < left, (c.lane >> 2) + 8 < left, a.scale, c.lane);
                                 if (here) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // before the place's next copy
                             }
-                            dc_release<1>(em, 16U, c.lane);
+                            dc_release<1>(c, em, 16U);
                         }
                         advance((uint32_t)(kr.iters * DC_WARPS));
                         float *ml = reinterpret_cast<float *>(generic + g.lay.scratch) + at * DC_PARTIALS;
@@ -825,6 +848,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                         state.merge_groups(ml + item * 2, ml + DC_WARPS * 2 + item * 64, c.lane);
                     }
                     dc_sync();
+                    dc_check(c);
                     // Merge of the splits of all units at once (decode_combine_query), one thread per output: weights, sum and output over the
                     // splits in order. (Unit by unit, by the warps of that unit's outputs: 64 sequences 122 us per step.)
 #pragma unroll 1
@@ -873,7 +897,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                     float acc[1][NT][4];
                     if (!up) {
                         dc_ranges<T, D, NT, 1>(acc, tile, s_attn + brow * LDA + bcol + (((uint32_t)c.warp >> 2) & 1U) * D, (uint32_t)c.warp & 3U, c.lane);
-                        dc_release<2>(em, 4U, c.lane);
+                        dc_release<2>(c, em, 4U);
                         advance(8U);
                     } else {
 #pragma unroll
@@ -909,13 +933,14 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
 #pragma unroll 1
                                 for (uint32_t i = 0; i < kw / 16U; ++i) k16(w + i * 1024U, x + i * 32U);
                             }
-                            dc_release<2>(em, kw / 16U, c.lane);   // (of 256 / kw warps)
+                            dc_release<2>(c, em, kw / 16U);   // (of 256 / kw warps)
                         }
                         advance(F / 64U);
                     }
                     // the ranges' sums through shared memory, then a thread per output; the new rows go to every CTA
                     dc_leave_range<NT>(acc[0], s_red + (uint32_t)c.warp * (NT * 512U) + (uint32_t)c.lane * 16U);
                     asm volatile("bar.sync %0, 256;" ::"r"(DC_BAR_SUM + (uint32_t)ou) : "memory");
+                    dc_check(c);
                     const uint32_t src = s_red + (uint32_t)ou * (NT * 4096U) + (NT == 2 ? (uint32_t)(oi >> 7) * 512U : 0U) + (uint32_t)((oi & 7) * 4 + ((oi >> 3) & 7) / 2) * 16U +
                                          (uint32_t)(ohalf * 2 + ((oi >> 3) & 1)) * 4U;
                     float v = 0.0f;
@@ -940,28 +965,33 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                 }
             }
         }
-        receive(DX_LM, key_bytes);
-        if (c.warp < rows) {
+        if (going) receive(DX_LM, key_bytes);
+        else if (c.tid == 0) dead[0] = 1;   // (a warp may have given up without a wait of its own; the producers stop)
+        if (going && c.warp < rows) {
             const int id = best_id(c.warp, a.n_steps - 1);
-            if (c.rank == 0U && c.lane == 0) {
+            if (c.rank == 0U && c.lane == 0 && c.alive) {
                 a.tokens[b0 + c.warp] = id;
                 a.positions[b0 + c.warp] += a.n_steps;
             }
         }
-        if (c.rank == 0U && c.tid == 0) {
-            // every cluster has read the counter before it counts itself here; the last one advances it
+        if (c.rank == 0U && c.tid == 0 && going && c.alive) {
+            // every cluster has read the counter before it counts itself here; the last one advances it (one that gave up does not count)
             __threadfence();
             if (atomicAdd(a.sync, 1U) == gridDim.x / CS - 1U) *a.step_counter = t0 + a.n_steps;
         }
     }
-    // No block ends while another may still write to its shared memory; after a wait that gave up, copies in flight get time to land.
+    // No block ends while another may still write to its shared memory: after a wait that gave up, sends and copies in flight get a
+    // millisecond to land, in every CTA and from when none of them issues any more.
     __syncthreads();
-    if (dead != 0) {
+    if (dead[0] != 0 && c.tid < (int)CS) asm volatile("st.shared::cluster.b32 [%0], 1;" ::"r"(mapa_shared(smem_u32(&dead[2]), (uint32_t)c.tid)) : "memory");
+    __syncwarp();
+    gdb_t5::cluster_sync_all();
+    if (c.dead[2] != 0) {
         const long long until = clock64() + 2000000LL;
         while (clock64() < until) { }
+        __syncwarp();
+        gdb_t5::cluster_sync_all();
     }
-    __syncthreads();
-    gdb_t5::cluster_sync_all();
 }
 
 // K-major weights as tiles of 16 rows (two groups of eight, `gap` rows apart, at multiples of `step` rows) x half of k, in shared memory
@@ -1072,6 +1102,10 @@ gd_status gdb_decode_cluster_launch(gd_backend *be, uint32_t dtype, const gdb_de
     cfg.numAttrs = 1;
     dc_args g;
     g.a = *a;
+    g.mute = be->decode_mute;
+    g.mute_step = be->decode_mute_step;
+    g.wait_polls = be->decode_mute < 0 ? DC_WAIT_POLLS : be->decode_mute_polls;
+    be->decode_mute = -1;
     dc_kernel kern = nullptr;
     auto prepare = [&](int rows) {   // kernel, layout and launch shape for `rows` sequences per cluster
         if (!dc_make_layout(&g.lay, (uint32_t)rows, D, F, (uint32_t)a->H, (uint32_t)a->splits)) return false;

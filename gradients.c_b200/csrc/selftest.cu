@@ -3,11 +3,13 @@
 // Every wait in the kernels of this backend (on an mbarrier, a ticket or a flag) is bounded; when the limit runs out the
 // kernel stores a code in the backend's device error word and returns normally, and gd_backend_flush / fence_wait turn
 // the word into GD_ERR_INTERNAL (the reference maps a failed Metal command buffer to GD_ERR_INTERNAL at flush in the same
-// way, src/backends/metal/backend_metal.m:569-573). The two entries here let a test drive that path on purpose:
+// way, src/backends/metal/backend_metal.m:569-573). The three entries here let a test drive that path on purpose:
 //   gdb200_inject_device_error     stores a code in the error word in stream order (a host-injected failure)
 //   gdb200_selftest_bounded_wait   runs a one-warp kernel that waits, with a caller-chosen iteration limit, on an mbarrier
 //                                  nobody ever arrives at, stores code 399 when the limit runs out and returns
-// Neither traps, spins without bound or touches memory it does not own; the CUDA context stays usable.
+//   gdb200_selftest_decode_give_up has one CTA of each cluster fall silent in the next run of decode steps, so that the waits
+//                                  of the others run out after a caller-chosen number of polls (code 398)
+// None of them traps, spins without bound or touches memory it does not own; the CUDA context stays usable.
 #include "tcgen05.cuh"
 
 namespace {
@@ -70,6 +72,17 @@ gd_status gdb200_selftest_bounded_wait(gd_backend *be, uint32_t max_iters)
     cudaSetDevice(be->device);
     gdb_launch(bounded_wait_kernel, 1, 32, 0, be->stream, be->err_flag, (unsigned)max_iters, (unsigned *)nullptr);
     return gdb_launched(be, "selftest_bounded_wait");
+}
+
+gd_status gdb200_selftest_decode_give_up(gd_backend *be, int32_t cta, int32_t step, uint32_t max_polls)
+{
+    if (be == NULL || cta < 0 || cta > 15 || step < 0 || max_polls == 0U || max_polls > (1U << 12)) {
+        return GD_ERR_INVALID_ARGUMENT;
+    }
+    be->decode_mute = cta;
+    be->decode_mute_step = step;
+    be->decode_mute_polls = max_polls;
+    return GD_OK;
 }
 
 }  // extern "C"

@@ -645,7 +645,8 @@ gd_status gdb200_gpt_prefill(gd_backend *backend, const gdb200_gpt_spec *spec, c
  * step. use_graph != 0: where the shapes allow (16-bit storage, at most 64 sequences, head_dim 64, d_model 128 / 256 / 512,
  * mlp_hidden a multiple of 128 and what of it fits shared memory, vocab_size a multiple of 16) ALL steps run in one kernel of
  * independent thread-block clusters (d_model / 32 CTAs each, a few sequences each, the weights read from L2; a wait that gives up
- * stores code 398 in the error word); otherwise the first step runs eagerly, the second is
+ * stores code 398 in the error word, and its cluster's sequences keep their ids and positions and all of them the step counter of
+ * before the call; out_tokens holds the steps that were done); otherwise the first step runs eagerly, the second is
  * recorded as a CUDA graph and the rest replay it. All forms generate the same ids and caches. */
 gd_status gdb200_gpt_decode_steps(gd_backend *backend, const gdb200_gpt_spec *spec, const gdb200_gpt_decode_state *state,
                                   int32_t n_steps, int32_t use_graph, size_t *scratch_used);
@@ -654,10 +655,13 @@ gd_status gdb200_gpt_decode_steps(gd_backend *backend, const gdb200_gpt_spec *sp
  * src/backends/metal/backend_metal.m:569-573; here every device-side wait is bounded and reports through an error word
  * that flush / fence_wait read). gdb200_inject_device_error stores `code` in that word in stream order;
  * gdb200_selftest_bounded_wait runs a one-warp kernel that polls an mbarrier nobody arrives at for at most max_iters
- * (<= 2^20) iterations, stores code 399 and returns. After either, gd_backend_flush returns GD_ERR_INTERNAL once,
+ * (<= 2^20) iterations, stores code 399 and returns; gdb200_selftest_decode_give_up has CTA `cta` (0 .. 15) of each cluster
+ * fall silent at step `step` of the next run of decode steps that is one launch, and the waits of the others give up after
+ * max_polls (<= 2^12) polls of up to 0.1 ms with code 398. After any of them, gd_backend_flush returns GD_ERR_INTERNAL once,
  * gdb200_last_error names the code, and the backend stays usable. */
 gd_status gdb200_inject_device_error(gd_backend *backend, int32_t code);
 gd_status gdb200_selftest_bounded_wait(gd_backend *backend, uint32_t max_iters);
+gd_status gdb200_selftest_decode_give_up(gd_backend *backend, int32_t cta, int32_t step, uint32_t max_polls);
 
 /* Data-parallel gradient exchange (the reference has no collective; one process per GPU).
  * id_bytes is the 128-byte ncclUniqueId produced by gdb200_dp_unique_id on rank 0. */
