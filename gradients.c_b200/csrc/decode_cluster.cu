@@ -59,7 +59,10 @@ constexpr uint32_t DC_BARS = 256U;
 constexpr uint32_t DC_BAR_ALL = 1U, DC_BAR_PAIR = 2U, DC_PAIRS = 8U, DC_BAR_SUM = DC_BAR_PAIR + DC_PAIRS, DC_SUMS = 2U;
 static_assert(DC_BAR_ALL > 0U && DC_BAR_PAIR > DC_BAR_ALL && DC_BAR_SUM >= DC_BAR_PAIR + DC_PAIRS && DC_BAR_SUM + DC_SUMS <= 16U,
               "barrier 0 is __syncthreads, a block has 16, and no barrier is used with two numbers of threads");
-constexpr unsigned DC_WAIT_POLLS = 1U << 21;
+// Time a wait may take before it gives up. What is waited for comes from the CTA's own copies or from CTAs that are resident with it: some
+// microseconds; a second or two leave room for other processes' time slices. (Time, not polls: how long a poll sleeps is the
+// hardware's choice, up to the hint of 0.1 ms, and 2^21 of them would be minutes.)
+constexpr unsigned DC_WAIT_US = 2000000U;
 constexpr int DC_ERR_WAIT = 398;
 
 enum { DC_QKV = 0, DC_OUT = 1, DC_UP = 2, DC_DOWN = 3, DC_LM = 4 };
@@ -80,14 +83,14 @@ struct dc_args {
     CUtensorMap kv[GDB_DECODE_MAX_LAYERS][2];         // keys, values; a head x 16 positions
     CUtensorMap kv_ahead[GDB_DECODE_MAX_LAYERS][2];   // the heads of an attention unit x 64 positions, for prefetches
     int mute, mute_step;      // for tests: consumer warps of CTA `mute` of every cluster give up at that step (mute < 0: none)
-    unsigned wait_polls;      // of a wait before it gives up
+    unsigned wait_us;         // a wait may take
 };
 
 // One CTA's side of the exchanges and of the ring.
 struct dc_ctx {
     uint32_t sm;                  // shared-memory address of the ring; everything else lies behind it
     uint32_t full, empty;         // addresses of the uses' barriers
-    volatile int *dead;           // [0] a wait of this CTA gave up, [1] polls before one does, [2] another CTA of the cluster gave up
+    volatile int *dead;           // [0] a wait of this CTA gave up, [1] microseconds before one does, [2] another CTA of the cluster gave up
     int *err_flag;
     uint32_t rank, places, n, place;   // ring cursor: use and place of the next phase's first tile
     int tid, warp, lane;
@@ -187,10 +190,15 @@ __device__ __noinline__ float2 dc_cos_sin(const gdb_decode_args &a, unsigned pai
     cs.y *= a.rope.sin_sign;   // (the sign is 1 or -1: its place for the caller is behind the table's values, which have none)
     return cs;
 }
-__device__ __noinline__ void dc_stamp(const gdb_decode_args &a, int *stamp)
+__device__ __forceinline__ unsigned long long dc_now()
 {
     unsigned long long ns;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(ns));
+    return ns;
+}
+__device__ __noinline__ void dc_stamp(const gdb_decode_args &a, int *stamp)
+{
+    const unsigned long long ns = dc_now();
     if (*stamp < a.n_steps * (5 * a.L + 1)) a.timeline[(*stamp)++] = ns;
 }
 __device__ __forceinline__ bool dc_try_wait(uint32_t bar, uint32_t parity)
@@ -207,11 +215,11 @@ __device__ __forceinline__ bool dc_try_wait(uint32_t bar, uint32_t parity)
 }
 __device__ __noinline__ bool dc_wait_more(uint32_t bar, uint32_t parity, volatile int *dead, int *err_flag)
 {
-#pragma unroll 1
-    for (unsigned it = (unsigned)dead[1]; it > 0U; --it) {
+    const unsigned long long since = dc_now(), limit = (unsigned long long)(unsigned)dead[1] * 1000ULL;
+    do {
         if (dc_try_wait(bar, parity)) return true;
         if (*dead != 0) return false;
-    }
+    } while (dc_now() - since < limit);
     *dead = 1;
     atomicCAS(err_flag, 0, DC_ERR_WAIT);
     return false;
@@ -465,7 +473,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
     }
     if (c.tid == 0) {
         dead[0] = dead[2] = 0;
-        dead[1] = (int)g.wait_polls;
+        dead[1] = (int)g.wait_us;
         for (int i = 0; i < DX_COUNT; ++i) gdb_t5::mbar_init(bar(i), i == DX_LM ? CS + 1U : 1U);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         gdb_t5::mbar_expect_tx(bar(DX_QKV), qkv_bytes);
@@ -1104,7 +1112,7 @@ gd_status gdb_decode_cluster_launch(gd_backend *be, uint32_t dtype, const gdb_de
     g.a = *a;
     g.mute = be->decode_mute;
     g.mute_step = be->decode_mute_step;
-    g.wait_polls = be->decode_mute < 0 ? DC_WAIT_POLLS : be->decode_mute_polls;
+    g.wait_us = be->decode_mute >= 0 && be->decode_wait_us != 0U ? be->decode_wait_us : DC_WAIT_US;
     be->decode_mute = -1;
     dc_kernel kern = nullptr;
     auto prepare = [&](int rows) {   // kernel, layout and launch shape for `rows` sequences per cluster

@@ -8,7 +8,7 @@
 //   gdb200_selftest_bounded_wait   runs a one-warp kernel that waits, with a caller-chosen iteration limit, on an mbarrier
 //                                  nobody ever arrives at, stores code 399 when the limit runs out and returns
 //   gdb200_selftest_decode_give_up has one CTA of each cluster fall silent in the next run of decode steps, so that the waits
-//                                  of the others run out after a caller-chosen number of polls (code 398)
+//                                  of the others run out after a caller-chosen time (code 398)
 // None of them traps, spins without bound or touches memory it does not own; the CUDA context stays usable.
 #include "tcgen05.cuh"
 
@@ -74,14 +74,14 @@ gd_status gdb200_selftest_bounded_wait(gd_backend *be, uint32_t max_iters)
     return gdb_launched(be, "selftest_bounded_wait");
 }
 
-gd_status gdb200_selftest_decode_give_up(gd_backend *be, int32_t cta, int32_t step, uint32_t max_polls)
+gd_status gdb200_selftest_decode_give_up(gd_backend *be, int32_t cta, int32_t step, uint32_t max_wait_us)
 {
-    if (be == NULL || cta < 0 || cta > 15 || step < 0 || max_polls == 0U || max_polls > (1U << 12)) {
+    if (be == NULL || cta < 0 || cta > 15 || step < 0 || max_wait_us > 1000000U) {
         return GD_ERR_INVALID_ARGUMENT;
     }
     be->decode_mute = cta;
     be->decode_mute_step = step;
-    be->decode_mute_polls = max_polls;
+    be->decode_wait_us = max_wait_us;
     return GD_OK;
 }
 

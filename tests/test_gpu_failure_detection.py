@@ -3,6 +3,7 @@ backend usable. The failure is made without a fault: a code stored in the backen
 one-warp kernel whose bounded wait on a barrier nobody arrives at runs out (a few thousand polls) and returns; a CTA of the
 decode kernel that falls silent, so that the exchanges of its cluster run out."""
 import ctypes as C
+import time
 
 import numpy as np
 import pytest
@@ -96,7 +97,7 @@ def test_decode_that_gives_up_leaves_ids_and_positions_where_they_were(d_model, 
     with pkg.runtime.Context(params_bytes=256 << 20, state_bytes=256 << 20, scratch_bytes=1 << 30) as ctx:
         run = DecodeRun(ctx, d_model, mlp_hidden, batch, new=8)
         before = run.words()
-        assert ctx.lib.gdb200_selftest_decode_give_up(ctx.backend, cta, step, 4096) == abi.GD_OK
+        assert ctx.lib.gdb200_selftest_decode_give_up(ctx.backend, cta, step, 50000) == abi.GD_OK
         assert run.decode() == abi.GD_ERR_INTERNAL and b"code 398" in ctx.lib.gdb200_last_error(ctx.backend)
         failed = run.words()
         assert np.array_equal(failed[0], before[0]) and np.array_equal(failed[1], before[1]) and failed[3] == before[3] == 1
@@ -108,3 +109,13 @@ def test_decode_that_gives_up_leaves_ids_and_positions_where_they_were(d_model, 
         assert still_usable(ctx)
         want = pkg.gpt_lm.greedy_generate_native(run.model, run.io.read()[:batch * 9].reshape(batch, 9), 8, 17, use_graph=False)
         assert np.array_equal(ids.T, want)
+
+
+def test_decode_gives_up_within_seconds():
+    with pkg.runtime.Context(params_bytes=256 << 20, state_bytes=256 << 20, scratch_bytes=1 << 30) as ctx:
+        run = DecodeRun(ctx, 512, 1024, 3, new=4)
+        assert ctx.lib.gdb200_selftest_decode_give_up(ctx.backend, 5, 1, 0) == abi.GD_OK
+        start = time.monotonic()
+        assert run.decode() == abi.GD_ERR_INTERNAL and b"code 398" in ctx.lib.gdb200_last_error(ctx.backend)
+        assert 1.5 < time.monotonic() - start < 10.0        # two seconds, once: no CTA waits a second time
+        assert run.decode() == abi.GD_OK
