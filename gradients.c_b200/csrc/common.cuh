@@ -59,7 +59,7 @@ struct gd_backend {
     unsigned *tickets;
     // of the next run of decode steps in one launch (gdb200_selftest_decode_give_up): the CTA that gives up, -1 for none
     int decode_mute, decode_mute_step;
-    unsigned decode_wait_us;   // microseconds before its waits give up, 0 for the kernel's own limit
+    unsigned decode_wait_ms;   // milliseconds before its waits give up, 0 for the kernel's own limit
     // scratch offsets of the parameter gradients of the last gdb200_gpt_train_step (valid until the arena is reused)
     int32_t last_grad_count;
     size_t last_grad_offset[GDB200_GPT_MAX_PARAMS];

@@ -24,9 +24,11 @@
 // 1345 cycles by st.async, 1550 by bulk copies, 2400 by remote stores and a releasing arrive.
 //
 // Waits are bounded. One that gives up stores code 398 in the backend's error word and raises the CTA's flag; from then on its thread
-// neither waits nor sends nor releases a place of the ring, nor does a thread that shares a block barrier with it. An exchange that
-// completes therefore carries rows that were formed from complete ones only, the other CTAs of the cluster give up at the next one, and
-// each leaves at the vote its consumer warps take once per norm: their sequences keep the ids, positions and step counter they had.
+// neither waits nor sends nor releases a place of the ring. The consumer warps vote once per step, ahead of sending the CTA's best
+// classes: a CTA in which one gave up sends none and leaves, so no CTA of the cluster completes that step's last exchange. Rows formed from
+// incomplete ones may have gone round within the step, but no id of it is recorded or fed back and the cache rows it wrote lie behind
+// every position: the sequences keep the ids, positions and step counter of before the launch. (The vote is in place of a block barrier
+// that is there anyway; behind every norm, or as one more barrier per step, it cost 1.1 and 0.7 us of a step of 41.)
 #include "common.cuh"
 #include "decode_parts.cuh"
 #include "tcgen05.cuh"
@@ -62,7 +64,7 @@ static_assert(DC_BAR_ALL > 0U && DC_BAR_PAIR > DC_BAR_ALL && DC_BAR_SUM >= DC_BA
 // Time a wait may take before it gives up. What is waited for comes from the CTA's own copies or from CTAs that are resident with it: some
 // microseconds; a second or two leave room for other processes' time slices. (Time, not polls: how long a poll sleeps is the
 // hardware's choice, up to the hint of 0.1 ms, and 2^21 of them would be minutes.)
-constexpr unsigned DC_WAIT_US = 2000000U;
+constexpr unsigned DC_WAIT_MS = 2000U;
 constexpr int DC_ERR_WAIT = 398;
 
 enum { DC_QKV = 0, DC_OUT = 1, DC_UP = 2, DC_DOWN = 3, DC_LM = 4 };
@@ -83,14 +85,14 @@ struct dc_args {
     CUtensorMap kv[GDB_DECODE_MAX_LAYERS][2];         // keys, values; a head x 16 positions
     CUtensorMap kv_ahead[GDB_DECODE_MAX_LAYERS][2];   // the heads of an attention unit x 64 positions, for prefetches
     int mute, mute_step;      // for tests: consumer warps of CTA `mute` of every cluster give up at that step (mute < 0: none)
-    unsigned wait_us;         // a wait may take
+    unsigned wait_ms;         // a wait may take (of 2^20 ns)
 };
 
 // One CTA's side of the exchanges and of the ring.
 struct dc_ctx {
     uint32_t sm;                  // shared-memory address of the ring; everything else lies behind it
     uint32_t full, empty;         // addresses of the uses' barriers
-    volatile int *dead;           // [0] a wait of this CTA gave up, [1] microseconds before one does, [2] another CTA of the cluster gave up
+    volatile int *dead;           // [0] a wait of this CTA gave up, [1] time before one does, [2] another CTA of the cluster gave up
     int *err_flag;
     uint32_t rank, places, n, place;   // ring cursor: use and place of the next phase's first tile
     int tid, warp, lane;
@@ -190,15 +192,10 @@ __device__ __noinline__ float2 dc_cos_sin(const gdb_decode_args &a, unsigned pai
     cs.y *= a.rope.sin_sign;   // (the sign is 1 or -1: its place for the caller is behind the table's values, which have none)
     return cs;
 }
-__device__ __forceinline__ unsigned long long dc_now()
+__device__ __noinline__ void dc_stamp(const gdb_decode_args &a, int *stamp)
 {
     unsigned long long ns;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(ns));
-    return ns;
-}
-__device__ __noinline__ void dc_stamp(const gdb_decode_args &a, int *stamp)
-{
-    const unsigned long long ns = dc_now();
     if (*stamp < a.n_steps * (5 * a.L + 1)) a.timeline[(*stamp)++] = ns;
 }
 __device__ __forceinline__ bool dc_try_wait(uint32_t bar, uint32_t parity)
@@ -213,13 +210,20 @@ __device__ __forceinline__ bool dc_try_wait(uint32_t bar, uint32_t parity)
         : "memory");
     return done != 0U;
 }
+// The time in units of 2^20 ns (32 bits: a wait that keeps 64-bit times takes registers from the kernel, 0.4 us a step)
+__device__ __forceinline__ uint32_t dc_now_ms()
+{
+    uint32_t lo, hi;
+    asm volatile("{\n.reg .b64 t;\nmov.u64 t, %%globaltimer;\nmov.b64 {%0, %1}, t;\n}" : "=r"(lo), "=r"(hi));
+    return __funnelshift_r(lo, hi, 20);
+}
 __device__ __noinline__ bool dc_wait_more(uint32_t bar, uint32_t parity, volatile int *dead, int *err_flag)
 {
-    const unsigned long long since = dc_now(), limit = (unsigned long long)(unsigned)dead[1] * 1000ULL;
+    const uint32_t since = dc_now_ms();
     do {
         if (dc_try_wait(bar, parity)) return true;
         if (*dead != 0) return false;
-    } while (dc_now() - since < limit);
+    } while (dc_now_ms() - since < (uint32_t)dead[1]);
     *dead = 1;
     atomicCAS(err_flag, 0, DC_ERR_WAIT);
     return false;
@@ -228,8 +232,6 @@ __device__ __forceinline__ void dc_wait(dc_ctx &c, uint32_t bar, uint32_t parity
 {
     if (c.alive && !dc_try_wait(bar, parity)) c.alive = dc_wait_more(bar, parity, c.dead, c.err_flag);
 }
-// Behind a block barrier: what the others left in shared memory is complete if none of them had given up before it.
-__device__ __forceinline__ void dc_check(dc_ctx &c) { c.alive = c.alive && *c.dead == 0; }
 
 // First unit and number of units of this CTA in a phase of `n` units shared by the cluster.
 __device__ __forceinline__ void dc_share(uint32_t n, uint32_t rank, uint32_t ctas, uint32_t *first, uint32_t *count)
@@ -293,10 +295,9 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
         return s;
     };
 #pragma unroll 1
-    for (int step = 0; step < a.n_steps; ++step) {
+    for (int step = 0; step < a.n_steps && __all_sync(0xffffffffU, c.alive); ++step) {
 #pragma unroll 1
         for (int ph = 0; ph <= 4 * a.L; ++ph) {
-            if (!__all_sync(0xffffffffU, c.alive)) return;
             const int kind = ph == 4 * a.L ? (int)DC_LM : (ph & 3), layer = ph >> 2;
             if (kind == DC_OUT) {
                 // keys and values of this CTA's attention units: use (i, w) for the i-th 16 keys of warp w's (head, split)
@@ -473,7 +474,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
     }
     if (c.tid == 0) {
         dead[0] = dead[2] = 0;
-        dead[1] = (int)g.wait_us;
+        dead[1] = (int)g.wait_ms;
         for (int i = 0; i < DX_COUNT; ++i) gdb_t5::mbar_init(bar(i), i == DX_LM ? CS + 1U : 1U);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         gdb_t5::mbar_expect_tx(bar(DX_QKV), qkv_bytes);
@@ -654,8 +655,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                             }
                         }
                     }
-                    going = dc_sync_vote(c.alive);
-                    if (!going) break;
+                    dc_sync();
 
                     // ---- QKV, up / gate or LM head ----
                     const uint32_t acts = s_normed + brow * LDA + bcol;
@@ -704,7 +704,6 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                         if (!mine) continue;
                         if (!whole) {
                             asm volatile("bar.sync %0, 64;" ::"r"(DC_BAR_PAIR + u) : "memory");
-                            dc_check(c);
 #pragma unroll
                             for (int s = 0; s < 4; ++s)
 #pragma unroll
@@ -772,7 +771,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                                 const uint32_t dst = s_qkv + ((at * 3U + what) * (uint32_t)hpc + (head & ((uint32_t)hpc - 1U))) * 128U + (col & 63U) * 2U;
                                 if (c.alive) dc_send(mapa_shared(dst, to), val, mapa_shared(bar(DX_QKV), to));
                                 const int pos = positions[row] + step;
-                                if (c.alive && what != 0U && pos >= 0 && pos < a.CAP)
+                                if (what != 0U && pos >= 0 && pos < a.CAP)
                                     *reinterpret_cast<uint4 *>((T *)(what == 1U ? a.kc[j >> 1] : a.vc[j >> 1]) + ((size_t)(b0 + row) * a.CAP + (size_t)pos) * D + col) = val;
                             }
                             __syncwarp();
@@ -792,8 +791,8 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                                 }
                                 if (c.lane < 4) asm volatile("st.shared.b64 [%0], %1;" ::"r"(s_wkeys + (uint32_t)(c.warp * DC_MAX_ROWS + t * 8 + t2 + e) * 8U), "l"(best[t][e]) : "memory");
                             }
-                        dc_sync();
-                        dc_check(c);
+                        going = dc_sync_vote(c.alive);
+                        if (!going) break;
                         const uint32_t row = (uint32_t)c.tid & 15U, to = (uint32_t)c.tid >> 4;
                         if (to < CS) {
                             if ((int)row < rows) {
@@ -856,7 +855,6 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                         state.merge_groups(ml + item * 2, ml + DC_WARPS * 2 + item * 64, c.lane);
                     }
                     dc_sync();
-                    dc_check(c);
                     // Merge of the splits of all units at once (decode_combine_query), one thread per output: weights, sum and output over the
                     // splits in order. (Unit by unit, by the warps of that unit's outputs: 64 sequences 122 us per step.)
 #pragma unroll 1
@@ -948,7 +946,6 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                     // the ranges' sums through shared memory, then a thread per output; the new rows go to every CTA
                     dc_leave_range<NT>(acc[0], s_red + (uint32_t)c.warp * (NT * 512U) + (uint32_t)c.lane * 16U);
                     asm volatile("bar.sync %0, 256;" ::"r"(DC_BAR_SUM + (uint32_t)ou) : "memory");
-                    dc_check(c);
                     const uint32_t src = s_red + (uint32_t)ou * (NT * 4096U) + (NT == 2 ? (uint32_t)(oi >> 7) * 512U : 0U) + (uint32_t)((oi & 7) * 4 + ((oi >> 3) & 7) / 2) * 16U +
                                          (uint32_t)(ohalf * 2 + ((oi >> 3) & 1)) * 4U;
                     float v = 0.0f;
@@ -1112,7 +1109,7 @@ gd_status gdb_decode_cluster_launch(gd_backend *be, uint32_t dtype, const gdb_de
     g.a = *a;
     g.mute = be->decode_mute;
     g.mute_step = be->decode_mute_step;
-    g.wait_us = be->decode_mute >= 0 && be->decode_wait_us != 0U ? be->decode_wait_us : DC_WAIT_US;
+    g.wait_ms = be->decode_mute >= 0 && be->decode_wait_ms != 0U ? be->decode_wait_ms : DC_WAIT_MS;
     be->decode_mute = -1;
     dc_kernel kern = nullptr;
     auto prepare = [&](int rows) {   // kernel, layout and launch shape for `rows` sequences per cluster

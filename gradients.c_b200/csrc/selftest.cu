@@ -74,14 +74,14 @@ gd_status gdb200_selftest_bounded_wait(gd_backend *be, uint32_t max_iters)
     return gdb_launched(be, "selftest_bounded_wait");
 }
 
-gd_status gdb200_selftest_decode_give_up(gd_backend *be, int32_t cta, int32_t step, uint32_t max_wait_us)
+gd_status gdb200_selftest_decode_give_up(gd_backend *be, int32_t cta, int32_t step, uint32_t max_wait_ms)
 {
-    if (be == NULL || cta < 0 || cta > 15 || step < 0 || max_wait_us > 1000000U) {
+    if (be == NULL || cta < 0 || cta > 15 || step < 0 || max_wait_ms > 1000U) {
         return GD_ERR_INVALID_ARGUMENT;
     }
     be->decode_mute = cta;
     be->decode_mute_step = step;
-    be->decode_wait_us = max_wait_us;
+    be->decode_wait_ms = max_wait_ms;
     return GD_OK;
 }
 

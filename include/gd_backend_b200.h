@@ -657,11 +657,11 @@ gd_status gdb200_gpt_decode_steps(gd_backend *backend, const gdb200_gpt_spec *sp
  * gdb200_selftest_bounded_wait runs a one-warp kernel that polls an mbarrier nobody arrives at for at most max_iters
  * (<= 2^20) iterations, stores code 399 and returns; gdb200_selftest_decode_give_up has CTA `cta` (0 .. 15) of each cluster
  * fall silent at step `step` of the next run of decode steps that is one launch, and the waits of the others give up after
- * max_wait_us microseconds (<= 10^6; 0: the kernel's own limit of two seconds) with code 398. After any of them, gd_backend_flush returns GD_ERR_INTERNAL once,
+ * max_wait_ms milliseconds (<= 1000; 0: the kernel's own limit of two seconds) with code 398. After any of them, gd_backend_flush returns GD_ERR_INTERNAL once,
  * gdb200_last_error names the code, and the backend stays usable. */
 gd_status gdb200_inject_device_error(gd_backend *backend, int32_t code);
 gd_status gdb200_selftest_bounded_wait(gd_backend *backend, uint32_t max_iters);
-gd_status gdb200_selftest_decode_give_up(gd_backend *backend, int32_t cta, int32_t step, uint32_t max_wait_us);
+gd_status gdb200_selftest_decode_give_up(gd_backend *backend, int32_t cta, int32_t step, uint32_t max_wait_ms);
 
 /* Data-parallel gradient exchange (the reference has no collective; one process per GPU).
  * id_bytes is the 128-byte ncclUniqueId produced by gdb200_dp_unique_id on rank 0. */

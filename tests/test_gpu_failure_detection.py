@@ -97,7 +97,7 @@ def test_decode_that_gives_up_leaves_ids_and_positions_where_they_were(d_model, 
     with pkg.runtime.Context(params_bytes=256 << 20, state_bytes=256 << 20, scratch_bytes=1 << 30) as ctx:
         run = DecodeRun(ctx, d_model, mlp_hidden, batch, new=8)
         before = run.words()
-        assert ctx.lib.gdb200_selftest_decode_give_up(ctx.backend, cta, step, 50000) == abi.GD_OK
+        assert ctx.lib.gdb200_selftest_decode_give_up(ctx.backend, cta, step, 50) == abi.GD_OK
         assert run.decode() == abi.GD_ERR_INTERNAL and b"code 398" in ctx.lib.gdb200_last_error(ctx.backend)
         failed = run.words()
         assert np.array_equal(failed[0], before[0]) and np.array_equal(failed[1], before[1]) and failed[3] == before[3] == 1
