@@ -73,7 +73,7 @@ enum { DC_QKV = 0, DC_OUT = 1, DC_UP = 2, DC_DOWN = 3, DC_LM = 4 };
 enum { DX_QKV = 0, DX_ATTN = 1, DX_RESID = 2, DX_ACT = 3, DX_X = 4, DX_LM = 5, DX_COUNT = 6 };
 
 struct dc_layout {
-    uint32_t places;
+    uint32_t places, inverse;   // of the ring, and ceil(2^32 / places)
     uint32_t x, resid, normed, act, attn, scratch, qkv, red, staging, keys, total;   // byte offsets from the ring's start
 };
 
@@ -94,7 +94,7 @@ struct dc_ctx {
     uint32_t full, empty;         // addresses of the uses' barriers
     volatile int *dead;           // [0] a wait of this CTA gave up, [1] time before one does, [2] another CTA of the cluster gave up
     int *err_flag;
-    uint32_t rank, places, n, place;   // ring cursor: use and place of the next phase's first tile
+    uint32_t rank, places, inverse, n, place;   // ring cursor: use and place of the next phase's first tile
     int tid, warp, lane;
     bool alive;
 };
@@ -233,6 +233,11 @@ __device__ __forceinline__ void dc_wait(dc_ctx &c, uint32_t bar, uint32_t parity
     if (c.alive && !dc_try_wait(bar, parity)) c.alive = dc_wait_more(bar, parity, c.dead, c.err_flag);
 }
 
+// Place of what lies s places behind the ring's first one. (For s < 2^32 / places, and the keys and values of one phase are fewer. Where each
+// tile's place was reduced by subtracting from its phase's first one, a sequence's attention took time with the square of its keys:
+// 64 sequences of 4000, 680 us a step.)
+__device__ __forceinline__ uint32_t dc_wrap(const dc_ctx &c, uint32_t s) { return s - __umulhi(s, c.inverse) * c.places; }
+
 // First unit and number of units of this CTA in a phase of `n` units shared by the cluster.
 __device__ __forceinline__ void dc_share(uint32_t n, uint32_t rank, uint32_t ctas, uint32_t *first, uint32_t *count)
 {
@@ -289,11 +294,7 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
     auto claim = [&](uint32_t use) {   // its place is free
         if (use >= c.places) dc_wait(c, c.empty + ((use - c.places) % DC_BARS) * 8U, ((use - c.places) / DC_BARS) & 1U);
     };
-    auto wrap = [&](uint32_t s) {
-#pragma unroll 1
-        while (s >= c.places) s -= c.places;
-        return s;
-    };
+    auto wrap = [&](uint32_t s) { return dc_wrap(c, s); };
 #pragma unroll 1
     for (int step = 0; step < a.n_steps && __all_sync(0xffffffffU, c.alive); ++step) {
 #pragma unroll 1
@@ -448,6 +449,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
     c.err_flag = a.err_flag;
     c.rank = gdb_t5::cluster_ctarank();
     c.places = g.lay.places;
+    c.inverse = g.lay.inverse;
     c.n = 0U;
     c.place = 0U;
     c.tid = threadIdx.x;
@@ -514,10 +516,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
         const uint32_t hpc_log = 31U - (uint32_t)__clz(hpc), groups_log = 31U - (uint32_t)__clz(groups);   // (both divide the head count, a power of two)
 
         auto wait_use = [&](uint32_t i, uint32_t *empty_bar) {   // use i of this phase: its shared-memory address
-            uint32_t place = c.place + i;
-#pragma unroll 1
-            while (place >= c.places) place -= c.places;
-            const uint32_t n = c.n + i, which = (n % DC_BARS) * 8U;
+            const uint32_t place = dc_wrap(c, c.place + i), n = c.n + i, which = (n % DC_BARS) * 8U;
             *empty_bar = c.empty + which;
             dc_wait(c, c.full + which, (n / DC_BARS) & 1U);
             return c.sm + place * DC_PLACE;
@@ -525,9 +524,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
         auto wait_tile = [&](uint32_t i, uint32_t *empty_bar) { return wait_use(2U * i, empty_bar); };   // weight tile i of this phase
         auto advance = [&](uint32_t uses) {
             c.n += uses;
-            c.place += uses;
-#pragma unroll 1
-            while (c.place >= c.places) c.place -= c.places;
+            c.place = dc_wrap(c, c.place + uses);
         };
         // The id that sequence r is at: the best of the CTAs' classes. CTA 0 records it as the choice of step `step`.
         auto best_id = [&](int r, int step) {
@@ -1073,6 +1070,7 @@ bool dc_make_layout(dc_layout *l, uint32_t rows, uint32_t D, uint32_t F, uint32_
     l->keys = take(CS * DC_MAX_ROWS * 8U);
     if (top + DC_MIN_PLACES * DC_PLACE > limit) return false;
     l->places = std::min((limit - top) / DC_PLACE & ~1U, DC_MAX_PLACES);
+    l->inverse = 0xffffffffU / l->places + 1U;
     const uint32_t ring = l->places * DC_PLACE;
     for (uint32_t *o : {&l->x, &l->resid, &l->normed, &l->act, &l->attn, &l->scratch, &l->qkv, &l->red, &l->staging, &l->keys}) *o += ring;
     l->total = top + ring;
