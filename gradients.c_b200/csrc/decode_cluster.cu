@@ -83,7 +83,6 @@ struct dc_args {
     int rows;                 // sequences per cluster
     CUtensorMap lm, w[GDB_DECODE_MAX_LAYERS][4];
     CUtensorMap kv[GDB_DECODE_MAX_LAYERS][2];         // keys, values; a head x 16 positions
-    CUtensorMap kv_ahead[GDB_DECODE_MAX_LAYERS][2];   // the heads of an attention unit x 64 positions, for prefetches
     int mute, mute_step;      // for tests: consumer warps of CTA `mute` of every cluster give up at that step (mute < 0: none)
     unsigned wait_ms;         // a wait may take (of 2^20 ns)
 };
@@ -332,17 +331,6 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
                     }
                     n += (uint32_t)(kr.iters * DC_WARPS);
                     place = wrap(place + (uint32_t)(kr.iters * DC_WARPS));
-                    // The next attention's keys and values on their way from DRAM to L2 while the phases in between leave DRAM idle (64
-                    // sequences, 256 + 256 tokens: all clusters fetch them in the same phases, 38 MB a layer)
-                    if (kr.span >= 64 && c.lane == 0) {
-                        const int ahead = layer + 1 == a.L ? 0 : layer + 1;
-#pragma unroll 1
-                        for (int i = (int)which; i < (kr.span + 63) / 64; i += DC_PRODUCERS) {
-                            gdb_t5::tma_prefetch_3d(&g.kv_ahead[ahead][0], h0 * 64, kr.lo + i * 64, b0 + row);
-                            gdb_t5::tma_prefetch_3d(&g.kv_ahead[ahead][1], h0 * 64, kr.lo + i * 64, b0 + row);
-                        }
-                    }
-                    __syncwarp();
                 }
             }
             const CUtensorMap *map = kind == DC_LM ? &g.lm : &g.w[layer][kind];
@@ -1022,19 +1010,6 @@ bool dc_map_down(CUtensorMap *m, uint32_t dtype, const void *base, uint64_t F, u
               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// A cache [batch, positions, D] in boxes of `cols` columns x 64 positions (at most 256 columns: the rest is fetched when it is read).
-bool dc_map_ahead(CUtensorMap *m, uint32_t dtype, const void *base, uint64_t batch, uint64_t positions, uint32_t D, uint32_t cols)
-{
-    gdb_t5::encode_tiled_fn fn = gdb_t5::get_encode_fn();
-    if (fn == nullptr) return false;
-    const cuuint64_t dims[3] = {D, positions, batch};
-    const cuuint64_t strides[2] = {D * 2U, positions * D * 2U};
-    const cuuint32_t box[3] = {std::min(cols, 256U), 64, 1}, estr[3] = {1, 1, 1};
-    const CUtensorMapDataType dt = dtype == GDB_DTYPE_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    return fn(m, dt, 3, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 typedef void (*dc_kernel)(const dc_args);
 template <typename T>
 dc_kernel dc_pick(uint32_t D, int tiles)
@@ -1140,7 +1115,6 @@ gd_status gdb_decode_cluster_launch(gd_backend *be, uint32_t dtype, const gdb_de
     for (int i = 0; i < a->L && mapped; ++i) {
         mapped = dc_map_rows(&g.w[i][DC_QKV], dtype, a->lw[i][1], 32U, 32U, 3U * D / 32U, D) && dc_map_rows(&g.w[i][DC_OUT], dtype, a->lw[i][3], 8U, 8U, D / 8U, D) &&
                  dc_map_rows(&g.w[i][DC_UP], dtype, a->lw[i][6], F, F, 2U, D) && dc_map_down(&g.w[i][DC_DOWN], dtype, a->lw[i][8], F, D);
-        for (int j = 0; j < 2 && mapped; ++j) mapped = dc_map_ahead(&g.kv_ahead[i][j], dtype, j == 0 ? a->kc[i] : a->vc[i], (uint64_t)a->B, cap, D, 64U * (16U / (uint32_t)a->splits));
         for (int j = 0; j < 2 && mapped; ++j)
             mapped = gdb_t5::make_tmap_batched(&g.kv[i][j], dtype, j == 0 ? a->kc[i] : a->vc[i], (uint64_t)a->B, cap, D, D * 2U, cap * D * 2U, 64U, 16U);
     }
