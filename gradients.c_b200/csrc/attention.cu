@@ -527,7 +527,7 @@ gd_status decode_common(gd_backend *be, const gd_backend_tensor_view *q, const g
             const char *env = getenv("GDB200_DECODE_WARPS_PER_SM");
             wps = env != NULL && atoi(env) > 0 ? atoi(env) : 32;
         }
-        const int splits = gdb_dec::decode_choose_splits(be->sm_count, p.batch, p.tq, p.hq, p.dh, p.tmax, wps);
+        const int splits = gdb_dec::decode_choose_splits(be->sm_count, p, wps);
         const size_t need = (size_t)total * splits * (2U + (size_t)p.dh) * sizeof(float);
         if (need <= be->ws_bytes) {
             float *ml = (float *)be->ws;

@@ -248,32 +248,52 @@ __device__ __forceinline__ bool decode_allowed(int qpos, int j, int window, int 
     return mask_allowed(qpos, j, 1, window, prefix);
 }
 
-// Number of key splits per query. One new token per sequence, head_dim 64 and at most 64 sequences (the shapes the kernel of all
-// steps takes): the 16 warps of a CTA are `heads_per_cta` heads x `splits` key ranges of ONE sequence, merged through shared memory;
-// heads_per_cta is the smallest power of two (dividing hq, at most 16) that leaves at most DECODE_UNITS units, one for every CTA of the
-// seven clusters of 16 that a B200 holds, else the largest: a second unit per CTA costs its latency in every layer (us per step, units
-// within 112 / within twice the SMs: 20 sequences 42.9 / 49.4, 32 52.9 / 59.9, 64 of 20-84 tokens 71 / 81, 64 of 256-512 123.2 / 122.7).
-// Other shapes: as many splits as keep `warps_per_sm` warps per SM busy, at least 32 keys of the cache per split, at most 16.
-constexpr int DECODE_UNITS = 112;
-static inline int decode_heads_per_cta(int batch, int hq)
+// Number of key splits per query, the same in every form of a decode step (the same partition gives the same bits).
+//
+// Shapes of the kernel of all steps (decode_cluster.cu): 16 warps of a CTA are `heads` heads x 16 / heads key ranges of ONE sequence, and a
+// cluster of 2 hq CTAs deals the hq / heads units of each of its sequences one to a CTA, in rounds. A round costs as much as some 256
+// keys of a head beside its own keys, so rounds x (256 + heads x keys) is made smallest; the finer partition where two are equal.
+// The keys are three quarters of what a query may see: a cache that is filled to half at first. us per step of the benchmark model (8
+// heads) with 2 / 4 / 8 / 16 ranges: 64 sequences of 120 keys 78 / 81 / 80 / 82, 250 99 / 100 / 95 / 99, 500 130 / 133 / 121 / 120, 1000
+// 187 / 190 / 165 / 158; 32 of 250 67 / 54 / 57 / 58, 1000 131 / 88 / 92 / 83; 4 heads, 64 of 250 - / 51 / 54 / 55, 4000 - / 208 / 217 /
+// 182; 2 heads, 64 of 250 - / - / 45 / 43. (For as many units as the seven clusters of 16 have CTAs, whatever the keys: 2, 4 and 8 ranges
+// for 64 sequences of 8, 4 and 2 heads.)
+static inline int decode_cluster_splits(int batch, int hq, int keys)
 {
-    int largest = 0, chosen = 0;
-    for (int hg = 16; hg >= 1; hg >>= 1) {
-        if (hg > hq || (hq % hg) != 0) continue;
-        if (largest == 0) largest = hg;
-        if ((long long)batch * (hq / hg) > DECODE_UNITS) break;
-        chosen = hg;
+    const int clusters = hq == 8 ? 7 : (hq == 4 ? 15 : 33);   // of 16, 8 and 4 CTAs that a B200 holds at once
+    const int rows = (batch + clusters - 1) / clusters;
+    long long least = 0;
+    int chosen = hq;
+    for (int heads = hq; heads >= 1; heads >>= 1) {
+        const long long rounds = (rows * (hq / heads) + 2 * hq - 1) / (2 * hq), cost = rounds * (1024 + 3LL * heads * keys);
+        if (heads == hq || cost <= least) {
+            least = cost;
+            chosen = heads;
+        }
     }
-    return chosen != 0 ? chosen : largest;
+    return 16 / chosen;
 }
-static inline int decode_choose_splits(int sm_count, int batch, int tq, int hq, int dh, int tmax, int warps_per_sm)
+// Other shapes of one new token, head_dim 64 and at most 64 sequences: heads x ranges likewise, `heads` the smallest power of two (dividing
+// hq, at most 16) that leaves at most a unit per SM, else the largest. The rest: as many splits as keep `warps_per_sm` warps per SM
+// busy, at least 32 keys of the cache per split, at most 16.
+static inline int decode_choose_splits(int sm_count, const decode_params &p, int warps_per_sm)
 {
-    if (tq == 1 && dh == 64 && batch <= 64) {
-        return 16 / decode_heads_per_cta(batch, hq);
+    if (p.tq == 1 && p.dh == 64 && p.batch <= 64) {
+        if (p.hq == p.hkv && p.prefix <= 0 && (p.hq == 2 || p.hq == 4 || p.hq == 8)) {
+            return decode_cluster_splits(p.batch, p.hq, p.window > 0 && p.window < p.tmax ? p.window : p.tmax);
+        }
+        int largest = 0, chosen = 0;
+        for (int heads = 16; heads >= 1; heads >>= 1) {
+            if (heads > p.hq || (p.hq % heads) != 0) continue;
+            if (largest == 0) largest = heads;
+            if ((long long)p.batch * (p.hq / heads) > sm_count) break;
+            chosen = heads;
+        }
+        return 16 / (chosen != 0 ? chosen : largest);
     }
-    const long long total_queries = (long long)batch * tq * hq;
+    const long long total_queries = (long long)p.batch * p.tq * p.hq;
     int splits = (int)(((long long)sm_count * warps_per_sm) / total_queries);
-    const int max_splits = (tmax + 31) / 32;
+    const int max_splits = (p.tmax + 31) / 32;
     if (splits > max_splits) splits = max_splits;
     if (splits < 1) splits = 1;
     if (splits > 16) splits = 16;

@@ -1260,7 +1260,14 @@ gd_status decode_steps_persistent(gd_backend *be, const gdb200_gpt_spec *s, cons
     a.CAP = (int)CAP;
     a.window = s->sdpa_window;
     // the key splits the stand-alone attention entry uses for this shape (the same partition gives the same bits)
-    a.splits = gdb_dec::decode_choose_splits(be->sm_count, (int)B, 1, (int)H, (int)Dh, (int)CAP, 32);
+    gdb_dec::decode_params dp = {};
+    dp.batch = (int)B;
+    dp.tq = 1;
+    dp.tmax = (int)CAP;
+    dp.hq = dp.hkv = (int)H;
+    dp.dh = (int)Dh;
+    dp.window = s->sdpa_window;
+    a.splits = gdb_dec::decode_choose_splits(be->sm_count, dp, 32);
     a.max_steps = d->max_steps;
     a.n_steps = n_steps;
     a.eps = s->rms_eps;
