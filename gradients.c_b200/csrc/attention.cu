@@ -246,25 +246,40 @@ using gdb_dec::decode_params;
 using gdb_dec::decode_allowed;
 using gdb_dec::decode_combine_query;
 
+// How the stand-alone kernel reads its keys. One new token per sequence (and no prefix), head_dim 64: through tiles in shared memory, with
+// the arithmetic of the kernel of all steps, three tiles to a warp and several splits where they are many (decode_splits_per_warp).
+// Otherwise in registers, at 108 of them a thread (four blocks to an SM), or at 80 (six) where that saves a wave. Everything else as
+// it is, us with keys in registers / in tiles: 64 sequences x 8 heads x 4000 keys 108 / 94, 1 x 64 (8) x 4000 28 / 22, 64 x 32 (8) x 500 39 /
+// 32, 128 x 16 x 2000 171 / 180; 200 x 8 (2) x 2000 with 108 / 80 registers 130 / 97; several tokens, registers at 108 / tiles: 32 x 16
+// tokens x 8 x 900 115 / 139, 8 x 2 tokens x 8 (2) x 2000 22 / 26. (With two tiles to a warp and one split, 64 x 8 x 4000 took 105.)
+enum { DECODE_REGS = 0, DECODE_TIGHT = 1, DECODE_TILES = 2 };
+int decode_register_form(int sm_count, long long blocks)
+{
+    const long long four = 4LL * sm_count, six = 6LL * sm_count;
+    return (blocks + six - 1) / six < (blocks + four - 1) / four ? DECODE_TIGHT : DECODE_REGS;
+}
+
 // Split-K decode: grid (ceil(queries / warps), splits). Each warp owns one (b, t, hq) query and the keys
 // [split*chunk, split*chunk+chunk) of its live range (gdb_dec::decode_split_item); partial (m, l, acc) per split
 // go to the workspace and are merged by decode_combine_query.
 // `tickets` != NULL: the block that arrives last for its group of queries (over the splits) merges the
 // partials and writes `out`, so no combine launch follows.
-template <typename T, int DH>
-__global__ void decode_split_kernel(const T *q, const T *kc, const T *vc, const int *pos_buf, float *part_ml,
-                                    float *part_acc, decode_params p, int splits, T *out, unsigned *tickets)
+template <typename T, int DH, int FORM>
+__global__ void __launch_bounds__(128, FORM == DECODE_REGS ? 4 : (FORM == DECODE_TIGHT ? 6 : 1))
+decode_split_kernel(const T *q, const T *kc, const T *vc, const int *pos_buf, float *part_ml, float *part_acc, decode_params p, int splits, int count, T *out,
+                    unsigned *tickets)
 {
     gdb_pdl_sync();
-    __shared__ __align__(128) unsigned char tiles[DH == 64 ? 4 : 1][gdb_dec::DECODE_TILES_BYTES];   // (DH 128 keeps its keys in registers)
+    constexpr bool TILES = FORM == DECODE_TILES;
+    extern __shared__ __align__(128) unsigned char decode_tiles[];   // TILES: DECODE_TILES_BYTES of each warp
     const int lane = threadIdx.x & 31;
     const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const long long total = (long long)p.batch * p.tq * p.hq;
     const bool active = w < total;
     if (active) {
-        const size_t item = (size_t)w * splits + blockIdx.y;
-        gdb_dec::decode_split_item<T, DH>(q, kc, vc, pos_buf, part_ml + item * 2U, part_acc + item * DH, p, splits, w, (int)blockIdx.y, lane,
-                                          tiles[DH == 64 ? threadIdx.x >> 5 : 0]);
+        const size_t item = (size_t)w * splits + blockIdx.y * count;
+        gdb_dec::decode_split_item<T, DH, TILES>(q, kc, vc, pos_buf, part_ml + item * 2U, part_acc + item * DH, p, splits, w, (int)blockIdx.y * count, count, lane,
+                                                    decode_tiles + (TILES ? threadIdx.x >> 5 : 0) * gdb_dec::DECODE_TILES_BYTES);
     }   // active
     if (tickets == nullptr) {
         return;
@@ -532,14 +547,29 @@ gd_status decode_common(gd_backend *be, const gd_backend_tensor_view *q, const g
         if (need <= be->ws_bytes) {
             float *ml = (float *)be->ws;
             float *pa = ml + (size_t)total * splits * 2U;
-            dim3 grid((unsigned)((total + 3) / 4), (unsigned)splits);
+            const int form = p.dh == 64 && p.tq == 1 && p.prefix <= 0 ? DECODE_TILES : decode_register_form(be->sm_count, (total + 3) / 4 * splits);
+            const int count = form == DECODE_TILES ? gdb_dec::decode_splits_per_warp(be->sm_count, p, splits) : 1;
+            const size_t smem = form == DECODE_TILES ? 4U * gdb_dec::DECODE_TILES_BYTES : 0U;
+            dim3 grid((unsigned)((total + 3) / 4), (unsigned)(splits / count));
             const bool fused = grid.x <= (unsigned)GDB_TICKET_WORDS;
-#define GDB_DECODE(T, DH) gdb_launch(decode_split_kernel<T, DH>, grid, 128, 0, be->stream, (const T *)qp, (const T *)kp, (const T *)vp, pp, ml, pa, p, splits, (T *)op, fused ? gdb_tickets(be) : (unsigned *)nullptr)
-            if (dt == GDB_DTYPE_F16) {
-                if (p.dh == 64) GDB_DECODE(__half, 64); else GDB_DECODE(__half, 128);
-            } else {
-                if (p.dh == 64) GDB_DECODE(__nv_bfloat16, 64); else GDB_DECODE(__nv_bfloat16, 128);
+            static bool tiles_allowed = false;   // more shared memory than a kernel has without asking
+            if (form == DECODE_TILES && !tiles_allowed) {
+                cudaError_t e = cudaFuncSetAttribute(decode_split_kernel<__half, 64, DECODE_TILES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                if (e == cudaSuccess) e = cudaFuncSetAttribute(decode_split_kernel<__nv_bfloat16, 64, DECODE_TILES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                if (e != cudaSuccess) return gdb_fail(be, e, "sdpa_decode: shared memory");
+                tiles_allowed = true;
             }
+#define GDB_DECODE(T, DH, FORM) gdb_launch(decode_split_kernel<T, DH, FORM>, grid, 128, smem, be->stream, (const T *)qp, (const T *)kp, (const T *)vp, pp, ml, pa, p, splits, count, (T *)op, fused ? gdb_tickets(be) : (unsigned *)nullptr)
+#define GDB_DECODE_FORMS(T) \
+    do { \
+        if (p.dh == 128) GDB_DECODE(T, 128, DECODE_REGS); \
+        else if (form == DECODE_TILES) GDB_DECODE(T, 64, DECODE_TILES); \
+        else if (form == DECODE_TIGHT) GDB_DECODE(T, 64, DECODE_TIGHT); \
+        else GDB_DECODE(T, 64, DECODE_REGS); \
+    } while (0)
+            if (dt == GDB_DTYPE_F16) GDB_DECODE_FORMS(__half);
+            else GDB_DECODE_FORMS(__nv_bfloat16);
+#undef GDB_DECODE_FORMS
 #undef GDB_DECODE
             gd_status st = gdb_launched(be, "sdpa_decode split");
             if (st != GD_OK || fused) return st;

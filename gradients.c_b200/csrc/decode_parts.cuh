@@ -276,10 +276,22 @@ static inline int decode_cluster_splits(int batch, int hq, int keys)
 // Other shapes of one new token, head_dim 64 and at most 64 sequences: heads x ranges likewise, `heads` the smallest power of two (dividing
 // hq, at most 16) that leaves at most a unit per SM, else the largest. The rest: as many splits as keep `warps_per_sm` warps per SM
 // busy, at least 32 keys of the cache per split, at most 16.
+static inline bool decode_cluster_shape(const decode_params &p)
+{
+    return p.tq == 1 && p.dh == 64 && p.batch <= 64 && p.hq == p.hkv && p.prefix <= 0 && (p.hq == 2 || p.hq == 4 || p.hq == 8);
+}
+// Splits of a query that one warp of the stand-alone kernel takes one after the other, so that its pipeline starts once: as many as leave six
+// warps per SM. (One each: 32 sequences x 8 heads of 1000 keys 27 us instead of 23, 64 of 400 21.4 instead of 18.4.)
+static inline int decode_splits_per_warp(int sm_count, const decode_params &p, int splits)
+{
+    int count = 1;
+    while (count < splits && (long long)p.batch * p.tq * p.hq * (splits / (2 * count)) >= 6LL * sm_count) count *= 2;
+    return count;
+}
 static inline int decode_choose_splits(int sm_count, const decode_params &p, int warps_per_sm)
 {
     if (p.tq == 1 && p.dh == 64 && p.batch <= 64) {
-        if (p.hq == p.hkv && p.prefix <= 0 && (p.hq == 2 || p.hq == 4 || p.hq == 8)) {
+        if (decode_cluster_shape(p)) {
             return decode_cluster_splits(p.batch, p.hq, p.window > 0 && p.window < p.tmax ? p.window : p.tmax);
         }
         int largest = 0, chosen = 0;
@@ -340,21 +352,22 @@ struct decode_fold {
 #pragma unroll
         for (int c = 0; c < 16; ++c) acc[c] = 0.0f;
     }
-    // Both scores, ONE running-max update, both keys folded into (l, acc). No branches: a key that is not valid counts with
-    // probability 0 and value 0.
+    // Both scores, ONE running-max update, both keys folded into (l, acc).
     __device__ __forceinline__ void fold2(const bool (&valid)[2], const uint4 (&k0)[2], const uint4 (&k1)[2], const uint4 (&v0)[2], const uint4 (&v1)[2])
     {
         float s[2];
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-            float ka[8], kb[8];
-            unpack8<T>(k0[u], ka);
-            unpack8<T>(k1[u], kb);
             s[u] = 0.0f;
+            if (valid[u]) {
+                float ka[8], kb[8];
+                unpack8<T>(k0[u], ka);
+                unpack8<T>(k1[u], kb);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) s[u] = fmaf(qr[e], ka[e], s[u]);
+                for (int e = 0; e < 8; ++e) s[u] = fmaf(qr[e], ka[e], s[u]);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) s[u] = fmaf(qr[8 + e], kb[e], s[u]);
+                for (int e = 0; e < 8; ++e) s[u] = fmaf(qr[8 + e], kb[e], s[u]);
+            }
         }
 #pragma unroll
         for (int o = 1; o < LPK; o <<= 1) {
@@ -362,20 +375,35 @@ struct decode_fold {
             s[1] += __shfl_xor_sync(0xffffffffU, s[1], o);
         }
         const float s0 = valid[0] ? s[0] : -INFINITY, s1 = valid[1] ? s[1] : -INFINITY;
-        const float mnew = fmaxf(m, fmaxf(s0, s1)), base = mnew == -INFINITY ? 0.0f : mnew;
-        const float corr = __expf(m - base), e0 = __expf(s0 - base), e1 = __expf(s1 - base);   // exp(-inf) = 0
-        l = l * corr + e0 + e1;
-        m = mnew;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
+        const float mnew = fmaxf(m, fmaxf(s0, s1));
+        if (mnew != -INFINITY) {
+            const float corr = __expf(m - mnew), e0 = __expf(s0 - mnew), e1 = __expf(s1 - mnew);   // exp(-inf) = 0
+            l = l * corr + e0 + e1;
             float va[8], vb[8];
-            unpack8<T>(only(half == 0 ? v0[0] : v1[0], valid[0]), va);
-            unpack8<T>(only(half == 0 ? v0[1] : v1[1], valid[1]), vb);
+            if (valid[0]) {
+                unpack8<T>(v0[0], va);
+                unpack8<T>(v1[0], vb);
 #pragma unroll
-            for (int c = 0; c < 8; ++c) acc[half * 8 + c] = fmaf(e1, vb[c], fmaf(e0, va[c], acc[half * 8 + c] * corr));
+                for (int c = 0; c < 8; ++c) {
+                    acc[c] = fmaf(e0, va[c], acc[c] * corr);
+                    acc[8 + c] = fmaf(e0, vb[c], acc[8 + c] * corr);
+                }
+            } else {
+#pragma unroll
+                for (int c = 0; c < 16; ++c) acc[c] *= corr;
+            }
+            if (valid[1]) {
+                unpack8<T>(v0[1], va);
+                unpack8<T>(v1[1], vb);
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    acc[c] = fmaf(e1, va[c], acc[c]);
+                    acc[8 + c] = fmaf(e1, vb[c], acc[8 + c]);
+                }
+            }
+            m = mnew;
         }
     }
-    static __device__ __forceinline__ uint4 only(const uint4 &v, bool valid) { return make_uint4(valid ? v.x : 0U, valid ? v.y : 0U, valid ? v.z : 0U, valid ? v.w : 0U); }
     template <int N>
     static __device__ __forceinline__ int give_half(float (&a)[16], int lane, int o)
     {
@@ -493,12 +521,14 @@ struct decode_fold64 {
     }
 };
 
-// One warp: query w = (b, t, hq) against the keys of split `split` of its live range; the partial goes to ml_item and acc_item
-// (8-byte aligned). DH 64: `tiles` is shared memory of this warp, DECODE_TILES_BYTES, 128-byte aligned.
-constexpr int DECODE_TILES_BYTES = 2 * 4096;   // two tiles of 16 keys and values, one on its way while the other is folded
-template <typename T, int DH>
+// One warp: query w = (b, t, hq) against the keys of splits split .. split + count - 1 of its live range; the partials go to ml_item and
+// acc_item (8-byte aligned), one behind the other. TILES (head_dim 64 only): keys through `tiles`, shared memory of this warp,
+// DECODE_TILES_BYTES, 128-byte aligned, and scores as the kernel of all steps forms them; otherwise keys in registers, FP32 scores and
+// one split.
+constexpr int DECODE_SLOTS = 3, DECODE_TILES_BYTES = DECODE_SLOTS * 4096;   // tiles of 16 keys and values: one is folded, the others are on their way
+template <typename T, int DH, bool TILES>
 __device__ __forceinline__ void decode_split_item(const T *q, const T *kc, const T *vc, const int *pos_buf, float *ml_item, float *acc_item,
-                                                  const decode_params &p, int splits, long long w, int split, int lane, unsigned char *tiles)
+                                                  const decode_params &p, int splits, long long w, int split, int count, int lane, unsigned char *tiles)
 {
     const int h = (int)(w % p.hq);
     const int t = (int)((w / p.hq) % p.tq);
@@ -515,60 +545,77 @@ __device__ __forceinline__ void decode_split_item(const T *q, const T *kc, const
     if (p.window > 0 && p.prefix <= 0 && qpos - p.window + 1 > 0) j_lo = qpos - p.window + 1;
     const int span = pos >= 0 && j_hi > j_lo ? j_hi - j_lo : 0;
     const int chunk = (span + splits - 1) / splits;
-    const int s_lo = j_lo + split * chunk;
-    int s_hi = s_lo + chunk;
-    if (s_hi > j_hi) s_hi = j_hi;
-    if (span == 0) s_hi = s_lo;
+    const int end = j_lo + span;
     const T *qh = q + (((size_t)b * p.tq + t) * p.hq + h) * DH;
     const size_t head = ((size_t)b * p.tmax * p.hkv + hk) * DH, pitch = (size_t)p.hkv * DH;   // key j at head + j * pitch
-    auto key_valid = [&](int j) { return j < s_hi && decode_allowed(qpos, j, p.window, p.prefix); };
-    if constexpr (DH == 64) {
+    if constexpr (TILES) {
+        static_assert(DH == 64, "tiles are laid out for head_dim 64");
         decode_fold64<T> state;
         state.init(lane, [&](int i, int hh) {
             const unsigned short *e = reinterpret_cast<const unsigned short *>(qh) + i * 16 + hh * 8 + lane * 2;
             return (uint32_t)e[0] | ((uint32_t)e[1] << 16);
         });
         const int piece = lane & 7, krow = lane >> 3;   // copy: lane -> (key within a group of 4, 16-byte piece)
-        auto issue = [&](int jb, int slot) {
-            if (jb < s_hi) {
+        auto split_end = [&](int s) { return min(j_lo + (s + 1) * chunk, end); };
+        // The tiles of all splits in one sequence, so that a split's first ones are on their way while the one before is folded.
+        int next_split = split, next = j_lo + split * chunk;
+        auto issue = [&](int slot) {
+            while (next >= split_end(next_split) && next_split + 1 < split + count) {
+                ++next_split;
+                next = j_lo + next_split * chunk;
+            }
+            const int stop = split_end(next_split);
+            if (next < stop) {
                 unsigned char *base = tiles + slot * 4096;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const int kl = i * 4 + krow, j = jb + kl;
-                    const bool ok = key_valid(j);
-                    const size_t src = head + (size_t)(ok ? j : s_lo) * pitch + (size_t)piece * 8U;
+                    const int kl = i * 4 + krow, j = next + kl;
+                    const bool ok = j < stop;
+                    const size_t src = head + (size_t)(ok ? j : next) * pitch + (size_t)piece * 8U;
                     unsigned char *dst = base + kl * 128 + ((piece ^ (kl & 7)) << 4);
                     sk_cp16(dst, kc + src, ok);
                     sk_cp16(dst + 2048, vc + src, ok);
                 }
+                next += 16;
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
-        issue(s_lo, 0);
+#pragma unroll
+        for (int i = 0; i < DECODE_SLOTS - 1; ++i) issue(i);
         int slot = 0;
 #pragma unroll 1
-        for (int jb = s_lo; jb < s_hi; jb += 16) {
-            issue(jb + 16, slot ^ 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-            __syncwarp();   // every lane's copies of this tile have landed
-            const uint32_t tile = sk_smem(tiles + slot * 4096);
-            state.fold(tile, tile + 2048U, key_valid(jb + (lane >> 2)), key_valid(jb + 8 + (lane >> 2)), p.scale, lane);
-            __syncwarp();   // every lane is done with the slot before it is refilled
-            slot ^= 1;
+        for (int s = split; s < split + count; ++s) {
+            const int stop = split_end(s);
+#pragma unroll 1
+            for (int jb = j_lo + s * chunk; jb < stop; jb += 16) {
+                issue(slot == 0 ? DECODE_SLOTS - 1 : slot - 1);
+                asm volatile("cp.async.wait_group %0;" ::"n"(DECODE_SLOTS - 1) : "memory");
+                __syncwarp();   // every lane's copies of this tile have landed
+                const uint32_t tile = sk_smem(tiles + slot * 4096);
+                state.fold(tile, tile + 2048U, jb + (lane >> 2) < stop, jb + 8 + (lane >> 2) < stop, p.scale, lane);
+                __syncwarp();   // every lane is done with the slot before it is refilled
+                slot = slot == DECODE_SLOTS - 1 ? 0 : slot + 1;
+            }
+            state.merge_groups(ml_item + (s - split) * 2, acc_item + (size_t)(s - split) * DH, lane);
+            state.s.init();
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
-        state.merge_groups(ml_item, acc_item, lane);
     } else {
         typedef decode_fold<T, DH> fold;
         constexpr int LPK = fold::LPK, KPW = fold::KPW, TILE = fold::TILE;
-        const int sub = lane % LPK, kg = lane / LPK;
+        const int sub = lane % LPK, kg = lane / LPK, s_lo = j_lo + split * chunk, s_hi = min(s_lo + chunk, end);
+        auto key_valid = [&](int j) { return j < s_hi && decode_allowed(qpos, j, p.window, p.prefix); };
         fold state;
         state.init();
 #pragma unroll
         for (int c = 0; c < 16; ++c) state.qr[c] = gdb_io<T>::ld(qh, (size_t)(sub * 16 + c)) * p.scale;
 #pragma unroll 1
         for (int jb = s_lo; jb < s_hi; jb += TILE) {
-            uint4 k0[2] = {}, k1[2] = {}, v0[2] = {}, v1[2] = {};
+            if (DH == 64) {   // the tile after this one on its way to L2: a line of K or V per lane
+                const int j = jb + TILE + (lane & 15);
+                if (j < s_hi) asm volatile("prefetch.global.L2 [%0];" ::"l"((lane < 16 ? kc : vc) + head + (size_t)j * pitch));
+            }
+            uint4 k0[2], k1[2], v0[2], v1[2];
             bool valid[2];
 #pragma unroll
             for (int u = 0; u < 2; ++u) {

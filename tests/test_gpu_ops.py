@@ -387,10 +387,12 @@ def test_sdpa_varlen_forward_backward(step, dtype, lengths, hq, hkv, dh, window,
 
 # the keys of a warp are multiplied 16 at a time: ranges that end on, before and behind a tile's edge, caches that hold NaN wherever no live key lies
 @pytest.mark.parametrize("dtype", [F16, BF16])
-@pytest.mark.parametrize("tq,hq,hkv,window,prefix", [(1, 8, 8, 0, 0), (1, 4, 2, 20, 0), (2, 4, 4, 0, 0), (1, 2, 2, 9, 24)])
-def test_decode_attention_reads_live_keys_only(step, dtype, tq, hq, hkv, window, prefix):
+@pytest.mark.parametrize("tq,hq,hkv,window,prefix,copies", [(1, 8, 8, 0, 0, 1), (1, 4, 2, 20, 0, 1), (2, 4, 4, 0, 0, 1), (1, 2, 2, 9, 24, 1), (1, 2, 2, 9, 0, 1),
+                                                            (1, 8, 8, 300, 0, 4),         # several key ranges to a warp, some without keys
+                                                            (1, 4, 4, 0, 0, 4), (4, 16, 16, 0, 0, 4)])
+def test_decode_attention_reads_live_keys_only(step, dtype, tq, hq, hkv, window, prefix, copies):
     ctx, sd = step, storage_name(dtype)
-    pos = np.array([0, 1, 14, 15, 16, 17, 30, 31, 32, 33, 255, 256, 257, 511, 509 - tq], dtype=np.int32)
+    pos = np.array([0, 1, 14, 15, 16, 17, 30, 31, 32, 33, 255, 256, 257, 511, 509 - tq] * copies, dtype=np.int32)
     b, tmax, dh = len(pos), 512 + tq - 1, 64
     kc, vc, q = (rnd_np(rng(50 + i).standard_normal(shape).astype(np.float32), dtype) for i, shape in enumerate(((b, tmax, hkv, dh), (b, tmax, hkv, dh), (b, tq, hq, dh))))
     dirty = [c.copy() for c in (kc, vc)]
