@@ -51,10 +51,14 @@ constexpr uint32_t DC_PLACE = 4096U, DC_TILE = 2U * DC_PLACE;
 constexpr uint32_t DC_MAX_PLACES = 48U, DC_MIN_PLACES = 16U;
 // Use n of a place has barriers n % 256 of its own (full: its bytes have landed; empty: its readers are done), not the place's: a warp
 // may wait for a tile whose place is still to be used once or twice before, and a parity cannot tell those phases apart. A barrier's use
-// before, n - 256, is over by then: the warps lie at most 88 places apart (a block barrier ends every 16 units of two tiles and every
-// four tiles per warp of the attention, whose warps may start while others have their part of the 12 QKV tiles to do; an exchange that
-// needs all warps ends the other phases), and at most 48 more are in flight.
-constexpr uint32_t DC_BARS = 256U;
+// before, n - 256, is over by then. Outside the down projection because the warps lie at most 160 places apart (a block barrier ends every 16
+// units of two tiles, 64 places, and every four tiles per warp of the attention, whose warps may start while others have their part of
+// the 12 QKV tiles to do; an exchange that needs all warps ends the other phases, and a pass of DC_PASS_COLS gate columns, 96 places, is
+// followed by the first 64 of the next one), and at most 48 more are in flight. Within the down projection, where nothing holds the
+// warps together and F / 64 places may lie between them, because tiles 128 apart have the same readers (those of one k range in four,
+// two or one) and the same producer, each of which has been through use n - 256 itself.
+constexpr uint32_t DC_BARS = 256U, DC_PASS_COLS = 6144U;
+static_assert(DC_BARS % (2U * 4U) == 0U && DC_PASS_COLS / 64U + 64U + DC_MAX_PLACES <= DC_BARS, "readers of uses that share a barrier");
 // Hardware barriers of the consumer warps: all of them; the two warps of a unit whose halves of k are formed apart (up to eight units);
 // the eight warps of one of the two units of a residual projection. A barrier has ONE number of threads: only the exchanges keep the
 // last two uses apart, and a CTA that gave a wait up skips those, so they share no barrier.
@@ -75,6 +79,15 @@ enum { DX_QKV = 0, DX_ATTN = 1, DX_RESID = 2, DX_ACT = 3, DX_X = 4, DX_LM = 5, D
 struct dc_layout {
     uint32_t places, inverse;   // of the ring, and ceil(2^32 / places)
     uint32_t x, resid, normed, act, attn, scratch, qkv, red, staging, keys, total;   // byte offsets from the ring's start
+    uint32_t pass_cols, act_bytes;   // gate columns of a pass, and the bytes of its rows
+};
+
+// Gate rows that do not fit shared memory are formed and multiplied in passes of `pass_cols` columns (a multiple of the down projection's
+// chunks, so every sum is formed in the same order; its partial sums wait where its ranges meet), in two places by turns. A CTA sends
+// rows of pass p + 1 when it has all of pass p; those were sent behind a block barrier that follows their CTA's last read of pass p - 1.
+struct dc_pass {
+    uint32_t col, cols;       // first column and number of columns
+    uint32_t first, n;        // this CTA's units of eight columns
 };
 
 struct dc_args {
@@ -243,6 +256,15 @@ __device__ __forceinline__ void dc_share(uint32_t n, uint32_t rank, uint32_t cta
     *first = n * rank / ctas;
     *count = n * (rank + 1U) / ctas - *first;
 }
+__device__ __forceinline__ dc_pass dc_gate_pass(uint32_t pass, uint32_t pass_cols, uint32_t F, uint32_t rank, uint32_t ctas)
+{
+    dc_pass p;
+    p.col = pass * pass_cols;
+    p.cols = min(F - p.col, pass_cols);
+    dc_share(p.cols / 8U, rank, ctas, &p.first, &p.n);
+    p.first += p.col / 8U;
+    return p;
+}
 // Weight rows lo .. lo + 7 and hi .. hi + 7 of unit u of the CTA (the 16 outputs of the unit).
 __device__ __forceinline__ void dc_unit_rows(int kind, uint32_t u, uint32_t first, uint32_t rank, uint32_t D, uint32_t F, uint32_t *lo, uint32_t *hi)
 {
@@ -278,18 +300,18 @@ __device__ __forceinline__ dc_keys dc_key_range(int pos, int window, int cap, ui
 // Every tile of every step in the order of use; warp `which` of the producers issues tiles which, which + DC_PRODUCERS, ... of a phase,
 // and of the attention the tiles of consumer warps 4 which .. 4 which + 3, one per lane (a warp that shares its scheduler with working
 // ones takes some five cycles per instruction: one tile at a time, keys and values came at 19 bytes per cycle and SM).
-template <typename T, int D>
+template <typename T, int D, bool PASSES>
 __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, int rows, const int *positions, uint32_t lm_bar)
 {
     static_assert(DC_WARPS == 4 * DC_PRODUCERS, "four consumer warps to a producer");
     constexpr uint32_t CS = D / 32U;
     const gdb_decode_args &a = g.a;
-    const uint32_t F = (uint32_t)a.F, splits_log = 31U - (uint32_t)__clz(a.splits), hpc_log = 4U - splits_log;
+    const uint32_t F = (uint32_t)a.F, pass_cols = PASSES ? g.lay.pass_cols : F, splits_log = 31U - (uint32_t)__clz(a.splits), hpc_log = 4U - splits_log;
     const int groups = a.H >> hpc_log, attn_units = rows * groups;
-    uint32_t up_first, up_n, lm_first, lm_n;
-    dc_share(F / 8U, c.rank, CS, &up_first, &up_n);
+    uint32_t lm_first, lm_n;
     dc_share((uint32_t)a.V / 16U, c.rank, CS, &lm_first, &lm_n);
-    uint32_t n = 0U, place = 0U;
+    uint32_t n = 0U, place = 0U, pass = 0U;
+    dc_pass gate = dc_gate_pass(0U, pass_cols, F, c.rank, CS);
     auto claim = [&](uint32_t use) {   // its place is free
         if (use >= c.places) dc_wait(c, c.empty + ((use - c.places) % DC_BARS) * 8U, ((use - c.places) / DC_BARS) & 1U);
     };
@@ -334,9 +356,9 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
                 }
             }
             const CUtensorMap *map = kind == DC_LM ? &g.lm : &g.w[layer][kind];
-            const uint32_t units = kind == DC_QKV ? 6U : (kind == DC_OUT ? 2U : (kind == DC_UP ? up_n : lm_n)), first = kind == DC_UP ? up_first : lm_first;
-            const uint32_t tiles = kind == DC_DOWN ? F / 128U : 2U * units;
-            const bool whole = (kind == DC_UP || kind == DC_LM) && units > DC_PAIRS;   // a warp to a unit: the first halves of 16 units, then the second
+            const uint32_t units = kind == DC_QKV ? 6U : (kind == DC_OUT ? 2U : (kind == DC_UP ? gate.n : lm_n)), first = kind == DC_UP ? gate.first : lm_first;
+            const uint32_t tiles = kind == DC_DOWN ? gate.cols / 128U : 2U * units;
+            const bool whole = (kind == DC_LM && units > DC_PAIRS) || (kind == DC_UP && (PASSES || units > DC_PAIRS));   // a warp to a unit: the first halves of 16 units, then the second
             uint32_t s = wrap(place + 2U * which);
 #pragma unroll 1
             for (uint32_t i = which; i < tiles; i += DC_PRODUCERS, s = wrap(s + 2U * DC_PRODUCERS)) {
@@ -348,7 +370,7 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
                     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full + 8U) : "memory");   // (nobody waits for the second place's use)
                     if (kind == DC_DOWN) {
                         gdb_t5::mbar_expect_tx(full, DC_TILE);
-                        gdb_t5::tma_load_2d(dst, map, (int)(c.rank * 32U), (int)(i * 128U), full);
+                        gdb_t5::tma_load_2d(dst, map, (int)(c.rank * 32U), (int)(gate.col + i * 128U), full);
                     } else {
                         uint32_t u = i >> 1, half = i & 1U, lo, hi;
                         if (whole) {
@@ -366,6 +388,12 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
             }
             n += 2U * tiles;
             place = wrap(place + 2U * tiles);
+            if (PASSES && kind == DC_DOWN) {
+                const bool more = gate.col + gate.cols < F;
+                pass = more ? pass + 1U : 0U;
+                gate = dc_gate_pass(pass, pass_cols, F, c.rank, CS);
+                if (more) ph -= 2;   // back to up / gate
+            }
         }
     }
 }
@@ -419,7 +447,7 @@ __device__ __forceinline__ void dc_release(const dc_ctx &c, uint32_t empty, uint
     if (c.lane < PLACES && c.alive) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(empty + (uint32_t)c.lane * 8U), "r"(shares) : "memory");
 }
 
-template <typename T, int D, int NT>
+template <typename T, int D, int NT, bool PASSES>
 __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __grid_constant__ dc_args g)
 {
     constexpr uint32_t CS = D / 32U;             // CTAs of a cluster
@@ -445,14 +473,14 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
     c.lane = threadIdx.x & 31;
     c.alive = true;
     const int b0 = (int)(blockIdx.x / CS) * g.rows, rows = min(g.rows, a.B - b0);   // this cluster's sequences
-    const uint32_t F = (uint32_t)a.F, LDF = (F + 8U) * 2U;
+    const uint32_t F = (uint32_t)a.F, pass_cols = PASSES ? g.lay.pass_cols : F, LDF = (pass_cols + 8U) * 2U;
     const int L = a.L, hpc = 16 / a.splits, groups = a.H / hpc, attn_units = rows * groups;
     const uint32_t my_attn = attn_units > (int)c.rank ? ((uint32_t)attn_units - c.rank - 1U) / CS + 1U : 0U;
     const uint32_t s_x = c.sm + g.lay.x, s_resid = c.sm + g.lay.resid, s_normed = c.sm + g.lay.normed, s_act = c.sm + g.lay.act, s_attn = c.sm + g.lay.attn;
     const uint32_t s_qkv = c.sm + g.lay.qkv, s_red = c.sm + g.lay.red, s_stage = c.sm + g.lay.staging + (uint32_t)(c.warp & 15) * (NT * 256U);
     const uint32_t s_keys = c.sm + g.lay.keys, s_wkeys = c.sm + g.lay.staging;   // (the LM head's epilogue stages nothing)
     unsigned char *const generic = dc_raw + (c.sm - smem_u32(dc_raw));
-    const uint32_t row_bytes = (uint32_t)rows * D * 2U, act_bytes = (uint32_t)rows * F * 2U, qkv_bytes = my_attn * (uint32_t)hpc * 384U, key_bytes = (uint32_t)rows * CS * 8U;
+    const uint32_t row_bytes = (uint32_t)rows * D * 2U, act_bytes = (uint32_t)rows * pass_cols * 2U, qkv_bytes = my_attn * (uint32_t)hpc * 384U, key_bytes = (uint32_t)rows * CS * 8U;
     auto bar = [&](int i) { return smem_u32(xch) + (uint32_t)i * 8U; };
 
     if (c.tid < rows) positions[c.tid] = a.positions[b0 + c.tid];
@@ -478,21 +506,21 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
     gdb_t5::cluster_sync_all();
 
     if (c.warp >= DC_WARPS) {
-        dc_produce<T, D>(c, g, (uint32_t)(c.warp - DC_WARPS), b0, rows, positions, bar(DX_LM));
+        dc_produce<T, D, PASSES>(c, g, (uint32_t)(c.warp - DC_WARPS), b0, rows, positions, bar(DX_LM));
     } else {
+        uint32_t lm_first, lm_n, pass = 0U;
+        dc_share((uint32_t)a.V / 16U, c.rank, CS, &lm_first, &lm_n);
+        dc_pass gate = dc_gate_pass(0U, pass_cols, F, c.rank, CS);
         int stamp = 0;
         uint32_t phase_bits = 0U;   // parity of each exchange's next use
         auto receive = [&](int i, uint32_t bytes) {
             dc_wait(c, bar(i), (phase_bits >> i) & 1U);
             phase_bits ^= 1U << i;
             if (c.tid == 0) {
-                if (a.timeline != nullptr && blockIdx.x == 0U) dc_stamp(a, &stamp);
+                if (a.timeline != nullptr && blockIdx.x == 0U && (!PASSES || pass == 0U)) dc_stamp(a, &stamp);
                 if (c.alive) gdb_t5::mbar_expect_tx(bar(i), bytes);   // the next use
             }
         };
-        uint32_t up_first, up_n, lm_first, lm_n;
-        dc_share(F / 8U, c.rank, CS, &up_first, &up_n);
-        dc_share((uint32_t)a.V / 16U, c.rank, CS, &lm_first, &lm_n);
         const int grow = c.lane >> 2, t2 = (c.lane & 3) * 2;   // fragment: weight rows grow, grow + 8; sequences t2, t2 + 1
         // the activation row this lane addresses in a product (rows that no sequence fills repeat the last one; their outputs are dropped)
         const uint32_t brow = (uint32_t)min((c.lane & 7) + (NT == 2 ? (c.lane >> 4) * 8 : 0), rows - 1), bcol = ((uint32_t)(c.lane >> 3) & 1U) * 16U;
@@ -547,13 +575,15 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
             // head. One body of code for all of them (with a copy per kind, 100 KB of code instead of 70, a step of one sequence took
             // 45.0 us instead of 44.4).
 #pragma unroll 1
-            for (int j = 0; j <= 2 * L; ++j) {
+            for (int j = 0; j <= 2 * L;) {
                 const int kind = j == 2 * L ? (int)DC_LM : ((j & 1) != 0 ? (int)DC_UP : (int)DC_QKV);
                 const void *const *lw = a.lw[kind == DC_LM ? 0 : j >> 1];
                 const bool up = (j & 1) != 0;
-                const uint32_t n = kind == DC_QKV ? 6U : (kind == DC_UP ? up_n : lm_n), first = kind == DC_UP ? up_first : lm_first;
-                // Two warps to a unit (a half of k each) when there are up to eight units, else one, in rounds of 16.
-                const bool whole = n > DC_PAIRS;
+                const uint32_t s_gate = PASSES ? s_act + (pass & 1U) * g.lay.act_bytes : s_act;
+                const uint32_t n = kind == DC_QKV ? 6U : (kind == DC_UP ? gate.n : lm_n), first = kind == DC_UP ? gate.first : lm_first;
+                // Two warps to a unit (a half of k each) when there are up to eight units, else one, in rounds of 16. (One in a pass of several: the
+                // down projection's sums lie where the halves would meet.)
+                const bool whole = n > DC_PAIRS || (PASSES && up);
                 const T *bias = (const T *)(kind == DC_LM ? a.b_lm : lw[kind == DC_QKV ? 2 : 7]);
                 {
                     // ---- the rows' norm; what depends on no exchange is read ahead of it ----
@@ -591,8 +621,8 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                     uint32_t em0 = 0U, tile0 = 0U;
                     const uint32_t i_first = whole ? u_first : (uint32_t)c.warp;
                     if (u_first < n && 2U * i_first + 1U < c.places) tile0 = wait_tile(i_first, &em0);
-                    if (j != 0 || step > 0) receive(j == 0 ? DX_LM : (up ? DX_RESID : DX_X), j == 0 ? key_bytes : row_bytes);
-                    if (c.warp < rows) {
+                    if ((j != 0 || step > 0) && (!PASSES || pass == 0U)) receive(j == 0 ? DX_LM : (up ? DX_RESID : DX_X), j == 0 ? key_bytes : row_bytes);
+                    if (c.warp < rows && (!PASSES || pass == 0U)) {
                         const uint32_t at = (up ? s_resid : s_x) + (uint32_t)c.warp * (D * 2U) + (uint32_t)c.lane * 16U;
                         if (j == 0) {
                             const int id = step == 0 ? a.tokens[b0 + c.warp] : best_id(c.warp, step - 1);
@@ -718,7 +748,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
 #pragma unroll
                                 for (uint32_t i = 0; i < (CS * NT + 3U) / 4U; ++i) {
                                     const uint32_t to = i * (4U / NT) + (uint32_t)c.lane / (NT * 8U);
-                                    if (to < CS) dc_send(mapa_shared(s_act + vec * LDF + lo * 2U, to), val, mapa_shared(bar(DX_ACT), to));
+                                    if (to < CS) dc_send(mapa_shared(s_gate + vec * LDF + (PASSES ? lo - gate.col : lo) * 2U, to), val, mapa_shared(bar(DX_ACT), to));
                                 }
                             }
                             __syncwarp();
@@ -884,17 +914,29 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                     // (down) ranges are eighths of chunks of k (sk_chunk_for), a tile is 128 k
                     const uint32_t ch = (F % 512U) == 0U ? 512U : ((F % 256U) == 0U ? 256U : 128U), kw = ch / 8U, off = ((uint32_t)c.warp & 7U) * kw;
                     uint32_t em, tile = wait_tile(up ? off / 128U : (uint32_t)ou * 2U + (((uint32_t)c.warp >> 2) & 1U), &em);
-                    receive(up ? DX_ACT : DX_ATTN, up ? act_bytes : row_bytes);
+                    const bool more = PASSES && up && gate.col + gate.cols < F;   // a pass of the gate rows behind this one
+                    receive(up ? DX_ACT : DX_ATTN, up ? (more ? (uint32_t)rows * min(F - gate.col - gate.cols, pass_cols) * 2U : act_bytes) : row_bytes);
                     float acc[1][NT][4];
                     if (!up) {
                         dc_ranges<T, D, NT, 1>(acc, tile, s_attn + brow * LDA + bcol + (((uint32_t)c.warp >> 2) & 1U) * D, (uint32_t)c.warp & 3U, c.lane);
                         dc_release<2>(c, em, 4U);
                         advance(8U);
                     } else {
+                        const uint32_t kept = s_red + (uint32_t)c.warp * (NT * 512U) + (uint32_t)c.lane * 16U;
 #pragma unroll
                         for (int t = 0; t < NT; ++t)
 #pragma unroll
                             for (int e = 0; e < 4; ++e) acc[0][t][e] = 0.0f;
+                        if (PASSES && pass != 0U) {
+#pragma unroll
+                            for (int t = 0; t < NT; ++t) {
+                                const uint4 w = dc_lds16(kept + (uint32_t)t * 512U);
+                                acc[0][t][0] = __uint_as_float(w.x);
+                                acc[0][t][1] = __uint_as_float(w.y);
+                                acc[0][t][2] = __uint_as_float(w.z);
+                                acc[0][t][3] = __uint_as_float(w.w);
+                            }
+                        }
                         const uint32_t r = c.lane & 7, half = (c.lane >> 3) & 1, kc = c.lane >> 4;
                         // (k steps are multiples of 16, eight rows apart within a step: the swizzle term does not depend on k)
                         const uint32_t w_at = (off % 128U + kc * 8U + r) * 64U + ((((uint32_t)ou * 2U + half) ^ ((r >> 1) & 3U)) << 4);
@@ -914,9 +956,9 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                             }
                         };
 #pragma unroll 1
-                        for (uint32_t k0 = off; k0 < F; k0 += ch) {
+                        for (uint32_t k0 = off; k0 < (PASSES ? gate.cols : F); k0 += ch) {
                             if (k0 != off) tile = wait_tile(k0 / 128U, &em);
-                            const uint32_t w = tile + w_at, x = s_act + brow * LDF + bcol + k0 * 2U;
+                            const uint32_t w = tile + w_at, x = s_gate + brow * LDF + bcol + k0 * 2U;
                             if (kw == 64U) {
 #pragma unroll
                                 for (uint32_t i = 0; i < 4U; ++i) k16(w + i * 1024U, x + i * 32U);
@@ -926,7 +968,15 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                             }
                             dc_release<2>(c, em, kw / 16U);   // (of 256 / kw warps)
                         }
-                        advance(F / 64U);
+                        advance((PASSES ? gate.cols : F) / 64U);
+                        if (PASSES) {
+                            pass = more ? pass + 1U : 0U;
+                            gate = dc_gate_pass(pass, pass_cols, F, c.rank, CS);
+                            if (more) {
+                                dc_leave_range<NT>(acc[0], kept);
+                                continue;
+                            }
+                        }
                     }
                     // the ranges' sums through shared memory, then a thread per output; the new rows go to every CTA
                     dc_leave_range<NT>(acc[0], s_red + (uint32_t)c.warp * (NT * 512U) + (uint32_t)c.lane * 16U);
@@ -953,6 +1003,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                         }
                     }
                 }
+                ++j;
             }
         }
         if (going) receive(DX_LM, key_bytes);
@@ -1011,11 +1062,11 @@ bool dc_map_down(CUtensorMap *m, uint32_t dtype, const void *base, uint64_t F, u
 }
 
 typedef void (*dc_kernel)(const dc_args);
-template <typename T>
+template <typename T, bool PASSES>
 dc_kernel dc_pick(uint32_t D, int tiles)
 {
-    if (D == 512U) return tiles == 1 ? decode_cluster_kernel<T, 512, 1> : decode_cluster_kernel<T, 512, 2>;
-    return D == 256U ? decode_cluster_kernel<T, 256, 1> : decode_cluster_kernel<T, 128, 1>;   // (of these enough clusters are resident)
+    if (D == 512U) return tiles == 1 ? decode_cluster_kernel<T, 512, 1, PASSES> : decode_cluster_kernel<T, 512, 2, PASSES>;
+    return D == 256U ? decode_cluster_kernel<T, 256, 1, PASSES> : decode_cluster_kernel<T, 128, 1, PASSES>;   // (of these enough clusters are resident)
 }
 
 // Shared memory of a CTA whose cluster has `rows` sequences; false when fewer than DC_MIN_PLACES places fit beside it.
@@ -1032,17 +1083,33 @@ bool dc_make_layout(dc_layout *l, uint32_t rows, uint32_t D, uint32_t F, uint32_
     l->x = take(rows * D * 2U);
     l->resid = take(rows * D * 2U);
     l->normed = take(rows * (D + 8U) * 2U);
-    // The attention's output rows and partials share the gate rows' place: those are read in the down projection only, whose sums all
-    // CTAs have sent before any can be in the next attention, and attention rows are multiplied before any residual row leaves.
-    const uint32_t attn_bytes = (rows * (D + 8U) * 2U + 127U) & ~127U;
-    // (the merge of a head's splits reads 16 items' worth of words from its first one on)
-    l->act = take(std::max(rows * (F + 8U) * 2U, attn_bytes + (units * DC_PARTIALS + 16U * 64U) * 4U));
-    l->attn = l->act;
-    l->scratch = l->act + attn_bytes;
     l->qkv = take(units * hpc * 384U);
     l->red = take(16U * tiles * 1024U);   // eight units of four k ranges, or two of eight
     l->staging = take(16U * std::max(tiles * 256U, (uint32_t)DC_MAX_ROWS * 8U));
     l->keys = take(CS * DC_MAX_ROWS * 8U);
+    // The attention's output rows and partials share the gate rows' place: those are read in the down projection only, whose sums all
+    // CTAs have sent before any can be in the next attention, and attention rows are multiplied before any residual row leaves.
+    const uint32_t attn_bytes = (rows * (D + 8U) * 2U + 127U) & ~127U;
+    // (the merge of a head's splits reads 16 items' worth of words from its first one on)
+    const uint32_t attn = attn_bytes + (units * DC_PARTIALS + 16U * 64U) * 4U;
+    auto gate_bytes = [&](uint32_t cols) { return (rows * (cols + 8U) * 2U + 127U) & ~127U; };
+    l->pass_cols = F;
+    // One pass, or as few of equal width, with two places for their rows, as leave the ring 24 places; 16 where the cluster has more than
+    // eight sequences, whose passes would be narrow. (us per step, three layers of hidden 8192, 48 sequences: one pass beside 16 places 142, four beside
+    // 26 132; 64 sequences, passes beside 16 / 20 / 24 places 197 / 206 / 210, one launch per operation 261.)
+    const uint32_t ring_bytes = (tiles == 1U ? 24U : DC_MIN_PLACES) * DC_PLACE;
+    if (top + std::max(gate_bytes(F), attn) + ring_bytes > limit) {
+        const uint32_t chunk = (F % 512U) == 0U ? 512U : ((F % 256U) == 0U ? 256U : 128U);
+        for (uint32_t passes = 2U;; ++passes) {
+            l->pass_cols = ((F + passes - 1U) / passes + chunk - 1U) / chunk * chunk;
+            const bool fits = top + std::max(2U * gate_bytes(l->pass_cols), attn) + ring_bytes <= limit;
+            if (l->pass_cols == chunk || (fits && l->pass_cols <= DC_PASS_COLS)) break;
+        }
+    }
+    l->act_bytes = gate_bytes(l->pass_cols);
+    l->act = take(std::max(l->pass_cols < F ? 2U * l->act_bytes : l->act_bytes, attn));
+    l->attn = l->act;
+    l->scratch = l->act + attn_bytes;
     if (top + DC_MIN_PLACES * DC_PLACE > limit) return false;
     l->places = std::min((limit - top) / DC_PLACE & ~1U, DC_MAX_PLACES);
     l->inverse = 0xffffffffU / l->places + 1U;
@@ -1087,7 +1154,10 @@ gd_status gdb_decode_cluster_launch(gd_backend *be, uint32_t dtype, const gdb_de
     dc_kernel kern = nullptr;
     auto prepare = [&](int rows) {   // kernel, layout and launch shape for `rows` sequences per cluster
         if (!dc_make_layout(&g.lay, (uint32_t)rows, D, F, (uint32_t)a->H, (uint32_t)a->splits)) return false;
-        kern = dtype == GDB_DTYPE_F16 ? dc_pick<__half>(D, rows > 8 ? 2 : 1) : dc_pick<__nv_bfloat16>(D, rows > 8 ? 2 : 1);
+        const bool half = dtype == GDB_DTYPE_F16;
+        const int tiles = rows > 8 ? 2 : 1;
+        if (g.lay.pass_cols < F) kern = half ? dc_pick<__half, true>(D, tiles) : dc_pick<__nv_bfloat16, true>(D, tiles);
+        else kern = half ? dc_pick<__half, false>(D, tiles) : dc_pick<__nv_bfloat16, false>(D, tiles);
         g.rows = rows;
         cfg.dynamicSmemBytes = g.lay.total + 1024U;
         cfg.gridDim = dim3((unsigned)((a->B + rows - 1) / rows) * CS);

@@ -46,6 +46,13 @@ def compare_decode_forms(monkeypatch, cfg, batch, prompt, new):
     assert all(np.array_equal(a, b) for a, b in zip(*forms))
 
 
+def other_model(dtype, d_model, mlp_hidden, vocab, layers, window):
+    cfg = g.GptConfig.baseline()
+    cfg.dropout_p, cfg.sdpa_window, cfg.n_layers, cfg.vocab_size, cfg.dtype = 0.0, window, layers, vocab, dtype
+    cfg.d_model, cfg.n_heads, cfg.mlp_hidden, cfg.context_length = d_model, d_model // 64, mlp_hidden, 1024
+    return cfg
+
+
 # weights resident in shared memory: one pass of rows and its edges (16 rows to a tile, 32 to a pass), a window, the largest batch
 @pytest.mark.parametrize("dtype", [abi.F16, abi.BF16])
 @pytest.mark.parametrize("batch,prompt,new,window", [(1, 16, 32, 0), (13, 77, 45, 64), (16, 40, 24, 0), (17, 40, 24, 0), (32, 30, 24, 0), (33, 100, 40, 0), (64, 200, 48, 0)])
@@ -68,11 +75,20 @@ def test_persistent_decode_of_a_larger_model_agrees_bit_for_bit(monkeypatch, dty
 
 # clusters of four and eight CTAs; more than 16 units of a phase to a CTA (rounds), a CTA with one unit more than another, k ranges of 16 and
 # 32, one 128-wide tile of the down projection; positions behind the cos / sin table (512) and more than 32 keys to a warp
+@pytest.mark.parametrize("dtype", [abi.F16, abi.BF16])
 @pytest.mark.parametrize("d_model,mlp_hidden,vocab,layers,batch,prompt,new,window", [
     (128, 128, 4096, 2, 5, 6, 12, 0), (128, 2560, 272, 1, 64, 4, 9, 3), (256, 640, 272, 2, 20, 30, 20, 0), (256, 768, 4112, 1, 3, 17, 8, 5),
     (512, 1536, 2048, 1, 3, 490, 40, 0), (512, 512, 16, 1, 59, 250, 12, 200)])
-def test_decode_of_other_shapes_agrees_bit_for_bit(monkeypatch, d_model, mlp_hidden, vocab, layers, batch, prompt, new, window):
-    cfg = g.GptConfig.baseline()
-    cfg.dropout_p, cfg.sdpa_window, cfg.n_layers, cfg.vocab_size = 0.0, window, layers, vocab
-    cfg.d_model, cfg.n_heads, cfg.mlp_hidden, cfg.context_length = d_model, d_model // 64, mlp_hidden, 1024
+def test_decode_of_other_shapes_agrees_bit_for_bit(monkeypatch, dtype, d_model, mlp_hidden, vocab, layers, batch, prompt, new, window):
+    cfg = other_model(dtype, d_model, mlp_hidden, vocab, layers, window)
     compare_decode_forms(monkeypatch, cfg, batch, prompt, new)
+
+
+# gate rows in one pass and in several: the last hidden width of one pass and the first of several for ten, nine, eight and two sequences to a
+# cluster, chunks of 512, 256 and 128, a short last pass; more places between two warps of the down projection than the ring has barriers
+@pytest.mark.parametrize("dtype", [abi.F16, abi.BF16])
+@pytest.mark.parametrize("d_model,mlp_hidden,batch", [
+    (512, 4096, 64), (512, 4224, 64), (512, 8192, 64), (512, 8960, 64), (512, 4736, 63), (512, 4864, 63), (512, 4736, 56), (512, 4864, 56), (512, 4992, 56),
+    (512, 8192, 49), (512, 8448, 45), (512, 16384, 30), (512, 16896, 1), (256, 9600, 64), (256, 9728, 64), (128, 26112, 64), (128, 26240, 64)])
+def test_decode_with_gate_rows_in_passes_agrees_bit_for_bit(monkeypatch, dtype, d_model, mlp_hidden, batch):
+    compare_decode_forms(monkeypatch, other_model(dtype, d_model, mlp_hidden, 272, 2, 0), batch, 5, 6)
