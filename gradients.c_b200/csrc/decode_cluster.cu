@@ -44,10 +44,12 @@ using gdb_t5::mapa_shared;
 constexpr int DC_WARPS = 16, DC_PRODUCERS = 4, DC_THREADS = (DC_WARPS + DC_PRODUCERS) * 32;
 constexpr int DC_MAX_ROWS = 16;              // sequences of a cluster
 constexpr int DC_PARTIALS = DC_WARPS * 2 + DC_WARPS * 64;   // (max, sum) and weighted sums of the 16 (head, split) items of an attention unit
-// The ring is used in places of 4 KB: a weight tile takes two (16 rows x half of k for d_model 512, or 128 k x 32 columns of the down
-// projection), 16 keys and values of a head take one. (Tiles of 32 keys in places of 8 KB: with 14 places and 16 warps the copy of a
+// The ring is used in places of 4 KB: a weight tile of 128 k x 32 columns of the down projection takes two, one of 16 rows x half of k two for
+// d_model 512 and else one (with two, d_model 256, hidden 2048: 3.9 us for 16 more gate units to a CTA, 1.8 with one), 16 keys and values of a
+// head take one. (Tiles of 32 keys in places of 8 KB: with 14 places and 16 warps the copy of a
 // warp's next tile began when it was done with this one, 27 bytes per cycle and SM for 64 sequences.)
 constexpr uint32_t DC_PLACE = 4096U, DC_TILE = 2U * DC_PLACE;
+template <int D> constexpr uint32_t DC_ROW_PLACES = D == 512 ? 2U : 1U;   // of a tile of 16 weight rows
 constexpr uint32_t DC_MAX_PLACES = 48U, DC_MIN_PLACES = 16U;
 // Use n of a place has barriers n % 256 of its own (full: its bytes have landed; empty: its readers are done), not the place's: a warp
 // may wait for a tile whose place is still to be used once or twice before, and a parity cannot tell those phases apart. A barrier's use
@@ -359,15 +361,16 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
             const uint32_t units = kind == DC_QKV ? 6U : (kind == DC_OUT ? 2U : (kind == DC_UP ? gate.n : lm_n)), first = kind == DC_UP ? gate.first : lm_first;
             const uint32_t tiles = kind == DC_DOWN ? gate.cols / 128U : 2U * units;
             const bool whole = (kind == DC_LM && units > DC_PAIRS) || (kind == DC_UP && (PASSES || units > DC_PAIRS));   // a warp to a unit: the first halves of 16 units, then the second
-            uint32_t s = wrap(place + 2U * which);
+            const uint32_t each = kind == DC_DOWN ? 2U : DC_ROW_PLACES<D>;   // places of a tile
+            uint32_t s = wrap(place + each * which);
 #pragma unroll 1
-            for (uint32_t i = which; i < tiles; i += DC_PRODUCERS, s = wrap(s + 2U * DC_PRODUCERS)) {
-                const uint32_t use = n + 2U * i;   // (even: a phase of the attention uses a multiple of 16 places, and their number is even)
+            for (uint32_t i = which; i < tiles; i += DC_PRODUCERS, s = wrap(s + each * DC_PRODUCERS)) {
+                const uint32_t use = n + each * i;   // (even for two places: all phases use an even number, and so is theirs)
                 claim(use);
-                claim(use + 1U);
+                if (each == 2U) claim(use + 1U);
                 if (c.alive && c.lane == 0) {
                     const uint32_t full = c.full + (use % DC_BARS) * 8U, dst = c.sm + s * DC_PLACE;
-                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full + 8U) : "memory");   // (nobody waits for the second place's use)
+                    if (each == 2U) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full + 8U) : "memory");   // (nobody waits for the second place's use)
                     if (kind == DC_DOWN) {
                         gdb_t5::mbar_expect_tx(full, DC_TILE);
                         gdb_t5::tma_load_2d(dst, map, (int)(c.rank * 32U), (int)(gate.col + i * 128U), full);
@@ -386,8 +389,8 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
                 }
                 __syncwarp();
             }
-            n += 2U * tiles;
-            place = wrap(place + 2U * tiles);
+            n += each * tiles;
+            place = wrap(place + each * tiles);
             if (PASSES && kind == DC_DOWN) {
                 const bool more = gate.col + gate.cols < F;
                 pass = more ? pass + 1U : 0U;
@@ -440,11 +443,11 @@ __device__ __forceinline__ void dc_ranges(float (&acc)[G][NT][4], uint32_t tile,
         }
 }
 // `shares` of the 16 reader shares of a tile of one or two places are done.
-template <int PLACES>
+template <uint32_t PLACES>
 __device__ __forceinline__ void dc_release(const dc_ctx &c, uint32_t empty, uint32_t shares)
 {
     __syncwarp();
-    if (c.lane < PLACES && c.alive) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(empty + (uint32_t)c.lane * 8U), "r"(shares) : "memory");
+    if ((uint32_t)c.lane < PLACES && c.alive) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(empty + (uint32_t)c.lane * 8U), "r"(shares) : "memory");
 }
 
 template <typename T, int D, int NT, bool PASSES>
@@ -537,7 +540,8 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
             dc_wait(c, c.full + which, (n / DC_BARS) & 1U);
             return c.sm + place * DC_PLACE;
         };
-        auto wait_tile = [&](uint32_t i, uint32_t *empty_bar) { return wait_use(2U * i, empty_bar); };   // weight tile i of this phase
+        constexpr uint32_t ROW_PLACES = DC_ROW_PLACES<D>;
+        auto wait_tile = [&](uint32_t i, uint32_t *empty_bar) { return wait_use(ROW_PLACES * i, empty_bar); };   // tile i of 16 weight rows of this phase
         auto advance = [&](uint32_t uses) {
             c.n += uses;
             c.place = dc_wrap(c, c.place + uses);
@@ -620,7 +624,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                     // tile of this phase must leave first is waited for behind the block barrier that the other's readers need.)
                     uint32_t em0 = 0U, tile0 = 0U;
                     const uint32_t i_first = whole ? u_first : (uint32_t)c.warp;
-                    if (u_first < n && 2U * i_first + 1U < c.places) tile0 = wait_tile(i_first, &em0);
+                    if (u_first < n && ROW_PLACES * (i_first + 1U) <= c.places) tile0 = wait_tile(i_first, &em0);
                     if ((j != 0 || step > 0) && (!PASSES || pass == 0U)) receive(j == 0 ? DX_LM : (up ? DX_RESID : DX_X), j == 0 ? key_bytes : row_bytes);
                     if (c.warp < rows && (!PASSES || pass == 0U)) {
                         const uint32_t at = (up ? s_resid : s_x) + (uint32_t)c.warp * (D * 2U) + (uint32_t)c.lane * 16U;
@@ -699,9 +703,9 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                             float acc[4][NT][4];
                             uint32_t em = em0, tile = tile0;
                             if (u0 != 0U || (whole && half != 0U)) tile = wait_tile(2U * u0 + half * min(n - u0, 16U) + (u - u0), &em);
-                            else if (2U * i_first + 1U >= c.places) tile = wait_tile(i_first, &em);
+                            else if (ROW_PLACES * (i_first + 1U) > c.places) tile = wait_tile(i_first, &em);
                             dc_ranges<T, D, NT, 4>(acc, tile, acts + half * D, 0U, c.lane);
-                            dc_release<2>(c, em, 16U);
+                            dc_release<ROW_PLACES>(c, em, 16U);
                             if (whole || half == 0U) {
 #pragma unroll
                                 for (int t = 0; t < NT; ++t)
@@ -792,7 +796,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                             __syncwarp();
                         }
                     }
-                    advance(4U * n);
+                    advance(2U * ROW_PLACES * n);
                     if (kind == DC_LM) {
                         // over the eight weight rows of the fragment, then over the warps, then to every CTA
 #pragma unroll
@@ -913,14 +917,14 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                     const float b = gdb_io<T>::ld((const T *)lw[up ? 9 : 4], ocol);
                     // (down) ranges are eighths of chunks of k (sk_chunk_for), a tile is 128 k
                     const uint32_t ch = (F % 512U) == 0U ? 512U : ((F % 256U) == 0U ? 256U : 128U), kw = ch / 8U, off = ((uint32_t)c.warp & 7U) * kw;
-                    uint32_t em, tile = wait_tile(up ? off / 128U : (uint32_t)ou * 2U + (((uint32_t)c.warp >> 2) & 1U), &em);
+                    uint32_t em, tile = wait_use(up ? off / 128U * 2U : ((uint32_t)ou * 2U + (((uint32_t)c.warp >> 2) & 1U)) * ROW_PLACES, &em);
                     const bool more = PASSES && up && gate.col + gate.cols < F;   // a pass of the gate rows behind this one
                     receive(up ? DX_ACT : DX_ATTN, up ? (more ? (uint32_t)rows * min(F - gate.col - gate.cols, pass_cols) * 2U : act_bytes) : row_bytes);
                     float acc[1][NT][4];
                     if (!up) {
                         dc_ranges<T, D, NT, 1>(acc, tile, s_attn + brow * LDA + bcol + (((uint32_t)c.warp >> 2) & 1U) * D, (uint32_t)c.warp & 3U, c.lane);
-                        dc_release<2>(c, em, 4U);
-                        advance(8U);
+                        dc_release<ROW_PLACES>(c, em, 4U);
+                        advance(4U * ROW_PLACES);
                     } else {
                         const uint32_t kept = s_red + (uint32_t)c.warp * (NT * 512U) + (uint32_t)c.lane * 16U;
 #pragma unroll
@@ -957,7 +961,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                         };
 #pragma unroll 1
                         for (uint32_t k0 = off; k0 < (PASSES ? gate.cols : F); k0 += ch) {
-                            if (k0 != off) tile = wait_tile(k0 / 128U, &em);
+                            if (k0 != off) tile = wait_use(k0 / 128U * 2U, &em);
                             const uint32_t w = tile + w_at, x = s_gate + brow * LDF + bcol + k0 * 2U;
                             if (kw == 64U) {
 #pragma unroll
