@@ -50,6 +50,9 @@ constexpr int DC_PARTIALS = DC_WARPS * 2 + DC_WARPS * 64;   // (max, sum) and we
 // warp's next tile began when it was done with this one, 27 bytes per cycle and SM for 64 sequences.)
 constexpr uint32_t DC_PLACE = 4096U, DC_TILE = 2U * DC_PLACE;
 template <int D> constexpr uint32_t DC_ROW_PLACES = D == 512 ? 2U : 1U;   // of a tile of 16 weight rows
+// d_model 128: both halves of k in one tile, but for the LM head (whose units may be odd in number: a phase takes an even number of places).
+// (Two tiles of 2 KB each: four layers of hidden 2560 96 us per step, 74 with one.)
+template <int D> constexpr bool DC_JOINED = D == 128;
 constexpr uint32_t DC_MAX_PLACES = 48U, DC_MIN_PLACES = 16U;
 // Use n of a place has barriers n % 256 of its own (full: its bytes have landed; empty: its readers are done), not the place's: a warp
 // may wait for a tile whose place is still to be used once or twice before, and a parity cannot tell those phases apart. A barrier's use
@@ -359,7 +362,8 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
             }
             const CUtensorMap *map = kind == DC_LM ? &g.lm : &g.w[layer][kind];
             const uint32_t units = kind == DC_QKV ? 6U : (kind == DC_OUT ? 2U : (kind == DC_UP ? gate.n : lm_n)), first = kind == DC_UP ? gate.first : lm_first;
-            const uint32_t tiles = kind == DC_DOWN ? gate.cols / 128U : 2U * units;
+            const bool joined = DC_JOINED<D> && kind != DC_LM;
+            const uint32_t tiles = kind == DC_DOWN ? gate.cols / 128U : (joined ? units : 2U * units);
             const bool whole = (kind == DC_LM && units > DC_PAIRS) || (kind == DC_UP && (PASSES || units > DC_PAIRS));   // a warp to a unit: the first halves of 16 units, then the second
             const uint32_t each = kind == DC_DOWN ? 2U : DC_ROW_PLACES<D>;   // places of a tile
             uint32_t s = wrap(place + each * which);
@@ -375,14 +379,14 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
                         gdb_t5::mbar_expect_tx(full, DC_TILE);
                         gdb_t5::tma_load_2d(dst, map, (int)(c.rank * 32U), (int)(gate.col + i * 128U), full);
                     } else {
-                        uint32_t u = i >> 1, half = i & 1U, lo, hi;
-                        if (whole) {
+                        uint32_t u = joined ? i : i >> 1, half = joined ? 0U : i & 1U, lo, hi;
+                        if (whole && !joined) {
                             const uint32_t u0 = i / 32U * 16U, in = i % 32U, nr = min(units - u0, 16U);
                             half = in >= nr ? 1U : 0U;
                             u = u0 + in - half * nr;
                         }
                         dc_unit_rows(kind, u, first, c.rank, D, F, &lo, &hi);
-                        gdb_t5::mbar_expect_tx(full, 16U * D);
+                        gdb_t5::mbar_expect_tx(full, joined ? 32U * D : 16U * D);
                         gdb_t5::tma_load_4d(dst, map, 0, (int)(kind == DC_UP ? lo : (kind == DC_QKV ? lo & 31U : 0U)),
                                             (int)(kind == DC_UP ? 0U : (kind == DC_QKV ? lo >> 5 : lo >> 3)), (int)(half * (D / 128U)), full);
                     }
@@ -623,7 +627,8 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                     // The weights are there before the rows are, as a rule: their wait is not behind the rows'. (A tile whose place another
                     // tile of this phase must leave first is waited for behind the block barrier that the other's readers need.)
                     uint32_t em0 = 0U, tile0 = 0U;
-                    const uint32_t i_first = whole ? u_first : (uint32_t)c.warp;
+                    const bool joined = DC_JOINED<D> && kind != DC_LM;
+                    const uint32_t i_first = whole || joined ? u_first : (uint32_t)c.warp;
                     if (u_first < n && ROW_PLACES * (i_first + 1U) <= c.places) tile0 = wait_tile(i_first, &em0);
                     if ((j != 0 || step > 0) && (!PASSES || pass == 0U)) receive(j == 0 ? DX_LM : (up ? DX_RESID : DX_X), j == 0 ? key_bytes : row_bytes);
                     if (c.warp < rows && (!PASSES || pass == 0U)) {
@@ -698,14 +703,17 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                             for (int e = 0; e < 4; ++e) v[t][e] = 0.0f;
                         const uint32_t part = (uint32_t)c.warp & 1U, slot0 = s_red + u * (NT * 2048U) + (uint32_t)c.lane * 16U;   // the second half's four ranges
                         bool mine = true;
+                        uint32_t em = em0, tile = tile0;
 #pragma unroll 1
                         for (uint32_t half = whole ? 0U : part; half < 2U; half += whole ? 1U : 2U) {
                             float acc[4][NT][4];
-                            uint32_t em = em0, tile = tile0;
-                            if (u0 != 0U || (whole && half != 0U)) tile = wait_tile(2U * u0 + half * min(n - u0, 16U) + (u - u0), &em);
-                            else if (ROW_PLACES * (i_first + 1U) > c.places) tile = wait_tile(i_first, &em);
-                            dc_ranges<T, D, NT, 4>(acc, tile, acts + half * D, 0U, c.lane);
-                            dc_release<ROW_PLACES>(c, em, 16U);
+                            if (!joined || !whole || half == 0U) {
+                                if (u0 != 0U || (whole && half != 0U)) tile = wait_tile(joined ? u : 2U * u0 + half * min(n - u0, 16U) + (u - u0), &em);
+                                else if (ROW_PLACES * (i_first + 1U) > c.places) tile = wait_tile(i_first, &em);
+                            }
+                            dc_ranges<T, D, NT, 4>(acc, joined ? tile + half * 2048U : tile, acts + half * D, 0U, c.lane);
+                            if (!joined) dc_release<ROW_PLACES>(c, em, 16U);
+                            else if (!whole || half != 0U) dc_release<ROW_PLACES>(c, em, whole ? 16U : 8U);
                             if (whole || half == 0U) {
 #pragma unroll
                                 for (int t = 0; t < NT; ++t)
@@ -796,7 +804,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                             __syncwarp();
                         }
                     }
-                    advance(2U * ROW_PLACES * n);
+                    advance(joined ? n : 2U * ROW_PLACES * n);
                     if (kind == DC_LM) {
                         // over the eight weight rows of the fragment, then over the warps, then to every CTA
 #pragma unroll
@@ -917,14 +925,15 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                     const float b = gdb_io<T>::ld((const T *)lw[up ? 9 : 4], ocol);
                     // (down) ranges are eighths of chunks of k (sk_chunk_for), a tile is 128 k
                     const uint32_t ch = (F % 512U) == 0U ? 512U : ((F % 256U) == 0U ? 256U : 128U), kw = ch / 8U, off = ((uint32_t)c.warp & 7U) * kw;
-                    uint32_t em, tile = wait_use(up ? off / 128U * 2U : ((uint32_t)ou * 2U + (((uint32_t)c.warp >> 2) & 1U)) * ROW_PLACES, &em);
+                    const uint32_t khalf = ((uint32_t)c.warp >> 2) & 1U;
+                    uint32_t em, tile = wait_use(up ? off / 128U * 2U : (DC_JOINED<D> ? (uint32_t)ou : ((uint32_t)ou * 2U + khalf) * ROW_PLACES), &em);
                     const bool more = PASSES && up && gate.col + gate.cols < F;   // a pass of the gate rows behind this one
                     receive(up ? DX_ACT : DX_ATTN, up ? (more ? (uint32_t)rows * min(F - gate.col - gate.cols, pass_cols) * 2U : act_bytes) : row_bytes);
                     float acc[1][NT][4];
                     if (!up) {
-                        dc_ranges<T, D, NT, 1>(acc, tile, s_attn + brow * LDA + bcol + (((uint32_t)c.warp >> 2) & 1U) * D, (uint32_t)c.warp & 3U, c.lane);
-                        dc_release<ROW_PLACES>(c, em, 4U);
-                        advance(4U * ROW_PLACES);
+                        dc_ranges<T, D, NT, 1>(acc, DC_JOINED<D> ? tile + khalf * 2048U : tile, s_attn + brow * LDA + bcol + khalf * D, (uint32_t)c.warp & 3U, c.lane);
+                        dc_release<ROW_PLACES>(c, em, DC_JOINED<D> ? 2U : 4U);
+                        advance(DC_JOINED<D> ? 2U : 4U * ROW_PLACES);
                     } else {
                         const uint32_t kept = s_red + (uint32_t)c.warp * (NT * 512U) + (uint32_t)c.lane * 16U;
 #pragma unroll
@@ -1039,15 +1048,15 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
     }
 }
 
-// K-major weights as tiles of 16 rows (two groups of eight, `gap` rows apart, at multiples of `step` rows) x half of k, in shared memory
-// D / 128 blocks of 16 rows x 128 bytes.
-bool dc_map_rows(CUtensorMap *m, uint32_t dtype, const void *base, uint32_t inner_rows, uint64_t gap, uint64_t groups, uint32_t D)
+// K-major weights as tiles of 16 rows (two groups of eight, `gap` rows apart) x `blocks` times 64 k, in shared memory as blocks of 16 rows x
+// 128 bytes.
+bool dc_map_rows(CUtensorMap *m, uint32_t dtype, const void *base, uint32_t inner_rows, uint64_t gap, uint64_t groups, uint32_t D, uint32_t blocks)
 {
     gdb_t5::encode_tiled_fn fn = gdb_t5::get_encode_fn();
     if (fn == nullptr) return false;
     const cuuint64_t dims[4] = {64, inner_rows, groups, D / 64U};
     const cuuint64_t strides[3] = {D * 2U, gap * D * 2U, 128};
-    const cuuint32_t box[4] = {64, 8, 2, D / 128U}, estr[4] = {1, 1, 1, 1};
+    const cuuint32_t box[4] = {64, 8, 2, blocks}, estr[4] = {1, 1, 1, 1};
     const CUtensorMapDataType dt = dtype == GDB_DTYPE_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
     return fn(m, dt, 4, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
@@ -1185,10 +1194,11 @@ gd_status gdb_decode_cluster_launch(gd_backend *be, uint32_t dtype, const gdb_de
         return GD_ERR_UNSUPPORTED;
     }
     const uint64_t cap = (uint64_t)a->CAP;
-    bool mapped = dc_map_rows(&g.lm, dtype, a->w_lm, 8U, 8U, (uint64_t)a->V / 8U, D);
+    const uint32_t blocks = DC_JOINED<128> && D == 128U ? 2U : D / 128U;
+    bool mapped = dc_map_rows(&g.lm, dtype, a->w_lm, 8U, 8U, (uint64_t)a->V / 8U, D, D / 128U);
     for (int i = 0; i < a->L && mapped; ++i) {
-        mapped = dc_map_rows(&g.w[i][DC_QKV], dtype, a->lw[i][1], 32U, 32U, 3U * D / 32U, D) && dc_map_rows(&g.w[i][DC_OUT], dtype, a->lw[i][3], 8U, 8U, D / 8U, D) &&
-                 dc_map_rows(&g.w[i][DC_UP], dtype, a->lw[i][6], F, F, 2U, D) && dc_map_down(&g.w[i][DC_DOWN], dtype, a->lw[i][8], F, D);
+        mapped = dc_map_rows(&g.w[i][DC_QKV], dtype, a->lw[i][1], 32U, 32U, 3U * D / 32U, D, blocks) && dc_map_rows(&g.w[i][DC_OUT], dtype, a->lw[i][3], 8U, 8U, D / 8U, D, blocks) &&
+                 dc_map_rows(&g.w[i][DC_UP], dtype, a->lw[i][6], F, F, 2U, D, blocks) && dc_map_down(&g.w[i][DC_DOWN], dtype, a->lw[i][8], F, D);
         for (int j = 0; j < 2 && mapped; ++j)
             mapped = gdb_t5::make_tmap_batched(&g.kv[i][j], dtype, j == 0 ? a->kc[i] : a->vc[i], (uint64_t)a->B, cap, D, D * 2U, cap * D * 2U, 64U, 16U);
     }
