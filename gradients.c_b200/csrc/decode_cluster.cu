@@ -57,7 +57,7 @@ constexpr uint32_t DC_MAX_PLACES = 48U, DC_MIN_PLACES = 16U;
 // Use n of a place has barriers n % 256 of its own (full: its bytes have landed; empty: its readers are done), not the place's: a warp
 // may wait for a tile whose place is still to be used once or twice before, and a parity cannot tell those phases apart. A barrier's use
 // before, n - 256, is over by then. Outside the down projection because the warps lie at most 160 places apart (a block barrier ends every 16
-// units of two tiles, 64 places, and every four tiles per warp of the attention, whose warps may start while others have their part of
+// units of two tiles, 64 places, and every eight tiles per warp of the attention, 128 places, whose warps may start while others have their part of
 // the 12 QKV tiles to do; an exchange that needs all warps ends the other phases, and a pass of DC_PASS_COLS gate columns, 96 places, is
 // followed by the first 64 of the next one), and at most 48 more are in flight. Within the down projection, where nothing holds the
 // warps together and F / 64 places may lie between them, because tiles 128 apart have the same readers (those of one k range in four,
@@ -858,7 +858,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                         state.init(c.lane, [&](int i, int hh) { return dc_lds4(fresh + (uint32_t)(i * 32 + hh * 16 + c.lane * 4)); });
 #pragma unroll 1
                         for (int it = 0; it < kr.iters; ++it, ++turn) {
-                            if (turn != 0 && (turn & 3) == 0) dc_sync();
+                            if (turn != 0 && (turn & 7) == 0) dc_sync();
                             if (at != 0U || it != 0) tile = wait_use((uint32_t)(it * DC_WARPS + c.warp), &em);
                             const int key = s_lo + it * 16, left = s_hi - key, newest = pos - key;
                             if (left > 0) {

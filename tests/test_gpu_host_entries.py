@@ -49,7 +49,7 @@ def compare_decode_forms(monkeypatch, cfg, batch, prompt, new):
 def other_model(dtype, d_model, mlp_hidden, vocab, layers, window):
     cfg = g.GptConfig.baseline()
     cfg.dropout_p, cfg.sdpa_window, cfg.n_layers, cfg.vocab_size, cfg.dtype = 0.0, window, layers, vocab, dtype
-    cfg.d_model, cfg.n_heads, cfg.mlp_hidden, cfg.context_length = d_model, d_model // 64, mlp_hidden, 1024
+    cfg.d_model, cfg.n_heads, cfg.mlp_hidden, cfg.context_length = d_model, d_model // 64, mlp_hidden, 4096
     return cfg
 
 
@@ -74,11 +74,13 @@ def test_persistent_decode_of_a_larger_model_agrees_bit_for_bit(monkeypatch, dty
 
 
 # clusters of four and eight CTAs; more than 16 units of a phase to a CTA (rounds), a CTA with one unit more than another, k ranges of 16 and
-# 32, one 128-wide tile of the down projection; positions behind the cos / sin table (512) and more than 32 keys to a warp
+# 32, one 128-wide tile of the down projection; positions behind the cos / sin table (512); more than eight tiles of keys to
+# a warp, and several units to a CTA
 @pytest.mark.parametrize("dtype", [abi.F16, abi.BF16])
 @pytest.mark.parametrize("d_model,mlp_hidden,vocab,layers,batch,prompt,new,window", [
     (128, 128, 4096, 2, 5, 6, 12, 0), (128, 2560, 272, 1, 64, 4, 9, 3), (256, 640, 272, 2, 20, 30, 20, 0), (256, 768, 4112, 1, 3, 17, 8, 5),
-    (512, 1536, 2048, 1, 3, 490, 40, 0), (512, 512, 16, 1, 59, 250, 12, 200)])
+    (512, 1536, 2048, 1, 3, 490, 40, 0), (512, 512, 16, 1, 59, 250, 12, 200),
+    (512, 512, 272, 1, 2, 3000, 9, 0), (512, 512, 272, 2, 58, 900, 5, 0), (256, 256, 272, 1, 61, 700, 5, 0), (128, 128, 272, 1, 35, 600, 5, 0)])
 def test_decode_of_other_shapes_agrees_bit_for_bit(monkeypatch, dtype, d_model, mlp_hidden, vocab, layers, batch, prompt, new, window):
     cfg = other_model(dtype, d_model, mlp_hidden, vocab, layers, window)
     compare_decode_forms(monkeypatch, cfg, batch, prompt, new)
