@@ -278,7 +278,7 @@ decode_split_kernel(const T *q, const T *kc, const T *vc, const int *pos_buf, fl
     const bool active = w < total;
     if (active) {
         const size_t item = (size_t)w * splits + blockIdx.y * count;
-        gdb_dec::decode_split_item<T, DH, TILES>(q, kc, vc, pos_buf, part_ml + item * 2U, part_acc + item * DH, p, splits, w, (int)blockIdx.y * count, count, lane,
+        gdb_dec::decode_split_item<T, DH, TILES>(q, kc, vc, pos_buf, part_ml + item * 2U, part_acc + item * DH, p, splits, w, (int)blockIdx.y * count, min(count, splits - (int)blockIdx.y * count), lane,
                                                     decode_tiles + (TILES ? threadIdx.x >> 5 : 0) * gdb_dec::DECODE_TILES_BYTES);
     }   // active
     if (tickets == nullptr) {
@@ -550,7 +550,7 @@ gd_status decode_common(gd_backend *be, const gd_backend_tensor_view *q, const g
             const int form = p.dh == 64 && p.tq == 1 && p.prefix <= 0 ? DECODE_TILES : decode_register_form(be->sm_count, (total + 3) / 4 * splits);
             const int count = form == DECODE_TILES ? gdb_dec::decode_splits_per_warp(be->sm_count, p, splits) : 1;
             const size_t smem = form == DECODE_TILES ? 4U * gdb_dec::DECODE_TILES_BYTES : 0U;
-            dim3 grid((unsigned)((total + 3) / 4), (unsigned)(splits / count));
+            dim3 grid((unsigned)((total + 3) / 4), (unsigned)((splits + count - 1) / count));
             const bool fused = grid.x <= (unsigned)GDB_TICKET_WORDS;
             static bool tiles_allowed = false;   // more shared memory than a kernel has without asking
             if (form == DECODE_TILES && !tiles_allowed) {

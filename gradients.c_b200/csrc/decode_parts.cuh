@@ -284,9 +284,8 @@ static inline bool decode_cluster_shape(const decode_params &p)
 // warps per SM. (One each: 32 sequences x 8 heads of 1000 keys 27 us instead of 23, 64 of 400 21.4 instead of 18.4.)
 static inline int decode_splits_per_warp(int sm_count, const decode_params &p, int splits)
 {
-    int count = 1;
-    while (count < splits && (long long)p.batch * p.tq * p.hq * (splits / (2 * count)) >= 6LL * sm_count) count *= 2;
-    return count;
+    const long long queries = (long long)p.batch * p.tq * p.hq, groups = (6LL * sm_count + queries - 1) / queries;
+    return groups >= splits ? 1 : (int)((splits + groups - 1) / groups);
 }
 static inline int decode_choose_splits(int sm_count, const decode_params &p, int warps_per_sm)
 {

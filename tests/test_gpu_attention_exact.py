@@ -103,3 +103,31 @@ def test_backward_of_128_dimensions_repeats_bit_for_bit(ctx, dtype, lengths, hq,
         ctx.end_step()
         first = first or grads
         assert all(np.array_equal(a, b) for a, b in zip(grads, first))
+
+
+# Scores, probabilities and weighted sums are FP32 sums of 16-bit factors (products of the tensor cores for one new token at head_dim 64): their
+# error is at most 64 x 2^-22 x sum |q k| x scale, some 1e-4 of a probability, and a third of that in the 2-norm of a result over
+# dozens of keys. Beside the result's own rounding (2e-4 for 11 bits) that is 2 %; probabilities in 16 bits would be 5e-4 each. (Three, five
+# and seven key ranges of a query are among the shapes, with some but not all of them to a warp.)
+@pytest.mark.parametrize("dtype", [F16, BF16])
+@pytest.mark.parametrize("b,tq,hq,hkv,dh,tmax,window", [(1, 1, 8, 8, 64, 48, 0), (13, 1, 8, 8, 64, 122, 50), (64, 1, 8, 8, 64, 512, 0), (30, 1, 4, 4, 64, 900, 0), (64, 1, 2, 2, 64, 300, 0),
+                                                        (100, 1, 12, 4, 64, 200, 0), (100, 1, 8, 8, 64, 160, 0), (200, 1, 3, 3, 64, 400, 90), (5, 1, 8, 8, 128, 200, 0), (9, 3, 8, 2, 64, 150, 0), (100, 2, 16, 16, 64, 70, 0)])
+def test_decode_attention_has_the_rounding_of_its_result(ctx, dtype, b, tq, hq, hkv, dh, tmax, window):
+    rng = np.random.default_rng(b * tmax)
+    q, k, v = (rnd_np((rng.standard_normal(shape) * f).astype(np.float32), dtype) for shape, f in (((b, tq, hq, dh), 1.5), ((b, tmax, hkv, dh), 1.0), ((b, tmax, hkv, dh), 1.0)))
+    pos = rng.integers(0, tmax - tq + 1, size=b).astype(np.int32)
+    ctx.begin_step()
+    got = host(ops.gd_sdpa_decode_positions(ctx, dev(ctx, q, dtype), dev(ctx, k, dtype), dev(ctx, v, dtype), dev(ctx, pos, I32), sliding_window=window)).astype(np.float64)
+    ctx.end_step()
+    want = np.zeros((b, tq, hq, dh))
+    for i in range(b):
+        for t in range(tq):
+            hi = pos[i] + t + 1
+            lo = max(0, hi - window) if window > 0 else 0
+            for h in range(hq):
+                kk, vv = (c[i, lo:hi, h // (hq // hkv)].astype(np.float64) for c in (k, v))
+                s = kk @ q[i, t, h].astype(np.float64) / np.sqrt(dh)
+                p = np.exp(s - s.max())
+                want[i, t, h] = p @ vv / p.sum()
+    rounding = np.linalg.norm(rnd_np(want.astype(np.float32), dtype) - want)
+    assert np.linalg.norm(got.reshape(want.shape) - want) <= 1.02 * rounding

@@ -181,8 +181,8 @@ def test_greedy_decode_matches_oracle():
 def test_native_decode_feeds_back_on_the_device_and_matches_the_host_loop(batch, window, mlp_hidden, use_graph):
     """gdb200_gpt_decode_steps (device argmax, ids / positions kept on the device) generates exactly the ids of the
     per-step host loop: same arithmetic, same logits, same tie rule. use_graph = False enqueues one launch per
-    operation; with use_graph the run is ONE persistent kernel when the shapes allow (mlp_hidden 256: 13 steps in one
-    launch after the memset of its barrier words), else a replayed CUDA graph of the per-operation launches (192)."""
+    operation; with use_graph the run is ONE kernel when the shapes allow (mlp_hidden 256: 13 steps in one
+    launch after the memset of its counter), else a replayed CUDA graph of the per-operation launches (192)."""
     cfg = small_cfg(dropout_p=0.0, tied_lm_head=(batch == 4), sdpa_window=window, mlp_hidden=mlp_hidden)
     hp = g.init_params(cfg, seed=12, residual_scaled=False)
     prompts = np.random.default_rng(5).integers(0, cfg.vocab_size, size=(batch, 9)).astype(np.int32)
@@ -199,8 +199,8 @@ def test_native_decode_feeds_back_on_the_device_and_matches_the_host_loop(batch,
         assert timing["decode_launches"] >= 13, timing
 
 
-def test_persistent_decode_kernel_past_the_cache_capacity_and_bf16():
-    """The persistent decode kernel with rows whose position runs past the cache capacity (the append is dropped and
+def test_decode_kernel_past_the_cache_capacity_and_bf16():
+    """The kernel of all decode steps with rows whose position runs past the cache capacity (the append is dropped and
     attention reads the live part only, as the per-operation path does), in BF16."""
     cfg = small_cfg(dropout_p=0.0, mlp_hidden=256, dtype=abi.BF16)
     hp = g.init_params(cfg, seed=3, residual_scaled=False)
@@ -214,12 +214,12 @@ def test_persistent_decode_kernel_past_the_cache_capacity_and_bf16():
 
 
 @pytest.mark.parametrize("d_model,n_heads,mlp_hidden,vocab,batch,window,tied", [
-    (256, 4, 512, 1024, 64, 0, False),     # 2 heads x 8 key ranges per CTA, two K chunks of 256 in the down projection
+    (256, 4, 512, 1024, 64, 0, False),     # 4 heads x 4 key ranges per CTA, one K chunk of 512 in the down projection
     (256, 4, 384, 512, 7, 12, True),       # odd batch: 1 head x 16 key ranges, K chunks of 128, sliding window, tied head
-    (512, 8, 1024, 2048, 33, 0, True),     # the reference-default widths at a batch that leaves rows of the 64-row tile empty
+    (512, 8, 1024, 2048, 33, 0, True),     # the reference-default widths; a last cluster with fewer sequences
 ])
-def test_persistent_decode_kernel_shapes(d_model, n_heads, mlp_hidden, vocab, batch, window, tied):
-    """The persistent decode kernel on other partitions of its work (heads per CTA, key ranges, K chunks, unit counts above
+def test_decode_kernel_shapes(d_model, n_heads, mlp_hidden, vocab, batch, window, tied):
+    """The kernel of all decode steps on other partitions of its work (heads per CTA, key ranges, K chunks, unit counts above
     and below the number of CTAs): the ids equal the per-operation host loop's, in one launch."""
     cfg = small_cfg(dropout_p=0.0, d_model=d_model, n_heads=n_heads, mlp_hidden=mlp_hidden, vocab_size=vocab, tied_lm_head=tied,
                     sdpa_window=window, n_layers=2)
