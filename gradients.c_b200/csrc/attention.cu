@@ -293,7 +293,7 @@ decode_split_kernel(const T *q, const T *kc, const T *vc, const int *pos_buf, fl
     __syncthreads();
     if (last) {
         __threadfence();
-        if (active) decode_combine_query<T, true>(part_ml + (size_t)w * splits * 2U, part_acc + (size_t)w * splits * DH, out + (size_t)w * DH, DH, splits, lane);
+        if (active) decode_combine_query<T>(part_ml + (size_t)w * splits * 2U, part_acc + (size_t)w * splits * DH, out + (size_t)w * DH, DH, splits, lane);
         if (threadIdx.x == 0) tickets[blockIdx.x] = 0U;
     }
 }
@@ -307,7 +307,7 @@ __global__ void decode_combine_kernel(const float *part_ml, const float *part_ac
     if (w >= total) {
         return;
     }
-    decode_combine_query<T, true>(part_ml + (size_t)w * splits * 2U, part_acc + (size_t)w * splits * dh, out + (size_t)w * dh, dh, splits, lane);
+    decode_combine_query<T>(part_ml + (size_t)w * splits * 2U, part_acc + (size_t)w * splits * dh, out + (size_t)w * dh, dh, splits, lane);
 }
 
 // General head_dim decode: one warp per query, lanes split head_dim.

@@ -1,7 +1,7 @@
 // Device-side building blocks of one KV-cache decode step, shared by the stand-alone kernels (one
 // launch per operation: gemm_skinny.cu, embedding_rope.cu, attention.cu, the argmax of gpt_lm_native.cu)
 // and by the kernel of all steps (decode_cluster.cu). Both sides call the same functions, so a
-// step computed by one launch per operation and a step computed by the persistent kernel perform the
+// step computed by one launch per operation and a step computed by that kernel perform the
 // same floating-point operations in the same order and produce the same bits.
 #ifndef GDB200_DECODE_PARTS_CUH
 #define GDB200_DECODE_PARTS_CUH
@@ -312,12 +312,11 @@ static inline int decode_choose_splits(int sm_count, const decode_params &p, int
 }
 
 // Merge of the per-split partials of one query: out = sum_s acc_s e^(m_s - m) / sum_s l_s e^(m_s - m). `ml` [splits, 2] and
-// `acc` [splits, dh] are the query's partials, `out` its dh outputs. GLOBAL: the partials were written by other CTAs
-// (L2 loads); otherwise they lie in shared memory.
-template <typename T, bool GLOBAL>
+// `acc` [splits, dh] are the query's partials, written by other CTAs (L2 loads), `out` its dh outputs.
+template <typename T>
 __device__ __forceinline__ void decode_combine_query(const float *ml, const float *acc, T *out, int dh, int splits, int lane)
 {
-    auto ld = [](const float *p) { return GLOBAL ? __ldcg(p) : *p; };
+    auto ld = [](const float *p) { return __ldcg(p); };
     float m = -INFINITY;
     for (int s = 0; s < splits; ++s) m = fmaxf(m, ld(&ml[s * 2]));
     float l = 0.0f;

@@ -1205,7 +1205,7 @@ gd_status decode_step_body(gd_backend *be, const gdb200_gpt_spec *s, const gdb20
 
 // The whole run of decode steps in one launch (decode_cluster.cu) where its shapes allow; GD_ERR_UNSUPPORTED
 // otherwise (the caller then enqueues one launch per operation).
-gd_status decode_steps_persistent(gd_backend *be, const gdb200_gpt_spec *s, const gdb200_gpt_decode_state *d, int32_t n_steps, size_t *scratch_used)
+gd_status decode_steps_one_launch(gd_backend *be, const gdb200_gpt_spec *s, const gdb200_gpt_decode_state *d, int32_t n_steps, size_t *scratch_used)
 {
     const int64_t B = d->batch, D = s->d_model, F = s->mlp_hidden, V = s->vocab_size, H = s->n_heads, Dh = s->head_dim, CAP = d->capacity;
     const int L = s->n_layers;
@@ -1476,7 +1476,7 @@ extern "C" gd_status gdb200_gpt_decode_steps(gd_backend *be, const gdb200_gpt_sp
         return GD_OK;
     }
     if (use_graph) {
-        gd_status pst = decode_steps_persistent(be, s, d, n_steps, scratch_used);
+        gd_status pst = decode_steps_one_launch(be, s, d, n_steps, scratch_used);
         if (pst != GD_ERR_UNSUPPORTED) {
             return pst;
         }

@@ -90,9 +90,9 @@ class DecodeRun:
 
 
 # clusters of 16 and of four CTAs; CTAs without an attention unit (one sequence); up to eight gate units to a CTA (hidden 1024) and more;
-# the CTA that records the ids; the first step and later ones
+# the CTA that records the ids; the first step and later ones; gate rows in passes (hidden 8192)
 @pytest.mark.parametrize("d_model,mlp_hidden,batch,cta,step", [(512, 1024, 1, 15, 0), (512, 1024, 1, 0, 3), (512, 1536, 20, 7, 2), (512, 1536, 64, 3, 1),
-                                                               (256, 512, 7, 2, 4), (128, 256, 64, 1, 2)])
+                                                               (256, 512, 7, 2, 4), (128, 256, 64, 1, 2), (512, 8192, 64, 9, 2)])
 def test_decode_that_gives_up_leaves_ids_and_positions_where_they_were(d_model, mlp_hidden, batch, cta, step):
     with pkg.runtime.Context(params_bytes=256 << 20, state_bytes=256 << 20, scratch_bytes=1 << 30) as ctx:
         run = DecodeRun(ctx, d_model, mlp_hidden, batch, new=8)
