@@ -63,6 +63,8 @@ constexpr uint32_t DC_MAX_PLACES = 48U, DC_MIN_PLACES = 16U;
 // warps together and F / 64 places may lie between them, because tiles 128 apart have the same readers (those of one k range in four,
 // two or one) and the same producer, each of which has been through use n - 256 itself.
 constexpr uint32_t DC_BARS = 256U, DC_PASS_COLS = 6144U;
+// Uses are counted modulo 2^32 (thousands of steps over a million keys come round), from a little before it so that every run does.
+constexpr uint32_t DC_FIRST_USE = 0U - 2U * DC_BARS;
 static_assert(DC_BARS % (2U * 4U) == 0U && DC_PASS_COLS / 64U + 64U + DC_MAX_PLACES <= DC_BARS, "readers of uses that share a barrier");
 // Hardware barriers of the consumer warps: all of them; the two warps of a unit whose halves of k are formed apart (up to eight units);
 // the eight warps of one of the two units of a residual projection. A barrier has ONE number of threads: only the exchanges keep the
@@ -315,10 +317,10 @@ __device__ void dc_produce(dc_ctx &c, const dc_args &g, uint32_t which, int b0, 
     const int groups = a.H >> hpc_log, attn_units = rows * groups;
     uint32_t lm_first, lm_n;
     dc_share((uint32_t)a.V / 16U, c.rank, CS, &lm_first, &lm_n);
-    uint32_t n = 0U, place = 0U, pass = 0U;
+    uint32_t n = DC_FIRST_USE, place = 0U, pass = 0U;
     dc_pass gate = dc_gate_pass(0U, pass_cols, F, c.rank, CS);
     auto claim = [&](uint32_t use) {   // its place is free
-        if (use >= c.places) dc_wait(c, c.empty + ((use - c.places) % DC_BARS) * 8U, ((use - c.places) / DC_BARS) & 1U);
+        dc_wait(c, c.empty + ((use - c.places) % DC_BARS) * 8U, ((use - c.places) / DC_BARS) & 1U);   // (the first uses: of a phase before the first)
     };
     auto wrap = [&](uint32_t s) { return dc_wrap(c, s); };
 #pragma unroll 1
@@ -473,7 +475,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
     c.rank = gdb_t5::cluster_ctarank();
     c.places = g.lay.places;
     c.inverse = g.lay.inverse;
-    c.n = 0U;
+    c.n = DC_FIRST_USE;
     c.place = 0U;
     c.tid = threadIdx.x;
     c.warp = threadIdx.x >> 5;
