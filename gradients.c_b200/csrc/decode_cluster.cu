@@ -6,8 +6,9 @@
 // up / gate + SwiGLU, down projection; then the LM head): each ends in an exchange of activations. Inside a cluster that exchange
 // is a 16-byte store into the shared memory of the other CTAs that also counts its bytes on their barrier (st.async): no counter
 // in global memory, no fence, and the next phase reads its operand where it landed. The price is that every cluster needs all
-// weights in every step. They stay in L2 (seven clusters drew 18 TB/s in a probe, 89 bytes per cycle and SM, with three or four issuing
-// warps; 40 with one); each CTA's share is streamed by its producer warps through a ring of TMA tiles that runs
+// weights in every step. They come from L2 (seven clusters drew 18 TB/s in a probe, 89 bytes per cycle and SM, with three or four issuing
+// warps; 40 with one), and since the clusters walk through them side by side also where they do not fit there (16 layers of hidden 2048,
+// 143 MB: 64 sequences 669 -> 456 us per step, one 562 -> 229; vocabulary 50304, 72 MB: 206 -> 154, 169 -> 90); each CTA's share is streamed by its producer warps through a ring of TMA tiles that runs
 // ahead of the phases, across exchanges, layers and steps, and so are the keys and values of its attention units.
 //
 // A CTA owns 32 columns of the residual stream: half a head of q, k and v (so a rotation pair lies in one thread), 32 columns of
@@ -18,9 +19,10 @@
 // key splits), so ids and caches are those of one launch per operation, bit for bit. The newest key and value reach the attention
 // through the exchange, the cache row is read from global memory from the next step on (ordered by the step's last exchange).
 //
-// Benchmark model (d 512, 3 layers, vocabulary 2048), us per step, against the grid-wide kernel before (weights resident in the
-// shared memory of all SMs, exchanges through global memory): 1 sequence 53.5 -> 40.8, 13 59 -> 41.0, 32 80 -> 50.5, 64 of 256-512 tokens
-// 148 -> 117.4. A phase of one sequence is some 5 k cycles, of which the exchange 1.0-1.4 k; an all-to-all of 8 KB in a cluster of 16 took
+// Benchmark model (d 512, 3 layers, vocabulary 2048), us per step, against the grid-wide kernels before (weights resident in the
+// shared memory of all SMs or read once per step by all of them, exchanges through global memory): 1 sequence 52.5 -> 39.5, 13 59 -> 40.3,
+// 32 of 128-256 tokens 80 -> 50.0, 64 of 256-512 146 -> 102.6, 64 of 4000 358-372 -> 368 and of 6000 480 -> 529 (112 of 148 SMs fetch the keys,
+// and ten sequences of a cluster are more than a seventh of 64). A phase of one sequence is some 5 k cycles, of which the exchange 1.0-1.4 k; an all-to-all of 8 KB in a cluster of 16 took
 // 1345 cycles by st.async, 1550 by bulk copies, 2400 by remote stores and a releasing arrive.
 //
 // Waits are bounded. One that gives up stores code 398 in the backend's error word and raises the CTA's flag; from then on its thread

@@ -643,7 +643,7 @@ gd_status gdb200_gpt_prefill(gd_backend *backend, const gdb200_gpt_spec *spec, c
                              size_t last_rows_offset, const gdb200_gpt_decode_state *state, size_t *scratch_used);
 /* Enqueues n_steps decode steps without any host synchronisation. use_graph == 0: one launch per operation, step after
  * step. use_graph != 0: where the shapes allow (16-bit storage, at most 64 sequences, head_dim 64, d_model 128 / 256 / 512,
- * mlp_hidden a multiple of 128 and what of it fits shared memory, vocab_size a multiple of 16) ALL steps run in one kernel of
+ * mlp_hidden a multiple of 128, vocab_size a multiple of 16) ALL steps run in one kernel of
  * independent thread-block clusters (d_model / 32 CTAs each, a few sequences each, the weights read from L2; a wait that gives up
  * stores code 398 in the error word, and its cluster's sequences keep their ids and positions and all of them the step counter of
  * before the call; out_tokens holds the steps that were done); otherwise the first step runs eagerly, the second is
