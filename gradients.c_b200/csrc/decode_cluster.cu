@@ -75,9 +75,9 @@ constexpr uint32_t DC_BAR_ALL = 1U, DC_BAR_PAIR = 2U, DC_PAIRS = 8U, DC_BAR_SUM 
 static_assert(DC_BAR_ALL > 0U && DC_BAR_PAIR > DC_BAR_ALL && DC_BAR_SUM >= DC_BAR_PAIR + DC_PAIRS && DC_BAR_SUM + DC_SUMS <= 16U,
               "barrier 0 is __syncthreads, a block has 16, and no barrier is used with two numbers of threads");
 // Time a wait may take before it gives up. What is waited for comes from the CTA's own copies or from CTAs that are resident with it: some
-// microseconds; a second or two leave room for other processes' time slices. (Time, not polls: how long a poll sleeps is the
-// hardware's choice, up to the hint of 0.1 ms, and 2^21 of them would be minutes.)
-constexpr unsigned DC_WAIT_MS = 2000U;
+// microseconds; two seconds leave room for other processes' time slices, and the polls, some 50 ms of them, for a process that was off
+// the GPU for longer. (Not polls alone: how long one sleeps is the hardware's choice, up to the hint of 0.1 ms, and 2^21 would be minutes.)
+constexpr unsigned DC_WAIT_MS = 2000U, DC_WAIT_POLLS = 512U;
 constexpr int DC_ERR_WAIT = 398;
 
 enum { DC_QKV = 0, DC_OUT = 1, DC_UP = 2, DC_DOWN = 3, DC_LM = 4 };
@@ -241,10 +241,11 @@ __device__ __forceinline__ uint32_t dc_now_ms()
 __device__ __noinline__ bool dc_wait_more(uint32_t bar, uint32_t parity, volatile int *dead, int *err_flag)
 {
     const uint32_t since = dc_now_ms();
+    uint32_t polls = 0U;
     do {
         if (dc_try_wait(bar, parity)) return true;
         if (*dead != 0) return false;
-    } while (dc_now_ms() - since < (uint32_t)dead[1]);
+    } while (++polls < DC_WAIT_POLLS || dc_now_ms() - since < (uint32_t)dead[1]);
     *dead = 1;
     atomicCAS(err_flag, 0, DC_ERR_WAIT);
     return false;
